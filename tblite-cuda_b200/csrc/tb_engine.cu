@@ -299,6 +299,7 @@ struct tb_calculator {
     double a = 0, b = 0;  // in-house latency of one structure: a N^2 + b N^3 seconds
     double c = 0, d = 0;  // one cuSOLVER call: c + d N^3 seconds
     double t_in[2] = {0, 0}, t_lib[2] = {0, 0};  // the measured points (256/512 and 256/1024 AOs)
+    double scale = 1;  // measured in-house time over SyevPlan's model, mean of the two points
   } eig;
   // small structures: the one-warp Jacobi variant against the one-CTA
   // eigensolver, measured once per calculator (batched throughput per size)
@@ -420,6 +421,7 @@ struct tb_batch {
   int* d_wflag = nullptr;
   int* d_jlist = nullptr;  // structures on the one-warp Jacobi eigensolver
   int njac = 0;
+  SyevPlan syev;            // k_syev's clusters over the batch's order
   TridPlan trid;            // structures tridiagonalised by k_trid_smem, per class
   int* d_tlist = nullptr;
   int4 *d_tiles64, *d_tiles32, *d_tiles128;
@@ -484,10 +486,11 @@ tb_status calibrate_tiles(tb_calculator* c);
 // Automatic eigensolver choice for a batch (tb_options.solver = 0): the k
 // largest structures go to cuSOLVER, the rest to the batched in-house solver,
 // with k minimising the modelled time of one SCF iteration's eigensolve:
-//   sum_{i<k} t_lib(N_i) + max(t_in(N_k), sum_{i>=k} t_in(N_i) / slots)
-// (library calls run one after another; in-house structures run concurrently,
-// one CTA each, up to `slots` at a time; t_in and t_lib are measured once per
-// calculator).  Returns lib_above: structures with more AOs go to the library.
+//   sum_{i<k} t_lib(N_i) + span(N_k, N_{k+1}, ...)
+// (library calls run one after another, then k_syev runs the rest; t_lib is
+// measured once per calculator, span is the plan's model scaled by the
+// measured in-house times).  Returns lib_above: structures with more AOs go
+// to the library.
 int choose_lib_above(tb_calculator* c, std::vector<int> sizes) {
   std::sort(sizes.begin(), sizes.end(), std::greater<int>());
   const int nmol = (int)sizes.size();
@@ -497,19 +500,14 @@ int choose_lib_above(tb_calculator* c, std::vector<int> sizes) {
   if (sizes[k0] < 384) return kSyevMaxN;  // small structures: the batched solver always wins
   if (calibrate_eigensolvers(c) != TB_OK) return kSyevMaxN;
   const auto& M = c->eig;
-  auto t_in = [&](double n) { return M.a * n * n + M.b * n * n * n; };
   auto t_lib = [&](double n) { return M.c + M.d * n * n * n; };
-  auto slots = [&](int n) {
-    const int per = (int)std::min<size_t>(3, (227 * 1024) / std::max<size_t>(syev_smem_bytes(n), 1));
-    return 148.0 * std::max(per, 1);
-  };
-  std::vector<double> tail(nmol + 1, 0.0);
-  for (int i = nmol - 1; i >= 0; --i) tail[i] = tail[i + 1] + t_in(sizes[i]);
   double lib_sum = 0.0, best = 1e300;
   int best_k = k0;
   for (int i = 0; i < k0; ++i) lib_sum += t_lib(sizes[i]);
-  for (int k = k0; k <= nmol; ++k) {
-    const double in_t = k == nmol ? 0.0 : std::max(t_in(sizes[k]), tail[k] / slots(sizes[k]));
+  for (int k = k0; k <= nmol && lib_sum < best; ++k) {
+    SyevPlan rest;
+    rest.build(std::vector<int>(sizes.begin() + k, sizes.end()), 0, 0);
+    const double in_t = 1e-3 * rest.span * M.scale;
     if (lib_sum + in_t < best) { best = lib_sum + in_t; best_k = k; }
     if (k < nmol) lib_sum += t_lib(sizes[k]);
   }
@@ -902,6 +900,11 @@ tb_status batch_build(tb_calculator* calc, const tb_structure* mols, int nmol, c
     return b->h_ooff[a + 1] - b->h_ooff[a] > b->h_ooff[c + 1] - b->h_ooff[c];
   });
   put(o_order, order.data(), NM * I4);
+  {
+    std::vector<int> sizes(nmol);
+    for (int i = 0; i < nmol; ++i) sizes[i] = b->h_ooff[order[i] + 1] - b->h_ooff[order[i]];
+    b->syev.build(sizes, lib_above, jacobi_max);
+  }
   if (!jlist.empty()) put(o_jlist, jlist.data(), jlist.size() * I4);
   if (!b->trid.list.empty()) put(o_tlist, b->trid.list.data(), b->trid.list.size() * I4);
   TB_CUDA(cudaMemcpy(base, blob, meta_end, cudaMemcpyHostToDevice));
@@ -1113,7 +1116,6 @@ tb_status mixed_core(tb_batch* b, cudaStream_t st, double n3_lo, double n3_hi, d
   const int nmol = b->nmol, nt = (int)b->tiles64.size();
   const int4* T = b->d_tiles64;
   const size_t smem32 = syev_smem_bytes(std::max(b->nmax_in, 1), sizeof(float));
-  const size_t eig_smem = syev_smem_bytes(std::max(b->nmax_in, 1));
   int *lo = b->act_lo, *hi = b->act_hi;
   const int nt128 = (int)b->tiles128.size(), tc_grid = std::min(nt128, 148);
   const int4* T128 = b->d_tiles128;
@@ -1136,7 +1138,8 @@ tb_status mixed_core(tb_batch* b, cudaStream_t st, double n3_lo, double n3_hi, d
     if (ts != TB_OK) return ts;
   }
   TB_K("syev", 4.0 * n3_hi, 1,
-       k_syev<<<nmol, kEigThreads, eig_smem, st>>>(B, b->F, b->Z, b->W, b->w, b->perm, S.status, hi));
+       TB_CUDA(launch_syev(b->syev, B, b->F, b->Z, b->W, b->w, b->perm, S.status, hi, st, &b->launches)));
+  --b->launches;  // launch_syev has counted
   if (b->njac > 0)
     TB_K("syev_jacobi", 0, 0,
          k_syev_jacobi<<<nblk(b->njac, kJacobiWarps), kJacobiWarps * 32, jacobi_smem_bytes(), st>>>(
@@ -1198,7 +1201,7 @@ tb_status raise_smem_limits() {
   int dev = 0, optin = 0;
   TB_CUDA(cudaGetDevice(&dev));
   TB_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-  const void* ks[] = {(const void*)k_syev, (const void*)k_syev_f32, (const void*)k_fermi, (const void*)k_oa_step,
+  const void* ks[] = {(const void*)k_syev, (const void*)k_syev_wide, (const void*)k_syev_ql, (const void*)k_syev_f32, (const void*)k_fermi, (const void*)k_oa_step,
                       (const void*)k_gemm_tc, (const void*)k_fock, (const void*)k_syev_jacobi};
   for (const void* k : ks) {
     cudaFuncAttributes a;
@@ -1272,9 +1275,10 @@ tb_status calibrate_eigensolvers(tb_calculator* c) {
         if (tp.off[cl + 1] > tp.off[cl])
           TB_CUDA(launch_trid(B, at<double>(base, oA), at<double>(base, oW), at<int>(base, os), nullptr,
                               at<int>(base, ol), 1, kTridClusterSizes[cl], n, 0));
-      k_syev<<<1, kEigThreads, syev_smem_bytes(n)>>>(B, at<double>(base, oA), at<double>(base, oZ),
-                                                     at<double>(base, oW), at<double>(base, ow), at<int>(base, op),
-                                                     at<int>(base, os), nullptr);
+      SyevPlan sp;
+      sp.build({n}, 0, 0);
+      TB_CUDA(launch_syev(sp, B, at<double>(base, oA), at<double>(base, oZ), at<double>(base, oW),
+                          at<double>(base, ow), at<int>(base, op), at<int>(base, os), nullptr, 0, nullptr));
       TB_CUDA(cudaEventRecord(e1));
       TB_CUDA(cudaEventSynchronize(e1));
       TB_CUDA(cudaEventElapsedTime(&ms, e0, e1));
@@ -1314,6 +1318,12 @@ tb_status calibrate_eigensolvers(tb_calculator* c) {
   c->eig.d = std::max(0.0, (l2 - l1) / (m2 * m2 * m2 - m1 * m1 * m1));
   c->eig.c = std::max(0.0, l1 - c->eig.d * m1 * m1 * m1);
   c->eig.t_in[0] = t1; c->eig.t_in[1] = t2;
+  {
+    SyevPlan p1, p2;
+    p1.build({256}, 0, 0);
+    p2.build({512}, 0, 0);
+    c->eig.scale = 500.0 * (t1 / p1.span + t2 / p2.span);
+  }
   c->eig.t_lib[0] = l1; c->eig.t_lib[1] = l2;
   c->eig.ready = true;
   return TB_OK;
@@ -1386,9 +1396,9 @@ tb_status calibrate_small(tb_calculator* c) {
         cudaMemset(base + os, 0, cnt * 4);
         cudaEventRecord(e0);
         if (variant == 0)
-          k_syev<<<cnt, kEigThreads, syev_smem_bytes(n)>>>(Bk, at<double>(base, oA), at<double>(base, oZ),
-                                                           at<double>(base, oW), at<double>(base, ow),
-                                                           at<int>(base, op), at<int>(base, os), nullptr);
+          k_syev_ql<<<cnt, kEigThreads, syev_smem_bytes(n)>>>(Bk, at<double>(base, oA), at<double>(base, oZ),
+                                                              at<double>(base, ow), at<int>(base, op),
+                                                              at<int>(base, os), nullptr);
         else
           k_syev_jacobi<<<nblk(cnt, kJacobiWarps), kJacobiWarps * 32, jacobi_smem_bytes()>>>(
               Bk, at<double>(base, oA), at<double>(base, oZ), at<double>(base, ow), at<int>(base, op),
@@ -1694,8 +1704,8 @@ tb_status iterate_body(tb_batch* b, cudaStream_t st) {
       if (ts != TB_OK) return ts;
     }
     TB_K("syev", 4.0 * n3, 1,
-         k_syev<<<nmol, kEigThreads, syev_smem_bytes(std::max(b->nmax_in, 1)), st>>>(
-             B, b->F, b->Z, b->W, b->w, b->perm, S.status, S.active));
+         TB_CUDA(launch_syev(b->syev, B, b->F, b->Z, b->W, b->w, b->perm, S.status, S.active, st, &b->launches)));
+    --b->launches;  // launch_syev has counted
     if (b->njac > 0)
       TB_K("syev_jacobi", 0, 0,
            k_syev_jacobi<<<nblk(b->njac, kJacobiWarps), kJacobiWarps * 32, jacobi_smem_bytes(), st>>>(
@@ -2268,10 +2278,11 @@ int32_t tb_bounds_check_build(void) {
 
 tb_status tb_bounds_violations(int64_t* count, int32_t* site, int64_t* index, int64_t* lo, int64_t* hi,
                                int32_t reset) {
-  OobRecord r[3];
+  OobRecord r[4];
   cudaError_t e = oob_setup(&r[0], reset != 0);
   if (e == cudaSuccess) e = oob_scf(&r[1], reset != 0);
   if (e == cudaSuccess) e = oob_linalg(&r[2], reset != 0);
+  if (e == cudaSuccess) e = oob_syev(&r[3], reset != 0);
   if (e != cudaSuccess) return fail(TB_CUDA_ERROR, cudaGetErrorString(e));
   int64_t total = 0;
   const OobRecord* first = nullptr;
@@ -2739,6 +2750,7 @@ struct MatBatch {
   size_t lib_bytes = 0;
   int* lib_info = nullptr;
   TridPlan trid;
+  SyevPlan syev;
   int* d_tlist = nullptr;
   tb_status build(int nmat, const int32_t* n, int smem_tridiag = kTridMin) {
     std::vector<int> ooff(nmat + 1, 0);
@@ -2770,8 +2782,15 @@ struct MatBatch {
     h_ooff = ooff;
     n2 = moff[nmat];
     no = ooff[nmat];
+    // largest matrices first: the order k_syev's plan and the factorisations take
+    std::vector<int> order(nmat), sorted(nmat);
+    for (int m = 0; m < nmat; ++m) order[m] = m;
+    std::stable_sort(order.begin(), order.end(), [&](int a, int c) { return n[a] > n[c]; });
+    for (int i = 0; i < nmat; ++i) sorted[i] = n[order[i]];
+    syev.build(sorted, kSyevMaxN, 0);
     Layout L;
     size_t o_ooff = L.add((nmat + 1) * 4), o_moff = L.add((nmat + 1) * 8), o_t = L.add(tiles.size() * sizeof(int4));
+    size_t o_ord = L.add(nmat * 4);
     size_t o_S = L.add(n2 * 8), o_X = L.add(n2 * 8), o_W = L.add(n2 * 8), o_F = L.add(n2 * 8), o_Z = L.add(n2 * 8);
     size_t o_w = L.add(no * 8), o_f = L.add(no * 8), o_p = L.add(no * 4), o_k = L.add(nmat * 4);
     size_t o_st = L.add(nmat * 4), o_act = L.add(nmat * 4), o_nel = L.add(2 * nmat * 8), o_ets = L.add(nmat * 8),
@@ -2784,7 +2803,9 @@ struct MatBatch {
     TB_CUDA(cudaMemcpy(base + o_ooff, ooff.data(), (nmat + 1) * 4, cudaMemcpyHostToDevice));
     TB_CUDA(cudaMemcpy(base + o_moff, moff.data(), (nmat + 1) * 8, cudaMemcpyHostToDevice));
     TB_CUDA(cudaMemcpy(base + o_t, tiles.data(), tiles.size() * sizeof(int4), cudaMemcpyHostToDevice));
+    TB_CUDA(cudaMemcpy(base + o_ord, order.data(), nmat * 4, cudaMemcpyHostToDevice));
     db.nmol = nmat;
+    db.order = at<int>(base, o_ord);
     db.ooff = at<int>(base, o_ooff);
     db.moff = at<long long>(base, o_moff);
     db.lib_above = kSyevMaxN;
@@ -2834,7 +2855,6 @@ tb_status tb_sygvd_batch(int32_t nmat, const int32_t* n, const double* H, const 
                                  kGemmKUpToJ);
   k_gemm<<<grid, kGemmThreads>>>(B, mb.d_tiles, nt, mb.X, 1, mb.W, 0, nullptr, nullptr, nullptr, mb.F, 1.0, 0.0, mb.ms.active,
                                  kGemmKUpToI | kGemmSym);
-  const size_t smem = syev_smem_bytes(std::max(mb.nmax_in, 1));
   {
     const tb_status ss = raise_smem_limits();
     if (ss != TB_OK) return ss;
@@ -2845,7 +2865,7 @@ tb_status tb_sygvd_batch(int32_t nmat, const int32_t* n, const double* H, const 
     TB_CUDA(launch_trid(B, mb.F, mb.W, mb.ms.status, mb.ms.active, mb.d_tlist + mb.trid.off[c], cnt,
                         kTridClusterSizes[c], mb.trid.nmax[c], 0));
   }
-  k_syev<<<nmat, kEigThreads, smem>>>(B, mb.F, mb.Z, mb.W, mb.w, mb.perm, mb.ms.status, mb.ms.active);
+  TB_CUDA(launch_syev(mb.syev, B, mb.F, mb.Z, mb.W, mb.w, mb.perm, mb.ms.status, mb.ms.active, 0, nullptr));
   std::vector<int> fstat(nmat, 0);
   if (!mb.big.empty()) TB_CUDA(cudaMemcpy(fstat.data(), mb.ms.status, nmat * 4, cudaMemcpyDeviceToHost));
   for (size_t k = 0; k < mb.big.size(); ++k) {

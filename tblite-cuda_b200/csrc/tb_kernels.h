@@ -152,10 +152,32 @@ __global__ void k_gemm(DevBatch B, const int4* tiles, int ntiles, const double* 
 __global__ void k_gemm32(DevBatch B, const int4* tiles, int ntiles, const double* Ab, int ta, const double* Bb,
                          int tb_, const int* perm, const double* ks, const int* kdim, double* Cb, double alpha,
                          double beta, const int* active, int shape = 0);
-// Sb: optional n x n scratch per structure (same offsets as Ab); with it,
-// structures of at least kDcMin (64) AOs take divide and conquer instead of QL
+// FP64 eigensolver (tb_syev.cu; structures of kDcMin+ AOs): Sb an n x n scratch
+// per structure (same offsets as Ab); the grid is clusters of C CTAs, the first
+// ncoop of them each on one structure, then one structure per CTA (SyevPlan)
 __global__ void k_syev(DevBatch B, double* Ab, double* Zb, double* Sb, double* wout, int* perm, int* status,
-                       const int* active);
+                       const int* active, int ncoop);
+__global__ void k_syev_wide(DevBatch B, double* Ab, double* Zb, double* Sb, double* wout, int* perm, int* status,
+                            const int* active, int ncoop);
+constexpr int kSyevMaxCluster = 8;
+constexpr size_t kSyevSmemTwo = 110 * 1024;  // dynamic shared memory up to which two CTAs fit an SM
+struct SyevPlan {
+  int n64 = 0;          // structures of kDcMin+ AOs on the in-house solver lead the order
+  int nsmall = 0;       // structures below kDcMin AOs that k_syev_ql solves
+  int cluster = 1, ncoop = 0;
+  bool wide = true;     // k_syev_wide (one CTA per SM)
+  double span = 0.0;    // modelled time of one launch, ms
+  int nmax = 0;         // largest in-house structure
+  // sizes in the batch's order (decreasing; those of the library path first)
+  void build(const std::vector<int>& sizes, int lib_above, int jacobi_max);
+};
+// k_syev (and k_syev_ql where the plan has small structures) on st; *launches
+// counts them.  The shared-memory limits must have been raised.
+cudaError_t launch_syev(const SyevPlan& P, const DevBatch& B, double* A, double* Z, double* Sb, double* w, int* perm,
+                        int* status, const int* active, cudaStream_t st, int64_t* launches);
+// one CTA per structure, FP64, below kDcMin AOs: implicit QL
+__global__ void k_syev_ql(DevBatch B, double* Ab, double* Zb, double* wout, int* perm, int* status,
+                          const int* active);
 // the same eigensolver in FP32 (A and Z float, eigenvalues written as double)
 __global__ void k_syev_f32(DevBatch B, float* Ab, float* Zb, double* wout, int* perm, int* status, const int* active);
 // small-structure variant: one warp per structure of N <= kJacobiMaxN (cyclic Jacobi
@@ -195,6 +217,7 @@ __global__ void k_oa_step(DevBatch B, double* G, double* Sm, double* V, double* 
 cudaError_t oob_setup(OobRecord* r, bool reset);
 cudaError_t oob_scf(OobRecord* r, bool reset);
 cudaError_t oob_linalg(OobRecord* r, bool reset);
+cudaError_t oob_syev(OobRecord* r, bool reset);
 
 // D4 dispersion (tb_disp.cu; only when DevParams::d4): per atom cn, W and dW
 // (kD4MaxRef each), energy share e_at, dE/dCN and gradient g [3 nat]; per

@@ -121,12 +121,14 @@ extern "C" tb_status tb_sygvd_noalloc(int32_t n, const double* H, const double* 
       // memory opt-in for the largest accepted n (raised only: the batched
       // paths may already have set a higher limit), then the scratch address
       // (cached last, so that a failed set-up is retried by the next call)
-      cudaFuncAttributes fa;
-      e = cudaFuncGetAttributes(&fa, (const void*)k_syev);
       const int need = (int)syev_smem_bytes(kNoAllocMaxN);
-      if (e == cudaSuccess && fa.maxDynamicSharedSizeBytes < need)
-        e = cudaFuncSetAttribute((const void*)k_syev, cudaFuncAttributeMaxDynamicSharedMemorySize, need);
-      if (e != cudaSuccess) return noalloc_fail(TB_CUDA_ERROR, cudaGetErrorString(e));
+      for (const void* k : {(const void*)k_syev, (const void*)k_syev_wide, (const void*)k_syev_ql}) {
+        cudaFuncAttributes fa;
+        e = cudaFuncGetAttributes(&fa, k);
+        if (e == cudaSuccess && fa.maxDynamicSharedSizeBytes < need)
+          e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, need);
+        if (e != cudaSuccess) return noalloc_fail(TB_CUDA_ERROR, cudaGetErrorString(e));
+      }
       double* addr = nullptr;
       e = cudaGetSymbolAddress(reinterpret_cast<void**>(&addr), g_noalloc_scratch);
       if (e != cudaSuccess) return noalloc_fail(TB_CUDA_ERROR, cudaGetErrorString(e));
@@ -149,7 +151,10 @@ extern "C" tb_status tb_sygvd_noalloc(int32_t n, const double* H, const double* 
                                  v.active, kGemmKUpToJ);
   k_gemm<<<ntiles, kGemmThreads, 0, st>>>(B, v.tiles, ntiles, v.X, 1, v.W, 0, nullptr, nullptr, nullptr, v.A, 1.0, 0.0,
                                  v.active, kGemmKUpToI | kGemmSym);
-  k_syev<<<1, kEigThreads, syev_smem_bytes(n), st>>>(B, v.A, v.Z, v.W, w, v.perm, v.status, v.active);
+  SyevPlan sp;
+  sp.build({n}, 0, 0);
+  e = launch_syev(sp, B, v.A, v.Z, v.W, w, v.perm, v.status, v.active, st, nullptr);
+  if (e != cudaSuccess) return noalloc_fail(TB_CUDA_ERROR, cudaGetErrorString(e));
   // C = X Z with the eigenvectors in ascending order
   k_gemm<<<ntiles, kGemmThreads, 0, st>>>(B, v.tiles, ntiles, v.X, 0, v.Z, 1, v.perm, nullptr, nullptr, C, 1.0, 0.0,
                                  v.active, kGemmKFromI);

@@ -1,0 +1,1410 @@
+// FP64 symmetric eigensolver for structures of kDcMin+ AOs (k_syev): one CTA
+// or one thread block cluster per structure, the same bits either way.
+//
+//  1. Householder tridiagonalisation in panels of kPanel reflectors
+//     (tridiag_tiles): within a panel the trailing block keeps its value from
+//     the panel start, each step forms its product with one read-only walk of
+//     the upper triangle and corrects it with the panel's pairs; the
+//     panel-closing walk applies the rank-2 kPanel update on the FP64 tensor
+//     instruction, fused with the next product.
+//  2. Zc = Q^T accumulated backwards in compact-WY blocks (form_q).
+//  3. Tridiagonal eigenproblem by divide and conquer (dc_solve).
+//  4. Ascending order by rank (ties by index).
+// Together with k_cholesky, k_trinv and k_gemm this is sygvd (reference
+// src/lapack/sygvd.h:4-23).
+//
+// Work is cut into units whose boundaries and order of additions depend on
+// the matrix order alone (row/column tiles of the walks, 64-row tiles of Q,
+// 64 x 64 tiles of the merge products, teams of four lanes per secular root),
+// never on how many warps share them.  So a structure gives the same bits on
+// one CTA (a large batch: 444 structures resident on 148 SMs, throughput) and
+// on a cluster of 2..16 (a few structures: latency).  The CTAs of a cluster keep
+// identical copies of the vectors (d, e, tau, v, p, w, the panel) in their
+// shared memory and repeat the O(n) arithmetic on them; only the units are
+// divided, their results exchanged through global memory (walk partials, Z,
+// merge blocks) or the peers' shared memory (roots, recomputed z), with one
+// cluster barrier per Householder step and three per shared merge.
+#include <algorithm>
+#include <functional>
+
+#include "tb_common.cuh"
+#include "tb_kernels.h"
+
+namespace tb {
+
+namespace {
+
+constexpr double kEps = 2.220446049250313e-16;
+constexpr int kPanel = 8;    // reflectors per tridiagonalisation panel
+constexpr int kQBlock = 16;  // reflectors per compact-WY block of the Q accumulation
+constexpr int kWarps = kEigThreads / 32;
+static_assert(kEigThreads == 256, "the tile shapes below assume eight warps");
+static_assert(kPanel <= kRing, "panel exceeds the shared-memory ring");
+
+// ------------------------------------------------------------ CTAs of one structure
+struct Group {
+  int rank, size;  // this CTA's rank in the structure's cluster; size 1: a CTA of its own
+};
+
+__device__ __forceinline__ void group_sync(const Group& g) {
+  if (g.size == 1) {
+    __syncthreads();
+  } else {
+    asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;\n" ::: "memory");
+  }
+}
+
+// *p = v in the shared memory of CTA r of the group (the same variable there)
+__device__ __forceinline__ void put_at(double* p, double v, const Group& g, int r) {
+  if (r == g.rank) {
+    *p = v;
+  } else {
+    const unsigned a = (unsigned)__cvta_generic_to_shared(p);
+    unsigned ra;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(a), "r"(r));
+    asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(ra), "d"(v) : "memory");
+  }
+}
+__device__ __forceinline__ void put_at(int* p, int v, const Group& g, int r) {
+  if (r == g.rank) {
+    *p = v;
+  } else {
+    const unsigned a = (unsigned)__cvta_generic_to_shared(p);
+    unsigned ra;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(a), "r"(r));
+    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(ra), "r"(v) : "memory");
+  }
+}
+
+// D = A B + D for one 8 x 8 x 4 step.  Lane l = 4 g + t holds A[g][t], B[t][g]
+// and D[g][2t], D[g][2t+1].  Volatile: without it the compiler may sink the
+// instruction into a branch that only some lanes take (a guarded store of its
+// result), where a warp-wide instruction hangs.
+__device__ __forceinline__ void dmma(double& d0, double& d1, double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
+               : "+d"(d0), "+d"(d1)
+               : "d"(a), "d"(b));
+}
+
+// Block-wide sum in a fixed order with one barrier.  The caller alternates
+// between two `red` buffers of kWarps entries: a buffer is rewritten only
+// after the barrier of the call in between, by when everyone has read it.
+__device__ __forceinline__ double block_sum_once(double v, double* red) {
+  v = warp_sum(v);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+  __syncthreads();
+  double t = 0.0;
+#pragma unroll
+  for (int w = 0; w < kWarps; ++w) t += red[w];
+  return t;
+}
+
+// 1/x for the divide-and-conquer inner loops: the hardware reciprocal
+// estimate (rcp.approx.ftz.f64) refined by two Newton-Raphson steps for
+// f(r) = 1/r - x, r <- r + r (1 - x r), each squaring the relative error;
+// within a few units in the last place, not correctly rounded.  x = 0 gives
+// inf and |x| = inf gives 0, as 1/x does (the refinement is NaN there).
+__device__ __forceinline__ double dc_rcp(double x) {
+  double r0;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r0) : "d"(x));
+  double r = fma(r0, fma(-x, r0, 1.0), r0);
+  r = fma(r, fma(-x, r, 1.0), r);
+  return r == r ? r : r0;
+}
+
+// ------------------------------------------------------------ 1. tridiagonalisation
+// Tiles of a walk over an nm x nm block, upper triangle: row tiles of 2^RS
+// rows, column strips of 2^CS; unit (I, J) exists where the strip's last
+// column reaches the tile's first row.  A unit adds its column products
+// (entries on and above the diagonal) into col[I][c] and its row products
+// (entries above the diagonal) into row[J][r] of the scratch, each written
+// once, and p is their sum in a fixed order.  Wider tiles for larger blocks
+// keep at most 19 column and 10 row partials per entry (every CTA of a group
+// reads them all); 32 x 64 for 225..448 rows gives up to 56 units, one per
+// warp of a cluster of seven or eight.
+constexpr int kWalk1 = 224, kWalk2 = 448;  // 32 x 32, 32 x 64, above: 64 x 128
+__host__ __device__ constexpr int parts(int nm, int shift) { return (nm + (1 << shift) - 1) >> shift; }
+
+// Position in the unit list of one warp: units are numbered strip by strip.
+template <int RS, int CS>
+struct Units {
+  int nI, nJ, J = 0, base = 0;
+  __device__ __forceinline__ explicit Units(int nm) : nI(parts(nm, RS)), nJ(parts(nm, CS)) {}
+  // row tile of unit u (>= the previous one's); -1 past the last
+  __device__ __forceinline__ int seek(int u) {
+    for (;;) {
+      const int cnt = min(nI, parts((J + 1) << CS, RS));
+      if (u - base < cnt) return u - base;
+      base += cnt;
+      if (++J >= nJ) return -1;
+    }
+  }
+};
+
+// Read-only walk: partials of M x over the upper triangle of the block at Mb
+// (nm x nm, row stride n).  A warp reads whole row segments (32 Q contiguous
+// entries), U rows of them before using any (U Q loads in flight per lane).
+// The row sums of eight rows are reduced on the FP64 tensor instruction: with
+// lane l's products of row i as the 4 x 8 operand B_i (entry [l % 4][l / 4])
+// and A_i the matrix with ones in row i only, sum_i A_i B_i holds eight partial
+// sums of row i in its row i; one addition and two exchanges finish them (the
+// same sums by exchanges alone took four times the instructions, and the walk
+// is bound by its instructions when three CTAs share an SM).  U changes no
+// sum's order.
+template <int RS, int CS, int U>
+__device__ __noinline__ void walk_read(const double* Mb, int n, int nm, const double* x, double* part, int gw,
+                                       int ngw) {
+  constexpr int Q = 1 << (CS - 5);
+  static_assert(U % 8 == 0, "rows are reduced in eights");
+  const int lane = threadIdx.x & 31, g = lane >> 2;
+  Units<RS, CS> un(nm);
+  double* col = part;
+  double* row = part + (long long)un.nI * nm;
+  for (int u = gw;; u += ngw) {
+    const int I = un.seek(u);
+    if (I < 0) return;
+    const int c0 = un.J << CS, rbeg = I << RS;
+    const int rend = min(min(nm, rbeg + (1 << RS)), c0 + (1 << CS));
+    double xs[Q], acc[Q];
+    int cc[Q];  // column, -1 past the block
+#pragma unroll
+    for (int j = 0; j < Q; ++j) {
+      const int c = c0 + lane + 32 * j;
+      cc[j] = c < nm ? c : -1;
+      xs[j] = c < nm ? x[c] : 0.0;
+      acc[j] = 0.0;
+    }
+    double* rowp = row + (long long)un.J * nm;
+    for (int rb = rbeg; rb < rend; rb += U) {
+      double a[U][Q];
+      const double* Mr = Mb + (long long)rb * n + c0 + lane;
+      const bool inside = rb + U <= c0 && c0 + (1 << CS) <= nm;  // wholly above the diagonal
+      if (inside) {
+#pragma unroll
+        for (int i = 0; i < U; ++i) {
+#pragma unroll
+          for (int j = 0; j < Q; ++j) a[i][j] = Mr[32 * j];
+          Mr += n;
+        }
+      } else {
+#pragma unroll
+        for (int i = 0; i < U; ++i) {
+#pragma unroll
+          for (int j = 0; j < Q; ++j) a[i][j] = cc[j] - rb >= i ? Mr[32 * j] : 0.0;
+          Mr += n;
+        }
+      }
+      double v[U];  // lane's products of each row
+#pragma unroll
+      for (int i = 0; i < U; ++i) {
+        // (rows past the block hold zeros; x is finite there)
+        const double xr = x[rb + i];
+        v[i] = 0.0;
+        if (inside) {
+#pragma unroll
+          for (int j = 0; j < Q; ++j) {
+            acc[j] += a[i][j] * xr;
+            v[i] += a[i][j] * xs[j];
+          }
+        } else {
+#pragma unroll
+          for (int j = 0; j < Q; ++j) {
+            acc[j] += a[i][j] * xr;
+            if (cc[j] - rb > i) v[i] += a[i][j] * xs[j];
+          }
+        }
+      }
+      double s0[U / 4], s1[U / 4];  // two chains (even and odd rows) per eight rows
+#pragma unroll
+      for (int k = 0; k < U / 4; ++k) s0[k] = s1[k] = 0.0;
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int k = 0; k < U / 8; ++k) dmma(s0[2 * k + (i & 1)], s1[2 * k + (i & 1)], g == i ? 1.0 : 0.0, v[8 * k + i]);
+#pragma unroll
+      for (int k = 0; k < U / 8; ++k) {
+        double t = (s0[2 * k] + s1[2 * k]) + (s0[2 * k + 1] + s1[2 * k + 1]);
+        t += __shfl_xor_sync(0xffffffffu, t, 1);
+        t += __shfl_xor_sync(0xffffffffu, t, 2);
+        const int r = rb + 8 * k + g;
+        if ((lane & 3) == 0 && r < nm) rowp[r] = t;
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < Q; ++j)
+      if (cc[j] >= 0) col[(long long)I * nm + cc[j]] = acc[j];
+  }
+}
+
+// Panel-closing walk over the same units: with the
+// panel's pairs as K = [PV; PW] and L = [PW; PV] (16 x n, absolute index), the
+// upper triangle is updated as M -= K^T L on 16 x 16 sub-tiles of the FP64
+// tensor instruction (accumulators initialised from M, stored back), and the
+// partials of M_new x are formed from the same fragments.  NB sub-tiles of a
+// 16-column block are loaded before the first is used.
+template <int RS, int CS, int NB>
+__device__ __noinline__ void walk_close(double* Mb, int n, int r0, int nm, const double* PV, const double* PW,
+                                        const double* x, double* part, int gw, int ngw) {
+  constexpr int RB = 1 << (RS - 4);
+  static_assert(RB % NB == 0, "sub-tiles per load round");
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  Units<RS, CS> un(nm);
+  double* col = part;
+  double* row = part + (long long)un.nI * nm;
+  for (int u = gw;; u += ngw) {
+    const int I = un.seek(u);
+    if (I < 0) return;
+    const int J = un.J, c0 = J << CS, rbeg = I << RS;
+    double rp[RB][2];
+#pragma unroll
+    for (int i = 0; i < RB; ++i) rp[i][0] = rp[i][1] = 0.0;
+    for (int cw = c0; cw < min(nm, c0 + (1 << CS)); cw += 16) {
+      double cs[4] = {0.0, 0.0, 0.0, 0.0};  // column sums, index 2y + h
+      double* M0 = Mb + (long long)(rbeg + g) * n + cw + 2 * t;
+#pragma unroll
+      for (int rb0 = 0; rb0 < RB; rb0 += NB) {
+        double d[NB][2][2][2];
+#pragma unroll
+        for (int i = 0; i < NB; ++i) {
+          const int rt = rbeg + 16 * (rb0 + i);
+          const bool inside = rt + 16 <= cw && cw + 16 <= nm;
+#pragma unroll
+          for (int xx = 0; xx < 2; ++xx)
+#pragma unroll
+            for (int y = 0; y < 2; ++y)
+#pragma unroll
+              for (int h = 0; h < 2; ++h) {
+                const int r = rt + 8 * xx + g, c = cw + 8 * y + 2 * t + h;
+                d[i][xx][y][h] = (inside || (r < nm && c < nm && c >= r))
+                                     ? M0[(long long)(16 * (rb0 + i) + 8 * xx) * n + 8 * y + h] : 0.0;
+              }
+        }
+#pragma unroll
+        for (int ks = 0; ks < 4; ++ks) {
+          const double* Lc = (ks < 2 ? PW : PV) + (long long)(4 * (ks & 1) + t) * n + r0;
+          const double* Kr = (ks < 2 ? PV : PW) + (long long)(4 * (ks & 1) + t) * n + r0;
+          double b[2];
+#pragma unroll
+          for (int y = 0; y < 2; ++y) {
+            const int c = cw + 8 * y + g;
+            b[y] = c < nm ? Lc[c] : 0.0;
+          }
+#pragma unroll
+          for (int i = 0; i < NB; ++i)
+#pragma unroll
+            for (int xx = 0; xx < 2; ++xx) {
+              const int r = rbeg + 16 * (rb0 + i) + 8 * xx + g;
+              const double a = r < nm ? -Kr[r] : 0.0;
+#pragma unroll
+              for (int y = 0; y < 2; ++y) dmma(d[i][xx][y][0], d[i][xx][y][1], a, b[y]);
+            }
+        }
+        // store the upper entries, drop the others from the products
+#pragma unroll
+        for (int i = 0; i < NB; ++i) {
+          const int rt = rbeg + 16 * (rb0 + i);
+          const bool inside = rt + 16 <= cw && cw + 16 <= nm;
+#pragma unroll
+          for (int xx = 0; xx < 2; ++xx) {
+            const int r = rt + 8 * xx + g;
+            const double xr = r < nm ? x[r] : 0.0;
+#pragma unroll
+            for (int y = 0; y < 2; ++y)
+#pragma unroll
+              for (int h = 0; h < 2; ++h) {
+                const int c = cw + 8 * y + 2 * t + h;
+                if (inside || (r < nm && c < nm && c >= r)) {
+                  const double z = d[i][xx][y][h];
+                  M0[(long long)(16 * (rb0 + i) + 8 * xx) * n + 8 * y + h] = z;
+                  cs[2 * y + h] += z * xr;
+                  if (inside || c > r) rp[rb0 + i][xx] += z * x[c];
+                }
+              }
+          }
+        }
+      }
+      // column sums over the eight row lanes g (lane bits 4, 3, 2): lane bit 4
+      // ends with y, bit 3 with h
+      {
+        const bool u16 = lane & 16, u8 = lane & 8;
+        const double s0 = u16 ? cs[0] : cs[2], s1 = u16 ? cs[1] : cs[3];
+        const double k0 = (u16 ? cs[2] : cs[0]) + __shfl_xor_sync(0xffffffffu, s0, 16);
+        const double k1 = (u16 ? cs[3] : cs[1]) + __shfl_xor_sync(0xffffffffu, s1, 16);
+        const double s = u8 ? k0 : k1;
+        double k = (u8 ? k1 : k0) + __shfl_xor_sync(0xffffffffu, s, 8);
+        k += __shfl_xor_sync(0xffffffffu, k, 4);
+        const int c = cw + (u16 ? 8 : 0) + 2 * t + (u8 ? 1 : 0);
+        if (!(lane & 4) && c < nm) col[(long long)I * nm + c] = k;
+      }
+    }
+#pragma unroll
+    for (int rbk = 0; rbk < RB; ++rbk) {  // row sums over the four column lanes t
+      const bool u1 = lane & 1;
+      double k = (u1 ? rp[rbk][1] : rp[rbk][0]) +
+                 __shfl_xor_sync(0xffffffffu, u1 ? rp[rbk][0] : rp[rbk][1], 1);
+      k += __shfl_xor_sync(0xffffffffu, k, 2);
+      const int r = rbeg + 16 * rbk + (u1 ? 8 : 0) + g;
+      if (!(lane & 2) && r < nm) row[(long long)J * nm + r] = k;
+    }
+  }
+}
+
+// Sum of entry c's partials: column tiles I with rows I <= c, then the strips
+// with columns beyond c.  Every load is issued before `between` runs and the
+// first addition follows it.
+template <int RS, int CS, int NI, int NJ, typename F>
+__device__ __forceinline__ double walk_gather(const double* part, int nm, int c, F between) {
+  const int ni = (c >> RS) + 1, j0 = (c + 1) >> CS, nj = parts(nm, CS) - j0;  // strips whose last column is > c
+  const double* col = part + c;
+  const double* row = col + (long long)(parts(nm, RS) + j0) * nm;
+  double a[NI], b[NJ];
+#pragma unroll
+  for (int i = 0; i < NI; ++i) {
+    a[i] = i < ni ? *col : 0.0;
+    col += nm;
+  }
+#pragma unroll
+  for (int j = 0; j < NJ; ++j) {
+    b[j] = j < nj ? *row : 0.0;
+    row += nm;
+  }
+  between();
+  double t = 0.0;
+#pragma unroll
+  for (int i = 0; i < NI; ++i) t += a[i];
+#pragma unroll
+  for (int j = 0; j < NJ; ++j) t += b[j];
+  return t;
+}
+template <typename F>
+__device__ __forceinline__ double walk_gather(const double* part, int nm, int c, F between) {
+  if (nm <= kWalk1) return walk_gather<5, 5, parts(kWalk1, 5), parts(kWalk1, 5)>(part, nm, c, between);
+  if (nm <= kWalk2) return walk_gather<5, 6, parts(kWalk2, 5), parts(kWalk2, 6)>(part, nm, c, between);
+  return walk_gather<6, 7, parts(kSyevMaxN, 6), parts(kSyevMaxN, 7)>(part, nm, c, between);
+}
+
+// A (n x n, upper triangle used, row-major) to tridiagonal form: reflector k
+// (leading 1) in row k of A from column k+1 on, its scale in tau[k], the
+// diagonal in d, the off-diagonal in e; d, e and tau complete in every CTA.
+// gs: scratch for the walk partials (at most n^2 doubles).
+template <bool W>
+__device__ __noinline__ void tridiag_tiles(double* A, int n, double* d, double* e, double* tau, double* v, double* vn,
+                                           double* p, double* w, double* ring, double* gs, const Group g) {
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const int gw = g.rank + g.size * wid, ngw = g.size * kWarps;
+  double* PV = ring;               // kPanel x n: v_i of the open panel (absolute index)
+  double* PW = ring + kPanel * n;  // kPanel x n: w_i
+  __shared__ double dots[2][2 * kPanel], red[2][kWarps], s_alpha;
+  // the walks read up to 31 entries of x past the block (against zeros): keep what
+  // follows v and vn finite
+  for (int i = tid; i < n; i += kEigThreads) v[i] = vn[i] = p[i] = w[i] = 0.0;
+  __syncthreads();
+  const int nref = n - 2;  // reflectors 0 .. n-3
+  int np = 0;              // pairs in the open panel
+  for (int r = 0;; ++r) {
+    // row r brought up to date with pair r-1 (formed here from the last walk)
+    const int mm = n - r;  // columns r .. n-1, entry j = column r + j
+    double part2 = 0.0;
+    if (r == 0) {
+      for (int j = tid; j < mm; j += kEigThreads) {
+        const double x = A[j];
+        if (j == 0) d[0] = x;
+        else if (j == 1) s_alpha = x;
+        else { vn[j - 1] = x; part2 += x * x; }
+      }
+    } else {
+      const double tk = tau[r - 1];
+      double* rowr = A + (long long)r * n + r;
+      const double* dot = dots[r & 1];
+      double part = 0.0;
+      for (int j = tid; j < mm; j += kEigThreads) {
+        const double raw = rowr[j];
+        // the open pairs' part of p and of row r, while the partials arrive
+        double cp = 0.0, cx = 0.0;
+        const double sum = walk_gather(gs, mm, j, [&]() {
+          for (int i = 0; i < np; ++i) {
+            const double pv = PV[i * n + r + j], pw = PW[i * n + r + j];
+            cp += pv * dot[i] + pw * dot[kPanel + i];
+            cx += PV[i * n + r] * pw + PW[i * n + r] * pv;
+          }
+        });
+        const double pj = tk * (sum - cp);
+        p[j] = pj;
+        w[j] = raw - cx;
+        part += pj * v[j];
+      }
+      // reflector r-1 into row r-1: every CTA has read that row's old values
+      // before the last group barrier
+      if (g.size == 1 || (r - 1) % g.size == g.rank)
+        for (int j = tid; j < mm; j += kEigThreads) A[(long long)(r - 1) * n + r + j] = v[j];
+      const double kk = 0.5 * tk * block_sum_once(part, red[0]);
+      const double w0 = p[0] - kk;  // v[0] = 1
+      for (int j = tid; j < mm; j += kEigThreads) {
+        const double vj = v[j], wj = p[j] - kk * vj, x = w[j] - (wj + w0 * vj);
+        PV[np * n + r + j] = vj;
+        PW[np * n + r + j] = wj;
+        if (j == 0) d[r] = x;
+        else if (j == 1) s_alpha = x;
+        else { vn[j - 1] = x; part2 += x * x; }
+      }
+      ++np;
+    }
+    const double sigma = block_sum_once(part2, red[1]);
+    const double alpha = s_alpha;
+    if (r == nref) {  // the last 2 x 2 block
+      if (tid == 0) {
+        e[r] = alpha;
+        double x = A[(long long)(n - 1) * n + n - 1];
+        for (int i = 0; i < np; ++i) x -= 2.0 * PV[i * n + n - 1] * PW[i * n + n - 1];
+        d[n - 1] = x;
+      }
+      break;
+    }
+    // reflector r: v_new = (1, x / (alpha - beta)), beta = -sign(alpha) |(alpha, x)|,
+    // tau = (beta - alpha) / beta = 1 + |alpha| / |beta|; every thread the same
+    // scalars, from one reciprocal square root and one refined reciprocal
+    const int mr = n - r - 1;
+    double scal = 0.0, tr = 0.0, beta = alpha;
+    if (sigma != 0.0) {
+      const double s2 = alpha * alpha + sigma, ri = rsqrt(s2), rr = s2 * ri;
+      beta = alpha <= 0.0 ? rr : -rr;
+      tr = 1.0 + fabs(alpha) * ri;
+      scal = copysign(dc_rcp(fabs(alpha) + rr), -beta);
+    }
+    if (tid == 0) { tau[r] = tr; e[r] = beta; vn[0] = 1.0; }
+    for (int i = 1 + tid; i < mr; i += kEigThreads) vn[i] *= scal;
+    __syncthreads();
+    // products with the new reflector over rows and columns r+1 .. n-1
+    double* Mb = A + (long long)(r + 1) * n + r + 1;
+    if (np == kPanel) {
+      if (mr <= kWalk1) walk_close<5, 5, 2>(Mb, n, r + 1, mr, PV, PW, vn, gs, gw, ngw);
+      else if (mr <= kWalk2) walk_close<5, 6, 2>(Mb, n, r + 1, mr, PV, PW, vn, gs, gw, ngw);
+      else walk_close<6, 7, W ? 4 : 2>(Mb, n, r + 1, mr, PV, PW, vn, gs, gw, ngw);
+      np = 0;
+    } else {
+      if (mr <= kWalk1) walk_read<5, 5, 32>(Mb, n, mr, vn, gs, gw, ngw);
+      else if (mr <= kWalk2) walk_read<5, 6, W ? 32 : 16>(Mb, n, mr, vn, gs, gw, ngw);
+      else walk_read<6, 7, W ? 16 : 8>(Mb, n, mr, vn, gs, gw, ngw);
+      // the next step's w_i . v and v_i . v, one warp each, in every CTA; the
+      // last warps of the group first (the walk's units start at warp 0).  Two
+      // buffers: a CTA one step behind may still read the other
+      double* dot = dots[(r + 1) & 1];
+      for (int q = ngw - 1 - gw; q < 2 * np; q += ngw) {
+        const double* src = (q < np ? PW + q * n : PV + (q - np) * n) + r + 1;
+        double acc = 0.0;
+        for (int j = lane; j < mr; j += 32) acc += src[j] * vn[j];
+        acc = warp_sum(acc);
+        if (lane < g.size) put_at(dot + (q < np ? q : kPanel + q - np), acc, g, lane);
+      }
+    }
+    group_sync(g);
+    double* s = v; v = vn; vn = s;
+  }
+  group_sync(g);  // A's reflectors are written; the partials have been read
+}
+
+// ------------------------------------------------------------ 2. Q
+// One compact-WY block applied to eight rows of Z by one warp, on the FP64
+// tensor instruction: with Zt the rows row0..row0+7 (lane (g, t) = (lane / 4,
+// lane % 4) owns row row0 + g) and columns c0..n-1 (m of them) of Z, Vs the
+// block's reflectors (kQBlock x m, shared memory, row stride mp) and Ts its T:
+//   Wm = Zt Vs^T, Wt = Wm T^T, Zt -= Wt Vs.
+// Wm and Wt (8 x kQBlock) stay in registers -- an accumulator becomes the next
+// product's left operand by exchanges among the four lanes of a row -- so the
+// warps share nothing but Vs and Ts and meet no barrier inside a block.  U
+// steps of four columns are loaded before the first is used.
+template <int U>
+__device__ __forceinline__ void formq_rows(double* Z, int n, int row0, int c0, int m, const double* Vs, int mp,
+                                           const double (*Ts)[kQBlock + 4]) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int r = row0 + g;
+  const bool valid = r >= c0 && r < n;
+  double* zr = Z + (long long)r * n + c0;
+  double a0[2] = {0.0, 0.0}, a1[2] = {0.0, 0.0};  // Wm[g][8y + 2t], Wm[g][8y + 2t + 1]
+  const double* Vg = Vs + g * mp + t;
+  for (int k0 = 0; k0 < m; k0 += 4 * U) {
+    double z[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int c = k0 + 4 * u + t;
+      z[u] = (valid && c < m) ? zr[c] : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int k = k0 + 4 * u;
+      if (k >= m) break;
+      const bool in = k + t < m;
+#pragma unroll
+      for (int y = 0; y < 2; ++y) {
+        const double b = in ? Vg[8 * y * mp + k] : 0.0;
+        dmma(a0[y], a1[y], z[u], b);
+      }
+    }
+  }
+  // left-operand fragment s (columns 4s + t) of an 8 x 16 accumulator
+  auto left = [&](const double* d0, const double* d1, int s) {
+    const int src = (lane & ~3) | ((4 * (s & 1) + t) >> 1);
+    const double x0 = __shfl_sync(0xffffffffu, d0[s >> 1], src), x1 = __shfl_sync(0xffffffffu, d1[s >> 1], src);
+    return (t & 1) ? x1 : x0;
+  };
+  double w0[2] = {0.0, 0.0}, w1[2] = {0.0, 0.0};  // Wt
+#pragma unroll
+  for (int s = 0; s < 4; ++s) {
+    const double a = left(a0, a1, s);
+#pragma unroll
+    for (int y = 0; y < 2; ++y) dmma(w0[y], w1[y], a, Ts[8 * y + g][4 * s + t]);
+  }
+  double wf[4];
+#pragma unroll
+  for (int s = 0; s < 4; ++s) wf[s] = -left(w0, w1, s);
+  const double* Vt = Vs + t * mp + g;
+  constexpr int V = U / 2;  // 8-column fragments per round
+  for (int ct = 0; ct < m; ct += 8 * V) {
+    double d0[V], d1[V];
+#pragma unroll
+    for (int y = 0; y < V; ++y) {
+      const int c = ct + 8 * y + 2 * t;
+      d0[y] = (valid && c < m) ? zr[c] : 0.0;
+      d1[y] = (valid && c + 1 < m) ? zr[c + 1] : 0.0;
+    }
+#pragma unroll
+    for (int y = 0; y < V; ++y) {
+      if (ct + 8 * y >= m) break;
+      const bool in = ct + 8 * y + g < m;
+#pragma unroll
+      for (int s = 0; s < 4; ++s) {
+        const double b = in ? Vt[4 * s * mp + ct + 8 * y] : 0.0;
+        dmma(d0[y], d1[y], wf[s], b);
+      }
+    }
+#pragma unroll
+    for (int y = 0; y < V; ++y) {
+      const int c = ct + 8 * y + 2 * t;
+      if (valid && c < m) zr[c] = d0[y];
+      if (valid && c + 1 < m) zr[c + 1] = d1[y];
+    }
+  }
+}
+
+// Zc = Q^T (row c of Zc = column c of Q), Q = H_0 H_1 ... H_{n-3}, accumulated
+// backwards in blocks of kQBlock reflectors in compact WY form: H_k0 ... H_k1
+// = I - V T V^T (V = [v_k0 .. v_k1], T upper triangular), so
+// Zc <- Zc H_k1 ... H_k0 = Zc - (Zc V) T^T V^T on rows and columns >= k0+1.
+// Every row of Zc is transformed independently of the others: warp gw of the
+// group's ngw takes the rows of the 8-row groups gw, gw + ngw, ... throughout,
+// and the CTAs never wait for one another; each forms V and T of the block
+// itself.  vbuf: 20 n elements of shared memory.
+template <bool W>
+__device__ __noinline__ void form_q(const double* A, double* Z, int n, const double* tau, double* vbuf,
+                                    const Group grp) {
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, g = lane >> 2, t = lane & 3;
+  const int gw = grp.rank + grp.size * wid, ngw = grp.size * kWarps;
+  for (int q = gw; 8 * q < n; q += ngw)
+    for (int i = 8 * q; i < min(n, 8 * q + 8); ++i)
+      for (int j = lane; j < n; j += 32) Z[(long long)i * n + j] = i == j ? 1.0 : 0.0;
+  __shared__ double Ts[kQBlock][kQBlock + 4];  // T of the block (rows padded against bank conflicts)
+  __shared__ double yv[2][3][64];              // V V^T: fragments (0,0), (0,1), (1,1) of 8 x 8, two halves of the columns
+  double* Vs = vbuf;
+  const int nref = n - 2;
+  for (int k1 = nref - 1; k1 >= 0; k1 -= kQBlock) {
+    const int k0 = k1 - kQBlock + 1 > 0 ? k1 - kQBlock + 1 : 0, bb = k1 - k0 + 1;
+    const int c0 = k0 + 1, m = n - c0;
+    const int mp = m + ((20 - (m & 15)) & 15);  // row stride 4 mod 16: conflict-free fragments of both kinds
+    __syncthreads();  // Vs and Ts of the previous block have been read
+    // Vs[j][cc] = v_{k0+j}[c0 + cc]: row k0+j of A from column k0+j+1 (which holds 1), zero before
+    for (int j = wid; j < kQBlock; j += kWarps) {
+      const double* Ar = A + (long long)(k0 + j) * n + c0;
+#pragma unroll 4
+      for (int cc = lane; cc < m; cc += 32) Vs[j * mp + cc] = (j < bb && cc >= j) ? Ar[cc] : 0.0;
+    }
+    __syncthreads();
+    if (wid < 6) {  // fragment (fa, fb) of V V^T over one half of the columns, one warp each
+      const int half = wid / 3, f = wid % 3, fa = f == 2, fb = f > 0;
+      const int steps = (m + 3) / 4, kb = half ? 4 * ((steps + 1) / 2) : 0, ke = half ? m : min(m, 4 * ((steps + 1) / 2));
+      double y0[2] = {0.0, 0.0}, y1[2] = {0.0, 0.0};
+      for (int k = kb; k < ke; k += 8) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int kk = k + 4 * h + t;
+          const double a = kk < ke ? Vs[(8 * fa + g) * mp + kk] : 0.0, b = kk < ke ? Vs[(8 * fb + g) * mp + kk] : 0.0;
+          dmma(y0[h], y1[h], a, b);
+        }
+      }
+      yv[half][f][8 * g + 2 * t] = y0[0] + y0[1];
+      yv[half][f][8 * g + 2 * t + 1] = y1[0] + y1[1];
+    }
+    __syncthreads();
+    if (tid < kQBlock) {  // T[i][i] = tau, T[0:i][i] = -tau T[0:i][0:i] (V^T v_i)[0:i]; lane r: row r
+      const int r = tid;
+      double acc[kQBlock];
+#pragma unroll
+      for (int i = 0; i < kQBlock; ++i) acc[i] = 0.0;
+#pragma unroll
+      for (int q = 0; q < kQBlock; ++q) {
+        const double tq = q < bb ? tau[k0 + q] : 0.0;
+        const double x = q == r ? tq : (q > r ? -tq * acc[q] : 0.0);
+        Ts[r][q] = x;
+#pragma unroll
+        for (int i = q + 1; i < kQBlock; ++i) {
+          const int f = (q >> 3) + (i >> 3), xy = 8 * (q & 7) + (i & 7);
+          acc[i] += x * (yv[0][f][xy] + yv[1][f][xy]);
+        }
+      }
+    }
+    __syncthreads();
+    for (int q = (c0 >> 3) + ((gw - (c0 >> 3)) % ngw + ngw) % ngw; 8 * q < n; q += ngw)
+      formq_rows<W ? 32 : 16>(Z, n, 8 * q, c0, m, Vs, mp, Ts);
+  }
+}
+
+// ------------------------------------------------------------ 3. divide and conquer (Cuppen)
+// Tridiagonal T (d, e) = diag(T_left, T_right) + rho v v^T torn at every node
+// of a halving tree down to leaves of at most kDcLeaf rows; the eigenvector
+// matrix G of each node (rows = eigenvectors in T's index space, an m x m
+// diagonal block of an n x n buffer) is built bottom-up by rank-one merges:
+//  * z = [last column of G_left ; sign(e) * first column of G_right], unit
+//    norm, rho' = |e| |z|^2; eigenvalues sorted;
+//  * deflation (tolerance 8 eps max(|delta|max, rho')): entries with rho'|z_i|
+//    below it keep their eigenpair; adjacent close pairs are rotated so that
+//    one z entry vanishes (LAPACK dlaed2's two tests);
+//  * roots of the secular equation 1 + rho' sum z_i^2 / (delta_i - lambda) = 0
+//    by bracketed two-pole rational interpolation (Bunch, Nielsen and Sorensen
+//    1978), each root kept as (nearest pole, offset) so that delta_i - lambda
+//    keeps full relative accuracy;
+//  * z recomputed from the roots (Gu and Eisenstat 1994) so the eigenvectors
+//    w_j = z_i / (delta_i - lambda_j) are orthogonal to working accuracy;
+//  * G_node = W G_children as a tiled product.
+// Finally Zc <- G Zc (Zc = Q^T), and the eigenvalues are left in d.
+// kDcMin, kDcK, kDcBs, kDcTileElems and dc_ws_elems (tb_kernels.h): the
+// workspace starts at tau and runs to the end of the dynamic shared memory,
+// which syev_smem_bytes sizes so that every structure of kDcMin+ rows has it.
+//
+// The roots, the recomputed z and the norms are each formed by a team of four
+// lanes (terms sub, sub + 4, ..., combined by two exchanges): a root's chain of
+// passes over the k terms is four times shorter than with one thread, and a
+// group's CTAs take every size-th root.
+
+__device__ __forceinline__ double team_sum(double v, unsigned mask) {
+  v += __shfl_xor_sync(mask, v, 1);
+  v += __shfl_xor_sync(mask, v, 2);
+  return v;
+}
+__device__ __forceinline__ double team_mul(double v, unsigned mask) {
+  v *= __shfl_xor_sync(mask, v, 1);
+  v *= __shfl_xor_sync(mask, v, 2);
+  return v;
+}
+
+// Root j of 1 + rho sum_i z_i^2 / (dl_i - lambda) = 0 (dl strictly ascending,
+// rho > 0): lambda = dl[*o] + *tau, by the four lanes of `mask` (sub 0..3).
+__device__ void secular_root(int j, int k, const double* dl, const double* z, double rho, int sub, unsigned mask,
+                             int* o_out, double* tau_out) {
+  int o;
+  double lo, hi;
+  if (j < k - 1) {
+    const double mid = 0.5 * (dl[j + 1] - dl[j]);
+    double f = 0.0;
+    for (int i = sub; i < k; i += 4) f += z[i] * z[i] * dc_rcp((dl[i] - dl[j]) - mid);
+    f = 1.0 + rho * team_sum(f, mask);
+    if (f >= 0.0) { o = j; lo = 0.0; hi = mid; }
+    else { o = j + 1; lo = -mid; hi = 0.0; }
+  } else {
+    double s = 0.0;
+    for (int i = sub; i < k; i += 4) s += z[i] * z[i];
+    o = k - 1; lo = 0.0; hi = rho * team_sum(s, mask);
+  }
+  const double base = dl[o];
+  double tau = 0.5 * (lo + hi);
+  for (int it = 0; it < 100; ++it) {
+    double psi = 0.0, phi = 0.0, dpsi = 0.0, dphi = 0.0;
+    int i = sub;
+    for (; i <= j; i += 4) {
+      const double r = dc_rcp((dl[i] - base) - tau);
+      const double q = z[i] * z[i] * r;
+      psi += q; dpsi += q * r;
+    }
+    for (; i < k; i += 4) {
+      const double r = dc_rcp((dl[i] - base) - tau);
+      const double q = z[i] * z[i] * r;
+      phi += q; dphi += q * r;
+    }
+    psi = rho * team_sum(psi, mask); phi = rho * team_sum(phi, mask);
+    dpsi = rho * team_sum(dpsi, mask); dphi = rho * team_sum(dphi, mask);
+    const double f = 1.0 + psi + phi;
+    const double err = kEps * (8.0 * (fabs(psi) + fabs(phi)) + 3.0 + fabs(tau) * (dpsi + dphi));
+    if (fabs(f) <= err) break;
+    if (f < 0.0) lo = tau; else hi = tau;
+    if (hi - lo <= 2.0 * kEps * fmax(fabs(lo), fabs(hi))) break;
+    const double a = (dl[j] - base) - tau;
+    double eta = 0.0;
+    bool ok = false;
+    if (j < k - 1) {  // psi ~ c1 + s1/(a - eta), phi ~ c2 + s2/(b - eta)
+      const double b = (dl[j + 1] - base) - tau;
+      const double s1 = dpsi * a * a, c1 = psi - dpsi * a, s2 = dphi * b * b, c2 = phi - dphi * b;
+      const double C = 1.0 + c1 + c2;
+      const double Bq = C * (a + b) + s1 + s2;
+      const double sq = sqrt(fmax(Bq * Bq - 4.0 * C * a * b * f, 0.0));
+      const double q = Bq >= 0.0 ? 0.5 * (Bq + sq) : 0.5 * (Bq - sq);
+      if (q != 0.0) { eta = a * b * f / q; ok = eta > a && eta < b; }
+      if (!ok && C != 0.0) { eta = q / C; ok = eta > a && eta < b; }
+    } else {
+      const double s1 = dpsi * a * a, C = 1.0 + psi - dpsi * a;
+      if (C > 0.0) { eta = a + s1 / C; ok = true; }
+    }
+    double tn = tau + eta;
+    if (!ok || !(tn > lo && tn < hi)) tn = 0.5 * (lo + hi);
+    tau = tn;
+  }
+  *o_out = o;
+  *tau_out = tau;
+}
+
+// Out[(r0 + j) ld + c0 + c] = sum_i gen(j, i) In[(srow ? srow[i] : i) ld + c0 + c]
+// for j < nrow, c < ncol, i < kdim, the group's CTAs taking every size-th of
+// the 64 x 64 output tiles (numbered from first); slabs of kDcK staged in
+// shared memory (Wt: 64 x kDcK, Bt: kDcK x 64 with padded rows), the next
+// slab (its loads and generated entries) fetched into registers while the
+// current one is multiplied on the FP64 tensor instruction (each warp a
+// 16 x 32 block as 2 x 4 fragments of 8 x 8).
+template <typename Gen>
+__device__ void dc_gemm(int nrow, int kdim, int ncol, Gen gen, const double* In, const int* srow, double* Out, int r0,
+                        int c0, int ld, double* Wt, double* Bt, const Group g, int first = 0) {
+  const int tid = threadIdx.x;
+  const int lane = tid & 31, warp = tid >> 5, gl = lane >> 2, tg = lane & 3;
+  const int wrow = (warp >> 1) * 16, wcol = (warp & 1) * 32;  // this warp's block of the tile
+  int idx = first;
+  for (int j0 = 0; j0 < nrow; j0 += 64) {
+    for (int cb = 0; cb < ncol; cb += 64, ++idx) {
+      if (g.size > 1 && idx % g.size != g.rank) continue;
+      double acc[2][4], acc2[2][4];
+#pragma unroll
+      for (int a = 0; a < 2; ++a)
+#pragma unroll
+        for (int b = 0; b < 4; ++b) acc[a][b] = acc2[a][b] = 0.0;
+      constexpr int kPer = 64 * kDcK / kEigThreads;  // slab entries per thread
+      double wr[kPer], br[kPer];
+      auto fetch = [&](int i0) {
+#pragma unroll
+        for (int u = 0; u < kPer; ++u) {
+          const int x = tid + u * kEigThreads;
+          const int jj = x / kDcK, kk = x - jj * kDcK, j = j0 + jj, i = i0 + kk;
+          wr[u] = (j < nrow && i < kdim) ? gen(j, i) : 0.0;
+          const int kb = x >> 6, cc = x & 63, ib = i0 + kb;
+          br[u] = (ib < kdim && cb + cc < ncol) ? In[(long long)(srow ? srow[ib] : ib) * ld + c0 + cb + cc] : 0.0;
+        }
+      };
+      fetch(0);
+      for (int i0 = 0; i0 < kdim; i0 += kDcK) {
+#pragma unroll
+        for (int u = 0; u < kPer; ++u) {
+          const int x = tid + u * kEigThreads;
+          Wt[x] = wr[u];
+          Bt[(x >> 6) * kDcBs + (x & 63)] = br[u];
+        }
+        __syncthreads();
+        if (i0 + kDcK < kdim) fetch(i0 + kDcK);
+#pragma unroll
+        for (int k4 = 0; k4 < kDcK; k4 += 4) {
+          double af[2], bf[4];
+#pragma unroll
+          for (int x = 0; x < 2; ++x) af[x] = Wt[(wrow + 8 * x + gl) * kDcK + k4 + tg];
+#pragma unroll
+          for (int y = 0; y < 4; ++y) bf[y] = Bt[(k4 + tg) * kDcBs + wcol + 8 * y + gl];
+#pragma unroll
+          for (int x = 0; x < 2; ++x)
+#pragma unroll
+            for (int y = 0; y < 4; ++y) dmma(acc[x][y], acc2[x][y], af[x], bf[y]);
+        }
+        __syncthreads();
+      }
+      // fragment (x, y): rows wrow + 8x + gl, columns wcol + 8y + 2 tg + {0, 1}
+#pragma unroll
+      for (int x = 0; x < 2; ++x) {
+        const int j = j0 + wrow + 8 * x + gl;
+        if (j >= nrow) continue;
+#pragma unroll
+        for (int y = 0; y < 4; ++y) {
+          const int c = cb + wcol + 8 * y + 2 * tg;
+          if (c < ncol) Out[(long long)(r0 + j) * ld + c0 + c] = acc[x][y];
+          if (c + 1 < ncol) Out[(long long)(r0 + j) * ld + c0 + c + 1] = acc2[x][y];
+        }
+      }
+    }
+  }
+}
+
+// One merge of the node [lo, hi) torn at t by the CTAs of g: children's G
+// blocks in Gi (the node's diagonal block), eigenvalues in d[lo, hi) of every
+// CTA.  The rows lo..hi-1 of V (columns vc0 .. vc0+vcols-1; V = Gi itself, or
+// the children's eigenvectors already applied to Zc) are combined into the
+// same rows of Out and the merged eigenvalues written to d[lo, hi) of every
+// CTA.  V is overwritten.  ws: dc_ws_elems(hi - lo) doubles.
+template <bool W>
+__device__ __noinline__ void dc_merge(double* d, const double* e, int n, int lo, int t, int hi, double* Gi, double* V,
+                                      int vc0, int vcols, double* Out, double* ws, const Group g) {
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const int gw = g.rank * kWarps + wid, ngw = g.size * kWarps;
+  const int m = hi - lo;
+  double* delta = ws;          // m: sorted eigenvalues (rotated pairs updated)
+  double* zs = delta + m;      // m: sorted z (unit norm)
+  double* dl = zs + m;         // k: non-deflated delta
+  double* zl = dl + m;         // k: their z, then the recomputed z
+  double* tv = zl + m;         // k: root offsets
+  double* inrm = tv + m;       // k: 1 / |w_j|
+  double* rc = inrm + m;       // rotations: cosine
+  double* rsn = rc + m;        //            sine
+  double* Wt = rsn + m;
+  double* Bt = Wt + 64 * kDcK;
+  int* rowof = reinterpret_cast<int*>(Wt + kDcTileElems);  // m: row of sorted entry s
+  int* flg = rowof + m;   // m: deflated
+  int* ndl = flg + m;     // m: sorted index of the k non-deflated, then of the deflated
+  int* rp = ndl + m;      // rotations: rows
+  int* rq = rp + m;
+  int* ori = rq + m;      // k: root origin (index into dl)
+  int* srow = ori + m;    // k: row of non-deflated entry
+  __shared__ int s_k, s_nrot;
+  __shared__ double red[kWarps];
+  const double ev = e[t - 1];
+  const double rho = fabs(ev), sg = ev >= 0.0 ? 1.0 : -1.0;
+  // children's blocks are diagonal sub-blocks: clear the rest of the node's block
+  if (V == Gi)
+    for (int r = lo + gw; r < hi; r += ngw)
+      for (int c = (r < t ? t : lo) + lane; c < (r < t ? hi : t); c += 32) Gi[(long long)r * n + c] = 0.0;
+  // z and its norm (in rc until the rotations are formed)
+  double part = 0.0;
+  for (int r = lo + tid; r < hi; r += kEigThreads) {
+    const double z = r < t ? Gi[(long long)r * n + t - 1] : sg * Gi[(long long)r * n + t];
+    rc[r - lo] = z;
+    rowof[r - lo] = r;  // valid rows even where non-finite eigenvalues leave ranks unset below
+    delta[r - lo] = zs[r - lo] = 0.0;
+    part += z * z;
+  }
+  const double zz = block_sum_once(part, red);
+  const double zsc = 1.0 / sqrt(zz), rhop = rho * zz;
+  // rank sort of the eigenvalues (ties by index)
+  for (int r = lo + tid; r < hi; r += kEigThreads) {
+    const double dr = d[r];
+    int rank = 0;
+    for (int q = lo; q < hi; ++q) {
+      const double dq = d[q];
+      rank += (dq < dr || (dq == dr && q < r)) ? 1 : 0;
+    }
+    rowof[rank] = r;
+    delta[rank] = dr;
+    zs[rank] = rc[r - lo] * zsc;
+  }
+  __syncthreads();
+  if (tid < 32) {  // deflation scan (lane 0, in order) and compaction (warp ballots), warp 0
+    double dmax = 0.0;
+    for (int s = lane; s < m; s += 32) dmax = fmax(dmax, fabs(delta[s]));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) dmax = fmax(dmax, __shfl_xor_sync(0xffffffffu, dmax, o));
+    const double tol = 8.0 * kEps * fmax(dmax, rhop);
+    for (int s = lane; s < m; s += 32) flg[s] = rhop * fabs(zs[s]) <= tol ? 1 : 0;
+    __syncwarp();
+    if (lane == 0) {
+      // close pair (prev, s): the rotation zeroing z_prev (c = z_s / tau, sn = -z_prev / tau,
+      // tau = |(z_prev, z_s)|) deflates when |(d_s - d_prev) c sn| <= tol, tested as
+      // |d_s - d_prev| |z_prev z_s| <= tol tau^2 without the square root
+      int nrot = 0, prev = -1;
+      for (int s = 0; s < m; ++s) {
+        if (flg[s]) continue;
+        if (prev >= 0) {
+          const double za = zs[prev], zb = zs[s], t2 = za * za + zb * zb;
+          if (fabs(delta[s] - delta[prev]) * fabs(za * zb) <= tol * t2) {
+            const double tau = sqrt(t2);
+            const double c = zb / tau, sn = -za / tau;
+            rp[nrot] = rowof[prev]; rq[nrot] = rowof[s]; rc[nrot] = c; rsn[nrot] = sn; ++nrot;
+            zs[s] = tau; zs[prev] = 0.0;
+            const double dp = delta[prev], ds = delta[s];
+            delta[prev] = dp * c * c + ds * sn * sn;
+            delta[s] = dp * sn * sn + ds * c * c;
+            flg[prev] = 1;
+          }
+        }
+        prev = s;
+      }
+      s_nrot = nrot;
+    }
+    __syncwarp();
+    // non-deflated entries first, then the deflated ones, each in order
+    int k = 0;
+    for (int s0 = 0; s0 < m; s0 += 32) {
+      const int s = s0 + lane;
+      const bool keep = s < m && !flg[s];
+      const unsigned bal = __ballot_sync(0xffffffffu, keep);
+      if (keep) {
+        const int pos = k + __popc(bal & ((1u << lane) - 1u));
+        ndl[pos] = s; dl[pos] = delta[s]; zl[pos] = zs[s]; srow[pos] = rowof[s];
+      }
+      k += __popc(bal);
+    }
+    int q = k;
+    for (int s0 = 0; s0 < m; s0 += 32) {
+      const int s = s0 + lane;
+      const bool defl = s < m && flg[s];
+      const unsigned bal = __ballot_sync(0xffffffffu, defl);
+      if (defl) ndl[q + __popc(bal & ((1u << lane) - 1u))] = s;
+      q += __popc(bal);
+    }
+    if (lane == 0) s_k = k;
+  }
+  __syncthreads();
+  const int k = s_k, nrot = s_nrot;
+  // close-pair rotations on the rows, one thread per column, in order (a group
+  // first waits until its CTAs have read z and cleared their rows)
+  if (nrot > 0 && g.size > 1) group_sync(g);
+  for (int c = vc0 + g.rank * kEigThreads + tid; c < vc0 + vcols; c += g.size * kEigThreads)
+    for (int q = 0; q < nrot; ++q) {
+      double* pa = V + (long long)rp[q] * n + c;
+      double* pb = V + (long long)rq[q] * n + c;
+      const double a = *pa, b = *pb;
+      *pa = rc[q] * a + rsn[q] * b;
+      *pb = rc[q] * b - rsn[q] * a;
+    }
+  // teams of four lanes: roots, recomputed z, norms
+  const int sub = lane & 3, team = tid >> 2, gteam = g.rank + g.size * team, nteam = g.size * (kEigThreads / 4);
+  const unsigned mask = 0xfu << (lane & ~3);
+  for (int j = gteam; j < k; j += nteam) {
+    int o;
+    double tj;
+    secular_root(j, k, dl, zl, rhop, sub, mask, &o, &tj);
+    for (int r = sub; r < g.size; r += 4) {
+      put_at(ori + j, o, g, r);
+      put_at(tv + j, tj, g, r);
+    }
+  }
+  group_sync(g);
+  // z of the k poles, recomputed from the roots (Gu and Eisenstat: every ratio
+  // in (0, 1]); the new entry keeps the old one's sign, so a lane of the team
+  // that reads it late reads the same sign
+  for (int i = gteam; i < k; i += nteam) {
+    const double di = dl[i];
+    double prod = 1.0;
+    int j = sub;
+    for (; j < i; j += 4) prod *= ((dl[ori[j]] - di) + tv[j]) * dc_rcp(dl[j] - di);
+    for (; j < k; j += 4)
+      if (j > i) prod *= ((dl[ori[j - 1]] - di) + tv[j - 1]) * dc_rcp(dl[j] - di);
+    prod = team_mul(prod, mask) * (((dl[ori[k - 1]] - di) + tv[k - 1]) / rhop);
+    const double z = copysign(sqrt(fmax(prod, 0.0)), zl[i]);
+    for (int r = sub; r < g.size; r += 4) put_at(zl + i, z, g, r);
+  }
+  group_sync(g);
+  // W formed once (row stride n) instead of once per 64-column tile of the
+  // product, where Gi has a free k x k block: at the root all of Gi is free
+  // once z has been read; below it, rows lo.. of Gi beside the node's block
+  // (columns hi.. or ..lo) belong to no node of this level
+  double* Wb = nullptr;
+  if (V != Gi) Wb = Gi;
+  else if (hi + k <= n) Wb = Gi + (long long)lo * n + hi;
+  else if (lo >= k) Wb = Gi + (long long)lo * n + (lo - k);
+  // norms: of this CTA's rows of W (rows gw, gw + ngw, ...), of all rows where
+  // every tile generates its own
+  const int r0w = g.rank * kWarps;
+  const int nq = !Wb ? k : (k > r0w ? kWarps * ((k - r0w + ngw - 1) / ngw) : 0);
+  for (int q = team; q < nq; q += kEigThreads / 4) {
+    const int j = Wb ? (q / kWarps) * ngw + r0w + q % kWarps : q;
+    if (j >= k) continue;
+    const double bj = dl[ori[j]], tj = tv[j];
+    double s = 0.0;
+    for (int i = sub; i < k; i += 4) {
+      const double w = zl[i] * dc_rcp((dl[i] - bj) - tj);
+      s += w * w;
+    }
+    s = team_sum(s, mask);
+    if (sub == 0) inrm[j] = 1.0 / sqrt(s);
+  }
+  __syncthreads();
+  // roots: Out rows lo .. lo+k-1; deflated: rows lo+k .. hi-1 copied
+  auto wgen = [&](int j, int i) { return zl[i] * dc_rcp((dl[i] - dl[ori[j]]) - tv[j]) * inrm[j]; };
+  if (Wb) {
+    for (int j = gw; j < k; j += ngw)
+      for (int i = lane; i < k; i += 32) Wb[(long long)j * n + i] = wgen(j, i);
+    group_sync(g);
+    dc_gemm(k, k, vcols, [&](int j, int i) { return Wb[(long long)j * n + i]; }, V, srow, Out, lo, vc0, n, Wt, Bt, g);
+  } else {
+    dc_gemm(k, k, vcols, wgen, V, srow, Out, lo, vc0, n, Wt, Bt, g);
+  }
+  for (int q = gw; q < m - k; q += ngw) {
+    const double* src = V + (long long)rowof[ndl[k + q]] * n;
+    double* dst = Out + (long long)(lo + k + q) * n;
+    for (int c = vc0 + lane; c < vc0 + vcols; c += 32) dst[c] = src[c];
+  }
+  __syncthreads();
+  for (int j = tid; j < m; j += kEigThreads) d[lo + j] = j < k ? dl[ori[j]] + tv[j] : delta[ndl[j]];
+  group_sync(g);
+}
+
+constexpr int kDcLeaf = 24;  // leaves of the merge tree: at most this many rows, solved by one warp
+
+// Leaf [lo, lo+s) of the tree (s <= kDcLeaf) by one warp: implicit QL with
+// Wilkinson shifts (the same sweep as the k_syev producer) on lane 0 over
+// d[lo..] and a private copy of the leaf's off-diagonal, each sweep's
+// rotations then applied by lanes (one per column) to the rows of the leaf's
+// eigenvector block U in shared memory; U is written to G's diagonal block.
+// Returns false if an eigenvalue took more than 60 sweeps.
+constexpr int kDcLeafWs = kDcLeaf * kDcLeaf + 3 * kDcLeaf;  // per leaf warp: U, off-diagonal, rotations
+static_assert(kDcLeafWs <= dc_ws_elems<double>(kDcMin), "leaf workspace exceeds the divide-and-conquer workspace");
+
+__device__ bool dc_leaf(double* d, const double* e, int lo, int s, double* U, double* le, double* rcs, double* G,
+                        int n) {
+  const int lane = threadIdx.x & 31;
+  for (int x = lane; x < s * s; x += 32) U[x] = (x / s == x % s) ? 1.0 : 0.0;
+  for (int i = lane; i < s; i += 32) le[i] = i < s - 1 ? e[lo + i] : 0.0;
+  __syncwarp();
+  double* dd = d + lo;
+  bool ok = true;
+  for (int l = 0; l < s && ok; ++l) {
+    int iter = 0;
+    for (;;) {
+      int mq = s - 1;
+      for (int i = l; i < s - 1; ++i)
+        if (fabs(le[i]) <= kEps * (fabs(dd[i]) + fabs(dd[i + 1]))) { mq = i; break; }
+      if (mq == l) break;
+      if (++iter > 60) { ok = false; break; }
+      int cnt = 0;
+      if (lane == 0) {
+        double g = (dd[l + 1] - dd[l]) / (2.0 * le[l]);
+        double r = sqrt(g * g + 1.0);
+        g = dd[mq] - dd[l] + le[l] / (g + (g >= 0.0 ? r : -r));
+        double sn = 1.0, c = 1.0, pp = 0.0;
+        bool underflow = false;
+        for (int i = mq - 1; i >= l; --i) {
+          const double f = sn * le[i], bb = c * le[i];
+          const double rr2 = f * f + g * g;
+          if (rr2 == 0.0) { dd[i + 1] -= pp; le[mq] = 0.0; underflow = true; break; }
+          const double ri = rsqrt(rr2);
+          r = rr2 * ri;
+          le[i + 1] = r;
+          sn = f * ri;
+          c = g * ri;
+          g = dd[i + 1] - pp;
+          r = (dd[i] - g) * sn + 2.0 * c * bb;
+          pp = sn * r;
+          dd[i + 1] = g + pp;
+          g = c * r - bb;
+          rcs[2 * cnt] = c;
+          rcs[2 * cnt + 1] = sn;
+          ++cnt;
+        }
+        if (!underflow) { dd[l] -= pp; le[l] = g; le[mq] = 0.0; }
+      }
+      cnt = __shfl_sync(0xffffffffu, cnt, 0);
+      __syncwarp();
+      if (lane < s) {  // rotation t acts on rows i = mq-1-t and i+1 of U
+        for (int t = 0; t < cnt; ++t) {
+          const int i = mq - 1 - t;
+          const double c = rcs[2 * t], sn = rcs[2 * t + 1];
+          const double x = U[i * s + lane], y = U[(i + 1) * s + lane];
+          U[(i + 1) * s + lane] = sn * x + c * y;
+          U[i * s + lane] = c * x - sn * y;
+        }
+      }
+      __syncwarp();
+    }
+  }
+  for (int x = lane; x < s * s; x += 32) G[(long long)(lo + x / s) * n + lo + x % s] = U[x];
+  __syncwarp();
+  return ok;
+}
+
+// Node b of depth dep of the halving tree: [lo, hi); *plen = its parent's size.
+__device__ inline void dc_node(int n, int dep, int b, int* lo_out, int* hi_out, int* plen) {
+  int lo = 0, hi = n, pl = n + 1;
+  for (int l = 0; l < dep; ++l) {
+    const int mid = (lo + hi) >> 1;
+    pl = hi - lo;
+    if ((b >> (dep - 1 - l)) & 1) lo = mid; else hi = mid;
+  }
+  *lo_out = lo; *hi_out = hi; *plen = pl;
+}
+
+// Eigenvalues (d, in every CTA) and eigenvector rows (Zc <- G Zc) of the
+// tridiagonal (d, e) by the merge tree; G0 and G1 are n x n buffers, ws
+// dc_ws_elems(n).  A level with at least as many nodes as CTAs gives each CTA
+// whole merges (no barriers between CTAs inside them), the levels above share
+// every merge.  Returns false if a leaf failed to converge.
+template <bool W>
+__device__ bool dc_solve(double* d, double* e, double* Z, double* G0, double* G1, int n, double* ws, long long ws_cap,
+                         const Group g) {
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const Group alone{0, 1};
+  __shared__ int s_fail;
+  int depth = 0;  // nodes at this depth have at most kDcLeaf rows
+  while (((n + (1 << depth) - 1) >> depth) > kDcLeaf) ++depth;
+  if (tid == 0) s_fail = 0;
+  // tear every internal node (rho = |e[t-1]| off both neighbours)
+  for (int dep = 0; dep < depth; ++dep) {
+    for (int b = tid; b < (1 << dep); b += kEigThreads) {
+      int lo, hi, pl;
+      dc_node(n, dep, b, &lo, &hi, &pl);
+      if (hi - lo <= kDcLeaf) continue;
+      const int t = (lo + hi) >> 1;
+      const double rho = fabs(e[t - 1]);
+      d[t - 1] -= rho;  // nodes of one depth are disjoint
+      d[t] -= rho;
+    }
+    __syncthreads();
+  }
+  group_sync(g);  // every CTA's d is torn before a peer writes a leaf's eigenvalues there
+  // as many leaf warps as the free shared memory holds blocks for
+  const int lw = (int)min((long long)kWarps, ws_cap / kDcLeafWs);
+  double* U = ws + wid * kDcLeafWs;
+  for (int dep = depth; dep >= 0; --dep) {
+    double* Gi = ((depth - dep - 1) & 1) ? G1 : G0;
+    double* Go = ((depth - dep) & 1) ? G1 : G0;
+    // leaves of this depth, one warp each
+    for (int b = g.rank + g.size * wid; wid < lw && b < (1 << dep); b += g.size * lw) {
+      int lo, hi, pl;
+      dc_node(n, dep, b, &lo, &hi, &pl);
+      if (hi - lo < 1 || hi - lo > kDcLeaf || pl <= kDcLeaf) continue;
+      if (!dc_leaf(d, e, lo, hi - lo, U, U + kDcLeaf * kDcLeaf, U + kDcLeaf * kDcLeaf + kDcLeaf, Go, n))
+        for (int r = lane; r < g.size; r += 32) put_at(&s_fail, 1, g, r);
+      for (int r = 0; g.size > 1 && r < g.size; ++r)
+        if (r != g.rank && lane < hi - lo) put_at(d + lo + lane, d[lo + lane], g, r);
+    }
+    if (dep > 0) {
+      const bool whole = (1 << dep) >= g.size;
+      if (whole) __syncthreads();  // the leaf blocks in ws have been read
+      else group_sync(g);
+      for (int b = 0; b < (1 << dep); ++b) {
+        if (whole && b % g.size != g.rank) continue;
+        int lo, hi, pl;
+        dc_node(n, dep, b, &lo, &hi, &pl);
+        if (hi - lo <= kDcLeaf) continue;
+        dc_merge<W>(d, e, n, lo, (lo + hi) >> 1, hi, Gi, Gi, lo, hi - lo, Go, ws, whole ? alone : g);
+        if (whole)
+          for (int r = 0; r < g.size; ++r)
+            if (r != g.rank)
+              for (int i = lo + tid; i < hi; i += kEigThreads) put_at(d + i, d[i], g, r);
+      }
+      group_sync(g);
+    } else {
+      // root: Y = diag(G_left, G_right) Zc into the free buffer, then the
+      // merge combines rows of Y straight into Zc
+      group_sync(g);
+      const int t = n >> 1;
+      double* Wt = ws;
+      double* Bt = Wt + 64 * kDcK;
+      int first = 0;  // tiles of the first product, so that the second's continue the round
+      for (int h = 0; h < 2; ++h) {
+        const int lc = h ? t : 0, sz = h ? n - t : t;
+        dc_gemm(sz, sz, n, [&](int j, int i) { return Gi[(long long)(lc + j) * n + lc + i]; }, Z + (long long)lc * n,
+                nullptr, Go, lc, 0, n, Wt, Bt, g, first);
+        first = ((sz + 63) / 64) * ((n + 63) / 64);
+      }
+      group_sync(g);
+      dc_merge<W>(d, e, n, 0, t, n, Gi, Go, 0, n, Z, ws, g);
+    }
+  }
+  return s_fail == 0;
+}
+
+// Structures of kDcMin+ AOs (those below: k_syev_ql).  The grid is ncoop groups
+// of C CTAs (C = the cluster size), each on one structure (the first ncoop of
+// B.order), then CTAs with a structure each, C to a cluster.
+template <bool W>
+__device__ __forceinline__ void syev_structure(const DevBatch& B, double* __restrict__ Ab, double* __restrict__ Zb,
+                                               double* __restrict__ Sb, double* __restrict__ wout,
+                                               int* __restrict__ perm, int* __restrict__ status,
+                                               const int* __restrict__ active, int ncoop) {
+  unsigned csize, crank;
+  asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(csize));
+  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(crank));
+  const int cid = (int)(blockIdx.x / csize);
+  const bool coop = cid < ncoop;
+  const Group g{coop ? (int)crank : 0, coop ? (int)csize : 1};
+  const int slot = coop ? cid : ncoop + (cid - ncoop) * (int)csize + (int)crank;
+  if (slot >= B.nmol) return;
+  const int m = B.order ? B.order[slot] : slot;  // largest structures first
+  // (the tests below read the same words in every CTA of a group)
+  if (active && !active[m]) return;
+  if (status[m] != kStOk) return;
+  const int n = B.ooff[m + 1] - B.ooff[m];
+  if (on_library(B, n) || n < kDcMin) return;
+  const long long mo = B.moff[m], vo = B.ooff[m];
+  double* A = Ab + mo;
+  double* Z = Zb + mo;
+  double* Sc = Sb + mo;
+  extern __shared__ __align__(16) unsigned char syev_smem[];
+  double* sm = reinterpret_cast<double*>(syev_smem);
+  double* d = sm;          // n
+  double* e = d + n;       // n
+  double* tau = e + n;     // n
+  double* v = tau + n;     // n
+  double* vn = v + n;      // n
+  double* p = vn + n;      // n
+  double* w = p + n;       // n
+  double* ring = w + n;    // 2 kRing n
+  __shared__ int q_fail;
+  const int tid = threadIdx.x;
+
+  if (B.trid_max > 0 && n >= B.trid_min && n >= kTridMin && n <= B.trid_max) {
+    // tridiagonalised in shared memory by k_trid_smem: reflectors in A's rows,
+    // d | e | tau in the first 3n entries of the scratch slice
+    for (int i = tid; i < n; i += kEigThreads) {
+      d[i] = Sc[i];
+      e[i] = i < n - 1 ? Sc[n + i] : 0.0;
+      tau[i] = i < n - 2 ? Sc[2 * n + i] : 0.0;
+    }
+    group_sync(g);
+  } else {
+    tridiag_tiles<W>(A, n, d, e, tau, v, vn, p, w, ring, Sc, g);
+  }
+  form_q<W>(A, Z, n, tau, v, g);
+  group_sync(g);  // Z is complete, A and the scratch are free
+
+  unsigned dyn_bytes;
+  asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dyn_bytes));
+  const long long ws_cap = (long long)(dyn_bytes / sizeof(double)) - 2LL * n;
+  if (tid == 0) { q_fail = 0; e[n - 1] = 0.0; }
+  __syncthreads();
+  const bool conv = dc_solve<W>(d, e, Z, A, Sc, n, tau, ws_cap, g);
+  for (int i = tid; i < n; i += kEigThreads)
+    if (!conv || !(fabs(d[i]) < 1e30)) q_fail = 1;  // a leaf did not converge, or non-finite input
+  __syncthreads();
+  if (q_fail) {
+    if (tid == 0 && g.rank == 0) status[m] = kStEigenFailed;  // k_fermi retires the structure
+    return;
+  }
+  // ascending order by rank (ties by index)
+  for (int i = g.rank * kEigThreads + tid; i < n; i += g.size * kEigThreads) {
+    const double di = d[i];
+    int rank = 0;
+    for (int j = 0; j < n; ++j) {
+      const double dj = d[j];
+      rank += (dj < di || (dj == di && j < i)) ? 1 : 0;
+    }
+    if (!TB_GUARD(9, rank, 0, n)) continue;
+    perm[vo + rank] = i;
+    wout[vo + rank] = di;
+  }
+}
+
+}  // namespace
+
+// Two CTAs per SM (128 registers) for batches that fill the GPU with a CTA per
+// structure, one CTA per SM with whole units in registers for clusters and for
+// orders whose vectors take more than half an SM's shared memory.  Both run
+// the same arithmetic in the same order.  (Three CTAs per SM at 80 registers
+// spilled in the walks and held 16 loads in flight per lane instead of 32:
+// 444 structures of 300 AOs took 4.1 ms of an SM each against 3.9.)
+__global__ void __launch_bounds__(kEigThreads, 2) k_syev(DevBatch B, double* __restrict__ Ab, double* __restrict__ Zb,
+                                                         double* __restrict__ Sb, double* __restrict__ wout,
+                                                         int* __restrict__ perm, int* __restrict__ status,
+                                                         const int* __restrict__ active, int ncoop) {
+  syev_structure<false>(B, Ab, Zb, Sb, wout, perm, status, active, ncoop);
+}
+__global__ void __launch_bounds__(kEigThreads, 1) k_syev_wide(DevBatch B, double* __restrict__ Ab,
+                                                              double* __restrict__ Zb, double* __restrict__ Sb,
+                                                              double* __restrict__ wout, int* __restrict__ perm,
+                                                              int* __restrict__ status,
+                                                              const int* __restrict__ active, int ncoop) {
+  syev_structure<true>(B, Ab, Zb, Sb, wout, perm, status, active, ncoop);
+}
+
+TB_OOB_EXPORT(oob_syev)
+
+namespace {
+// Time of one structure of n AOs on a group of C CTAs, in ms: what the CTAs
+// divide, plus what each repeats or waits for (the steps' barriers, gathers
+// and scalars, a merge's sort and scan).  Measured on one structure alone:
+// 1.6, 9.4, 44, 161 ms at 138, 384, 722, 1196 AOs on one CTA; 1.2, 5.9, 25.5,
+// 88 on two; 1.1, 4.2, 15.6, 52 on four; 1.1, 3.5, 11.3, 34 on eight.
+double syev_ms(double n, int C) {
+  const double serial = n * (6.0e-3 + 6.0e-6 * n), shared = n * n * (3.0e-5 + 6.0e-8 * n);
+  return serial + shared / C;
+}
+}  // namespace
+
+// The cluster size and the number of structures that get a whole cluster: the
+// combination with the shortest modelled span.  A span is list scheduling of
+// the order (largest first) over as many clusters as the GPU holds at once
+// (kCap: cudaOccupancyMaxActiveClusters on a B200, one and two CTAs per SM) for
+// every cluster size and a geometric set of splits into cluster and one-CTA
+// structures.  Two CTAs on an SM slow each other (kSlowTwo; the narrower
+// kernel alone, kSlowNarrow).  400 water clusters of 48..384 AOs: 13.3 ms on
+// one CTA each, 11.0 on two; 128: 11.1 and 6.2 (on four); 48 chains of
+// 122..1196 AOs: 172 and 40 (on eight).  Batches of several waves of CTAs keep
+// one CTA per structure: clusters repeat work and would only lose.
+void SyevPlan::build(const std::vector<int>& sizes, int lib_above, int jacobi_max) {
+  *this = SyevPlan();
+  int first = 0;  // structures of the library path lead the order and exit at once
+  for (size_t i = 0; i < sizes.size(); ++i) {
+    const int n = sizes[i];
+    if (lib_above != 0 && n > lib_above) { first = n64 = (int)i + 1; continue; }
+    nmax = n > nmax ? n : nmax;
+    if (n >= kDcMin) n64 = (int)i + 1;
+    else if (n > jacobi_max) ++nsmall;
+  }
+  if (n64 <= first) return;
+  std::vector<double> busy;  // finish times of the clusters in flight (a heap)
+  auto schedule = [&](int cap, int C, int k, double slow, double limit) {
+    busy.clear();
+    double end = 0.0;
+    for (int i = first; i < n64 && end < limit;) {
+      const bool coop = C > 1 && i < k;
+      double t = slow * syev_ms(sizes[i], coop ? C : 1);
+      i += coop ? 1 : C;
+      if ((int)busy.size() == cap) {
+        std::pop_heap(busy.begin(), busy.end(), std::greater<double>());
+        t += busy.back();
+        busy.pop_back();
+      }
+      busy.push_back(t);
+      std::push_heap(busy.begin(), busy.end(), std::greater<double>());
+      end = std::max(end, t);
+    }
+    return end;
+  };
+  constexpr int kCap[2][4] = {{148, 74, 33, 15}, {296, 148, 71, 33}};
+  constexpr double kSlowTwo = 1.42, kSlowNarrow = 1.1;
+  const int cnt = n64 - first;
+  span = 1e300;
+  for (int per = syev_smem_bytes(nmax) <= kSyevSmemTwo ? 2 : 1; per >= 1; --per)
+    for (int c = 0; c < 4; ++c) {
+      const int C = 1 << c;
+      if (C > 1 && cnt > 4 * 148) break;
+      for (int k = cnt; k >= 1; k = k > 1 ? (3 * k) / 4 : 0) {
+        const int items = C > 1 ? k + (cnt - k + C - 1) / C : cnt;
+        const double slow = per == 1 ? 1.0 : items > kCap[0][c] ? kSlowTwo : kSlowNarrow;
+        const double t = schedule(kCap[per - 1][c], C, first + k, slow, span);
+        if (t < 0.97 * span) { span = t; cluster = C; ncoop = C > 1 ? first + k : 0; wide = per == 1; }
+        if (C == 1) break;
+      }
+    }
+}
+
+cudaError_t launch_syev(const SyevPlan& P, const DevBatch& B, double* A, double* Z, double* Sb, double* w, int* perm,
+                        int* status, const int* active, cudaStream_t st, int64_t* launches) {
+  cudaError_t e = cudaSuccess;
+  const size_t smem = syev_smem_bytes(P.nmax > 1 ? P.nmax : 1);
+  if (P.n64 > 0 && P.nmax >= kDcMin) {
+    DevBatch Bs = B;
+    Bs.nmol = P.n64;  // the kernel's bound on its position in the order
+    const int C = P.cluster;
+    const int groups = P.ncoop + (P.n64 - P.ncoop + C - 1) / C;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)(groups * C));
+    cfg.blockDim = dim3(kEigThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)C;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = C > 1 ? 1 : 0;
+    e = cudaLaunchKernelEx(&cfg, P.wide ? k_syev_wide : k_syev, Bs, A, Z, Sb, w, perm, status, active, P.ncoop);
+    if (e != cudaSuccess) return e;
+    if (launches) ++*launches;
+  }
+  if (P.nsmall > 0) {
+    k_syev_ql<<<B.nmol, kEigThreads, smem, st>>>(B, A, Z, w, perm, status, active);
+    e = cudaGetLastError();
+    if (launches) ++*launches;
+  }
+  return e;
+}
+
+}  // namespace tb

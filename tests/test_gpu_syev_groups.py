@@ -1,0 +1,57 @@
+"""GPU: k_syev on one CTA and on clusters.
+
+The eigensolver's units of work depend on the matrix order alone, so a
+structure gives the same bits alone (a cluster of CTAs) and in a batch of
+several waves (one CTA per structure).  Orders at the edges of its tiles
+(walk shapes change at 224 and 448 rows, leaves at 24 rows, Q in 16-reflector
+blocks) are compared with numpy through the allocation-free entry point.
+"""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from tblite_b200 import capi
+from tblite_b200 import geometry as g
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n", [64, 65, 97, 112, 129, 193, 223, 224, 225, 226, 240, 255, 256])
+def test_orders_at_tile_edges(n):
+    import torch
+    rng = np.random.default_rng(n)
+    a = rng.standard_normal((n, n))
+    H = 0.5 * (a + a.T)
+    if n == 129:  # threefold degenerate
+        H = np.diag(np.repeat(np.arange(43.0), 3))
+    b = 0.1 * rng.standard_normal((n, n))
+    S = np.eye(n) + b @ b.T / n
+    h, s = torch.from_numpy(H).cuda(), torch.from_numpy(S).cuda()
+    w = torch.empty(n, dtype=torch.float64, device="cuda")
+    c = torch.empty((n, n), dtype=torch.float64, device="cuda")
+    st = capi.load_library().tb_sygvd_noalloc(C.c_int32(n), *[C.c_void_p(x.data_ptr()) for x in (h, s, w, c)],
+                                              C.c_void_p(0))
+    assert st == 0, capi.last_error()
+    W, V = w.cpu().numpy(), c.cpu().numpy()
+    li = np.linalg.inv(np.linalg.cholesky(S))
+    scale = max(1.0, np.abs(H).sum(axis=1).max())
+    tol = 8 * n * np.finfo(float).eps  # backward stable: a few n eps of the norm
+    np.testing.assert_allclose(W, np.linalg.eigvalsh(li @ H @ li.T), atol=tol * scale, rtol=0)
+    np.testing.assert_allclose(V.T @ S @ V, np.eye(n), atol=tol, rtol=0)
+    np.testing.assert_allclose(H @ V, S @ V * W, atol=tol * scale, rtol=0)
+
+
+def test_cluster_and_one_cta_give_the_same_bits(gpu_calc):
+    rng = np.random.default_rng(17)
+    mols = [g.water_cluster(k, rng) for k in (11, 16, 22, 37, 38, 64)]
+    mols += [g.alkane(k, rng) for k in (11, 37, 74, 75, 110)]  # 68, 224, 446, 452, 662 AOs
+    fill = g.water_clusters(700, seed=9, nmin=11, nmax=14)     # several waves: one CTA each
+    batch = gpu_calc.singlepoint_batch(mols + fill, solver=1)
+    few = gpu_calc.singlepoint_batch(mols, solver=1)
+    for i, m in enumerate(mols):
+        alone = gpu_calc.singlepoint_batch([m], solver=1)[0]
+        for r in (batch[i], few[i]):
+            assert alone["status"] == r["status"] == 0
+            assert alone["energy"] == r["energy"] and alone["iterations"] == r["iterations"]
+            np.testing.assert_array_equal(alone["qat"], r["qat"])
