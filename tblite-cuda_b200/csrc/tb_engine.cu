@@ -1201,7 +1201,7 @@ tb_status raise_smem_limits() {
   int dev = 0, optin = 0;
   TB_CUDA(cudaGetDevice(&dev));
   TB_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-  const void* ks[] = {(const void*)k_syev, (const void*)k_syev_wide, (const void*)k_syev_ql, (const void*)k_syev_f32, (const void*)k_fermi, (const void*)k_oa_step,
+  const void* ks[] = {(const void*)k_syev, (const void*)k_syev_wide, (const void*)k_syev_small, (const void*)k_syev_f32, (const void*)k_fermi, (const void*)k_oa_step,
                       (const void*)k_gemm_tc, (const void*)k_fock, (const void*)k_syev_jacobi};
   for (const void* k : ks) {
     cudaFuncAttributes a;
@@ -1396,9 +1396,9 @@ tb_status calibrate_small(tb_calculator* c) {
         cudaMemset(base + os, 0, cnt * 4);
         cudaEventRecord(e0);
         if (variant == 0)
-          k_syev_ql<<<cnt, kEigThreads, syev_smem_bytes(n)>>>(Bk, at<double>(base, oA), at<double>(base, oZ),
-                                                              at<double>(base, ow), at<int>(base, op),
-                                                              at<int>(base, os), nullptr);
+          k_syev_small<<<cnt, kEigThreads, small_smem_bytes(n)>>>(Bk, at<double>(base, oA), at<double>(base, oZ),
+                                                                  at<double>(base, ow), at<int>(base, op),
+                                                                  at<int>(base, os), nullptr, 0);
         else
           k_syev_jacobi<<<nblk(cnt, kJacobiWarps), kJacobiWarps * 32, jacobi_smem_bytes()>>>(
               Bk, at<double>(base, oA), at<double>(base, oZ), at<double>(base, ow), at<int>(base, op),

@@ -163,7 +163,7 @@ constexpr int kSyevMaxCluster = 8;
 constexpr size_t kSyevSmemTwo = 110 * 1024;  // dynamic shared memory up to which two CTAs fit an SM
 struct SyevPlan {
   int n64 = 0;          // structures of kDcMin+ AOs on the in-house solver lead the order
-  int nsmall = 0;       // structures below kDcMin AOs that k_syev_ql solves
+  int nsmall = 0, small_max = 1;  // structures below kDcMin AOs that k_syev_small solves, the largest
   int cluster = 1, ncoop = 0;
   bool wide = true;     // k_syev_wide (one CTA per SM)
   double span = 0.0;    // modelled time of one launch, ms
@@ -171,13 +171,23 @@ struct SyevPlan {
   // sizes in the batch's order (decreasing; those of the library path first)
   void build(const std::vector<int>& sizes, int lib_above, int jacobi_max);
 };
-// k_syev (and k_syev_ql where the plan has small structures) on st; *launches
+// k_syev (and k_syev_small where the plan has small structures) on st; *launches
 // counts them.  The shared-memory limits must have been raised.
 cudaError_t launch_syev(const SyevPlan& P, const DevBatch& B, double* A, double* Z, double* Sb, double* w, int* perm,
                         int* status, const int* active, cudaStream_t st, int64_t* launches);
-// one CTA per structure, FP64, below kDcMin AOs: implicit QL
-__global__ void k_syev_ql(DevBatch B, double* Ab, double* Zb, double* wout, int* perm, int* status,
-                          const int* active);
+// FP64 structures below kDcMin AOs, one CTA each in shared memory: B.order
+// from position `first` on; dynamic shared memory small_smem_bytes(largest)
+constexpr int kSmallLeaf = 13;  // leaves of its merge tree
+__host__ __device__ constexpr int small_ld(int n) {  // row stride: even, and no multiple of 16 (bank conflicts)
+  return (n + 1) / 2 * 2 + (((n + 1) / 2 * 2) % 16 == 0 ? 2 : 0);
+}
+__host__ __device__ constexpr int small_ws_elems(int n) {  // merge workspace; the reduction's vectors before it
+  const int red = (3 * (kEigThreads / 32) + 4) * 64, dc = dc_ws_elems<double>(n);
+  return ((dc > red ? dc : red) + 1) / 2 * 2;
+}
+inline size_t small_smem_bytes(int n) { return (3 * (size_t)n * small_ld(n) + 3 * n + small_ws_elems(n)) * sizeof(double); }
+__global__ void k_syev_small(DevBatch B, const double* Ab, double* Zb, double* wout, int* perm, int* status,
+                             const int* active, int first);
 // the same eigensolver in FP32 (A and Z float, eigenvalues written as double)
 __global__ void k_syev_f32(DevBatch B, float* Ab, float* Zb, double* wout, int* perm, int* status, const int* active);
 // small-structure variant: one warp per structure of N <= kJacobiMaxN (cyclic Jacobi

@@ -1,11 +1,10 @@
 // Batched FP64 dense linear algebra for uneven structure sizes:
 //  * k_cholesky / k_trinv: S = L L^T and X = L^-T (once per structure);
 //  * k_gemm: C = alpha op(A) diag(ks) op(B) + beta C over a tile list;
-//  * k_syev_ql, k_syev_f32: symmetric eigenproblem, one CTA per structure
+//  * k_syev_f32: the mixed form's FP32 eigensolver, one CTA per structure
 //    (Householder tridiagonalisation, explicit Q, implicit QL with the
 //    rotations of each sweep applied to the eigenvector rows by all threads,
-//    rank-based sort): FP64 below kDcMin AOs (k_syev in tb_syev.cu above) and
-//    the mixed form's FP32 solver.
+//    rank-based sort); FP64: tb_syev.cu, and k_syev_jacobi here.
 // Together these give sygvd (itype 1, jobz 'V'; reference src/lapack/sygvd.h:4-23):
 // H C = S C e  <=>  (X^T H X) Z = Z e, C = X Z.
 #include "tb_common.cuh"
@@ -363,16 +362,16 @@ __global__ void __launch_bounds__(kGemmThreads) k_gemm32(DevBatch B, const int4*
 }
 
 // ------------------------------------------------------------ eigensolver
-// Symmetric eigenproblem of A (n x n, row-major, overwritten) for every
-// active structure, one CTA of 256 threads per structure: w ascending,
+// FP32 symmetric eigenproblem (mixed form; FP64: tb_syev.cu) of A (n x n,
+// row-major, overwritten) for every active structure, one CTA of 256 threads per structure: w ascending,
 // eigenvector j = row perm[j] of Zc (n x n, one eigenvector per row).
 //
 //  1. Householder tridiagonalisation in panels (tridiagonalise): within a
 //     panel the trailing block keeps its value from the panel start, each
 //     step forms its product with one read-only walk (colwalk, row segments)
 //     and corrects it with the panel's pairs; the panel-closing walk
-//     (panel_walk_tc, panel_walk) applies the rank-2 width update fused with
-//     the next product.  Reflector k is kept in row k of A.
+//     (panel_walk) applies the rank-2 width update fused with the next
+//     product.  Reflector k is kept in row k of A.
 //  2. Zc = Q^T accumulated backwards in compact-WY blocks of kQBlock
 //     reflectors (form_q).
 //  3. Tridiagonal eigenproblem: implicit QL with Wilkinson shift (warp 0 runs
@@ -382,13 +381,10 @@ __global__ void __launch_bounds__(kGemmThreads) k_gemm32(DevBatch B, const int4*
 //  4. Ascending order by rank (ties by index).
 namespace {
 
-// Tridiagonalisation panel: reflectors per panel (2 panel n <= ring) and, for
-// the FP32 column form of the panel-closing walk, rows per load batch.  FP64
-// moves twice the bytes per element, so its walks are traffic-bound and wide
-// panels pay (its panel-closing walk is panel_walk_tc); in
-// FP32 a panel of one (each step's update fused with the next product) is as fast.
+// Tridiagonalisation panel: reflectors per panel (2 panel n <= ring) and rows
+// per load batch of the panel-closing walk; a panel of one (each step's update
+// fused with the next product) is as fast as a wider one in FP32.
 template <typename T> struct PanelCfg;
-template <> struct PanelCfg<double> { static constexpr int width = 8; };
 template <> struct PanelCfg<float> { static constexpr int width = 1, batch = 12; };
 // Read-only Householder walk (colwalk): the warps form kWalkRowGroups row
 // groups (interleaved rows) times nw / kWalkRowGroups column groups; a lane
@@ -397,18 +393,15 @@ template <> struct PanelCfg<float> { static constexpr int width = 1, batch = 12;
 // for DRAM) with cols * rows loads in flight per lane.
 constexpr int kWalkRowGroups = 4;
 template <typename T> struct WalkCfg { static constexpr int cols = 3, rows = 4; };
-static_assert(PanelCfg<double>::width <= kRing && PanelCfg<float>::width <= kRing, "panel exceeds the ring");
+static_assert(PanelCfg<float>::width <= kRing, "panel exceeds the ring");
 constexpr int kQBlock = 16;     // reflectors per compact-WY block of the Q accumulation
 constexpr int kWaveK = 4;            // QL sweeps applied per pass over Zc
 constexpr int kWin = 2 * kWaveK;     // rows of Zc in flight per column
 constexpr long long kSpinLimit = 1LL << 24;
 
 template <typename T> struct Eps;
-template <> struct Eps<double> { static constexpr double v = 2.220446049250313e-16; };
 template <> struct Eps<float> { static constexpr float v = 1.1920929e-07f; };
-__device__ inline double tb_sqrt(double x) { return sqrt(x); }
 __device__ inline float tb_sqrt(float x) { return sqrtf(x); }
-__device__ inline double tb_abs(double x) { return fabs(x); }
 __device__ inline float tb_abs(float x) { return fabsf(x); }
 // one Newton step y(3 - x y^2)/2 on the hardware estimate keeps Givens pairs orthogonal to ~1 ulp
 __device__ inline float tb_rsqrt(float x) {
@@ -416,9 +409,7 @@ __device__ inline float tb_rsqrt(float x) {
   return y * (1.5f - 0.5f * x * y * y);
 }
 
-// reciprocal square root on the QL rotation chain (FP32: one Newton step on the estimate)
-__device__ inline double chain_rsqrt(double x) { return rsqrt(x); }
-
+// reciprocal square root on the QL rotation chain (one Newton step on the estimate)
 __device__ inline float chain_rsqrt(float x) { return tb_rsqrt(x); }
 
 template <typename T>
@@ -567,88 +558,6 @@ __device__ __noinline__ void panel_walk(T* M, int n, int r0, int nm, const T* PV
   }
 }
 
-// FP64 panel-closing walk on the tensor instruction (mma.sync m8n8k4), same
-// result as panel_walk up to rounding: with the panel's 8 pairs as
-// K = [PV; PW] (16 x n) and L = [PW; PV], the block is updated as
-// M -= K^T L over 16 x 32 tiles per warp (accumulators initialised from M,
-// stored back), and out_c = scale * sum_r M_new[r][c] x_{r-r0} is formed from
-// the same fragments.  Warps as in colwalk: kWalkRowGroups groups of
-// interleaved 16-row tiles times nw / kWalkRowGroups column groups; the row
-// groups' partial sums go through out, p1, p2, p3 (nm entries each).
-__device__ __noinline__ void panel_walk_tc(double* M, int n, int r0, int nm, const double* PV, const double* PW,
-                                           const double* x, double* out, double scale, double* p1, double* p2,
-                                           double* p3) {
-  static_assert(PanelCfg<double>::width == 8, "two panel halves of four k-steps");
-  constexpr int kG = kWalkRowGroups;
-  const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
-  const int ncg = (nt >> 5) / kG, rg = warp % kG, cg = warp / kG;
-  double* mine = rg == 0 ? out : (rg == 1 ? p1 : (rg == 2 ? p2 : p3));
-  double* Mb = M + (long long)r0 * n + r0;
-  for (int c0 = 0; c0 < nm; c0 += 32 * ncg) {
-    const int cw = c0 + 32 * cg;  // this warp's first column (relative)
-    for (int rt = 16 * rg; rt < nm; rt += 16 * kG) {
-      double d[2][4][2];
-#pragma unroll
-      for (int xx = 0; xx < 2; ++xx)
-#pragma unroll
-        for (int y = 0; y < 4; ++y)
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const int r = rt + 8 * xx + g, c = cw + 8 * y + 2 * t + h;
-            d[xx][y][h] = (r < nm && c < nm) ? Mb[(long long)r * n + c] : 0.0;
-          }
-#pragma unroll
-      for (int ks = 0; ks < 4; ++ks) {
-        const int k = 4 * (ks & 1) + t;                                 // pair index
-        const double* Kr = (ks < 2 ? PV : PW) + (long long)k * n + r0;  // row side
-        const double* Lc = (ks < 2 ? PW : PV) + (long long)k * n + r0;  // column side
-        double a[2], b[4];
-#pragma unroll
-        for (int xx = 0; xx < 2; ++xx) {
-          const int r = rt + 8 * xx + g;
-          a[xx] = r < nm ? -Kr[r] : 0.0;
-        }
-#pragma unroll
-        for (int y = 0; y < 4; ++y) {
-          const int c = cw + 8 * y + g;
-          b[y] = c < nm ? Lc[c] : 0.0;
-        }
-#pragma unroll
-        for (int xx = 0; xx < 2; ++xx)
-#pragma unroll
-          for (int y = 0; y < 4; ++y) dmma(d[xx][y][0], d[xx][y][1], a[xx], b[y]);
-      }
-      const double x0 = rt + g < nm ? x[rt + g] : 0.0, x1 = rt + 8 + g < nm ? x[rt + 8 + g] : 0.0;
-#pragma unroll
-      for (int xx = 0; xx < 2; ++xx)
-#pragma unroll
-        for (int y = 0; y < 4; ++y)
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const int r = rt + 8 * xx + g, c = cw + 8 * y + 2 * t + h;
-            if (r < nm && c < nm) Mb[(long long)r * n + c] = d[xx][y][h];
-          }
-      // this tile's column sums over its 16 rows (the eight row lanes g are
-      // lanes t, t + 4, ..., t + 28), added to the warp's own entries of `mine`
-#pragma unroll
-      for (int y = 0; y < 4; ++y)
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          double v = d[0][y][h] * x0 + d[1][y][h] * x1;
-          v += __shfl_xor_sync(0xffffffffu, v, 4);
-          v += __shfl_xor_sync(0xffffffffu, v, 8);
-          v += __shfl_xor_sync(0xffffffffu, v, 16);
-          const int c = cw + 8 * y + 2 * t + h;
-          if (g == 0 && c < nm) mine[c] = rt == 16 * rg ? v : mine[c] + v;
-        }
-    }
-    if (16 * rg >= nm)  // a row group without rows still owns its partial entries
-      for (int c = cw + lane; c < cw + 32 && c < nm; c += 32) mine[c] = 0.0;
-  }
-  __syncthreads();
-  for (int c = tid; c < nm; c += nt) out[c] = scale * (((out[c] + p1[c]) + p2[c]) + p3[c]);
-}
-
 // Phase 1 of syev_body: A (n x n, symmetric, row-major) is reduced to
 // tridiagonal form in place; reflector k is stored in row k of A from column
 // k+1 on (leading 1), its scale in tau[k], the off-diagonal in e.  Out of line
@@ -767,10 +676,7 @@ __device__ __noinline__ void tridiagonalise(T* A, int n, T* e, T* tau, T* v, T* 
           __syncthreads();
         }
         if (np == kPanel) {  // close the panel: A -= V W^T + W V^T on the block, fused with p_r = tau_r A vn
-          if constexpr (sizeof(T) == 8) {
-            panel_walk_tc(A, n, r + 1, n - r - 1, PV, PW, vn, p, tau[r], w, d, v);  // v is in PV already
-          } else
-            panel_walk<T>(A, n, r + 1, n - r - 1, PV, PW, vn, p, tau[r], w);
+          panel_walk<T>(A, n, r + 1, n - r - 1, PV, PW, vn, p, tau[r], w);
           np = 0;
         } else {  // p_r = tau_r A0 vn
           colwalk<T>(A, n, r + 1, n - r - 1, vn, p, tau[r], w, d, v);  // v is in PV already
@@ -887,8 +793,6 @@ __device__ __forceinline__ void syev_body(const DevBatch& B, T* __restrict__ Ab,
   if (status[m] != kStOk) return;
   const int n = B.ooff[m + 1] - B.ooff[m];
   if (on_library(B, n)) return;
-  // FP64: the one-warp Jacobi variant (k_syev_jacobi) below, k_syev (tb_syev.cu) above
-  if (sizeof(T) == 8 && (n <= B.jacobi_max || n >= kDcMin)) return;
   const long long mo = B.moff[m];
   const long long vo = B.ooff[m];
   T* A = Ab + mo;
@@ -1256,13 +1160,6 @@ __global__ void __launch_bounds__(kJacobiWarps * 32) k_syev_jacobi(DevBatch B, d
     perm[vo + rank] = lane;
     wout[vo + rank] = di;
   }
-}
-
-__global__ void __launch_bounds__(kEigThreads, 3) k_syev_ql(DevBatch B, double* __restrict__ Ab,
-                                                            double* __restrict__ Zb, double* __restrict__ wout,
-                                                            int* __restrict__ perm, int* __restrict__ status,
-                                                            const int* __restrict__ active) {
-  syev_body<double>(B, Ab, Zb, wout, perm, status, active);
 }
 
 __global__ void __launch_bounds__(kEigThreads, 4) k_syev_f32(DevBatch B, float* __restrict__ Ab,

@@ -28,6 +28,7 @@
 
 #include <mutex>
 #include <string>
+#include <utility>
 
 #include "../../include/tblite_b200.h"
 #include "tb_common.cuh"
@@ -121,12 +122,14 @@ extern "C" tb_status tb_sygvd_noalloc(int32_t n, const double* H, const double* 
       // memory opt-in for the largest accepted n (raised only: the batched
       // paths may already have set a higher limit), then the scratch address
       // (cached last, so that a failed set-up is retried by the next call)
-      const int need = (int)syev_smem_bytes(kNoAllocMaxN);
-      for (const void* k : {(const void*)k_syev, (const void*)k_syev_wide, (const void*)k_syev_ql}) {
+      const std::pair<const void*, size_t> need[] = {{(const void*)k_syev, syev_smem_bytes(kNoAllocMaxN)},
+                                                     {(const void*)k_syev_wide, syev_smem_bytes(kNoAllocMaxN)},
+                                                     {(const void*)k_syev_small, small_smem_bytes(kDcMin - 1)}};
+      for (const auto& k : need) {
         cudaFuncAttributes fa;
-        e = cudaFuncGetAttributes(&fa, k);
-        if (e == cudaSuccess && fa.maxDynamicSharedSizeBytes < need)
-          e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, need);
+        e = cudaFuncGetAttributes(&fa, k.first);
+        if (e == cudaSuccess && fa.maxDynamicSharedSizeBytes < (int)k.second)
+          e = cudaFuncSetAttribute(k.first, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k.second);
         if (e != cudaSuccess) return noalloc_fail(TB_CUDA_ERROR, cudaGetErrorString(e));
       }
       double* addr = nullptr;

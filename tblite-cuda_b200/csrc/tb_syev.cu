@@ -27,6 +27,8 @@
 #include <algorithm>
 #include <functional>
 
+#include <cooperative_groups.h>
+
 #include "tb_common.cuh"
 #include "tb_kernels.h"
 
@@ -46,12 +48,17 @@ struct Group {
   int rank, size;  // this CTA's rank in the structure's cluster; size 1: a CTA of its own
 };
 
+// Barrier over the group's CTAs; what they wrote before it (global and peers'
+// shared memory) is visible after it.  The warp is brought together first: the
+// cluster barrier by itself lets the lanes of a warp that has diverged (the
+// four-lane teams leave their loops one by one) arrive and go on separately,
+// and a warp-wide instruction after it (mma.sync, a block barrier) is then
+// executed by part of a warp, which is an illegal instruction.
 __device__ __forceinline__ void group_sync(const Group& g) {
-  if (g.size == 1) {
-    __syncthreads();
-  } else {
-    asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;\n" ::: "memory");
-  }
+  __syncwarp();
+  if (g.size == 1) __syncthreads();
+  else cooperative_groups::this_cluster().sync();
+  __syncwarp();
 }
 
 // *p = v in the shared memory of CTA r of the group (the same variable there)
@@ -161,6 +168,7 @@ __device__ __noinline__ void walk_read(const double* Mb, int n, int nm, const do
   double* col = part;
   double* row = part + (long long)un.nI * nm;
   for (int u = gw;; u += ngw) {
+    __syncwarp();
     const int I = un.seek(u);
     if (I < 0) return;
     const int c0 = un.J << CS, rbeg = I << RS;
@@ -252,6 +260,7 @@ __device__ __noinline__ void walk_close(double* Mb, int n, int r0, int nm, const
   double* col = part;
   double* row = part + (long long)un.nI * nm;
   for (int u = gw;; u += ngw) {
+    __syncwarp();
     const int I = un.seek(u);
     if (I < 0) return;
     const int J = un.J, c0 = J << CS, rbeg = I << RS;
@@ -523,6 +532,7 @@ __device__ __forceinline__ void formq_rows(double* Z, int n, int row0, int c0, i
   double a0[2] = {0.0, 0.0}, a1[2] = {0.0, 0.0};  // Wm[g][8y + 2t], Wm[g][8y + 2t + 1]
   const double* Vg = Vs + g * mp + t;
   for (int k0 = 0; k0 < m; k0 += 4 * U) {
+    __syncwarp();
     double z[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
@@ -560,6 +570,7 @@ __device__ __forceinline__ void formq_rows(double* Z, int n, int row0, int c0, i
   const double* Vt = Vs + t * mp + g;
   constexpr int V = U / 2;  // 8-column fragments per round
   for (int ct = 0; ct < m; ct += 8 * V) {
+    __syncwarp();
     double d0[V], d1[V];
 #pragma unroll
     for (int y = 0; y < V; ++y) {
@@ -840,7 +851,7 @@ __device__ void dc_gemm(int nrow, int kdim, int ncol, Gen gen, const double* In,
 // same rows of Out and the merged eigenvalues written to d[lo, hi) of every
 // CTA.  V is overwritten.  ws: dc_ws_elems(hi - lo) doubles.
 template <bool W>
-__device__ __noinline__ void dc_merge(double* d, const double* e, int n, int lo, int t, int hi, double* Gi, double* V,
+__device__ __noinline__ void dc_merge(double* d, const double* e, int n, int ld, int lo, int t, int hi, double* Gi, double* V,
                                       int vc0, int vcols, double* Out, double* ws, const Group g) {
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const int gw = g.rank * kWarps + wid, ngw = g.size * kWarps;
@@ -869,11 +880,11 @@ __device__ __noinline__ void dc_merge(double* d, const double* e, int n, int lo,
   // children's blocks are diagonal sub-blocks: clear the rest of the node's block
   if (V == Gi)
     for (int r = lo + gw; r < hi; r += ngw)
-      for (int c = (r < t ? t : lo) + lane; c < (r < t ? hi : t); c += 32) Gi[(long long)r * n + c] = 0.0;
+      for (int c = (r < t ? t : lo) + lane; c < (r < t ? hi : t); c += 32) Gi[(long long)r * ld + c] = 0.0;
   // z and its norm (in rc until the rotations are formed)
   double part = 0.0;
   for (int r = lo + tid; r < hi; r += kEigThreads) {
-    const double z = r < t ? Gi[(long long)r * n + t - 1] : sg * Gi[(long long)r * n + t];
+    const double z = r < t ? Gi[(long long)r * ld + t - 1] : sg * Gi[(long long)r * ld + t];
     rc[r - lo] = z;
     rowof[r - lo] = r;  // valid rows even where non-finite eigenvalues leave ranks unset below
     delta[r - lo] = zs[r - lo] = 0.0;
@@ -956,8 +967,8 @@ __device__ __noinline__ void dc_merge(double* d, const double* e, int n, int lo,
   if (nrot > 0 && g.size > 1) group_sync(g);
   for (int c = vc0 + g.rank * kEigThreads + tid; c < vc0 + vcols; c += g.size * kEigThreads)
     for (int q = 0; q < nrot; ++q) {
-      double* pa = V + (long long)rp[q] * n + c;
-      double* pb = V + (long long)rq[q] * n + c;
+      double* pa = V + (long long)rp[q] * ld + c;
+      double* pb = V + (long long)rq[q] * ld + c;
       const double a = *pa, b = *pb;
       *pa = rc[q] * a + rsn[q] * b;
       *pb = rc[q] * b - rsn[q] * a;
@@ -974,7 +985,7 @@ __device__ __noinline__ void dc_merge(double* d, const double* e, int n, int lo,
       put_at(tv + j, tj, g, r);
     }
   }
-  group_sync(g);
+  group_sync(g);  // (brings the teams of a warp together again)
   // z of the k poles, recomputed from the roots (Gu and Eisenstat: every ratio
   // in (0, 1]); the new entry keeps the old one's sign, so a lane of the team
   // that reads it late reads the same sign
@@ -996,8 +1007,8 @@ __device__ __noinline__ void dc_merge(double* d, const double* e, int n, int lo,
   // (columns hi.. or ..lo) belong to no node of this level
   double* Wb = nullptr;
   if (V != Gi) Wb = Gi;
-  else if (hi + k <= n) Wb = Gi + (long long)lo * n + hi;
-  else if (lo >= k) Wb = Gi + (long long)lo * n + (lo - k);
+  else if (hi + k <= n) Wb = Gi + (long long)lo * ld + hi;
+  else if (lo >= k) Wb = Gi + (long long)lo * ld + (lo - k);
   // norms: of this CTA's rows of W (rows gw, gw + ngw, ...), of all rows where
   // every tile generates its own
   const int r0w = g.rank * kWarps;
@@ -1014,20 +1025,21 @@ __device__ __noinline__ void dc_merge(double* d, const double* e, int n, int lo,
     s = team_sum(s, mask);
     if (sub == 0) inrm[j] = 1.0 / sqrt(s);
   }
+  __syncwarp();
   __syncthreads();
   // roots: Out rows lo .. lo+k-1; deflated: rows lo+k .. hi-1 copied
   auto wgen = [&](int j, int i) { return zl[i] * dc_rcp((dl[i] - dl[ori[j]]) - tv[j]) * inrm[j]; };
   if (Wb) {
     for (int j = gw; j < k; j += ngw)
-      for (int i = lane; i < k; i += 32) Wb[(long long)j * n + i] = wgen(j, i);
+      for (int i = lane; i < k; i += 32) Wb[(long long)j * ld + i] = wgen(j, i);
     group_sync(g);
-    dc_gemm(k, k, vcols, [&](int j, int i) { return Wb[(long long)j * n + i]; }, V, srow, Out, lo, vc0, n, Wt, Bt, g);
+    dc_gemm(k, k, vcols, [&](int j, int i) { return Wb[(long long)j * ld + i]; }, V, srow, Out, lo, vc0, ld, Wt, Bt, g);
   } else {
-    dc_gemm(k, k, vcols, wgen, V, srow, Out, lo, vc0, n, Wt, Bt, g);
+    dc_gemm(k, k, vcols, wgen, V, srow, Out, lo, vc0, ld, Wt, Bt, g);
   }
   for (int q = gw; q < m - k; q += ngw) {
-    const double* src = V + (long long)rowof[ndl[k + q]] * n;
-    double* dst = Out + (long long)(lo + k + q) * n;
+    const double* src = V + (long long)rowof[ndl[k + q]] * ld;
+    double* dst = Out + (long long)(lo + k + q) * ld;
     for (int c = vc0 + lane; c < vc0 + vcols; c += 32) dst[c] = src[c];
   }
   __syncthreads();
@@ -1037,17 +1049,17 @@ __device__ __noinline__ void dc_merge(double* d, const double* e, int n, int lo,
 
 constexpr int kDcLeaf = 24;  // leaves of the merge tree: at most this many rows, solved by one warp
 
-// Leaf [lo, lo+s) of the tree (s <= kDcLeaf) by one warp: implicit QL with
+// Leaf [lo, lo+s) of the tree (s <= 32) by one warp: implicit QL with
 // Wilkinson shifts (the same sweep as the k_syev producer) on lane 0 over
 // d[lo..] and a private copy of the leaf's off-diagonal, each sweep's
 // rotations then applied by lanes (one per column) to the rows of the leaf's
 // eigenvector block U in shared memory; U is written to G's diagonal block.
 // Returns false if an eigenvalue took more than 60 sweeps.
-constexpr int kDcLeafWs = kDcLeaf * kDcLeaf + 3 * kDcLeaf;  // per leaf warp: U, off-diagonal, rotations
-static_assert(kDcLeafWs <= dc_ws_elems<double>(kDcMin), "leaf workspace exceeds the divide-and-conquer workspace");
+__host__ __device__ constexpr int dc_leaf_ws(int leaf) { return leaf * leaf + 3 * leaf; }  // U, off-diagonal, rotations
+static_assert(dc_leaf_ws(kDcLeaf) <= dc_ws_elems<double>(kDcMin), "leaf workspace exceeds the divide-and-conquer workspace");
 
 __device__ bool dc_leaf(double* d, const double* e, int lo, int s, double* U, double* le, double* rcs, double* G,
-                        int n) {
+                        int ld) {
   const int lane = threadIdx.x & 31;
   for (int x = lane; x < s * s; x += 32) U[x] = (x / s == x % s) ? 1.0 : 0.0;
   for (int i = lane; i < s; i += 32) le[i] = i < s - 1 ? e[lo + i] : 0.0;
@@ -1063,6 +1075,7 @@ __device__ bool dc_leaf(double* d, const double* e, int lo, int s, double* U, do
       if (mq == l) break;
       if (++iter > 60) { ok = false; break; }
       int cnt = 0;
+      __syncwarp();  // every lane has scanned d and the off-diagonal that lane 0 rewrites
       if (lane == 0) {
         double g = (dd[l + 1] - dd[l]) / (2.0 * le[l]);
         double r = sqrt(g * g + 1.0);
@@ -1103,7 +1116,7 @@ __device__ bool dc_leaf(double* d, const double* e, int lo, int s, double* U, do
       __syncwarp();
     }
   }
-  for (int x = lane; x < s * s; x += 32) G[(long long)(lo + x / s) * n + lo + x % s] = U[x];
+  for (int x = lane; x < s * s; x += 32) G[(long long)(lo + x / s) * ld + lo + x % s] = U[x];
   __syncwarp();
   return ok;
 }
@@ -1120,25 +1133,25 @@ __device__ inline void dc_node(int n, int dep, int b, int* lo_out, int* hi_out, 
 }
 
 // Eigenvalues (d, in every CTA) and eigenvector rows (Zc <- G Zc) of the
-// tridiagonal (d, e) by the merge tree; G0 and G1 are n x n buffers, ws
-// dc_ws_elems(n).  A level with at least as many nodes as CTAs gives each CTA
+// tridiagonal (d, e) by the merge tree with leaves of at most `leaf` rows
+// (n > leaf); G0, G1 and Z are n x n with row stride ld, ws dc_ws_elems(n).  A level with at least as many nodes as CTAs gives each CTA
 // whole merges (no barriers between CTAs inside them), the levels above share
 // every merge.  Returns false if a leaf failed to converge.
 template <bool W>
-__device__ bool dc_solve(double* d, double* e, double* Z, double* G0, double* G1, int n, double* ws, long long ws_cap,
-                         const Group g) {
+__device__ bool dc_solve(double* d, double* e, double* Z, double* G0, double* G1, int n, int ld, int leaf, double* ws,
+                         long long ws_cap, const Group g) {
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const Group alone{0, 1};
   __shared__ int s_fail;
-  int depth = 0;  // nodes at this depth have at most kDcLeaf rows
-  while (((n + (1 << depth) - 1) >> depth) > kDcLeaf) ++depth;
+  int depth = 0;  // nodes at this depth have at most leaf rows
+  while (((n + (1 << depth) - 1) >> depth) > leaf) ++depth;
   if (tid == 0) s_fail = 0;
   // tear every internal node (rho = |e[t-1]| off both neighbours)
   for (int dep = 0; dep < depth; ++dep) {
     for (int b = tid; b < (1 << dep); b += kEigThreads) {
       int lo, hi, pl;
       dc_node(n, dep, b, &lo, &hi, &pl);
-      if (hi - lo <= kDcLeaf) continue;
+      if (hi - lo <= leaf) continue;
       const int t = (lo + hi) >> 1;
       const double rho = fabs(e[t - 1]);
       d[t - 1] -= rho;  // nodes of one depth are disjoint
@@ -1148,8 +1161,8 @@ __device__ bool dc_solve(double* d, double* e, double* Z, double* G0, double* G1
   }
   group_sync(g);  // every CTA's d is torn before a peer writes a leaf's eigenvalues there
   // as many leaf warps as the free shared memory holds blocks for
-  const int lw = (int)min((long long)kWarps, ws_cap / kDcLeafWs);
-  double* U = ws + wid * kDcLeafWs;
+  const int lw = (int)min((long long)kWarps, ws_cap / dc_leaf_ws(leaf));
+  double* U = ws + wid * dc_leaf_ws(leaf);
   for (int dep = depth; dep >= 0; --dep) {
     double* Gi = ((depth - dep - 1) & 1) ? G1 : G0;
     double* Go = ((depth - dep) & 1) ? G1 : G0;
@@ -1157,8 +1170,8 @@ __device__ bool dc_solve(double* d, double* e, double* Z, double* G0, double* G1
     for (int b = g.rank + g.size * wid; wid < lw && b < (1 << dep); b += g.size * lw) {
       int lo, hi, pl;
       dc_node(n, dep, b, &lo, &hi, &pl);
-      if (hi - lo < 1 || hi - lo > kDcLeaf || pl <= kDcLeaf) continue;
-      if (!dc_leaf(d, e, lo, hi - lo, U, U + kDcLeaf * kDcLeaf, U + kDcLeaf * kDcLeaf + kDcLeaf, Go, n))
+      if (hi - lo < 1 || hi - lo > leaf || pl <= leaf) continue;
+      if (!dc_leaf(d, e, lo, hi - lo, U, U + leaf * leaf, U + leaf * leaf + leaf, Go, ld))
         for (int r = lane; r < g.size; r += 32) put_at(&s_fail, 1, g, r);
       for (int r = 0; g.size > 1 && r < g.size; ++r)
         if (r != g.rank && lane < hi - lo) put_at(d + lo + lane, d[lo + lane], g, r);
@@ -1171,8 +1184,8 @@ __device__ bool dc_solve(double* d, double* e, double* Z, double* G0, double* G1
         if (whole && b % g.size != g.rank) continue;
         int lo, hi, pl;
         dc_node(n, dep, b, &lo, &hi, &pl);
-        if (hi - lo <= kDcLeaf) continue;
-        dc_merge<W>(d, e, n, lo, (lo + hi) >> 1, hi, Gi, Gi, lo, hi - lo, Go, ws, whole ? alone : g);
+        if (hi - lo <= leaf) continue;
+        dc_merge<W>(d, e, n, ld, lo, (lo + hi) >> 1, hi, Gi, Gi, lo, hi - lo, Go, ws, whole ? alone : g);
         if (whole)
           for (int r = 0; r < g.size; ++r)
             if (r != g.rank)
@@ -1189,18 +1202,164 @@ __device__ bool dc_solve(double* d, double* e, double* Z, double* G0, double* G1
       int first = 0;  // tiles of the first product, so that the second's continue the round
       for (int h = 0; h < 2; ++h) {
         const int lc = h ? t : 0, sz = h ? n - t : t;
-        dc_gemm(sz, sz, n, [&](int j, int i) { return Gi[(long long)(lc + j) * n + lc + i]; }, Z + (long long)lc * n,
-                nullptr, Go, lc, 0, n, Wt, Bt, g, first);
+        dc_gemm(sz, sz, n, [&](int j, int i) { return Gi[(long long)(lc + j) * ld + lc + i]; }, Z + (long long)lc * ld,
+                nullptr, Go, lc, 0, ld, Wt, Bt, g, first);
         first = ((sz + 63) / 64) * ((n + 63) / 64);
       }
       group_sync(g);
-      dc_merge<W>(d, e, n, 0, t, n, Gi, Go, 0, n, Z, ws, g);
+      dc_merge<W>(d, e, n, ld, 0, t, n, Gi, Go, 0, n, Z, ws, g);
     }
   }
   return s_fail == 0;
 }
 
-// Structures of kDcMin+ AOs (those below: k_syev_ql).  The grid is ncoop groups
+// ------------------------------------------------------------ small structures
+// Structures below kDcMin AOs, one CTA each, wholly in registers and shared
+// memory: such a matrix is a few thousand entries, so a Householder step costs
+// what its chain of reductions and barriers costs.  Lane group r = tid / 4
+// holds row r, lane sub = tid % 4 of it the columns 8i + 2 sub + {0, 1} (the
+// operands shared by all rows are then read from shared memory 16 bytes at a
+// time without conflicts).  Every warp repeats the step's scalars on its own
+// copy of the vectors, so a step has one barrier (the exchange of p = A v).
+// The eigenvectors of the tridiagonal come from dc_solve with leaves of at
+// most kSmallLeaf rows (a leaf's chain of rotations grows with its square),
+// all buffers in shared memory.
+static_assert(kEigThreads / 4 >= kDcMin, "four lanes per row");
+
+__device__ __noinline__ void small_reduce(const double* A, int n, int ld, double* V, double* d, double* e, double* tau,
+                                          double* ws) {
+  // per warp: reflectors k and k-1 and w; shared: p and row k+1, two buffers each
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, r = tid >> 2, sub = tid & 3;
+  double* vS = ws + 192 * wid;  // [2][64]
+  double* wS = vS + 128;
+  double* pS = ws + 192 * kWarps;  // [2][64]
+  double* rowS = pS + 128;         // [2][64]
+  __shared__ double s_last;        // row n-1's diagonal
+  double a[16];
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    const int c = 8 * (i >> 1) + 2 * sub + (i & 1);
+    a[i] = (r < n && c < n) ? A[(long long)r * n + c] : 0.0;
+  }
+#pragma unroll
+  for (int i = 0; i < 6; ++i) vS[lane + 32 * i] = 0.0;
+  if (r == n - 1)
+#pragma unroll
+    for (int i = 0; i < 16; ++i)
+      if (8 * (i >> 1) + 2 * sub + (i & 1) == n - 1) s_last = a[i];
+  double x0 = lane < n ? A[lane] : 0.0, x1 = lane + 32 < n ? A[lane + 32] : 0.0;  // row k at columns lane, lane + 32
+  __syncthreads();
+  for (int k = 0;; ++k) {
+    if (wid == 0 && lane == (k & 31)) d[k] = k < 32 ? x0 : x1;
+    if (k == n - 1) break;
+    const int c1 = k + 1;
+    const double alpha = __shfl_sync(0xffffffffu, c1 < 32 ? x0 : x1, c1 & 31);
+    double* v = vS + 64 * (k & 1);
+    const double* vp = vS + 64 * (c1 & 1);
+    if (k == n - 2) {  // the last diagonal: the rows in registers carry every pair but the last
+      if (tid == 0) e[k] = alpha;
+      x0 = x1 = s_last - 2.0 * vp[n - 1] * wS[n - 1];
+      continue;
+    }
+    // reflector k (as in tridiag_tiles)
+    const double sigma = warp_sum((lane > c1 ? x0 * x0 : 0.0) + (lane + 32 > c1 ? x1 * x1 : 0.0));
+    double scal = 0.0, tk = 0.0, beta = alpha;
+    if (sigma != 0.0) {
+      const double s2 = alpha * alpha + sigma, ri = rsqrt(s2), rr = s2 * ri;
+      beta = alpha <= 0.0 ? rr : -rr;
+      tk = 1.0 + fabs(alpha) * ri;
+      scal = copysign(dc_rcp(fabs(alpha) + rr), -beta);
+    }
+    if (tid == 0) { e[k] = beta; tau[k] = tk; }
+    const double v0 = lane == c1 ? 1.0 : (lane > c1 ? x0 * scal : 0.0);
+    const double v1 = lane + 32 == c1 ? 1.0 : (lane + 32 > c1 ? x1 * scal : 0.0);
+    v[lane] = v0;
+    v[lane + 32] = v1;
+    __syncwarp();
+    // the previous pair applied to the rows, and p = A v
+    const double vr = vp[r], wr = wS[r];
+    double p = 0.0, q = 0.0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      if (8 * i >= n) break;
+      const int c = 8 * i + 2 * sub;
+      const double2 vv = *reinterpret_cast<const double2*>(v + c);
+      const double2 pp = *reinterpret_cast<const double2*>(vp + c);
+      const double2 ww = *reinterpret_cast<const double2*>(wS + c);
+      a[2 * i] -= vr * ww.x + wr * pp.x;
+      a[2 * i + 1] -= vr * ww.y + wr * pp.y;
+      p += a[2 * i] * vv.x;
+      q += a[2 * i + 1] * vv.y;
+    }
+    p += q;
+    p += __shfl_xor_sync(0xffffffffu, p, 1);
+    p += __shfl_xor_sync(0xffffffffu, p, 2);
+    double* pb = pS + 64 * (k & 1);
+    double* rb = rowS + 64 * (k & 1);
+    if (sub == 0) pb[r] = p;
+    if (r == c1)
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        *reinterpret_cast<double2*>(rb + 8 * i + 2 * sub) = make_double2(a[2 * i], a[2 * i + 1]);
+    if (k == n - 3 && r == n - 1)
+#pragma unroll
+      for (int i = 0; i < 16; ++i)
+        if (8 * (i >> 1) + 2 * sub + (i & 1) == n - 1) s_last = a[i];
+    __syncthreads();
+    if (wid == 0) {  // reflector k, for the eigenvectors
+      if (lane < n) V[k * ld + lane] = v0;
+      if (lane + 32 < n) V[k * ld + lane + 32] = v1;
+    }
+    const double p0 = lane > k ? tk * pb[lane] : 0.0, p1 = lane + 32 > k ? tk * pb[lane + 32] : 0.0;
+    const double kk = 0.5 * tk * warp_sum(p0 * v0 + p1 * v1);
+    const double w0 = p0 - kk * v0, w1 = p1 - kk * v1;
+    const double wn = __shfl_sync(0xffffffffu, c1 < 32 ? w0 : w1, c1 & 31);
+    x0 = rb[lane] - (w0 + wn * v0);  // v is 1 at c1
+    x1 = rb[lane + 32] - (w1 + wn * v1);
+    __syncwarp();  // every lane has read the previous w
+    wS[lane] = w0;
+    wS[lane + 32] = w1;
+    __syncwarp();
+  }
+}
+
+// Z = Q^T (as form_q) from the reflectors in V: row r in the registers of its
+// four lanes, so the rows meet nothing but their own two exchanges per reflector.
+__device__ __noinline__ void small_q(const double* V, int n, int ld, const double* tau, double* Z) {
+  const int tid = threadIdx.x, r = tid >> 2, sub = tid & 3;
+  double z[16];
+#pragma unroll
+  for (int i = 0; i < 16; ++i) z[i] = 8 * (i >> 1) + 2 * sub + (i & 1) == r ? 1.0 : 0.0;
+  for (int k = n - 3; k >= 0; --k) {
+    const double* v = V + k * ld + 2 * sub;
+    double p = 0.0, q = 0.0, u[16];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      u[2 * i] = u[2 * i + 1] = 0.0;
+      if (8 * i < n) {
+        const double2 vv = *reinterpret_cast<const double2*>(v + 8 * i);
+        u[2 * i] = 8 * i + 2 * sub < n ? vv.x : 0.0;  // past the row: whatever follows it
+        u[2 * i + 1] = 8 * i + 2 * sub + 1 < n ? vv.y : 0.0;
+      }
+      p += z[2 * i] * u[2 * i];
+      q += z[2 * i + 1] * u[2 * i + 1];
+    }
+    p += q;
+    p += __shfl_xor_sync(0xffffffffu, p, 1);
+    p += __shfl_xor_sync(0xffffffffu, p, 2);
+    p *= tau[k];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) z[i] -= p * u[i];
+  }
+  if (r < n)
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const int c = 8 * (i >> 1) + 2 * sub + (i & 1);
+      if (c < n) Z[r * ld + c] = z[i];
+    }
+}
+
+// Structures of kDcMin+ AOs (those below: k_syev_small).  The grid is ncoop groups
 // of C CTAs (C = the cluster size), each on one structure (the first ncoop of
 // B.order), then CTAs with a structure each, C to a cluster.
 template <bool W>
@@ -1259,7 +1418,7 @@ __device__ __forceinline__ void syev_structure(const DevBatch& B, double* __rest
   const long long ws_cap = (long long)(dyn_bytes / sizeof(double)) - 2LL * n;
   if (tid == 0) { q_fail = 0; e[n - 1] = 0.0; }
   __syncthreads();
-  const bool conv = dc_solve<W>(d, e, Z, A, Sc, n, tau, ws_cap, g);
+  const bool conv = dc_solve<W>(d, e, Z, A, Sc, n, n, kDcLeaf, tau, ws_cap, g);
   for (int i = tid; i < n; i += kEigThreads)
     if (!conv || !(fabs(d[i]) < 1e30)) q_fail = 1;  // a leaf did not converge, or non-finite input
   __syncthreads();
@@ -1303,6 +1462,70 @@ __global__ void __launch_bounds__(kEigThreads, 1) k_syev_wide(DevBatch B, double
   syev_structure<true>(B, Ab, Zb, Sb, wout, perm, status, active, ncoop);
 }
 
+// Structures of B.order from position `first` on, one CTA each.
+__global__ void __launch_bounds__(kEigThreads, 2) k_syev_small(DevBatch B, const double* __restrict__ Ab,
+                                                               double* __restrict__ Zb, double* __restrict__ wout,
+                                                               int* __restrict__ perm, int* __restrict__ status,
+                                                               const int* __restrict__ active, int first) {
+  const int slot = first + (int)blockIdx.x;
+  const int m = B.order ? B.order[slot] : slot;
+  if ((active && !active[m]) || status[m] != kStOk) return;
+  const int n = B.ooff[m + 1] - B.ooff[m];
+  if (on_library(B, n) || n >= kDcMin || n <= B.jacobi_max) return;
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, ld = small_ld(n);
+  extern __shared__ __align__(16) unsigned char syev_smem[];
+  double* ws = reinterpret_cast<double*>(syev_smem);  // small_ws_elems(n)
+  double* G0 = ws + small_ws_elems(n);                // n x ld: reflectors, then merge blocks
+  double* G1 = G0 + n * ld;
+  double* Z = G1 + n * ld;
+  double* d = Z + n * ld;
+  double* e = d + n;
+  double* tau = e + n;
+  __shared__ int q_fail;
+  const long long mo = B.moff[m], vo = B.ooff[m];
+  small_reduce(Ab + mo, n, ld, G0, d, e, tau, ws);
+  if (tid == 0) { e[n - 1] = 0.0; q_fail = 0; }
+  __syncthreads();
+  small_q(G0, n, ld, tau, Z);
+  __syncthreads();
+  bool conv = true;
+  if (n > kSmallLeaf) {
+    conv = dc_solve<false>(d, e, Z, G0, G1, n, ld, kSmallLeaf, ws, small_ws_elems(n), Group{0, 1});
+  } else {
+    if (wid == 0 && !dc_leaf(d, e, 0, n, ws, ws + kSmallLeaf * kSmallLeaf, ws + kSmallLeaf * (kSmallLeaf + 1), G0, ld) &&
+        lane == 0)
+      q_fail = 1;
+    __syncthreads();
+  }
+  for (int i = tid; i < n; i += kEigThreads)
+    if (!conv || !(fabs(d[i]) < 1e30)) q_fail = 1;  // a leaf did not converge, or non-finite input
+  __syncthreads();
+  if (q_fail) {
+    if (tid == 0) status[m] = kStEigenFailed;  // k_fermi retires the structure
+    return;
+  }
+  double* Zg = Zb + mo;
+  for (int r = wid; r < n; r += kWarps)
+    for (int c = lane; c < n; c += 32) {
+      double x = 0.0;
+      if (n > kSmallLeaf) x = Z[r * ld + c];
+      else
+        for (int i = 0; i < n; ++i) x += G0[r * ld + i] * Z[i * ld + c];
+      Zg[(long long)r * n + c] = x;
+    }
+  for (int i = tid; i < n; i += kEigThreads) {
+    const double di = d[i];
+    int rank = 0;
+    for (int j = 0; j < n; ++j) {
+      const double dj = d[j];
+      rank += (dj < di || (dj == di && j < i)) ? 1 : 0;
+    }
+    if (!TB_GUARD(11, rank, 0, n)) continue;
+    perm[vo + rank] = i;
+    wout[vo + rank] = di;
+  }
+}
+
 TB_OOB_EXPORT(oob_syev)
 
 namespace {
@@ -1335,7 +1558,7 @@ void SyevPlan::build(const std::vector<int>& sizes, int lib_above, int jacobi_ma
     if (lib_above != 0 && n > lib_above) { first = n64 = (int)i + 1; continue; }
     nmax = n > nmax ? n : nmax;
     if (n >= kDcMin) n64 = (int)i + 1;
-    else if (n > jacobi_max) ++nsmall;
+    else if (n > jacobi_max) { ++nsmall; small_max = std::max(small_max, n); }
   }
   if (n64 <= first) return;
   std::vector<double> busy;  // finish times of the clusters in flight (a heap)
@@ -1400,7 +1623,10 @@ cudaError_t launch_syev(const SyevPlan& P, const DevBatch& B, double* A, double*
     if (launches) ++*launches;
   }
   if (P.nsmall > 0) {
-    k_syev_ql<<<B.nmol, kEigThreads, smem, st>>>(B, A, Z, w, perm, status, active);
+    // in the order, the small structures follow n64 (with no order, anywhere)
+    const int first = B.order ? P.n64 : 0;
+    k_syev_small<<<B.nmol - first, kEigThreads, small_smem_bytes(P.small_max), st>>>(B, A, Z, w, perm, status, active,
+                                                                                    first);
     e = cudaGetLastError();
     if (launches) ++*launches;
   }

@@ -1,10 +1,11 @@
-"""GPU: k_syev on one CTA and on clusters.
+"""GPU: k_syev on one CTA and on clusters, k_syev_small below 64 AOs.
 
 The eigensolver's units of work depend on the matrix order alone, so a
 structure gives the same bits alone (a cluster of CTAs) and in a batch of
 several waves (one CTA per structure).  Orders at the edges of its tiles
 (walk shapes change at 224 and 448 rows, leaves at 24 rows, Q in 16-reflector
-blocks) are compared with numpy through the allocation-free entry point.
+blocks; the small kernel's leaves at 13, 26 and 52 rows, its padded row strides
+at multiples of 16, rows past one warp's 32 columns) are compared with numpy through the allocation-free entry point.
 """
 import ctypes as C
 
@@ -17,14 +18,14 @@ from tblite_b200 import geometry as g
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n", [64, 65, 97, 112, 129, 193, 223, 224, 225, 226, 240, 255, 256])
+@pytest.mark.parametrize("n", [1, 2, 3, 4, 13, 14, 15, 16, 26, 27, 31, 32, 33, 48, 51, 53, 62, 63, 64, 65, 97, 112, 129, 193, 223, 224, 225, 226, 240, 255, 256])
 def test_orders_at_tile_edges(n):
     import torch
     rng = np.random.default_rng(n)
     a = rng.standard_normal((n, n))
     H = 0.5 * (a + a.T)
-    if n == 129:  # threefold degenerate
-        H = np.diag(np.repeat(np.arange(43.0), 3))
+    if n in (33, 51, 129):  # threefold degenerate
+        H = np.diag(np.repeat(np.arange(n / 3.0), 3))
     b = 0.1 * rng.standard_normal((n, n))
     S = np.eye(n) + b @ b.T / n
     h, s = torch.from_numpy(H).cuda(), torch.from_numpy(S).cuda()
