@@ -177,12 +177,12 @@ cudaError_t launch_syev(const SyevPlan& P, const DevBatch& B, double* A, double*
                         int* status, const int* active, cudaStream_t st, int64_t* launches);
 // FP64 structures below kDcMin AOs, one CTA each in shared memory: B.order
 // from position `first` on; dynamic shared memory small_smem_bytes(largest)
-constexpr int kSmallLeaf = 13;  // leaves of its merge tree
+constexpr int kSmallLeaf = 16;  // leaves of its merge tree
 __host__ __device__ constexpr int small_ld(int n) {  // row stride: even, and no multiple of 16 (bank conflicts)
   return (n + 1) / 2 * 2 + (((n + 1) / 2 * 2) % 16 == 0 ? 2 : 0);
 }
 __host__ __device__ constexpr int small_ws_elems(int n) {  // merge workspace; the reduction's vectors before it
-  const int red = (3 * (kEigThreads / 32) + 4) * 64, dc = dc_ws_elems<double>(n);
+  const int red = (3 * (kEigThreads / 32) + 4) * 64, dc = dc_ws_elems<double>(n);  // red > a leaf of kSmallLeaf rows
   return ((dc > red ? dc : red) + 1) / 2 * 2;
 }
 inline size_t small_smem_bytes(int n) { return (3 * (size_t)n * small_ld(n) + 3 * n + small_ws_elems(n)) * sizeof(double); }

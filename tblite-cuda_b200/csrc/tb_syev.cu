@@ -43,6 +43,12 @@ constexpr int kWarps = kEigThreads / 32;
 static_assert(kEigThreads == 256, "the tile shapes below assume eight warps");
 static_assert(kPanel <= kRing, "panel exceeds the shared-memory ring");
 
+// The kernels' dynamic shared memory.  The out-of-line functions take offsets
+// into it, not pointers: through a generic pointer every access is a generic
+// load, several cycles slower on the chains that bound a step.
+extern __shared__ __align__(16) double syev_sm[];
+__device__ __forceinline__ int sm_off(const double* p) { return (int)(p - syev_sm); }
+
 // ------------------------------------------------------------ CTAs of one structure
 struct Group {
   int rank, size;  // this CTA's rank in the structure's cluster; size 1: a CTA of its own
@@ -159,10 +165,10 @@ struct Units {
 // is bound by its instructions when three CTAs share an SM).  U changes no
 // sum's order.
 template <int RS, int CS, int U>
-__device__ __noinline__ void walk_read(const double* Mb, int n, int nm, const double* x, double* part, int gw,
-                                       int ngw) {
+__device__ __noinline__ void walk_read(const double* Mb, int n, int nm, int xo, double* part, int gw, int ngw) {
   constexpr int Q = 1 << (CS - 5);
   static_assert(U % 8 == 0, "rows are reduced in eights");
+  const double* x = syev_sm + xo;
   const int lane = threadIdx.x & 31, g = lane >> 2;
   Units<RS, CS> un(nm);
   double* col = part;
@@ -251,8 +257,9 @@ __device__ __noinline__ void walk_read(const double* Mb, int n, int nm, const do
 // partials of M_new x are formed from the same fragments.  NB sub-tiles of a
 // 16-column block are loaded before the first is used.
 template <int RS, int CS, int NB>
-__device__ __noinline__ void walk_close(double* Mb, int n, int r0, int nm, const double* PV, const double* PW,
-                                        const double* x, double* part, int gw, int ngw) {
+__device__ __noinline__ void walk_close(double* Mb, int n, int r0, int nm, int pvo, int xo, double* part, int gw,
+                                        int ngw) {
+  const double *PV = syev_sm + pvo, *PW = PV + kPanel * n, *x = syev_sm + xo;
   constexpr int RB = 1 << (RS - 4);
   static_assert(RB % NB == 0, "sub-tiles per load round");
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
@@ -397,7 +404,7 @@ __device__ __forceinline__ double walk_gather(const double* part, int nm, int c,
 // diagonal in d, the off-diagonal in e; d, e and tau complete in every CTA.
 // gs: scratch for the walk partials (at most n^2 doubles).
 template <bool W>
-__device__ __noinline__ void tridiag_tiles(double* A, int n, double* d, double* e, double* tau, double* v, double* vn,
+__device__ __forceinline__ void tridiag_tiles(double* A, int n, double* d, double* e, double* tau, double* v, double* vn,
                                            double* p, double* w, double* ring, double* gs, const Group g) {
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const int gw = g.rank + g.size * wid, ngw = g.size * kWarps;
@@ -486,14 +493,14 @@ __device__ __noinline__ void tridiag_tiles(double* A, int n, double* d, double* 
     // products with the new reflector over rows and columns r+1 .. n-1
     double* Mb = A + (long long)(r + 1) * n + r + 1;
     if (np == kPanel) {
-      if (mr <= kWalk1) walk_close<5, 5, 2>(Mb, n, r + 1, mr, PV, PW, vn, gs, gw, ngw);
-      else if (mr <= kWalk2) walk_close<5, 6, 2>(Mb, n, r + 1, mr, PV, PW, vn, gs, gw, ngw);
-      else walk_close<6, 7, W ? 4 : 2>(Mb, n, r + 1, mr, PV, PW, vn, gs, gw, ngw);
+      if (mr <= kWalk1) walk_close<5, 5, 2>(Mb, n, r + 1, mr, sm_off(PV), sm_off(vn), gs, gw, ngw);
+      else if (mr <= kWalk2) walk_close<5, 6, 2>(Mb, n, r + 1, mr, sm_off(PV), sm_off(vn), gs, gw, ngw);
+      else walk_close<6, 7, W ? 4 : 2>(Mb, n, r + 1, mr, sm_off(PV), sm_off(vn), gs, gw, ngw);
       np = 0;
     } else {
-      if (mr <= kWalk1) walk_read<5, 5, 32>(Mb, n, mr, vn, gs, gw, ngw);
-      else if (mr <= kWalk2) walk_read<5, 6, W ? 32 : 16>(Mb, n, mr, vn, gs, gw, ngw);
-      else walk_read<6, 7, W ? 16 : 8>(Mb, n, mr, vn, gs, gw, ngw);
+      if (mr <= kWalk1) walk_read<5, 5, 32>(Mb, n, mr, sm_off(vn), gs, gw, ngw);
+      else if (mr <= kWalk2) walk_read<5, 6, W ? 32 : 16>(Mb, n, mr, sm_off(vn), gs, gw, ngw);
+      else walk_read<6, 7, W ? 16 : 8>(Mb, n, mr, sm_off(vn), gs, gw, ngw);
       // the next step's w_i . v and v_i . v, one warp each, in every CTA; the
       // last warps of the group first (the walk's units start at warp 0).  Two
       // buffers: a CTA one step behind may still read the other
@@ -606,7 +613,7 @@ __device__ __forceinline__ void formq_rows(double* Z, int n, int row0, int c0, i
 // and the CTAs never wait for one another; each forms V and T of the block
 // itself.  vbuf: 20 n elements of shared memory.
 template <bool W>
-__device__ __noinline__ void form_q(const double* A, double* Z, int n, const double* tau, double* vbuf,
+__device__ __forceinline__ void form_q(const double* A, double* Z, int n, const double* tau, double* vbuf,
                                     const Group grp) {
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, g = lane >> 2, t = lane & 3;
   const int gw = grp.rank + grp.size * wid, ngw = grp.size * kWarps;
@@ -695,9 +702,12 @@ __device__ __noinline__ void form_q(const double* A, double* Z, int n, const dou
 // passes over the k terms is four times shorter than with one thread, and a
 // group's CTAs take every size-th root.
 
+template <int T = 4>
 __device__ __forceinline__ double team_sum(double v, unsigned mask) {
-  v += __shfl_xor_sync(mask, v, 1);
-  v += __shfl_xor_sync(mask, v, 2);
+  if constexpr (T == 4) {
+    v += __shfl_xor_sync(mask, v, 1);
+    v += __shfl_xor_sync(mask, v, 2);
+  }
   return v;
 }
 __device__ __forceinline__ double team_mul(double v, unsigned mask) {
@@ -707,63 +717,84 @@ __device__ __forceinline__ double team_mul(double v, unsigned mask) {
 }
 
 // Root j of 1 + rho sum_i z_i^2 / (dl_i - lambda) = 0 (dl strictly ascending,
-// rho > 0): lambda = dl[*o] + *tau, by the four lanes of `mask` (sub 0..3).
-__device__ void secular_root(int j, int k, const double* dl, const double* z, double rho, int sub, unsigned mask,
+// rho > 0): lambda = dl[*o] + *tau, by the T (4 or 1) lanes of `mask` (sub 0..T-1).
+// The two poles p = min(j, k-2) and p+1 beside the root are treated apart: the
+// start solves the equation with the other terms frozen at the interval's
+// middle (for the last root, half way to its upper bound), each step replaces
+// the terms up to p and those beyond by one pole each with the same value and
+// slope; a step out of the bracket bisects it.
+template <int T>
+__device__ __forceinline__ void secular_root(int j, int k, const double* dl, const double* z, double rho, int sub, unsigned mask,
                              int* o_out, double* tau_out) {
-  int o;
-  double lo, hi;
-  if (j < k - 1) {
-    const double mid = 0.5 * (dl[j + 1] - dl[j]);
-    double f = 0.0;
-    for (int i = sub; i < k; i += 4) f += z[i] * z[i] * dc_rcp((dl[i] - dl[j]) - mid);
-    f = 1.0 + rho * team_sum(f, mask);
-    if (f >= 0.0) { o = j; lo = 0.0; hi = mid; }
-    else { o = j + 1; lo = -mid; hi = 0.0; }
-  } else {
-    double s = 0.0;
-    for (int i = sub; i < k; i += 4) s += z[i] * z[i];
-    o = k - 1; lo = 0.0; hi = rho * team_sum(s, mask);
+  if (k == 1) {
+    *o_out = 0;
+    *tau_out = rho * z[0] * z[0];
+    return;
   }
+  const bool last = j == k - 1;
+  const int p = last ? k - 2 : j;
+  const double del = dl[p + 1] - dl[p], zp = z[p] * z[p], zq = z[p + 1] * z[p + 1];
+  double top = 0.0;  // last root: upper bound of lambda - dl[k-1]
+  if (last) {
+    for (int i = sub; i < k; i += T) top += z[i] * z[i];
+    top = rho * team_sum<T>(top, mask);
+  }
+  const double mid = 0.5 * (last ? top : del);  // from dl[j]
+  double c = 0.0;  // the other terms at mid, plus 1 / rho
+#pragma unroll 4
+  for (int i = sub; i < k; i += T) {
+    const double q = z[i] * z[i] * dc_rcp((dl[i] - dl[j]) - mid);
+    c += i == p || i == p + 1 ? 0.0 : q;
+  }
+  c = dc_rcp(rho) + team_sum<T>(c, mask);
+  int o = j;
+  double lo = 0.0, hi = mid, tau;
+  const double rm = dc_rcp(mid);
+  if (!last && c + (zq - zp) * rm >= 0.0) {  // root in the lower half: x from dl[p], c x^2 - a x + b = 0
+    const double a = c * del + zp + zq, b = zp * del, sq = sqrt(fmax(a * a - 4.0 * b * c, 0.0));
+    tau = a > 0.0 ? 2.0 * b * dc_rcp(a + sq) : (a - sq) * dc_rcp(2.0 * c);
+  } else {  // x from dl[p + 1]: c x^2 + a x - b = 0, negative below it, positive past the last
+    const double a = c * del - zp - zq, b = zq * del, sq = sqrt(fmax(a * a + 4.0 * b * c, 0.0));
+    if (last) {
+      hi = top;
+      tau = a > 0.0 ? 2.0 * b * dc_rcp(a + sq) : (sq - a) * dc_rcp(2.0 * c);
+    } else {
+      o = j + 1;
+      lo = -mid;
+      hi = 0.0;
+      tau = a < 0.0 ? 2.0 * b * dc_rcp(a - sq) : -(a + sq) * dc_rcp(2.0 * c);
+    }
+  }
+  if (!(tau > lo && tau < hi)) tau = 0.5 * (lo + hi);
   const double base = dl[o];
-  double tau = 0.5 * (lo + hi);
   for (int it = 0; it < 100; ++it) {
     double psi = 0.0, phi = 0.0, dpsi = 0.0, dphi = 0.0;
-    int i = sub;
-    for (; i <= j; i += 4) {
+    // (one loop without branches: four terms' chains overlap)
+#pragma unroll 4
+    for (int i = sub; i < k; i += T) {
       const double r = dc_rcp((dl[i] - base) - tau);
-      const double q = z[i] * z[i] * r;
-      psi += q; dpsi += q * r;
+      const double q = z[i] * z[i] * r, dq = q * r;
+      const bool left = i <= p;
+      psi += left ? q : 0.0; dpsi += left ? dq : 0.0;
+      phi += left ? 0.0 : q; dphi += left ? 0.0 : dq;
     }
-    for (; i < k; i += 4) {
-      const double r = dc_rcp((dl[i] - base) - tau);
-      const double q = z[i] * z[i] * r;
-      phi += q; dphi += q * r;
-    }
-    psi = rho * team_sum(psi, mask); phi = rho * team_sum(phi, mask);
-    dpsi = rho * team_sum(dpsi, mask); dphi = rho * team_sum(dphi, mask);
+    psi = rho * team_sum<T>(psi, mask); phi = rho * team_sum<T>(phi, mask);
+    dpsi = rho * team_sum<T>(dpsi, mask); dphi = rho * team_sum<T>(dphi, mask);
     const double f = 1.0 + psi + phi;
     const double err = kEps * (8.0 * (fabs(psi) + fabs(phi)) + 3.0 + fabs(tau) * (dpsi + dphi));
     if (fabs(f) <= err) break;
     if (f < 0.0) lo = tau; else hi = tau;
     if (hi - lo <= 2.0 * kEps * fmax(fabs(lo), fabs(hi))) break;
-    const double a = (dl[j] - base) - tau;
-    double eta = 0.0;
-    bool ok = false;
-    if (j < k - 1) {  // psi ~ c1 + s1/(a - eta), phi ~ c2 + s2/(b - eta)
-      const double b = (dl[j + 1] - base) - tau;
-      const double s1 = dpsi * a * a, c1 = psi - dpsi * a, s2 = dphi * b * b, c2 = phi - dphi * b;
-      const double C = 1.0 + c1 + c2;
-      const double Bq = C * (a + b) + s1 + s2;
-      const double sq = sqrt(fmax(Bq * Bq - 4.0 * C * a * b * f, 0.0));
-      const double q = Bq >= 0.0 ? 0.5 * (Bq + sq) : 0.5 * (Bq - sq);
-      if (q != 0.0) { eta = a * b * f / q; ok = eta > a && eta < b; }
-      if (!ok && C != 0.0) { eta = q / C; ok = eta > a && eta < b; }
-    } else {
-      const double s1 = dpsi * a * a, C = 1.0 + psi - dpsi * a;
-      if (C > 0.0) { eta = a + s1 / C; ok = true; }
-    }
-    double tn = tau + eta;
-    if (!ok || !(tn > lo && tn < hi)) tn = 0.5 * (lo + hi);
+    // psi ~ c1 + s1 / (a - eta), phi ~ c2 + s2 / (b - eta)
+    const double a = (dl[p] - base) - tau, b = (dl[p + 1] - base) - tau;
+    const double s1 = dpsi * a * a, c1 = psi - dpsi * a, s2 = dphi * b * b, c2 = phi - dphi * b;
+    const double C = 1.0 + c1 + c2;
+    const double Bq = C * (a + b) + s1 + s2;
+    const double sq = sqrt(fmax(Bq * Bq - 4.0 * C * a * b * f, 0.0));
+    const double q = Bq >= 0.0 ? 0.5 * (Bq + sq) : 0.5 * (Bq - sq);
+    double tn = tau + a * b * f * dc_rcp(q);
+    if (!(tn > lo && tn < hi)) tn = tau + q * dc_rcp(C);
+    if (!(tn > lo && tn < hi)) tn = 0.5 * (lo + hi);
     tau = tn;
   }
   *o_out = o;
@@ -851,8 +882,10 @@ __device__ void dc_gemm(int nrow, int kdim, int ncol, Gen gen, const double* In,
 // same rows of Out and the merged eigenvalues written to d[lo, hi) of every
 // CTA.  V is overwritten.  ws: dc_ws_elems(hi - lo) doubles.
 template <bool W>
-__device__ __noinline__ void dc_merge(double* d, const double* e, int n, int ld, int lo, int t, int hi, double* Gi, double* V,
-                                      int vc0, int vcols, double* Out, double* ws, const Group g) {
+__device__ __noinline__ void dc_merge(int dofs, int eofs, int n, int ld, int lo, int t, int hi, double* Gi, double* V,
+                                      int vc0, int vcols, double* Out, int wofs, const Group g) {
+  double *d = syev_sm + dofs, *ws = syev_sm + wofs;
+  const double* e = syev_sm + eofs;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const int gw = g.rank * kWarps + wid, ngw = g.size * kWarps;
   const int m = hi - lo;
@@ -979,7 +1012,7 @@ __device__ __noinline__ void dc_merge(double* d, const double* e, int n, int ld,
   for (int j = gteam; j < k; j += nteam) {
     int o;
     double tj;
-    secular_root(j, k, dl, zl, rhop, sub, mask, &o, &tj);
+    secular_root<4>(j, k, dl, zl, rhop, sub, mask, &o, &tj);
     for (int r = sub; r < g.size; r += 4) {
       put_at(ori + j, o, g, r);
       put_at(tv + j, tj, g, r);
@@ -992,10 +1025,9 @@ __device__ __noinline__ void dc_merge(double* d, const double* e, int n, int ld,
   for (int i = gteam; i < k; i += nteam) {
     const double di = dl[i];
     double prod = 1.0;
-    int j = sub;
-    for (; j < i; j += 4) prod *= ((dl[ori[j]] - di) + tv[j]) * dc_rcp(dl[j] - di);
-    for (; j < k; j += 4)
-      if (j > i) prod *= ((dl[ori[j - 1]] - di) + tv[j - 1]) * dc_rcp(dl[j] - di);
+#pragma unroll 4
+    for (int j = sub; j < k - 1; j += 4)  // root j over pole j, from the entry's own pole on j + 1
+      prod *= ((dl[ori[j]] - di) + tv[j]) * dc_rcp(dl[j + (j >= i)] - di);
     prod = team_mul(prod, mask) * (((dl[ori[k - 1]] - di) + tv[k - 1]) / rhop);
     const double z = copysign(sqrt(fmax(prod, 0.0)), zl[i]);
     for (int r = sub; r < g.size; r += 4) put_at(zl + i, z, g, r);
@@ -1018,6 +1050,7 @@ __device__ __noinline__ void dc_merge(double* d, const double* e, int n, int ld,
     if (j >= k) continue;
     const double bj = dl[ori[j]], tj = tv[j];
     double s = 0.0;
+#pragma unroll 4
     for (int i = sub; i < k; i += 4) {
       const double w = zl[i] * dc_rcp((dl[i] - bj) - tj);
       s += w * w;
@@ -1049,76 +1082,247 @@ __device__ __noinline__ void dc_merge(double* d, const double* e, int n, int ld,
 
 constexpr int kDcLeaf = 24;  // leaves of the merge tree: at most this many rows, solved by one warp
 
-// Leaf [lo, lo+s) of the tree (s <= 32) by one warp: implicit QL with
-// Wilkinson shifts (the same sweep as the k_syev producer) on lane 0 over
-// d[lo..] and a private copy of the leaf's off-diagonal, each sweep's
-// rotations then applied by lanes (one per column) to the rows of the leaf's
-// eigenvector block U in shared memory; U is written to G's diagonal block.
-// Returns false if an eigenvalue took more than 60 sweeps.
-__host__ __device__ constexpr int dc_leaf_ws(int leaf) { return leaf * leaf + 3 * leaf; }  // U, off-diagonal, rotations
-static_assert(dc_leaf_ws(kDcLeaf) <= dc_ws_elems<double>(kDcMin), "leaf workspace exceeds the divide-and-conquer workspace");
+// Workspace of a leaf of s rows: W (rows and columns rounded up to fours, zero
+// past s; row stride leaf_ldw(s)), six vectors, the rotations' cosines and sines, and 8 s ints.
+__host__ __device__ constexpr int leaf_pad(int s) { return (s + 3) / 4 * 4; }
+__host__ __device__ constexpr int leaf_ldw(int s) { return leaf_pad(s) + 2; }
+__host__ __device__ constexpr int leaf_ws(int s) { return leaf_pad(s) * leaf_ldw(s) + 12 * s + 2; }
+static_assert(leaf_ws(kDcLeaf) <= dc_ws_elems<double>(kDcMin), "leaf workspace exceeds the divide-and-conquer workspace");
 
-__device__ bool dc_leaf(double* d, const double* e, int lo, int s, double* U, double* le, double* rcs, double* G,
-                        int ld) {
-  const int lane = threadIdx.x & 31;
-  for (int x = lane; x < s * s; x += 32) U[x] = (x / s == x % s) ? 1.0 : 0.0;
-  for (int i = lane; i < s; i += 32) le[i] = i < s - 1 ? e[lo + i] : 0.0;
-  __syncwarp();
-  double* dd = d + lo;
-  bool ok = true;
-  for (int l = 0; l < s && ok; ++l) {
-    int iter = 0;
-    for (;;) {
-      int mq = s - 1;
-      for (int i = l; i < s - 1; ++i)
-        if (fabs(le[i]) <= kEps * (fabs(dd[i]) + fabs(dd[i + 1]))) { mq = i; break; }
-      if (mq == l) break;
-      if (++iter > 60) { ok = false; break; }
-      int cnt = 0;
-      __syncwarp();  // every lane has scanned d and the off-diagonal that lane 0 rewrites
-      if (lane == 0) {
-        double g = (dd[l + 1] - dd[l]) / (2.0 * le[l]);
-        double r = sqrt(g * g + 1.0);
-        g = dd[mq] - dd[l] + le[l] / (g + (g >= 0.0 ? r : -r));
-        double sn = 1.0, c = 1.0, pp = 0.0;
-        bool underflow = false;
-        for (int i = mq - 1; i >= l; --i) {
-          const double f = sn * le[i], bb = c * le[i];
-          const double rr2 = f * f + g * g;
-          if (rr2 == 0.0) { dd[i + 1] -= pp; le[mq] = 0.0; underflow = true; break; }
-          const double ri = rsqrt(rr2);
-          r = rr2 * ri;
-          le[i + 1] = r;
-          sn = f * ri;
-          c = g * ri;
-          g = dd[i + 1] - pp;
-          r = (dd[i] - g) * sn + 2.0 * c * bb;
-          pp = sn * r;
-          dd[i + 1] = g + pp;
-          g = c * r - bb;
-          rcs[2 * cnt] = c;
-          rcs[2 * cnt + 1] = sn;
-          ++cnt;
-        }
-        if (!underflow) { dd[l] -= pp; le[l] = g; le[mq] = 0.0; }
-      }
-      cnt = __shfl_sync(0xffffffffu, cnt, 0);
-      __syncwarp();
-      if (lane < s) {  // rotation t acts on rows i = mq-1-t and i+1 of U
-        for (int t = 0; t < cnt; ++t) {
-          const int i = mq - 1 - t;
-          const double c = rcs[2 * t], sn = rcs[2 * t + 1];
-          const double x = U[i * s + lane], y = U[(i + 1) * s + lane];
-          U[(i + 1) * s + lane] = sn * x + c * y;
-          U[i * s + lane] = c * x - sn * y;
-        }
-      }
-      __syncwarp();
+// Leaf [lo0, lo0+s) of the tree (s <= S <= 32) by one warp: the same divide
+// and conquer down to single rows, every node of a level at once -- lane r is
+// row r of its node (its pole, root and row of W) and column r of the
+// eigenvector block, which it holds in registers, so a level costs what its
+// largest merge costs on one lane per row.  (Implicit QL, a serial chain of
+// some 500 rotations of 130 cycles for 24 rows, took ten times as long.)
+// Close-pair rotations enter as factors of W.  Eigenvalues to d[lo0, lo0+s),
+// the block to G's diagonal block (row stride ld).
+template <int S>
+__device__ __noinline__ void dc_leaf(int dofs, int eofs, int lo0, int s, int wofs, double* G, int ld) {
+  double *d = syev_sm + dofs, *ws = syev_sm + wofs;
+  const double* e = syev_sm + eofs;
+  const int lane = threadIdx.x & 31, ldw = leaf_ldw(s), sp = leaf_pad(s);
+  double* W = ws;
+  double* z = W + sp * ldw;
+  double* zs = z + s;      // sorted, unit norm
+  double* delta = zs + s;  // sorted eigenvalues
+  double* dl = delta + s;  // per node from its lo on: the k not deflated
+  double* zl = dl + s;
+  double* tv = zl + s;
+  double* rc = tv + s;     // rotations
+  double* rsn = rc + s;
+  int* rowof = reinterpret_cast<int*>(rsn + s);
+  int* srow = rowof + s;
+  int* ndl = srow + s;
+  int* ori = ndl + s;
+  int* rp = ori + s;
+  int* rq = rp + s;
+  int* fl = rq + s;    // per node at its lo: deflated entries (bits), rotations
+  int* nr = fl + s;
+  const bool row = lane < s;
+  const unsigned below = (1u << lane) - 1u;
+  double g[S];
+#pragma unroll
+  for (int r = 0; r < S; ++r) g[r] = r == lane ? 1.0 : 0.0;
+  // every boundary inside the leaf is torn at some level
+  double dr = 0.0;
+  if (row) dr = d[lo0 + lane] - (lane > 0 ? fabs(e[lo0 + lane - 1]) : 0.0) - (lane < s - 1 ? fabs(e[lo0 + lane]) : 0.0);
+  int depth = 0;
+  while ((1 << depth) < s) ++depth;
+  for (int dep = depth - 1; dep >= 0; --dep) {
+    int lo = 0, hi = s;
+    for (int l = 0; l < dep; ++l) {
+      const int mid = (lo + hi) >> 1;
+      if (lane >= mid) lo = mid; else hi = mid;
     }
+    const int m = hi - lo, t = (lo + hi) >> 1, j = lane - lo;
+    const bool act = row && m >= 2;
+    const unsigned node = m >= 32 ? 0xffffffffu : (((1u << (m & 31)) - 1u) << lo);
+    const double ev = act ? e[lo0 + t - 1] : 0.0, rho = fabs(ev), sg = ev >= 0.0 ? 1.0 : -1.0;
+    // z: the columns beside the tear publish their node's rows
+    if (act && (lane == t - 1 || lane == t)) {
+      const int ra = lane == t ? t : lo, rz = lane == t ? hi : t;
+      const double f = lane == t ? sg : 1.0;
+#pragma unroll
+      for (int r = 0; r < S; ++r)
+        if (r >= ra && r < rz) z[r] = f * g[r];
+    }
+    __syncwarp();
+    double rhop = 0.0;
+    if (act) {
+      double zz = 0.0;
+      for (int i = lo; i < hi; ++i) zz += z[i] * z[i];
+      rhop = rho * zz;
+      delta[lane] = dr;  // unsorted, for the ranks
+      zs[lane] = z[lane] * (1.0 / sqrt(zz));
+    }
+    __syncwarp();
+    int rank = lane;
+    const double zr = act ? zs[lane] : 0.0;
+    if (act) {
+      rank = lo;
+      for (int q = lo; q < hi; ++q) {
+        const double dq = delta[q];
+        rank += (dq < dr || (dq == dr && q < lane)) ? 1 : 0;
+      }
+    }
+    __syncwarp();
+    if (act) {
+      rowof[lane] = lane;  // valid rows even where non-finite values leave ranks unset
+      delta[lane] = zs[lane] = 0.0;
+    }
+    __syncwarp();
+    if (act) {
+      rowof[rank] = lane;
+      delta[rank] = dr;
+      zs[rank] = zr;
+    }
+    __syncwarp();
+    if (act && j == 0) {  // deflation scan of the node, in order (the tests of dc_merge)
+      double dmax = 0.0;
+      for (int i = lo; i < hi; ++i) dmax = fmax(dmax, fabs(delta[i]));
+      const double tol = 8.0 * kEps * fmax(dmax, rhop);
+      unsigned f = 0;
+      int n = 0, prev = -1;
+      double za = 0.0, da = 0.0;
+      for (int i = lo; i < hi; ++i) {
+        double zb = zs[i], db = delta[i];
+        if (rhop * fabs(zb) <= tol) { f |= 1u << i; continue; }
+        if (prev >= 0) {
+          const double t2 = za * za + zb * zb;
+          if (fabs(db - da) * fabs(za * zb) <= tol * t2) {
+            const double tau = sqrt(t2), c = zb / tau, sn = -za / tau;
+            rp[lo + n] = rowof[prev]; rq[lo + n] = rowof[i]; rc[lo + n] = c; rsn[lo + n] = sn; ++n;
+            delta[prev] = da * c * c + db * sn * sn;
+            db = da * sn * sn + db * c * c;
+            delta[i] = db;
+            zb = tau;
+            zs[i] = tau;
+            zs[prev] = 0.0;
+            f |= 1u << prev;
+          }
+        }
+        prev = i; za = zb; da = db;
+      }
+      fl[lo] = (int)f;
+      nr[lo] = n;
+    }
+    __syncwarp();
+    int k = 0, nrot = 0;
+    if (act) {  // not deflated first, then the deflated, each in order
+      const unsigned defl = (unsigned)fl[lo] & node, keep = node & ~defl;
+      nrot = nr[lo];
+      k = __popc(keep);
+      if ((keep >> lane) & 1u) {
+        const int pos = lo + __popc(keep & below);
+        dl[pos] = delta[lane]; zl[pos] = zs[lane]; srow[pos] = rowof[lane];
+      } else {
+        ndl[lo + k + __popc(defl & below)] = lane;
+      }
+    }
+    __syncwarp();
+    if (j < k) {
+      int o;
+      double tj;
+      secular_root<1>(j, k, dl + lo, zl + lo, rhop, 0, 0u, &o, &tj);
+      ori[lane] = o;
+      tv[lane] = tj;
+    }
+    __syncwarp();
+    double znew = 0.0;
+    if (j < k) {  // Gu and Eisenstat
+      const double di = dl[lane];
+      double prod = ((dl[lo + ori[lo + k - 1]] - di) + tv[lo + k - 1]) / rhop;
+#pragma unroll 4
+      for (int q = 0; q < k - 1; ++q)  // root q over pole q, or past the pole itself q + 1
+        prod *= ((dl[lo + ori[lo + q]] - di) + tv[lo + q]) * dc_rcp(dl[lo + q + (q >= j)] - di);
+      znew = copysign(sqrt(fmax(prod, 0.0)), zl[lane]);
+    }
+    __syncwarp();
+    if (j < k) zl[lane] = znew;
+    __syncwarp();
+    if (lane < sp) {  // row `lane` of W
+      double2* Wz = reinterpret_cast<double2*>(W + lane * ldw);
+      for (int c = 0; c < sp / 2; ++c) Wz[c] = make_double2(0.0, 0.0);
+    }
+    if (row) {
+      double* Wr = W + lane * ldw;
+      if (j < k) {
+        const double bj = dl[lo + ori[lane]], tj = tv[lane];
+        double nn = 0.0;
+#pragma unroll 4
+        for (int i = 0; i < k; ++i) {
+          const double w = zl[lo + i] * dc_rcp((dl[lo + i] - bj) - tj);
+          Wr[srow[lo + i]] = w;
+          nn += w * w;
+        }
+        const double inv = 1.0 / sqrt(nn);
+#pragma unroll 4
+        for (int i = lo; i < hi; ++i) Wr[i] *= inv;  // (the node's deflated columns hold 0)
+        dr = bj + tj;
+      } else if (act) {
+        Wr[rowof[ndl[lane]]] = 1.0;
+        dr = delta[ndl[lane]];
+      } else {
+        Wr[lane] = 1.0;
+      }
+      for (int q = nrot - 1; q >= 0; --q) {
+        const int pa = rp[lo + q], pb = rq[lo + q];
+        const double a = Wr[pa], b = Wr[pb];
+        Wr[pa] = rc[lo + q] * a - rsn[lo + q] * b;
+        Wr[pb] = rsn[lo + q] * a + rc[lo + q] * b;
+      }
+    }
+    __syncwarp();
+    // column `lane` of W G, in parts of 24 or 16 rows: the first of two parts
+    // waits in its place in G, so that a part and g fit the registers
+    constexpr int kPart = S <= 24 ? S : (S + 1) / 2;
+    double gn[kPart];
+    double* Gc = G + (long long)lo0 * ld + lo0 + lane;
+#pragma unroll
+    for (int r0 = 0; r0 < S; r0 += kPart) {
+#pragma unroll
+      for (int q0 = 0; q0 < kPart; q0 += 4) {
+        if (r0 + q0 < sp) {  // four rows at a time; W holds zeros past s
+          double b[4][2] = {};
+#pragma unroll
+          for (int c0 = 0; c0 < S; c0 += 4) {
+            if (c0 < sp) {
+#pragma unroll
+              for (int c = c0; c < c0 + 4; c += 2)
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                  const double2 w = *reinterpret_cast<const double2*>(W + (r0 + q0 + q) * ldw + c);
+                  b[q][0] += w.x * g[c];
+                  b[q][1] += w.y * g[c + 1];
+                }
+            }
+          }
+#pragma unroll
+          for (int q = 0; q < 4; ++q) gn[q0 + q] = b[q][0] + b[q][1];
+        } else {
+#pragma unroll
+          for (int q = 0; q < 4; ++q) gn[q0 + q] = 0.0;
+        }
+      }
+      if (r0 + kPart < S && row)
+#pragma unroll
+        for (int q = 0; q < kPart; ++q)
+          if (r0 + q < s) Gc[(long long)(r0 + q) * ld] = gn[q];
+    }
+#pragma unroll
+    for (int q = 0; q < kPart; ++q) g[S - kPart + q] = gn[q];
+#pragma unroll
+    for (int q = 0; q < S - kPart; ++q) g[q] = (row && q < s) ? Gc[(long long)q * ld] : 0.0;
+    __syncwarp();
   }
-  for (int x = lane; x < s * s; x += 32) G[(long long)(lo + x / s) * ld + lo + x % s] = U[x];
+  if (row) {
+    d[lo0 + lane] = dr;
+#pragma unroll
+    for (int r = 0; r < S; ++r)
+      if (r < s) G[(long long)(lo0 + r) * ld + lo0 + lane] = g[r];
+  }
   __syncwarp();
-  return ok;
 }
 
 // Node b of depth dep of the halving tree: [lo, hi); *plen = its parent's size.
@@ -1133,25 +1337,24 @@ __device__ inline void dc_node(int n, int dep, int b, int* lo_out, int* hi_out, 
 }
 
 // Eigenvalues (d, in every CTA) and eigenvector rows (Zc <- G Zc) of the
-// tridiagonal (d, e) by the merge tree with leaves of at most `leaf` rows
-// (n > leaf); G0, G1 and Z are n x n with row stride ld, ws dc_ws_elems(n).  A level with at least as many nodes as CTAs gives each CTA
+// tridiagonal (d, e) by the merge tree with leaves of at most S rows (n > S);
+// G0, G1 and Z are n x n with row stride ld, ws dc_ws_elems(n), lws lws_cap
+// elements for the leaves (even address).  A level with at least as many nodes as CTAs gives each CTA
 // whole merges (no barriers between CTAs inside them), the levels above share
-// every merge.  Returns false if a leaf failed to converge.
-template <bool W>
-__device__ bool dc_solve(double* d, double* e, double* Z, double* G0, double* G1, int n, int ld, int leaf, double* ws,
-                         long long ws_cap, const Group g) {
+// every merge.
+template <bool W, int S>
+__device__ void dc_solve(double* d, double* e, double* Z, double* G0, double* G1, int n, int ld, double* ws,
+                         double* lws, long long lws_cap, const Group g) {
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const Group alone{0, 1};
-  __shared__ int s_fail;
-  int depth = 0;  // nodes at this depth have at most leaf rows
-  while (((n + (1 << depth) - 1) >> depth) > leaf) ++depth;
-  if (tid == 0) s_fail = 0;
+  int depth = 0;  // nodes at this depth have at most S rows
+  while (((n + (1 << depth) - 1) >> depth) > S) ++depth;
   // tear every internal node (rho = |e[t-1]| off both neighbours)
   for (int dep = 0; dep < depth; ++dep) {
     for (int b = tid; b < (1 << dep); b += kEigThreads) {
       int lo, hi, pl;
       dc_node(n, dep, b, &lo, &hi, &pl);
-      if (hi - lo <= leaf) continue;
+      if (hi - lo <= S) continue;
       const int t = (lo + hi) >> 1;
       const double rho = fabs(e[t - 1]);
       d[t - 1] -= rho;  // nodes of one depth are disjoint
@@ -1160,9 +1363,9 @@ __device__ bool dc_solve(double* d, double* e, double* Z, double* G0, double* G1
     __syncthreads();
   }
   group_sync(g);  // every CTA's d is torn before a peer writes a leaf's eigenvalues there
-  // as many leaf warps as the free shared memory holds blocks for
-  const int lw = (int)min((long long)kWarps, ws_cap / dc_leaf_ws(leaf));
-  double* U = ws + wid * dc_leaf_ws(leaf);
+  // as many leaf warps as the workspace holds
+  const int lsize = leaf_ws((n + (1 << depth) - 1) >> depth) / 2 * 2;
+  const int lw = (int)min((long long)kWarps, lws_cap / lsize);
   for (int dep = depth; dep >= 0; --dep) {
     double* Gi = ((depth - dep - 1) & 1) ? G1 : G0;
     double* Go = ((depth - dep) & 1) ? G1 : G0;
@@ -1170,9 +1373,8 @@ __device__ bool dc_solve(double* d, double* e, double* Z, double* G0, double* G1
     for (int b = g.rank + g.size * wid; wid < lw && b < (1 << dep); b += g.size * lw) {
       int lo, hi, pl;
       dc_node(n, dep, b, &lo, &hi, &pl);
-      if (hi - lo < 1 || hi - lo > leaf || pl <= leaf) continue;
-      if (!dc_leaf(d, e, lo, hi - lo, U, U + leaf * leaf, U + leaf * leaf + leaf, Go, ld))
-        for (int r = lane; r < g.size; r += 32) put_at(&s_fail, 1, g, r);
+      if (hi - lo < 1 || hi - lo > S || pl <= S) continue;
+      dc_leaf<S>(sm_off(d), sm_off(e), lo, hi - lo, sm_off(lws) + wid * lsize, Go, ld);
       for (int r = 0; g.size > 1 && r < g.size; ++r)
         if (r != g.rank && lane < hi - lo) put_at(d + lo + lane, d[lo + lane], g, r);
     }
@@ -1184,8 +1386,9 @@ __device__ bool dc_solve(double* d, double* e, double* Z, double* G0, double* G1
         if (whole && b % g.size != g.rank) continue;
         int lo, hi, pl;
         dc_node(n, dep, b, &lo, &hi, &pl);
-        if (hi - lo <= leaf) continue;
-        dc_merge<W>(d, e, n, ld, lo, (lo + hi) >> 1, hi, Gi, Gi, lo, hi - lo, Go, ws, whole ? alone : g);
+        if (hi - lo <= S) continue;
+        dc_merge<W>(sm_off(d), sm_off(e), n, ld, lo, (lo + hi) >> 1, hi, Gi, Gi, lo, hi - lo, Go, sm_off(ws),
+                    whole ? alone : g);
         if (whole)
           for (int r = 0; r < g.size; ++r)
             if (r != g.rank)
@@ -1207,10 +1410,9 @@ __device__ bool dc_solve(double* d, double* e, double* Z, double* G0, double* G1
         first = ((sz + 63) / 64) * ((n + 63) / 64);
       }
       group_sync(g);
-      dc_merge<W>(d, e, n, ld, 0, t, n, Gi, Go, 0, n, Z, ws, g);
+      dc_merge<W>(sm_off(d), sm_off(e), n, ld, 0, t, n, Gi, Go, 0, n, Z, sm_off(ws), g);
     }
   }
-  return s_fail == 0;
 }
 
 // ------------------------------------------------------------ small structures
@@ -1221,12 +1423,12 @@ __device__ bool dc_solve(double* d, double* e, double* Z, double* G0, double* G1
 // operands shared by all rows are then read from shared memory 16 bytes at a
 // time without conflicts).  Every warp repeats the step's scalars on its own
 // copy of the vectors, so a step has one barrier (the exchange of p = A v).
-// The eigenvectors of the tridiagonal come from dc_solve with leaves of at
-// most kSmallLeaf rows (a leaf's chain of rotations grows with its square),
-// all buffers in shared memory.
+// The eigenvectors of the tridiagonal come from dc_solve with leaves of at most
+// kSmallLeaf rows (24 AOs: 0.14 ms as one leaf of a warp, 0.10 as two and a
+// merge by the CTA), all buffers in shared memory.
 static_assert(kEigThreads / 4 >= kDcMin, "four lanes per row");
 
-__device__ __noinline__ void small_reduce(const double* A, int n, int ld, double* V, double* d, double* e, double* tau,
+__device__ __forceinline__ void small_reduce(const double* A, int n, int ld, double* V, double* d, double* e, double* tau,
                                           double* ws) {
   // per warp: reflectors k and k-1 and w; shared: p and row k+1, two buffers each
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, r = tid >> 2, sub = tid & 3;
@@ -1325,7 +1527,7 @@ __device__ __noinline__ void small_reduce(const double* A, int n, int ld, double
 
 // Z = Q^T (as form_q) from the reflectors in V: row r in the registers of its
 // four lanes, so the rows meet nothing but their own two exchanges per reflector.
-__device__ __noinline__ void small_q(const double* V, int n, int ld, const double* tau, double* Z) {
+__device__ __forceinline__ void small_q(const double* V, int n, int ld, const double* tau, double* Z) {
   const int tid = threadIdx.x, r = tid >> 2, sub = tid & 3;
   double z[16];
 #pragma unroll
@@ -1385,9 +1587,7 @@ __device__ __forceinline__ void syev_structure(const DevBatch& B, double* __rest
   double* A = Ab + mo;
   double* Z = Zb + mo;
   double* Sc = Sb + mo;
-  extern __shared__ __align__(16) unsigned char syev_smem[];
-  double* sm = reinterpret_cast<double*>(syev_smem);
-  double* d = sm;          // n
+  double* d = syev_sm;     // n
   double* e = d + n;       // n
   double* tau = e + n;     // n
   double* v = tau + n;     // n
@@ -1418,9 +1618,9 @@ __device__ __forceinline__ void syev_structure(const DevBatch& B, double* __rest
   const long long ws_cap = (long long)(dyn_bytes / sizeof(double)) - 2LL * n;
   if (tid == 0) { q_fail = 0; e[n - 1] = 0.0; }
   __syncthreads();
-  const bool conv = dc_solve<W>(d, e, Z, A, Sc, n, n, kDcLeaf, tau, ws_cap, g);
+  dc_solve<W, kDcLeaf>(d, e, Z, A, Sc, n, n, tau, tau, ws_cap, g);  // (tau: at an even element)
   for (int i = tid; i < n; i += kEigThreads)
-    if (!conv || !(fabs(d[i]) < 1e30)) q_fail = 1;  // a leaf did not converge, or non-finite input
+    if (!(fabs(d[i]) < 1e30)) q_fail = 1;  // non-finite input
   __syncthreads();
   if (q_fail) {
     if (tid == 0 && g.rank == 0) status[m] = kStEigenFailed;  // k_fermi retires the structure
@@ -1473,8 +1673,7 @@ __global__ void __launch_bounds__(kEigThreads, 2) k_syev_small(DevBatch B, const
   const int n = B.ooff[m + 1] - B.ooff[m];
   if (on_library(B, n) || n >= kDcMin || n <= B.jacobi_max) return;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, ld = small_ld(n);
-  extern __shared__ __align__(16) unsigned char syev_smem[];
-  double* ws = reinterpret_cast<double*>(syev_smem);  // small_ws_elems(n)
+  double* ws = syev_sm;                               // small_ws_elems(n)
   double* G0 = ws + small_ws_elems(n);                // n x ld: reflectors, then merge blocks
   double* G1 = G0 + n * ld;
   double* Z = G1 + n * ld;
@@ -1488,17 +1687,17 @@ __global__ void __launch_bounds__(kEigThreads, 2) k_syev_small(DevBatch B, const
   __syncthreads();
   small_q(G0, n, ld, tau, Z);
   __syncthreads();
-  bool conv = true;
   if (n > kSmallLeaf) {
-    conv = dc_solve<false>(d, e, Z, G0, G1, n, ld, kSmallLeaf, ws, small_ws_elems(n), Group{0, 1});
+    // the leaves' workspace: ws or, since the deepest level's blocks go to G0, G1
+    const bool big = n * ld > small_ws_elems(n);
+    dc_solve<false, kSmallLeaf>(d, e, Z, G0, G1, n, ld, ws, big ? G1 : ws, big ? n * ld : small_ws_elems(n),
+                                Group{0, 1});
   } else {
-    if (wid == 0 && !dc_leaf(d, e, 0, n, ws, ws + kSmallLeaf * kSmallLeaf, ws + kSmallLeaf * (kSmallLeaf + 1), G0, ld) &&
-        lane == 0)
-      q_fail = 1;
+    if (wid == 0) dc_leaf<kSmallLeaf>(sm_off(d), sm_off(e), 0, n, sm_off(ws), G0, ld);
     __syncthreads();
   }
   for (int i = tid; i < n; i += kEigThreads)
-    if (!conv || !(fabs(d[i]) < 1e30)) q_fail = 1;  // a leaf did not converge, or non-finite input
+    if (!(fabs(d[i]) < 1e30)) q_fail = 1;  // non-finite input
   __syncthreads();
   if (q_fail) {
     if (tid == 0) status[m] = kStEigenFailed;  // k_fermi retires the structure
