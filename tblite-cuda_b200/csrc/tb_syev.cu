@@ -1363,8 +1363,10 @@ __device__ void dc_solve(double* d, double* e, double* Z, double* G0, double* G1
     __syncthreads();
   }
   group_sync(g);  // every CTA's d is torn before a peer writes a leaf's eigenvalues there
-  // as many leaf warps as the workspace holds
-  const int lsize = leaf_ws((n + (1 << depth) - 1) >> depth) / 2 * 2;
+  // as many leaf warps as the workspace holds blocks for the largest leaf: of the
+  // deepest level or, where a node of exactly S rows one level up is one, S
+  const int deepest = (n + (1 << depth) - 1) >> depth;
+  const int lsize = leaf_ws(depth > 0 && (n >> (depth - 1)) <= S ? S : deepest);
   const int lw = (int)min((long long)kWarps, lws_cap / lsize);
   for (int dep = depth; dep >= 0; --dep) {
     double* Gi = ((depth - dep - 1) & 1) ? G1 : G0;

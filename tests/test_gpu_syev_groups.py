@@ -46,7 +46,8 @@ def test_orders_at_tile_edges(n):
 def test_cluster_and_one_cta_give_the_same_bits(gpu_calc):
     rng = np.random.default_rng(17)
     mols = [g.water_cluster(k, rng) for k in (11, 16, 22, 37, 38, 64)]
-    mols += [g.alkane(k, rng) for k in (11, 37, 74, 75, 110)]  # 68, 224, 446, 452, 662 AOs
+    # 68, 224, 446, 452, 662 AOs, and 194, 386, 392, 770, 794 with leaves at two depths
+    mols += [g.alkane(k, rng) for k in (11, 37, 74, 75, 110, 32, 64, 65, 128, 132)]
     fill = g.water_clusters(700, seed=9, nmin=11, nmax=14)     # several waves: one CTA each
     batch = gpu_calc.singlepoint_batch(mols + fill, solver=1)
     few = gpu_calc.singlepoint_batch(mols, solver=1)
