@@ -608,7 +608,7 @@ def run_water_box(args, torch):
     elapsed = t0.elapsed_time(t1) * 1e-3 / args.steps
     iters = r["iterations"]
     scf_ms = sum(v[1] for k, v in prof_tot.items() if k not in ("atoms", "adjacency", "integrals", "cholesky",
-                                                                   "trinv", "factor_lib", "scf_init")) / args.steps
+                                                                   "factor", "factor_lib", "scf_init")) / args.steps
     flops = sum(v[2] for v in prof_tot.values() if v[3] == "flop") / args.steps
     flop_ms = sum(v[1] for v in prof_tot.values() if v[3] == "flop") / args.steps
     peak = fp64_peak_tflops(torch)

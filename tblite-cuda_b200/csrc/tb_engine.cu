@@ -422,6 +422,7 @@ struct tb_batch {
   int* d_jlist = nullptr;  // structures on the one-warp Jacobi eigensolver
   int njac = 0;
   SyevPlan syev;            // k_syev's clusters over the batch's order
+  FactorPlan fac;           // k_factor's
   TridPlan trid;            // structures tridiagonalised by k_trid_smem, per class
   int* d_tlist = nullptr;
   int4 *d_tiles64, *d_tiles32, *d_tiles128;
@@ -507,7 +508,7 @@ int choose_lib_above(tb_calculator* c, std::vector<int> sizes) {
   for (int k = k0; k <= nmol && lib_sum < best; ++k) {
     SyevPlan rest;
     rest.build(std::vector<int>(sizes.begin() + k, sizes.end()), 0, 0);
-    const double in_t = 1e-3 * rest.span * M.scale;
+    const double in_t = 1e-3 * rest.c.span * M.scale;
     if (lib_sum + in_t < best) { best = lib_sum + in_t; best_k = k; }
     if (k < nmol) lib_sum += t_lib(sizes[k]);
   }
@@ -904,6 +905,7 @@ tb_status batch_build(tb_calculator* calc, const tb_structure* mols, int nmol, c
     std::vector<int> sizes(nmol);
     for (int i = 0; i < nmol; ++i) sizes[i] = b->h_ooff[order[i] + 1] - b->h_ooff[order[i]];
     b->syev.build(sizes, lib_above, jacobi_max);
+    b->fac.build(sizes, lib_above);
   }
   if (!jlist.empty()) put(o_jlist, jlist.data(), jlist.size() * I4);
   if (!b->trid.list.empty()) put(o_tlist, b->trid.list.data(), b->trid.list.size() * I4);
@@ -1201,7 +1203,7 @@ tb_status raise_smem_limits() {
   int dev = 0, optin = 0;
   TB_CUDA(cudaGetDevice(&dev));
   TB_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-  const void* ks[] = {(const void*)k_syev, (const void*)k_syev_wide, (const void*)k_syev_small, (const void*)k_syev_f32, (const void*)k_fermi, (const void*)k_oa_step,
+  const void* ks[] = {(const void*)k_factor, (const void*)k_syev, (const void*)k_syev_wide, (const void*)k_syev_small, (const void*)k_syev_f32, (const void*)k_fermi, (const void*)k_oa_step,
                       (const void*)k_gemm_tc, (const void*)k_fock, (const void*)k_syev_jacobi};
   for (const void* k : ks) {
     cudaFuncAttributes a;
@@ -1322,7 +1324,7 @@ tb_status calibrate_eigensolvers(tb_calculator* c) {
     SyevPlan p1, p2;
     p1.build({256}, 0, 0);
     p2.build({512}, 0, 0);
-    c->eig.scale = 500.0 * (t1 / p1.span + t2 / p2.span);
+    c->eig.scale = 500.0 * (t1 / p1.c.span + t2 / p2.c.span);
   }
   c->eig.t_lib[0] = l1; c->eig.t_lib[1] = l2;
   c->eig.ready = true;
@@ -1573,6 +1575,10 @@ tb_status batch_setup(tb_batch* b, cudaStream_t st) {
   const DevBatch& B = b->db;
   MolState& S = b->ms;
   const int nmol = b->nmol;
+  {
+    const tb_status ss = raise_smem_limits();
+    if (ss != TB_OK) return ss;
+  }
   b->launches = 0;
   b->kclass.clear();
   b->pend.clear();
@@ -1620,8 +1626,7 @@ tb_status batch_setup(tb_batch* b, cudaStream_t st) {
                              b->sp_w, st, &b->launches));
     prof_stop(b, st, "integrals", e0, 0, 0);
   }
-  TB_K("cholesky", 0, 0, k_cholesky<<<nmol, 256, 0, st>>>(B, b->S, b->W, S.status, nullptr));
-  TB_K("trinv", 0, 0, k_trinv<<<nmol, 256, 0, st>>>(B, b->W, b->X, S.status));
+  TB_K("factor", 0, 0, TB_CUDA(launch_factor(b->fac, B, b->S, b->W, b->X, S.status, st)));
   for (size_t k = 0; k < b->big.size(); ++k) {
     const int m = b->big[k], n = b->h_ooff[m + 1] - b->h_ooff[m];
     const long long mo = b->h_moff[m];
@@ -1640,10 +1645,6 @@ tb_status batch_setup(tb_batch* b, cudaStream_t st) {
     TB_CUDA(cudaMemcpyAsync(b->d_guess_flag, b->h_guess_flag.data(), nmol * sizeof(int), cudaMemcpyHostToDevice,
                             st));
     TB_K("scf_init", 0, 0, k_apply_guess<<<nmol, 256, 0, st>>>(B, b->d_guess, b->d_guess_flag, b->q_in));
-  }
-  {
-    const tb_status ss = raise_smem_limits();
-    if (ss != TB_OK) return ss;
   }
   return read_flags(b, st);
 }
@@ -2751,6 +2752,7 @@ struct MatBatch {
   int* lib_info = nullptr;
   TridPlan trid;
   SyevPlan syev;
+  FactorPlan fac;
   int* d_tlist = nullptr;
   tb_status build(int nmat, const int32_t* n, int smem_tridiag = kTridMin) {
     std::vector<int> ooff(nmat + 1, 0);
@@ -2788,6 +2790,7 @@ struct MatBatch {
     std::stable_sort(order.begin(), order.end(), [&](int a, int c) { return n[a] > n[c]; });
     for (int i = 0; i < nmat; ++i) sorted[i] = n[order[i]];
     syev.build(sorted, kSyevMaxN, 0);
+    fac.build(sorted, kSyevMaxN);
     Layout L;
     size_t o_ooff = L.add((nmat + 1) * 4), o_moff = L.add((nmat + 1) * 8), o_t = L.add(tiles.size() * sizeof(int4));
     size_t o_ord = L.add(nmat * 4);
@@ -2842,8 +2845,11 @@ tb_status tb_sygvd_batch(int32_t nmat, const int32_t* n, const double* H, const 
   TB_CUDA(cudaMemcpy(mb.F, H, mb.n2 * 8, cudaMemcpyHostToDevice));
   const DevBatch& B = mb.db;
   const int nt = (int)mb.tiles.size(), grid = std::min(nt, 148 * 8);
-  k_cholesky<<<nmat, 256>>>(B, mb.S, mb.W, mb.ms.status, nullptr);
-  k_trinv<<<nmat, 256>>>(B, mb.W, mb.X, mb.ms.status);
+  {
+    const tb_status ss = raise_smem_limits();
+    if (ss != TB_OK) return ss;
+  }
+  TB_CUDA(launch_factor(mb.fac, B, mb.S, mb.W, mb.X, mb.ms.status, 0));
   for (size_t k = 0; k < mb.big.size(); ++k) {
     const int m = mb.big[k];
     const long long mo = mb.h_moff[m];
@@ -2855,10 +2861,6 @@ tb_status tb_sygvd_batch(int32_t nmat, const int32_t* n, const double* H, const 
                                  kGemmKUpToJ);
   k_gemm<<<grid, kGemmThreads>>>(B, mb.d_tiles, nt, mb.X, 1, mb.W, 0, nullptr, nullptr, nullptr, mb.F, 1.0, 0.0, mb.ms.active,
                                  kGemmKUpToI | kGemmSym);
-  {
-    const tb_status ss = raise_smem_limits();
-    if (ss != TB_OK) return ss;
-  }
   for (int c = 0; c < kTridClasses; ++c) {
     const int cnt = mb.trid.off[c + 1] - mb.trid.off[c];
     if (cnt == 0) continue;

@@ -141,8 +141,32 @@ cudaError_t launch_integrals(const DevParams& P, const DevBatch& B, const int* n
                              int lmask, const SpLists& W, cudaStream_t st, int64_t* launches);
 
 // linear algebra
-__global__ void k_cholesky(DevBatch B, const double* S, double* W, int* status, const int* active);
-__global__ void k_trinv(DevBatch B, const double* W, double* X, const int* status);
+// How a kernel that takes a structure on one CTA or on a cluster runs a batch:
+// clusters of `cluster` CTAs, the first ncoop structures of the order on one
+// each, then one structure per CTA; one CTA per SM (wide) or two; the modelled
+// span in ms.  ms(n, C): time of a structure of n AOs on C CTAs (tb_syev.cu).
+struct ClusterChoice {
+  int cluster = 1, ncoop = 0;
+  bool wide = true;
+  double span = 0.0;
+};
+ClusterChoice choose_clusters(const std::vector<int>& sizes, int first, int last, double (*ms)(double, int),
+                              bool two_per_sm, bool one_per_sm);
+
+// S = L L^T (W[k][i] = L[i][k]) and X = L^-T, 64 x 64 blocks (tb_factor.cu); a
+// structure whose S is not positive definite gets kStNotSpd
+constexpr int kFactorBlock = 64;
+__global__ void k_factor(DevBatch B, const double* S, double* Wb, double* Xb, int* status, int ncoop);
+struct FactorPlan {
+  int count = 0;  // structures
+  ClusterChoice c;
+  // sizes in the batch's order (decreasing; those of the library path first)
+  void build(const std::vector<int>& sizes, int lib_above);
+};
+size_t factor_smem_bytes();
+// the shared-memory limit must have been raised
+cudaError_t launch_factor(const FactorPlan& P, const DevBatch& B, const double* S, double* W, double* X, int* status,
+                          cudaStream_t st);
 // k_gemm shapes (bit mask): zeros of a triangular factor and symmetric results
 constexpr int kGemmKUpToJ = 1, kGemmKUpToI = 2, kGemmKFromI = 4, kGemmSym = 8;
 __global__ void k_gemm(DevBatch B, const int4* tiles, int ntiles, const double* Ab, int ta, const double* Bb, int tb_,
@@ -159,14 +183,11 @@ __global__ void k_syev(DevBatch B, double* Ab, double* Zb, double* Sb, double* w
                        const int* active, int ncoop);
 __global__ void k_syev_wide(DevBatch B, double* Ab, double* Zb, double* Sb, double* wout, int* perm, int* status,
                             const int* active, int ncoop);
-constexpr int kSyevMaxCluster = 8;
 constexpr size_t kSyevSmemTwo = 110 * 1024;  // dynamic shared memory up to which two CTAs fit an SM
 struct SyevPlan {
   int n64 = 0;          // structures of kDcMin+ AOs on the in-house solver lead the order
   int nsmall = 0, small_max = 1;  // structures below kDcMin AOs that k_syev_small solves, the largest
-  int cluster = 1, ncoop = 0;
-  bool wide = true;     // k_syev_wide (one CTA per SM)
-  double span = 0.0;    // modelled time of one launch, ms
+  ClusterChoice c;      // wide: k_syev_wide
   int nmax = 0;         // largest in-house structure
   // sizes in the batch's order (decreasing; those of the library path first)
   void build(const std::vector<int>& sizes, int lib_above, int jacobi_max);

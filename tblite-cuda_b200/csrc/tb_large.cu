@@ -1,12 +1,12 @@
 // Dense path for structures above the in-house eigensolver's stated size.
 //
-// The batched one-CTA-per-structure kernels (k_cholesky, k_trinv, k_syev)
+// The batched in-house kernels (k_factor, k_syev)
 // keep every matrix of a structure on one SM; past about a thousand AOs that
 // SM, not the GPU, sets the time.  Structures with more AOs than the stated
 // bound (tb_options.solver; 1216 by default) are therefore factorised and
 // diagonalised by cuSOLVER's 64-bit dense API, one structure at a time on the
 // run's stream, writing the SAME layouts the in-house kernels write:
-//  * X = L^-T, row-major upper triangular (k_trinv's output): Xpotrf (lower)
+//  * X = L^-T, row-major upper triangular (k_factor's output): Xpotrf (lower)
 //    and Xtrtri (lower, non-unit) on a column-major copy of S leave L^-1 in
 //    the lower triangle, which read row-major is L^-T; the strict lower
 //    triangle of the row-major view still holds S and is cleared.

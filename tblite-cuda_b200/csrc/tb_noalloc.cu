@@ -124,7 +124,8 @@ extern "C" tb_status tb_sygvd_noalloc(int32_t n, const double* H, const double* 
       // (cached last, so that a failed set-up is retried by the next call)
       const std::pair<const void*, size_t> need[] = {{(const void*)k_syev, syev_smem_bytes(kNoAllocMaxN)},
                                                      {(const void*)k_syev_wide, syev_smem_bytes(kNoAllocMaxN)},
-                                                     {(const void*)k_syev_small, small_smem_bytes(kDcMin - 1)}};
+                                                     {(const void*)k_syev_small, small_smem_bytes(kDcMin - 1)},
+                                                     {(const void*)k_factor, factor_smem_bytes()}};
       for (const auto& k : need) {
         cudaFuncAttributes fa;
         e = cudaFuncGetAttributes(&fa, k.first);
@@ -147,8 +148,10 @@ extern "C" tb_status tb_sygvd_noalloc(int32_t n, const double* H, const double* 
   B.moff = v.moff;
   const int nt = (n + 63) / 64, ntiles = nt * nt;
   k_noalloc_init<<<1, 64, 0, st>>>(base, n);
-  k_cholesky<<<1, 256, 0, st>>>(B, S, v.W, v.status, nullptr);
-  k_trinv<<<1, 256, 0, st>>>(B, v.W, v.X, v.status);
+  FactorPlan fp;
+  fp.build({n}, 0);
+  e = launch_factor(fp, B, S, v.W, v.X, v.status, st);
+  if (e != cudaSuccess) return noalloc_fail(TB_CUDA_ERROR, cudaGetErrorString(e));
   // A = X^T H X (T = H X kept in W, whose Cholesky factor is no longer needed)
   k_gemm<<<ntiles, kGemmThreads, 0, st>>>(B, v.tiles, ntiles, H, 0, v.X, 0, nullptr, nullptr, nullptr, v.W, 1.0, 0.0,
                                  v.active, kGemmKUpToJ);

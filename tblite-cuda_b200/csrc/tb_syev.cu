@@ -10,7 +10,7 @@
 //  2. Zc = Q^T accumulated backwards in compact-WY blocks (form_q).
 //  3. Tridiagonal eigenproblem by divide and conquer (dc_solve).
 //  4. Ascending order by rank (ties by index).
-// Together with k_cholesky, k_trinv and k_gemm this is sygvd (reference
+// Together with k_factor and k_gemm this is sygvd (reference
 // src/lapack/sygvd.h:4-23).
 //
 // Work is cut into units whose boundaries and order of additions depend on
@@ -1741,8 +1741,7 @@ double syev_ms(double n, int C) {
 }
 }  // namespace
 
-// The cluster size and the number of structures that get a whole cluster: the
-// combination with the shortest modelled span.  A span is list scheduling of
+// The combination with the shortest modelled span.  A span is list scheduling of
 // the order (largest first) over as many clusters as the GPU holds at once
 // (kCap: cudaOccupancyMaxActiveClusters on a B200, one and two CTAs per SM) for
 // every cluster size and a geometric set of splits into cluster and one-CTA
@@ -1751,24 +1750,16 @@ double syev_ms(double n, int C) {
 // one CTA each, 11.0 on two; 128: 11.1 and 6.2 (on four); 48 chains of
 // 122..1196 AOs: 172 and 40 (on eight).  Batches of several waves of CTAs keep
 // one CTA per structure: clusters repeat work and would only lose.
-void SyevPlan::build(const std::vector<int>& sizes, int lib_above, int jacobi_max) {
-  *this = SyevPlan();
-  int first = 0;  // structures of the library path lead the order and exit at once
-  for (size_t i = 0; i < sizes.size(); ++i) {
-    const int n = sizes[i];
-    if (lib_above != 0 && n > lib_above) { first = n64 = (int)i + 1; continue; }
-    nmax = n > nmax ? n : nmax;
-    if (n >= kDcMin) n64 = (int)i + 1;
-    else if (n > jacobi_max) { ++nsmall; small_max = std::max(small_max, n); }
-  }
-  if (n64 <= first) return;
+ClusterChoice choose_clusters(const std::vector<int>& sizes, int first, int last, double (*ms)(double, int),
+                              bool two_per_sm, bool one_per_sm) {
+  ClusterChoice best;
   std::vector<double> busy;  // finish times of the clusters in flight (a heap)
   auto schedule = [&](int cap, int C, int k, double slow, double limit) {
     busy.clear();
     double end = 0.0;
-    for (int i = first; i < n64 && end < limit;) {
+    for (int i = first; i < last && end < limit;) {
       const bool coop = C > 1 && i < k;
-      double t = slow * syev_ms(sizes[i], coop ? C : 1);
+      double t = slow * ms(sizes[i], coop ? C : 1);
       i += coop ? 1 : C;
       if ((int)busy.size() == cap) {
         std::pop_heap(busy.begin(), busy.end(), std::greater<double>());
@@ -1783,20 +1774,35 @@ void SyevPlan::build(const std::vector<int>& sizes, int lib_above, int jacobi_ma
   };
   constexpr int kCap[2][4] = {{148, 74, 33, 15}, {296, 148, 71, 33}};
   constexpr double kSlowTwo = 1.42, kSlowNarrow = 1.1;
-  const int cnt = n64 - first;
-  span = 1e300;
-  for (int per = syev_smem_bytes(nmax) <= kSyevSmemTwo ? 2 : 1; per >= 1; --per)
+  const int cnt = last - first;
+  best.span = 1e300;
+  for (int per = two_per_sm ? 2 : 1; per >= (one_per_sm ? 1 : 2); --per)
     for (int c = 0; c < 4; ++c) {
       const int C = 1 << c;
       if (C > 1 && cnt > 4 * 148) break;
       for (int k = cnt; k >= 1; k = k > 1 ? (3 * k) / 4 : 0) {
         const int items = C > 1 ? k + (cnt - k + C - 1) / C : cnt;
         const double slow = per == 1 ? 1.0 : items > kCap[0][c] ? kSlowTwo : kSlowNarrow;
-        const double t = schedule(kCap[per - 1][c], C, first + k, slow, span);
-        if (t < 0.97 * span) { span = t; cluster = C; ncoop = C > 1 ? first + k : 0; wide = per == 1; }
+        const double t = schedule(kCap[per - 1][c], C, first + k, slow, best.span);
+        if (t < 0.97 * best.span) best = {C, C > 1 ? first + k : 0, per == 1, t};
         if (C == 1) break;
       }
     }
+  return best;
+}
+
+void SyevPlan::build(const std::vector<int>& sizes, int lib_above, int jacobi_max) {
+  *this = SyevPlan();
+  int first = 0;  // structures of the library path lead the order and exit at once
+  for (size_t i = 0; i < sizes.size(); ++i) {
+    const int n = sizes[i];
+    if (lib_above != 0 && n > lib_above) { first = n64 = (int)i + 1; continue; }
+    nmax = n > nmax ? n : nmax;
+    if (n >= kDcMin) n64 = (int)i + 1;
+    else if (n > jacobi_max) { ++nsmall; small_max = std::max(small_max, n); }
+  }
+  if (n64 > first)
+    c = choose_clusters(sizes, first, n64, syev_ms, syev_smem_bytes(nmax) <= kSyevSmemTwo, true);
 }
 
 cudaError_t launch_syev(const SyevPlan& P, const DevBatch& B, double* A, double* Z, double* Sb, double* w, int* perm,
@@ -1806,8 +1812,8 @@ cudaError_t launch_syev(const SyevPlan& P, const DevBatch& B, double* A, double*
   if (P.n64 > 0 && P.nmax >= kDcMin) {
     DevBatch Bs = B;
     Bs.nmol = P.n64;  // the kernel's bound on its position in the order
-    const int C = P.cluster;
-    const int groups = P.ncoop + (P.n64 - P.ncoop + C - 1) / C;
+    const int C = P.c.cluster;
+    const int groups = P.c.ncoop + (P.n64 - P.c.ncoop + C - 1) / C;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)(groups * C));
     cfg.blockDim = dim3(kEigThreads);
@@ -1819,7 +1825,7 @@ cudaError_t launch_syev(const SyevPlan& P, const DevBatch& B, double* A, double*
     at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = C > 1 ? 1 : 0;
-    e = cudaLaunchKernelEx(&cfg, P.wide ? k_syev_wide : k_syev, Bs, A, Z, Sb, w, perm, status, active, P.ncoop);
+    e = cudaLaunchKernelEx(&cfg, P.c.wide ? k_syev_wide : k_syev, Bs, A, Z, Sb, w, perm, status, active, P.c.ncoop);
     if (e != cudaSuccess) return e;
     if (launches) ++*launches;
   }
