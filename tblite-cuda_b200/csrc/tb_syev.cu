@@ -402,7 +402,8 @@ __device__ __forceinline__ double walk_gather(const double* part, int nm, int c,
 // A (n x n, upper triangle used, row-major) to tridiagonal form: reflector k
 // (leading 1) in row k of A from column k+1 on, its scale in tau[k], the
 // diagonal in d, the off-diagonal in e; d, e and tau complete in every CTA.
-// gs: scratch for the walk partials (at most n^2 doubles).
+// gs: n^2 doubles of scratch for the walk partials, two halves: a CTA may write a
+// step's partials while a slower one still gathers the step before's.
 template <bool W>
 __device__ __forceinline__ void tridiag_tiles(double* A, int n, double* d, double* e, double* tau, double* v, double* vn,
                                            double* p, double* w, double* ring, double* gs, const Group g) {
@@ -415,6 +416,7 @@ __device__ __forceinline__ void tridiag_tiles(double* A, int n, double* d, doubl
   // follows v and vn finite
   for (int i = tid; i < n; i += kEigThreads) v[i] = vn[i] = p[i] = w[i] = 0.0;
   __syncthreads();
+  const int half = n * n / 2;
   const int nref = n - 2;  // reflectors 0 .. n-3
   int np = 0;              // pairs in the open panel
   for (int r = 0;; ++r) {
@@ -437,7 +439,7 @@ __device__ __forceinline__ void tridiag_tiles(double* A, int n, double* d, doubl
         const double raw = rowr[j];
         // the open pairs' part of p and of row r, while the partials arrive
         double cp = 0.0, cx = 0.0;
-        const double sum = walk_gather(gs, mm, j, [&]() {
+        const double sum = walk_gather(gs + ((r - 1) & 1) * half, mm, j, [&]() {
           for (int i = 0; i < np; ++i) {
             const double pv = PV[i * n + r + j], pw = PW[i * n + r + j];
             cp += pv * dot[i] + pw * dot[kPanel + i];
@@ -492,15 +494,16 @@ __device__ __forceinline__ void tridiag_tiles(double* A, int n, double* d, doubl
     __syncthreads();
     // products with the new reflector over rows and columns r+1 .. n-1
     double* Mb = A + (long long)(r + 1) * n + r + 1;
+    double* out = gs + (r & 1) * half;
     if (np == kPanel) {
-      if (mr <= kWalk1) walk_close<5, 5, 2>(Mb, n, r + 1, mr, sm_off(PV), sm_off(vn), gs, gw, ngw);
-      else if (mr <= kWalk2) walk_close<5, 6, 2>(Mb, n, r + 1, mr, sm_off(PV), sm_off(vn), gs, gw, ngw);
-      else walk_close<6, 7, W ? 4 : 2>(Mb, n, r + 1, mr, sm_off(PV), sm_off(vn), gs, gw, ngw);
+      if (mr <= kWalk1) walk_close<5, 5, 2>(Mb, n, r + 1, mr, sm_off(PV), sm_off(vn), out, gw, ngw);
+      else if (mr <= kWalk2) walk_close<5, 6, 2>(Mb, n, r + 1, mr, sm_off(PV), sm_off(vn), out, gw, ngw);
+      else walk_close<6, 7, W ? 4 : 2>(Mb, n, r + 1, mr, sm_off(PV), sm_off(vn), out, gw, ngw);
       np = 0;
     } else {
-      if (mr <= kWalk1) walk_read<5, 5, 32>(Mb, n, mr, sm_off(vn), gs, gw, ngw);
-      else if (mr <= kWalk2) walk_read<5, 6, W ? 32 : 16>(Mb, n, mr, sm_off(vn), gs, gw, ngw);
-      else walk_read<6, 7, W ? 16 : 8>(Mb, n, mr, sm_off(vn), gs, gw, ngw);
+      if (mr <= kWalk1) walk_read<5, 5, 32>(Mb, n, mr, sm_off(vn), out, gw, ngw);
+      else if (mr <= kWalk2) walk_read<5, 6, W ? 32 : 16>(Mb, n, mr, sm_off(vn), out, gw, ngw);
+      else walk_read<6, 7, W ? 16 : 8>(Mb, n, mr, sm_off(vn), out, gw, ngw);
       // the next step's w_i . v and v_i . v, one warp each, in every CTA; the
       // last warps of the group first (the walk's units start at warp 0).  Two
       // buffers: a CTA one step behind may still read the other
