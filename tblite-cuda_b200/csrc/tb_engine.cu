@@ -297,7 +297,7 @@ struct tb_calculator {
   struct EigModel {
     bool ready = false;
     double a = 0, b = 0;  // in-house latency of one structure: a N^2 + b N^3 seconds
-    double c = 0, d = 0;  // one cuSOLVER call: c + d N^3 seconds
+    double c = 0, d = 0;  // one cuSOLVER call: c + d N seconds
     double t_in[2] = {0, 0}, t_lib[2] = {0, 0};  // the measured points (256/512 and 256/1024 AOs)
     double scale = 1;  // measured in-house time over SyevPlan's model, mean of the two points
   } eig;
@@ -501,7 +501,7 @@ int choose_lib_above(tb_calculator* c, std::vector<int> sizes) {
   if (sizes[k0] < 384) return kSyevMaxN;  // small structures: the batched solver always wins
   if (calibrate_eigensolvers(c) != TB_OK) return kSyevMaxN;
   const auto& M = c->eig;
-  auto t_lib = [&](double n) { return M.c + M.d * n * n * n; };
+  auto t_lib = [&](double n) { return M.c + M.d * n; };
   double lib_sum = 0.0, best = 1e300;
   int best_k = k0;
   for (int i = 0; i < k0; ++i) lib_sum += t_lib(sizes[i]);
@@ -1210,13 +1210,17 @@ tb_status raise_smem_limits() {
     TB_CUDA(cudaFuncGetAttributes(&a, k));
     TB_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)a.sharedSizeBytes));
   }
+  // clusters of 16 (more than the portable eight)
+  for (const void* k : {(const void*)k_factor, (const void*)k_syev, (const void*)k_syev_wide})
+    TB_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   TB_CUDA(trid_raise_limits());
   return TB_OK;
 }
 
 // Measures the two eigensolvers once per calculator: the in-house k_syev on
 // one structure (latency, at 256 and 512 AOs, fitted by a N^2 + b N^3) and one
-// cuSOLVER syevd call (at 256 and 1024 AOs, fitted by c + d N^3), on
+// cuSOLVER syevd call (at 256 and 1024 AOs, fitted by c + d N: its calls are
+// bound by the launches of its steps, 3.9 ms at 384 AOs and 8.5 at 722), on
 // deterministic random symmetric matrices.
 tb_status calibrate_eigensolvers(tb_calculator* c) {
   std::lock_guard<std::mutex> lk(c->tune_mu);
@@ -1312,13 +1316,13 @@ tb_status calibrate_eigensolvers(tb_calculator* c) {
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   if (st != TB_OK) return st;
-  // t = a n^2 + b n^3 through (256, t1), (512, t2); t = c + d n^3 through (256, l1), (1024, l2)
+  // t = a n^2 + b n^3 through (256, t1), (512, t2); t = c + d n through (256, l1), (1024, l2)
   const double n1 = 256, n2 = 512, m1 = 256, m2 = NL;
   const double det = n1 * n1 * n2 * n2 * n2 - n2 * n2 * n1 * n1 * n1;
   c->eig.a = std::max(0.0, (t1 * n2 * n2 * n2 - t2 * n1 * n1 * n1) / det);
   c->eig.b = std::max(0.0, (n1 * n1 * t2 - n2 * n2 * t1) / det);
-  c->eig.d = std::max(0.0, (l2 - l1) / (m2 * m2 * m2 - m1 * m1 * m1));
-  c->eig.c = std::max(0.0, l1 - c->eig.d * m1 * m1 * m1);
+  c->eig.d = std::max(0.0, (l2 - l1) / (m2 - m1));
+  c->eig.c = l1 - c->eig.d * m1;
   c->eig.t_in[0] = t1; c->eig.t_in[1] = t2;
   {
     SyevPlan p1, p2;
@@ -2391,7 +2395,7 @@ int32_t tb_calculator_tuning(const tb_calculator* c, char* buf, int32_t len) {
     << ", \"inhouse_s\": {\"256\": " << c->eig.t_in[0] << ", \"512\": " << c->eig.t_in[1] << "}"
     << ", \"cusolver_s\": {\"256\": " << c->eig.t_lib[0] << ", \"1024\": " << c->eig.t_lib[1] << "}"
     << ", \"model\": {\"inhouse\": \"" << c->eig.a << " N^2 + " << c->eig.b << " N^3\", \"cusolver\": \""
-    << c->eig.c << " + " << c->eig.d << " N^3\"}, \"inhouse_limit\": " << kSyevMaxN << "}"
+    << c->eig.c << " + " << c->eig.d << " N\"}, \"inhouse_limit\": " << kSyevMaxN << "}"
     << ", \"smem_tridiag\": {\"min_n\": " << c->smem_tridiag << ", \"classes\": [";
   for (int k = 0; k < kTridClasses; ++k)
     o << (k ? ", " : "") << "{\"cluster\": " << kTridClusterSizes[k] << ", \"max_n\": " << kTridClassMax[k]

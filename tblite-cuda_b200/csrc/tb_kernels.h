@@ -183,7 +183,6 @@ __global__ void k_syev(DevBatch B, double* Ab, double* Zb, double* Sb, double* w
                        const int* active, int ncoop);
 __global__ void k_syev_wide(DevBatch B, double* Ab, double* Zb, double* Sb, double* wout, int* perm, int* status,
                             const int* active, int ncoop);
-constexpr size_t kSyevSmemTwo = 110 * 1024;  // dynamic shared memory up to which two CTAs fit an SM
 struct SyevPlan {
   int n64 = 0;          // structures of kDcMin+ AOs on the in-house solver lead the order
   int nsmall = 0, small_max = 1;  // structures below kDcMin AOs that k_syev_small solves, the largest

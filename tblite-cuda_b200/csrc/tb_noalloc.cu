@@ -131,6 +131,8 @@ extern "C" tb_status tb_sygvd_noalloc(int32_t n, const double* H, const double* 
         e = cudaFuncGetAttributes(&fa, k.first);
         if (e == cudaSuccess && fa.maxDynamicSharedSizeBytes < (int)k.second)
           e = cudaFuncSetAttribute(k.first, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k.second);
+        if (e == cudaSuccess && k.first != (const void*)k_syev_small)  // clusters of 16
+          e = cudaFuncSetAttribute(k.first, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         if (e != cudaSuccess) return noalloc_fail(TB_CUDA_ERROR, cudaGetErrorString(e));
       }
       double* addr = nullptr;

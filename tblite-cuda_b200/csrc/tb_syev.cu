@@ -17,7 +17,7 @@
 // the matrix order alone (row/column tiles of the walks, 64-row tiles of Q,
 // 64 x 64 tiles of the merge products, teams of four lanes per secular root),
 // never on how many warps share them.  So a structure gives the same bits on
-// one CTA (a large batch: 444 structures resident on 148 SMs, throughput) and
+// one CTA (a large batch: 296 structures resident on 148 SMs, throughput) and
 // on a cluster of 2..16 (a few structures: latency).  The CTAs of a cluster keep
 // identical copies of the vectors (d, e, tau, v, p, w, the panel) in their
 // shared memory and repeat the O(n) arithmetic on them; only the units are
@@ -132,21 +132,22 @@ __device__ __forceinline__ double dc_rcp(double x) {
 // (entries on and above the diagonal) into col[I][c] and its row products
 // (entries above the diagonal) into row[J][r] of the scratch, each written
 // once, and p is their sum in a fixed order.  Wider tiles for larger blocks
-// keep at most 19 column and 10 row partials per entry (every CTA of a group
-// reads them all); 32 x 64 for 225..448 rows gives up to 56 units, one per
-// warp of a cluster of seven or eight.
-constexpr int kWalk1 = 224, kWalk2 = 448;  // 32 x 32, 32 x 64, above: 64 x 128
+// keep at most 38 column and 10 row partials per entry (every CTA of a group
+// reads them all).  Coarser tiles (32 x 32, 32 x 64, 64 x 128) left most warps
+// of a cluster without a unit: 138 AOs alone 1.03 ms against 0.87, 384 3.40
+// against 2.87, 722 10.2 against 8.2, for 3% on a batch of one CTA each.
+constexpr int kWalk1 = 224, kWalk2 = 448;  // 16 x 32, 16 x 64, above: 32 x 128
 __host__ __device__ constexpr int parts(int nm, int shift) { return (nm + (1 << shift) - 1) >> shift; }
 
 // Position in the unit list of one warp: units are numbered strip by strip.
-template <int RS, int CS>
+template <int RS>
 struct Units {
-  int nI, nJ, J = 0, base = 0;
-  __device__ __forceinline__ explicit Units(int nm) : nI(parts(nm, RS)), nJ(parts(nm, CS)) {}
+  int cs, nI, nJ, J = 0, base = 0;
+  __device__ __forceinline__ Units(int nm, int cshift) : cs(cshift), nI(parts(nm, RS)), nJ(parts(nm, cshift)) {}
   // row tile of unit u (>= the previous one's); -1 past the last
   __device__ __forceinline__ int seek(int u) {
     for (;;) {
-      const int cnt = min(nI, parts((J + 1) << CS, RS));
+      const int cnt = min(nI, parts((J + 1) << cs, RS));
       if (u - base < cnt) return u - base;
       base += cnt;
       if (++J >= nJ) return -1;
@@ -170,7 +171,7 @@ __device__ __noinline__ void walk_read(const double* Mb, int n, int nm, int xo, 
   static_assert(U % 8 == 0, "rows are reduced in eights");
   const double* x = syev_sm + xo;
   const int lane = threadIdx.x & 31, g = lane >> 2;
-  Units<RS, CS> un(nm);
+  Units<RS> un(nm, CS);
   double* col = part;
   double* row = part + (long long)un.nI * nm;
   for (int u = gw;; u += ngw) {
@@ -192,21 +193,13 @@ __device__ __noinline__ void walk_read(const double* Mb, int n, int nm, int xo, 
     for (int rb = rbeg; rb < rend; rb += U) {
       double a[U][Q];
       const double* Mr = Mb + (long long)rb * n + c0 + lane;
-      const bool inside = rb + U <= c0 && c0 + (1 << CS) <= nm;  // wholly above the diagonal
-      if (inside) {
+      // one comparison per entry everywhere: a second copy of this code for the
+      // sub-blocks wholly above the diagonal cost a branch per row (11%)
 #pragma unroll
-        for (int i = 0; i < U; ++i) {
+      for (int i = 0; i < U; ++i) {
 #pragma unroll
-          for (int j = 0; j < Q; ++j) a[i][j] = Mr[32 * j];
-          Mr += n;
-        }
-      } else {
-#pragma unroll
-        for (int i = 0; i < U; ++i) {
-#pragma unroll
-          for (int j = 0; j < Q; ++j) a[i][j] = cc[j] - rb >= i ? Mr[32 * j] : 0.0;
-          Mr += n;
-        }
+        for (int j = 0; j < Q; ++j) a[i][j] = cc[j] - rb >= i ? Mr[32 * j] : 0.0;
+        Mr += n;
       }
       double v[U];  // lane's products of each row
 #pragma unroll
@@ -214,18 +207,10 @@ __device__ __noinline__ void walk_read(const double* Mb, int n, int nm, int xo, 
         // (rows past the block hold zeros; x is finite there)
         const double xr = x[rb + i];
         v[i] = 0.0;
-        if (inside) {
 #pragma unroll
-          for (int j = 0; j < Q; ++j) {
-            acc[j] += a[i][j] * xr;
-            v[i] += a[i][j] * xs[j];
-          }
-        } else {
-#pragma unroll
-          for (int j = 0; j < Q; ++j) {
-            acc[j] += a[i][j] * xr;
-            if (cc[j] - rb > i) v[i] += a[i][j] * xs[j];
-          }
+        for (int j = 0; j < Q; ++j) {
+          acc[j] += a[i][j] * xr;
+          if (cc[j] - rb > i) v[i] += a[i][j] * xs[j];
         }
       }
       double s0[U / 4], s1[U / 4];  // two chains (even and odd rows) per eight rows
@@ -256,14 +241,14 @@ __device__ __noinline__ void walk_read(const double* Mb, int n, int nm, int xo, 
 // tensor instruction (accumulators initialised from M, stored back), and the
 // partials of M_new x are formed from the same fragments.  NB sub-tiles of a
 // 16-column block are loaded before the first is used.
-template <int RS, int CS, int NB>
-__device__ __noinline__ void walk_close(double* Mb, int n, int r0, int nm, int pvo, int xo, double* part, int gw,
+template <int RS, int NB>
+__device__ __noinline__ void walk_close(double* Mb, int n, int r0, int nm, int CS, int pvo, int xo, double* part, int gw,
                                         int ngw) {
   const double *PV = syev_sm + pvo, *PW = PV + kPanel * n, *x = syev_sm + xo;
   constexpr int RB = 1 << (RS - 4);
   static_assert(RB % NB == 0, "sub-tiles per load round");
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  Units<RS, CS> un(nm);
+  Units<RS> un(nm, CS);
   double* col = part;
   double* row = part + (long long)un.nI * nm;
   for (int u = gw;; u += ngw) {
@@ -276,68 +261,62 @@ __device__ __noinline__ void walk_close(double* Mb, int n, int r0, int nm, int p
     for (int i = 0; i < RB; ++i) rp[i][0] = rp[i][1] = 0.0;
     for (int cw = c0; cw < min(nm, c0 + (1 << CS)); cw += 16) {
       double cs[4] = {0.0, 0.0, 0.0, 0.0};  // column sums, index 2y + h
+      double xc[4];
+      int cx[4];  // column, -1 past the block
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int c = cw + 8 * (k >> 1) + 2 * t + (k & 1);
+        cx[k] = c < nm ? c : -1;
+        xc[k] = c < nm ? x[c] : 0.0;
+      }
       double* M0 = Mb + (long long)(rbeg + g) * n + cw + 2 * t;
 #pragma unroll
       for (int rb0 = 0; rb0 < RB; rb0 += NB) {
-        double d[NB][2][2][2];
+        double d[NB][2][4];
 #pragma unroll
-        for (int i = 0; i < NB; ++i) {
-          const int rt = rbeg + 16 * (rb0 + i);
-          const bool inside = rt + 16 <= cw && cw + 16 <= nm;
+        for (int i = 0; i < NB; ++i)
 #pragma unroll
-          for (int xx = 0; xx < 2; ++xx)
+          for (int xx = 0; xx < 2; ++xx) {
+            const int r = rbeg + 16 * (rb0 + i) + 8 * xx + g;
 #pragma unroll
-            for (int y = 0; y < 2; ++y)
-#pragma unroll
-              for (int h = 0; h < 2; ++h) {
-                const int r = rt + 8 * xx + g, c = cw + 8 * y + 2 * t + h;
-                d[i][xx][y][h] = (inside || (r < nm && c < nm && c >= r))
-                                     ? M0[(long long)(16 * (rb0 + i) + 8 * xx) * n + 8 * y + h] : 0.0;
-              }
-        }
+            for (int k = 0; k < 4; ++k)
+              d[i][xx][k] = cx[k] >= r ? M0[(long long)(16 * (rb0 + i) + 8 * xx) * n + 8 * (k >> 1) + (k & 1)] : 0.0;
+          }
+        // (rows and columns past the block take its last one's pairs: their
+        // entries are neither stored nor added)
 #pragma unroll
         for (int ks = 0; ks < 4; ++ks) {
-          const double* Lc = (ks < 2 ? PW : PV) + (long long)(4 * (ks & 1) + t) * n + r0;
-          const double* Kr = (ks < 2 ? PV : PW) + (long long)(4 * (ks & 1) + t) * n + r0;
+          const double* Lc = (ks < 2 ? PW : PV) + (4 * (ks & 1) + t) * n + r0;
+          const double* Kr = (ks < 2 ? PV : PW) + (4 * (ks & 1) + t) * n + r0;
           double b[2];
 #pragma unroll
-          for (int y = 0; y < 2; ++y) {
-            const int c = cw + 8 * y + g;
-            b[y] = c < nm ? Lc[c] : 0.0;
-          }
+          for (int y = 0; y < 2; ++y) b[y] = Lc[min(cw + 8 * y + g, nm - 1)];
 #pragma unroll
           for (int i = 0; i < NB; ++i)
 #pragma unroll
             for (int xx = 0; xx < 2; ++xx) {
-              const int r = rbeg + 16 * (rb0 + i) + 8 * xx + g;
-              const double a = r < nm ? -Kr[r] : 0.0;
+              const double a = -Kr[min(rbeg + 16 * (rb0 + i) + 8 * xx + g, nm - 1)];
 #pragma unroll
-              for (int y = 0; y < 2; ++y) dmma(d[i][xx][y][0], d[i][xx][y][1], a, b[y]);
+              for (int y = 0; y < 2; ++y) dmma(d[i][xx][2 * y], d[i][xx][2 * y + 1], a, b[y]);
             }
         }
         // store the upper entries, drop the others from the products
 #pragma unroll
-        for (int i = 0; i < NB; ++i) {
-          const int rt = rbeg + 16 * (rb0 + i);
-          const bool inside = rt + 16 <= cw && cw + 16 <= nm;
+        for (int i = 0; i < NB; ++i)
 #pragma unroll
           for (int xx = 0; xx < 2; ++xx) {
-            const int r = rt + 8 * xx + g;
-            const double xr = r < nm ? x[r] : 0.0;
+            const int r = rbeg + 16 * (rb0 + i) + 8 * xx + g;
+            const double xr = x[min(r, nm - 1)];
 #pragma unroll
-            for (int y = 0; y < 2; ++y)
-#pragma unroll
-              for (int h = 0; h < 2; ++h) {
-                const int c = cw + 8 * y + 2 * t + h;
-                if (inside || (r < nm && c < nm && c >= r)) {
-                  const double z = d[i][xx][y][h];
-                  M0[(long long)(16 * (rb0 + i) + 8 * xx) * n + 8 * y + h] = z;
-                  cs[2 * y + h] += z * xr;
-                  if (inside || c > r) rp[rb0 + i][xx] += z * x[c];
-                }
+            for (int k = 0; k < 4; ++k) {
+              const double z = d[i][xx][k];
+              if (cx[k] >= r) {
+                M0[(long long)(16 * (rb0 + i) + 8 * xx) * n + 8 * (k >> 1) + (k & 1)] = z;
+                cs[k] += z * xr;
               }
+              if (cx[k] > r) rp[rb0 + i][xx] += z * xc[k];
+            }
           }
-        }
       }
       // column sums over the eight row lanes g (lane bits 4, 3, 2): lane bit 4
       // ends with y, bit 3 with h
@@ -392,11 +371,12 @@ __device__ __forceinline__ double walk_gather(const double* part, int nm, int c,
   for (int j = 0; j < NJ; ++j) t += b[j];
   return t;
 }
-template <typename F>
+template <bool W, typename F>
 __device__ __forceinline__ double walk_gather(const double* part, int nm, int c, F between) {
-  if (nm <= kWalk1) return walk_gather<5, 5, parts(kWalk1, 5), parts(kWalk1, 5)>(part, nm, c, between);
-  if (nm <= kWalk2) return walk_gather<5, 6, parts(kWalk2, 5), parts(kWalk2, 6)>(part, nm, c, between);
-  return walk_gather<6, 7, parts(kSyevMaxN, 6), parts(kSyevMaxN, 7)>(part, nm, c, between);
+  if (nm <= kWalk1) return walk_gather<4, 5, parts(kWalk1, 4), parts(kWalk1, 5)>(part, nm, c, between);
+  if (nm <= kWalk2) return walk_gather<4, 6, parts(kWalk2, 4), parts(kWalk2, 6)>(part, nm, c, between);
+  if constexpr (!W) return 0.0;  // (the two-CTA kernel takes orders up to kWalk2 + 1: less code, 3% in a batch)
+  else return walk_gather<5, 7, parts(kSyevMaxN, 5), parts(kSyevMaxN, 7)>(part, nm, c, between);
 }
 
 // A (n x n, upper triangle used, row-major) to tridiagonal form: reflector k
@@ -439,7 +419,7 @@ __device__ __forceinline__ void tridiag_tiles(double* A, int n, double* d, doubl
         const double raw = rowr[j];
         // the open pairs' part of p and of row r, while the partials arrive
         double cp = 0.0, cx = 0.0;
-        const double sum = walk_gather(gs + ((r - 1) & 1) * half, mm, j, [&]() {
+        const double sum = walk_gather<W>(gs + ((r - 1) & 1) * half, mm, j, [&]() {
           for (int i = 0; i < np; ++i) {
             const double pv = PV[i * n + r + j], pw = PW[i * n + r + j];
             cp += pv * dot[i] + pw * dot[kPanel + i];
@@ -496,14 +476,13 @@ __device__ __forceinline__ void tridiag_tiles(double* A, int n, double* d, doubl
     double* Mb = A + (long long)(r + 1) * n + r + 1;
     double* out = gs + (r & 1) * half;
     if (np == kPanel) {
-      if (mr <= kWalk1) walk_close<5, 5, 2>(Mb, n, r + 1, mr, sm_off(PV), sm_off(vn), out, gw, ngw);
-      else if (mr <= kWalk2) walk_close<5, 6, 2>(Mb, n, r + 1, mr, sm_off(PV), sm_off(vn), out, gw, ngw);
-      else walk_close<6, 7, W ? 4 : 2>(Mb, n, r + 1, mr, sm_off(PV), sm_off(vn), out, gw, ngw);
+      if (mr <= kWalk2) walk_close<4, 1>(Mb, n, r + 1, mr, mr <= kWalk1 ? 5 : 6, sm_off(PV), sm_off(vn), out, gw, ngw);
+      else if constexpr (W) walk_close<5, 2>(Mb, n, r + 1, mr, 7, sm_off(PV), sm_off(vn), out, gw, ngw);
       np = 0;
     } else {
-      if (mr <= kWalk1) walk_read<5, 5, 32>(Mb, n, mr, sm_off(vn), out, gw, ngw);
-      else if (mr <= kWalk2) walk_read<5, 6, W ? 32 : 16>(Mb, n, mr, sm_off(vn), out, gw, ngw);
-      else walk_read<6, 7, W ? 16 : 8>(Mb, n, mr, sm_off(vn), out, gw, ngw);
+      if (mr <= kWalk1) walk_read<4, 5, W ? 16 : 16>(Mb, n, mr, sm_off(vn), out, gw, ngw);
+      else if (mr <= kWalk2) walk_read<4, 6, 16>(Mb, n, mr, sm_off(vn), out, gw, ngw);
+      else if constexpr (W) walk_read<5, 7, W ? 16 : 8>(Mb, n, mr, sm_off(vn), out, gw, ngw);
       // the next step's w_i . v and v_i . v, one warp each, in every CTA; the
       // last warps of the group first (the walk's units start at warp 0).  Two
       // buffers: a CTA one step behind may still read the other
@@ -541,25 +520,29 @@ __device__ __forceinline__ void formq_rows(double* Z, int n, int row0, int c0, i
   double* zr = Z + (long long)r * n + c0;
   double a0[2] = {0.0, 0.0}, a1[2] = {0.0, 0.0};  // Wm[g][8y + 2t], Wm[g][8y + 2t + 1]
   const double* Vg = Vs + g * mp + t;
-  for (int k0 = 0; k0 < m; k0 += 4 * U) {
+  int k0 = 0;
+  for (; k0 + 4 * U <= m; k0 += 4 * U) {
     __syncwarp();
     double z[U];
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int c = k0 + 4 * u + t;
-      z[u] = (valid && c < m) ? zr[c] : 0.0;
-    }
+    for (int u = 0; u < U; ++u) z[u] = valid ? zr[k0 + 4 * u + t] : 0.0;
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int k = k0 + 4 * u;
-      if (k >= m) break;
-      const bool in = k + t < m;
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int y = 0; y < 2; ++y) dmma(a0[y], a1[y], z[u], Vg[8 * y * mp + k0 + 4 * u]);
+  }
+  for (; k0 < m; k0 += 16) {  // the rest, four steps at a time (past column m: zeros times zeros)
+    __syncwarp();
+    double z[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) z[u] = (valid && k0 + 4 * u + t < m) ? zr[k0 + 4 * u + t] : 0.0;
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
 #pragma unroll
       for (int y = 0; y < 2; ++y) {
-        const double b = in ? Vg[8 * y * mp + k] : 0.0;
+        const double b = k0 + 4 * u + t < m ? Vg[8 * y * mp + k0 + 4 * u] : 0.0;
         dmma(a0[y], a1[y], z[u], b);
       }
-    }
   }
   // left-operand fragment s (columns 4s + t) of an 8 x 16 accumulator
   auto left = [&](const double* d0, const double* d1, int s) {
@@ -579,27 +562,46 @@ __device__ __forceinline__ void formq_rows(double* Z, int n, int row0, int c0, i
   for (int s = 0; s < 4; ++s) wf[s] = -left(w0, w1, s);
   const double* Vt = Vs + t * mp + g;
   constexpr int V = U / 2;  // 8-column fragments per round
-  for (int ct = 0; ct < m; ct += 8 * V) {
+  int ct = 0;
+  for (; ct + 8 * V <= m; ct += 8 * V) {
     __syncwarp();
     double d0[V], d1[V];
 #pragma unroll
     for (int y = 0; y < V; ++y) {
       const int c = ct + 8 * y + 2 * t;
+      d0[y] = valid ? zr[c] : 0.0;
+      d1[y] = valid ? zr[c + 1] : 0.0;
+    }
+#pragma unroll
+    for (int s = 0; s < 4; ++s)
+#pragma unroll
+      for (int y = 0; y < V; ++y) dmma(d0[y], d1[y], wf[s], Vt[4 * s * mp + ct + 8 * y]);
+    if (valid)
+#pragma unroll
+      for (int y = 0; y < V; ++y) {
+        const int c = ct + 8 * y + 2 * t;
+        zr[c] = d0[y];
+        zr[c + 1] = d1[y];
+      }
+  }
+  for (; ct < m; ct += 16) {
+    __syncwarp();
+    double d0[2], d1[2];
+#pragma unroll
+    for (int y = 0; y < 2; ++y) {
+      const int c = ct + 8 * y + 2 * t;
       d0[y] = (valid && c < m) ? zr[c] : 0.0;
       d1[y] = (valid && c + 1 < m) ? zr[c + 1] : 0.0;
     }
 #pragma unroll
-    for (int y = 0; y < V; ++y) {
-      if (ct + 8 * y >= m) break;
-      const bool in = ct + 8 * y + g < m;
+    for (int s = 0; s < 4; ++s)
 #pragma unroll
-      for (int s = 0; s < 4; ++s) {
-        const double b = in ? Vt[4 * s * mp + ct + 8 * y] : 0.0;
+      for (int y = 0; y < 2; ++y) {
+        const double b = ct + 8 * y + g < m ? Vt[4 * s * mp + ct + 8 * y] : 0.0;
         dmma(d0[y], d1[y], wf[s], b);
       }
-    }
 #pragma unroll
-    for (int y = 0; y < V; ++y) {
+    for (int y = 0; y < 2; ++y) {
       const int c = ct + 8 * y + 2 * t;
       if (valid && c < m) zr[c] = d0[y];
       if (valid && c + 1 < m) zr[c + 1] = d1[y];
@@ -1648,8 +1650,8 @@ __device__ __forceinline__ void syev_structure(const DevBatch& B, double* __rest
 }  // namespace
 
 // Two CTAs per SM (128 registers) for batches that fill the GPU with a CTA per
-// structure, one CTA per SM with whole units in registers for clusters and for
-// orders whose vectors take more than half an SM's shared memory.  Both run
+// structure of at most kWalk2 + 1 AOs, one CTA per SM with whole units in
+// registers for clusters and larger orders.  Both run
 // the same arithmetic in the same order.  (Three CTAs per SM at 80 registers
 // spilled in the walks and held 16 loads in flight per lane instead of 32:
 // 444 structures of 300 AOs took 4.1 ms of an SM each against 3.9.)
@@ -1724,7 +1726,7 @@ __global__ void __launch_bounds__(kEigThreads, 2) k_syev_small(DevBatch B, const
       const double dj = d[j];
       rank += (dj < di || (dj == di && j < i)) ? 1 : 0;
     }
-    if (!TB_GUARD(11, rank, 0, n)) continue;
+    if (!TB_GUARD(9, rank, 0, n)) continue;
     perm[vo + rank] = i;
     wout[vo + rank] = di;
   }
@@ -1733,13 +1735,14 @@ __global__ void __launch_bounds__(kEigThreads, 2) k_syev_small(DevBatch B, const
 TB_OOB_EXPORT(oob_syev)
 
 namespace {
-// Time of one structure of n AOs on a group of C CTAs, in ms: what the CTAs
-// divide, plus what each repeats or waits for (the steps' barriers, gathers
-// and scalars, a merge's sort and scan).  Measured on one structure alone:
-// 1.6, 9.4, 44, 161 ms at 138, 384, 722, 1196 AOs on one CTA; 1.2, 5.9, 25.5,
-// 88 on two; 1.1, 4.2, 15.6, 52 on four; 1.1, 3.5, 11.3, 34 on eight.
+// Time of one structure of n AOs on a group of C CTAs, in ms: what each CTA
+// repeats or waits for (the steps' barriers, gathers and scalars, a merge's
+// sort and scan), plus what they divide.  Measured on one structure alone with
+// one CTA per SM, at 138, 384, 722, 1196 AOs: 1.1, 7.8, 41, 156 ms on one CTA;
+// 0.85, 4.8, 23, 84 on two; 0.72, 3.3, 13.5, 47 on four; 0.75, 2.6, 9.0, 29 on
+// eight; 0.74, 2.5, 7.2, 20 on sixteen.
 double syev_ms(double n, int C) {
-  const double serial = n * (6.0e-3 + 6.0e-6 * n), shared = n * n * (3.0e-5 + 6.0e-8 * n);
+  const double serial = n * (4.6e-3 + 2.05e-6 * n), shared = n * n * (6.6e-6 + 8.55e-8 * n);
   return serial + shared / C;
 }
 }  // namespace
@@ -1751,7 +1754,8 @@ double syev_ms(double n, int C) {
 // structures.  Two CTAs on an SM slow each other (kSlowTwo; the narrower
 // kernel alone, kSlowNarrow).  400 water clusters of 48..384 AOs: 13.3 ms on
 // one CTA each, 11.0 on two; 128: 11.1 and 6.2 (on four); 48 chains of
-// 122..1196 AOs: 172 and 40 (on eight).  Batches of several waves of CTAs keep
+// 122..1196 AOs: 172 and 40 (on eight) -- with the walks before their one
+// comparison per entry; the ratios since are the same.  Batches of several waves of CTAs keep
 // one CTA per structure: clusters repeat work and would only lose.
 ClusterChoice choose_clusters(const std::vector<int>& sizes, int first, int last, double (*ms)(double, int),
                               bool two_per_sm, bool one_per_sm) {
@@ -1775,12 +1779,12 @@ ClusterChoice choose_clusters(const std::vector<int>& sizes, int first, int last
     }
     return end;
   };
-  constexpr int kCap[2][4] = {{148, 74, 33, 15}, {296, 148, 71, 33}};
+  constexpr int kCap[2][5] = {{148, 74, 33, 15, 7}, {296, 148, 71, 33, 14}};
   constexpr double kSlowTwo = 1.42, kSlowNarrow = 1.1;
   const int cnt = last - first;
   best.span = 1e300;
   for (int per = two_per_sm ? 2 : 1; per >= (one_per_sm ? 1 : 2); --per)
-    for (int c = 0; c < 4; ++c) {
+    for (int c = 0; c < 5; ++c) {
       const int C = 1 << c;
       if (C > 1 && cnt > 4 * 148) break;
       for (int k = cnt; k >= 1; k = k > 1 ? (3 * k) / 4 : 0) {
@@ -1805,7 +1809,7 @@ void SyevPlan::build(const std::vector<int>& sizes, int lib_above, int jacobi_ma
     else if (n > jacobi_max) { ++nsmall; small_max = std::max(small_max, n); }
   }
   if (n64 > first)
-    c = choose_clusters(sizes, first, n64, syev_ms, syev_smem_bytes(nmax) <= kSyevSmemTwo, true);
+    c = choose_clusters(sizes, first, n64, syev_ms, nmax <= kWalk2 + 1, true);
 }
 
 cudaError_t launch_syev(const SyevPlan& P, const DevBatch& B, double* A, double* Z, double* Sb, double* w, int* perm,
