@@ -1106,7 +1106,7 @@ constexpr double kMixedSwitchScale = 10.0, kMixedSwitchFloorE = 1e-5, kMixedSwit
 // Eigen-decomposition and density of one SCF iteration in the mixed-precision
 // form (tb_mixed.cu).  Every matrix is stored in FP64.  Structures in the
 // mixed phase: F', C and P as TF32x3 tensor-core GEMMs (k_gemm_tc, tcgen05),
-// eigenpairs from the FP32 eigensolver and one FP64 Ogita-Aishima refinement
+// eigenpairs from an FP32 reduction and one FP64 Ogita-Aishima refinement
 // step.  Structures in the FP64 phase (the final iterations) run the plain
 // form's FP64 iteration: FP64 GEMMs and the FP64 eigensolver, so the
 // converged result carries no FP32 error.  Leaves w, focc, kdim and P as the
@@ -1130,10 +1130,19 @@ tb_status mixed_core(tb_batch* b, cudaStream_t st, double n3_lo, double n3_hi, d
   TB_K("gemm_tc", 2.0 * n3_lo, 1,
        k_gemm_tc<<<tc_grid, kTcThreads, tc_smem, st>>>(B, T128, nt128, b->X, 1, b->W, 0, nullptr, nullptr, nullptr, b->F, 1.0, 0.0, lo, S.status));
   TB_GEMM(2.0 * n3_hi, b->X, 1, b->W, 0, nullptr, nullptr, nullptr, b->F, 1.0, 0.0, hi, kGemmKUpToI | kGemmSym);
-  // mixed phase: FP32 eigensolve
+  // mixed phase: FP32 reduction, then the tridiagonal problem through k_syev
+  // (eigenvectors as rows of Vn; G and W are its scratch); structures below
+  // kDcMin AOs through the small FP64 kernels
   TB_K("convert", 0, 0, k_to_f32<<<gemm_grid, 256, 0, st>>>(B, T, nt, b->F, b->Af, lo));
   TB_K("syev_f32", 4.0 * n3_lo, 1,
-       k_syev_f32<<<nmol, kEigThreads, smem32, st>>>(B, b->Af, b->Zf, b->w, b->perm, S.status, lo));
+       k_reduce_f32<<<nmol, kEigThreads, smem32, st>>>(B, b->Af, b->Zf, b->Vn, b->W, S.status, lo));
+  TB_K("syev_f32", 0.0, 1,
+       TB_CUDA(launch_syev(b->syev, B, b->G, b->Vn, b->W, b->w, b->perm, S.status, lo, st, &b->launches, true, b->F)));
+  --b->launches;  // launch_syev has counted
+  if (b->njac > 0)
+    TB_K("syev_jacobi", 0, 0,
+         k_syev_jacobi<<<nblk(b->njac, kJacobiWarps), kJacobiWarps * 32, jacobi_smem_bytes(), st>>>(
+             B, b->F, b->Vn, b->w, b->perm, S.status, lo, b->d_jlist, b->njac));
   // FP64 phase: the FP64 eigensolver (eigenvectors as rows of Z, W as its scratch)
   {
     const tb_status ts = launch_trid_plan(b, hi, st);
@@ -1166,7 +1175,7 @@ tb_status mixed_core(tb_batch* b, cudaStream_t st, double n3_lo, double n3_hi, d
   // mixed phase: one FP64 refinement step (GEMMs included) of the FP32
   // eigenvectors, gathered into FP64 columns in ascending order (Z -> Vn)
   const size_t oa_smem = oa_smem_bytes(b->nmax);
-  TB_K("refine", 0, 0, k_gather_vectors<<<gemm_grid, 256, 0, st>>>(B, T, nt, b->Zf, b->perm, b->Z, lo));
+  TB_K("refine", 0, 0, k_gather_vectors<<<gemm_grid, 256, 0, st>>>(B, T, nt, b->Zf, b->Vn, b->perm, b->Z, lo));
   {
     double* V = b->Z;
     double* Vo = b->Vn;
@@ -1203,7 +1212,7 @@ tb_status raise_smem_limits() {
   int dev = 0, optin = 0;
   TB_CUDA(cudaGetDevice(&dev));
   TB_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-  const void* ks[] = {(const void*)k_factor, (const void*)k_syev, (const void*)k_syev_wide, (const void*)k_syev_small, (const void*)k_syev_f32, (const void*)k_fermi, (const void*)k_oa_step,
+  const void* ks[] = {(const void*)k_factor, (const void*)k_syev, (const void*)k_syev_wide, (const void*)k_syev_small, (const void*)k_reduce_f32, (const void*)k_fermi, (const void*)k_oa_step,
                       (const void*)k_gemm_tc, (const void*)k_fock, (const void*)k_syev_jacobi};
   for (const void* k : ks) {
     cudaFuncAttributes a;

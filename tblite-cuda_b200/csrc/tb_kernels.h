@@ -9,7 +9,7 @@
 namespace tb {
 
 constexpr int kEigThreads = 256;
-constexpr int kRing = 8;  // QL sweeps buffered between the k_syev producer and consumers
+constexpr int kRing = 8;  // n-vectors of the open panel, twice (v_i and w_i)
 // k_syev's divide and conquer: structures of kDcMin+ rows (more than two leaves of
 // 24), merge products in 64 x 64 tiles with reduction slabs of kDcK (Wt 64 x kDcK,
 // Bt kDcK x kDcBs, rows padded by 4 against bank conflicts)
@@ -22,7 +22,7 @@ template <typename T>
 __host__ __device__ constexpr int dc_ws_elems(int m) {
   return 8 * m + kDcTileElems + (7 * m * (int)sizeof(int) + (int)sizeof(T) - 1) / (int)sizeof(T);
 }
-// shared memory of k_syev: d, e, tau, v, vn, p, w (7n) + the rotation ring (2 n kRing);
+// shared memory of k_syev: d, e, tau, v, vn, p, w (7n) + the open panel's pairs (2 n kRing);
 // in FP64 at least d, e and the divide-and-conquer workspace (from tau on) for
 // kDcMin+ rows, so that the solver chosen for a structure depends on its size only
 inline size_t syev_smem_bytes(int n, size_t elem = sizeof(double)) {
@@ -179,10 +179,12 @@ __global__ void k_gemm32(DevBatch B, const int4* tiles, int ntiles, const double
 // FP64 eigensolver (tb_syev.cu; structures of kDcMin+ AOs): Sb an n x n scratch
 // per structure (same offsets as Ab); the grid is clusters of C CTAs, the first
 // ncoop of them each on one structure, then one structure per CTA (SyevPlan)
+// given: the tridiagonal problem is in Sb (d | e, 2n entries) and Q^T in Zb; Ab is
+// scratch
 __global__ void k_syev(DevBatch B, double* Ab, double* Zb, double* Sb, double* wout, int* perm, int* status,
-                       const int* active, int ncoop);
+                       const int* active, int ncoop, int given);
 __global__ void k_syev_wide(DevBatch B, double* Ab, double* Zb, double* Sb, double* wout, int* perm, int* status,
-                            const int* active, int ncoop);
+                            const int* active, int ncoop, int given);
 struct SyevPlan {
   int n64 = 0;          // structures of kDcMin+ AOs on the in-house solver lead the order
   int nsmall = 0, small_max = 1;  // structures below kDcMin AOs that k_syev_small solves, the largest
@@ -192,9 +194,11 @@ struct SyevPlan {
   void build(const std::vector<int>& sizes, int lib_above, int jacobi_max);
 };
 // k_syev (and k_syev_small where the plan has small structures) on st; *launches
-// counts them.  The shared-memory limits must have been raised.
+// counts them.  The shared-memory limits must have been raised.  given (see
+// k_syev): A is scratch and the small structures' matrices are in Asmall.
 cudaError_t launch_syev(const SyevPlan& P, const DevBatch& B, double* A, double* Z, double* Sb, double* w, int* perm,
-                        int* status, const int* active, cudaStream_t st, int64_t* launches);
+                        int* status, const int* active, cudaStream_t st, int64_t* launches, bool given = false,
+                        const double* Asmall = nullptr);
 // FP64 structures below kDcMin AOs, one CTA each in shared memory: B.order
 // from position `first` on; dynamic shared memory small_smem_bytes(largest)
 constexpr int kSmallLeaf = 16;  // leaves of its merge tree
@@ -208,8 +212,11 @@ __host__ __device__ constexpr int small_ws_elems(int n) {  // merge workspace; t
 inline size_t small_smem_bytes(int n) { return (3 * (size_t)n * small_ld(n) + 3 * n + small_ws_elems(n)) * sizeof(double); }
 __global__ void k_syev_small(DevBatch B, const double* Ab, double* Zb, double* wout, int* perm, int* status,
                              const int* active, int first);
-// the same eigensolver in FP32 (A and Z float, eigenvalues written as double)
-__global__ void k_syev_f32(DevBatch B, float* Ab, float* Zb, double* wout, int* perm, int* status, const int* active);
+// mixed form, structures of kDcMin+ AOs: reduction to tridiagonal form and Q in
+// FP32; Q^T in FP64 into Zd, d | e into the first 2n entries of Sd (k_syev with
+// `given` takes them from there)
+__global__ void k_reduce_f32(DevBatch B, float* Ab, float* Zb, double* Zd, double* Sd, const int* status,
+                             const int* active);
 // small-structure variant: one warp per structure of N <= kJacobiMaxN (cyclic Jacobi
 // in shared memory), structures list[0..nlist), kJacobiWarps structures per CTA;
 // same outputs as k_syev (w ascending, eigenvector j = row perm[j] of Z)
@@ -231,8 +238,8 @@ __global__ void k_gemm_tc(DevBatch B, const int4* tiles, int ntiles, const doubl
                           double beta, const int* active, int* status);
 size_t gemm_tc_smem_bytes();
 __global__ void k_to_f32(DevBatch B, const int4* tiles, int ntiles, const double* F, float* Af, const int* mask);
-__global__ void k_gather_vectors(DevBatch B, const int4* tiles, int ntiles, const float* Zf, const int* perm,
-                                 double* V, const int* mask);
+__global__ void k_gather_vectors(DevBatch B, const int4* tiles, int ntiles, const float* Zf, const double* Zd,
+                                 const int* perm, double* V, const int* mask);
 // refinement step (Rayleigh-Ritz in clusters + Ogita-Aishima coefficients)
 constexpr int kClusterMax = 64;
 inline size_t oa_smem_bytes(int nmax) {

@@ -1,9 +1,7 @@
 // Batched FP64 dense linear algebra for uneven structure sizes:
 //  * k_gemm: C = alpha op(A) diag(ks) op(B) + beta C over a tile list;
-//  * k_syev_f32: the mixed form's FP32 eigensolver, one CTA per structure
-//    (Householder tridiagonalisation, explicit Q, implicit QL with the
-//    rotations of each sweep applied to the eigenvector rows by all threads,
-//    rank-based sort); FP64: tb_syev.cu, and k_syev_jacobi here.
+//  * k_reduce_f32: the mixed form's FP32 reduction to tridiagonal form and Q;
+//    FP64 eigensolver: tb_syev.cu, and k_syev_jacobi here.
 // Together with k_factor (tb_factor.cu) these give sygvd (itype 1, jobz 'V'; reference src/lapack/sygvd.h:4-23):
 // H C = S C e  <=>  (X^T H X) Z = Z e, C = X Z.
 #include "tb_common.cuh"
@@ -215,10 +213,8 @@ __global__ void __launch_bounds__(kGemmThreads) k_gemm32(DevBatch B, const int4*
 }
 
 // ------------------------------------------------------------ eigensolver
-// FP32 symmetric eigenproblem (mixed form; FP64: tb_syev.cu) of A (n x n,
-// row-major, overwritten) for every active structure, one CTA of 256 threads per structure: w ascending,
-// eigenvector j = row perm[j] of Zc (n x n, one eigenvector per row).
-//
+// FP32 reduction of the mixed form's eigensolve (FP64: tb_syev.cu) of A (n x n,
+// row-major, overwritten), one CTA of 256 threads per structure:
 //  1. Householder tridiagonalisation in panels (tridiagonalise): within a
 //     panel the trailing block keeps its value from the panel start, each
 //     step forms its product with one read-only walk (colwalk, row segments)
@@ -227,11 +223,10 @@ __global__ void __launch_bounds__(kGemmThreads) k_gemm32(DevBatch B, const int4*
 //     product.  Reflector k is kept in row k of A.
 //  2. Zc = Q^T accumulated backwards in compact-WY blocks of kQBlock
 //     reflectors (form_q).
-//  3. Tridiagonal eigenproblem: implicit QL with Wilkinson shift (warp 0 runs
-//     the rotation chain, warps 1.. apply sweeps to Zc through a kRing-slot
-//     shared-memory ring; every wait is bounded, on timeout the structure is
-//     marked failed).
-//  4. Ascending order by rank (ties by index).
+// The tridiagonal problem and the product with Q go through k_syev's divide
+// and conquer: implicit QL on one CTA, a serial chain of rotations applied to
+// FP32 vectors, was more than half of the eigensolve (9.1 ms of a launch over
+// 64 clusters of 48..384 AOs), and FP32 merges cost an SCF iteration.
 namespace {
 
 // Tridiagonalisation panel: reflectors per panel (2 panel n <= ring) and rows
@@ -248,22 +243,8 @@ constexpr int kWalkRowGroups = 4;
 template <typename T> struct WalkCfg { static constexpr int cols = 3, rows = 4; };
 static_assert(PanelCfg<float>::width <= kRing, "panel exceeds the ring");
 constexpr int kQBlock = 16;     // reflectors per compact-WY block of the Q accumulation
-constexpr int kWaveK = 4;            // QL sweeps applied per pass over Zc
-constexpr int kWin = 2 * kWaveK;     // rows of Zc in flight per column
-constexpr long long kSpinLimit = 1LL << 24;
 
-template <typename T> struct Eps;
-template <> struct Eps<float> { static constexpr float v = 1.1920929e-07f; };
 __device__ inline float tb_sqrt(float x) { return sqrtf(x); }
-__device__ inline float tb_abs(float x) { return fabsf(x); }
-// one Newton step y(3 - x y^2)/2 on the hardware estimate keeps Givens pairs orthogonal to ~1 ulp
-__device__ inline float tb_rsqrt(float x) {
-  const float y = rsqrtf(x);
-  return y * (1.5f - 0.5f * x * y * y);
-}
-
-// reciprocal square root on the QL rotation chain (one Newton step on the estimate)
-__device__ inline float chain_rsqrt(float x) { return tb_rsqrt(x); }
 
 template <typename T>
 __device__ inline T block_sum_syev(T v, T* red) { return block_sum(v, red); }
@@ -411,7 +392,7 @@ __device__ __noinline__ void panel_walk(T* M, int n, int r0, int nm, const T* PV
   }
 }
 
-// Phase 1 of syev_body: A (n x n, symmetric, row-major) is reduced to
+// Phase 1 of k_reduce_f32: A (n x n, symmetric, row-major) is reduced to
 // tridiagonal form in place; reflector k is stored in row k of A from column
 // k+1 on (leading 1), its scale in tau[k], the off-diagonal in e.  Out of line
 // so that its registers are allocated apart from the later phases.
@@ -541,7 +522,7 @@ __device__ __noinline__ void tridiagonalise(T* A, int n, T* e, T* tau, T* v, T* 
   }
 }
 
-// Phase 2 of syev_body: Z = Q^T from the reflectors left in A and tau by
+// Phase 2 of k_reduce_f32: Z = Q^T from the reflectors left in A and tau by
 // tridiagonalise.  ring: kQBlock x n of shared memory.  Out of line like phase 1.
 template <typename T>
 __device__ __noinline__ void form_q(const T* A, T* Z, int n, const T* tau, T* ring) {
@@ -637,261 +618,55 @@ __device__ __noinline__ void form_q(const T* A, T* Z, int n, const T* tau, T* ri
 
 }
 
-template <typename T>
-__device__ __forceinline__ void syev_body(const DevBatch& B, T* __restrict__ Ab, T* __restrict__ Zb,
-                                          double* __restrict__ wout, int* __restrict__ perm,
-                                          int* __restrict__ status, const int* __restrict__ active) {
+}  // namespace
+
+// Structures of kDcMin+ AOs: reflectors and Q in FP32; Q^T (in FP64) into Zd, the
+// diagonal and off-diagonal into the first 2n entries of the scratch Sd, from
+// where k_syev takes the tridiagonal problem.
+__global__ void __launch_bounds__(kEigThreads, 4) k_reduce_f32(DevBatch B, float* __restrict__ Ab,
+                                                            float* __restrict__ Zb, double* __restrict__ Zd,
+                                                            double* __restrict__ Sd, const int* __restrict__ status,
+                                                            const int* __restrict__ active) {
   const int m = B.order ? B.order[blockIdx.x] : blockIdx.x;  // largest structures first
   if (active && !active[m]) return;
   if (status[m] != kStOk) return;
   const int n = B.ooff[m + 1] - B.ooff[m];
-  if (on_library(B, n)) return;
+  if (on_library(B, n) || n < kDcMin) return;
   const long long mo = B.moff[m];
-  const long long vo = B.ooff[m];
-  T* A = Ab + mo;
-  T* Z = Zb + mo;
-  extern __shared__ __align__(16) unsigned char syev_smem[];
-  T* sm = reinterpret_cast<T*>(syev_smem);
-  T* d = sm;          // n
-  T* e = d + n;       // n
-  T* tau = e + n;     // n
-  T* v = tau + n;     // n
-  T* vn = v + n;      // n
-  T* p = vn + n;      // n
-  T* w = p + n;       // n
-  T* ring = w + n;    // kRing slots x (n cosines + n sines)
-  __shared__ T red[kEigThreads / 32];
-  __shared__ T sh[4];
-  __shared__ int q_full, q_end, q_fail, sh_head[kRing][2];
-  __shared__ int q_done[kEigThreads / 32];  // sweeps finished, per consumer warp
+  float* A = Ab + mo;
+  float* Z = Zb + mo;
+  extern __shared__ __align__(16) float reduce_sm[];
+  float* d = reduce_sm;  // n
+  float* e = d + n;      // n
+  float* tau = e + n;    // n
+  float* v = tau + n;    // n
+  float* vn = v + n;     // n
+  float* p = vn + n;     // n
+  float* w = p + n;      // n
+  float* ring = w + n;   // kQBlock x n
+  __shared__ float red[kEigThreads / 32];
+  __shared__ float sh[4];
   const int tid = threadIdx.x, nt = blockDim.x;
-
   // symmetrise
   for (int i = tid >> 5; i < n; i += nt >> 5)
     for (int j = i + 1 + (tid & 31); j < n; j += 32) {
-      const T s = T(0.5) * (A[(long long)i * n + j] + A[(long long)j * n + i]);
+      const float s = 0.5f * (A[(long long)i * n + j] + A[(long long)j * n + i]);
       A[(long long)i * n + j] = s;
       A[(long long)j * n + i] = s;
     }
-  for (int i = tid; i < n; i += nt) { e[i] = T(0); tau[i] = T(0); }
+  for (int i = tid; i < n; i += nt) { e[i] = 0.0f; tau[i] = 0.0f; }
   __syncthreads();
   // d: scratch until the end
-  tridiagonalise<T>(A, n, e, tau, v, vn, p, w, d, ring, red, sh);
-  for (int i = tid; i < n; i += nt) d[i] = A[(long long)i * n + i];
-  if (tid == 0 && n >= 2) e[n - 2] = A[(long long)(n - 2) * n + n - 1];
-  __syncthreads();
-
-  form_q<T>(A, Z, n, tau, ring);
-
-  // ---- 3. implicit QL, producer (warp 0) / consumers (warps 1..)
-  if (tid == 0) { q_full = 0; q_end = 0; q_fail = 0; e[n - 1] = T(0); }
-  if (tid < kEigThreads / 32) q_done[tid] = 0;
-  __syncthreads();
-  const int ncons = (nt >> 5) - 1;
-  if (tid < 32) {
-    // producer warp: the deflation scan is warp-parallel (ballot over 32
-    // consecutive indices), the rotation chain runs on lane 0
-    const int lane = tid;
-    const T eps = Eps<T>::v;
-    int q = 0;
-    bool fail = false;
-    for (int l = 0; l < n && !fail; ++l) {
-      int iter = 0;
-      for (;;) {
-        int mq = n - 1;
-        for (int base = l; base < n - 1; base += 32) {
-          const int i = base + lane;
-          bool small = false;
-          if (i < n - 1) {
-            const T dd = tb_abs(d[i]) + tb_abs(d[i + 1]);
-            small = tb_abs(e[i]) <= eps * dd;
-          }
-          const unsigned bal = __ballot_sync(0xffffffffu, small);
-          if (bal) { mq = base + __ffs(bal) - 1; break; }
-        }
-        if (mq == l) break;
-        if (++iter > 60) { fail = true; break; }
-        // the ring slot of sweep q held sweep q-kRing: wait until EVERY consumer
-        // warp has finished it (warps progress unevenly)
-        const int slot = q % kRing;
-        if (q >= kRing) {
-          if (lane == 0) {
-            long long spins = 0;
-            for (int cw = 1; cw <= ncons && !fail; ++cw)
-              while (*(volatile int*)&q_done[cw] < q - kRing + 1) {
-                if (++spins > kSpinLimit) { fail = true; break; }
-                __nanosleep(64);
-              }
-          }
-          fail = __shfl_sync(0xffffffffu, fail, 0);
-          if (fail) break;
-          __threadfence_block();
-        }
-        if (lane == 0) {
-          T* rc = ring + (size_t)slot * 2 * n;
-          T* rs = rc + n;
-          T g = (d[l + 1] - d[l]) / (T(2) * e[l]);
-          T r = tb_sqrt(g * g + T(1));
-          g = d[mq] - d[l] + e[l] / (g + (g >= T(0) ? r : -r));
-          T s = T(1), c = T(1), pp = T(0);
-          int cnt = 0;
-          bool underflow = false;
-          // d[i+1], d[i], e[i] of the current rotation are carried in registers
-          // and the next rotation's d[i-1], e[i-1] are loaded one step ahead, so
-          // no shared-memory latency sits on the dependency chain (the sweep
-          // writes only d[i+1] and e[i+1], never an entry still to be read).
-          T dn = d[mq], di = d[mq - 1], ei = e[mq - 1];
-          for (int i = mq - 1; i >= l; --i) {
-            const T di_next = i > l ? d[i - 1] : T(0);
-            const T ei_next = i > l ? e[i - 1] : T(0);
-            const T f = s * ei;
-            const T bb = c * ei;
-            const T rr2 = f * f + g * g;
-            if (rr2 == T(0)) { d[i + 1] = dn - pp; e[mq] = T(0); underflow = true; break; }
-            const T ri = chain_rsqrt(rr2);
-            r = rr2 * ri;
-            e[i + 1] = r;
-            s = f * ri;
-            c = g * ri;
-            g = dn - pp;
-            r = (di - g) * s + T(2) * c * bb;
-            pp = s * r;
-            d[i + 1] = g + pp;
-            g = c * r - bb;
-            rc[cnt] = c;
-            rs[cnt] = s;
-            ++cnt;
-            dn = di;
-            di = di_next;
-            ei = ei_next;
-          }
-          if (!underflow) { d[l] -= pp; e[l] = g; e[mq] = T(0); }
-          sh_head[slot][0] = mq;
-          sh_head[slot][1] = cnt;
-          __threadfence_block();
-          *(volatile int*)&q_full = q + 1;
-        }
-        __syncwarp();  // d and e of this sweep are visible to the whole warp
-        ++q;
-      }
-    }
-    if (lane == 0) {
-      if (fail) *(volatile int*)&q_fail = 1;
-      __threadfence_block();
-      *(volatile int*)&q_end = 1;
-    }
-  } else {
-    // consumers: every column r of Zc owned by this thread (r = tid - 32 + k*(nt-32)).
-    // Sweeps are taken in groups of kWaveK and applied as a wavefront: sweep k
-    // of the group lags sweep k-1 by two rows, so each column streams through
-    // a window of 2*kWaveK rows held in registers and every element is loaded
-    // and stored once per group instead of once per sweep.
-    const int lane = tid & 31;
-    int q0 = 0;
-    for (;;) {
-      long long spins = 0;
-      int full;
-      bool quit = false;
-      while ((full = *(volatile int*)&q_full) < q0 + kWaveK) {
-        if (*(volatile int*)&q_end) {
-          __threadfence_block();
-          full = *(volatile int*)&q_full;
-          if (full <= q0) quit = true;
-          break;
-        }
-        if (++spins > kSpinLimit) { *(volatile int*)&q_fail = 1; quit = true; break; }
-        __nanosleep(32);
-      }
-      if (quit) break;
-      __threadfence_block();
-      const int kg = min(kWaveK, full - q0);
-      int mk[kWaveK], lk[kWaveK];
-      const T* ck[kWaveK];
-      int mx = 0, lmin = n;
-#pragma unroll
-      for (int k = 0; k < kWaveK; ++k) {
-        const int slot = (q0 + k) % kRing;
-        ck[k] = ring + (size_t)slot * 2 * n;
-        if (k < kg) {
-          mk[k] = sh_head[slot][0];
-          lk[k] = mk[k] - sh_head[slot][1];
-          mx = max(mx, mk[k]);
-          lmin = min(lmin, lk[k]);
-        } else {
-          mk[k] = -1;  // inactive: no index satisfies lk <= i <= mk - 1
-          lk[k] = 0;
-        }
-      }
-      const int J = mx - lmin + 2 * (kg - 1);
-      const int nblk = (J + kWin - 1) / kWin;
-      for (int r = tid - 32; r < n; r += nt - 32) {
-        T* zr = Z + r;
-        T wv[kWin];
-        wv[0] = T(0);
-#pragma unroll
-        for (int a = 1; a < kWin; ++a) {
-          const int row = mx - 1 + a;
-          wv[a] = row <= n - 1 ? zr[(long long)row * n] : T(0);
-        }
-        for (int blk = 0; blk < nblk; ++blk) {
-#pragma unroll
-          for (int p = 0; p < kWin; ++p) {
-            const int j = blk * kWin + p;
-            const int sl = (kWin - p) % kWin;
-            const int row_out = mx + kWin - 1 - j;
-            if (j >= 1 && row_out >= 0 && row_out <= n - 1) zr[(long long)row_out * n] = wv[sl];
-            const int row_in = mx - 1 - j;
-            wv[sl] = row_in >= 0 ? zr[(long long)row_in * n] : T(0);
-#pragma unroll
-            for (int k = 0; k < kWaveK; ++k) {
-              const int i = mx - 1 - j + 2 * k;
-              if (i >= lk[k] && i <= mk[k] - 1) {
-                const int t = mk[k] - 1 - i;
-                const T c = ck[k][t], sn = ck[k][n + t];
-                const int ia = (2 * k - p + 2 * kWin) % kWin, ib = (2 * k + 1 - p + 2 * kWin) % kWin;
-                const T x = wv[ia], y = wv[ib];
-                wv[ib] = sn * x + c * y;
-                wv[ia] = c * x - sn * y;
-              }
-            }
-          }
-        }
-        // flush the final window (last step has phase kWin - 1)
-        const int jl = nblk * kWin - 1;
-#pragma unroll
-        for (int a = 0; a < kWin; ++a) {
-          const int row = mx - 1 - jl + a;
-          if (row >= 0 && row <= n - 1) zr[(long long)row * n] = wv[(a + 1) % kWin];
-        }
-      }
-      __syncwarp();
-      q0 += kg;
-      if (lane == 0) {
-        __threadfence_block();
-        *(volatile int*)&q_done[tid >> 5] = q0;
-      }
-    }
-  }
-  __syncthreads();
-  if (q_fail) {
-    if (tid == 0) status[m] = kStEigenFailed;  // k_fermi retires the structure
-    return;
-  }
-  // ---- 4. ascending order by rank (ties by index)
+  tridiagonalise<float>(A, n, e, tau, v, vn, p, w, d, ring, red, sh);
   for (int i = tid; i < n; i += nt) {
-    const T di = d[i];
-    int rank = 0;
-    for (int j = 0; j < n; ++j) {
-      const T dj = d[j];
-      rank += (dj < di || (dj == di && j < i)) ? 1 : 0;
-    }
-    if (!TB_GUARD(9, rank, 0, n)) continue;
-    perm[vo + rank] = i;
-    wout[vo + rank] = di;
+    Sd[mo + i] = A[(long long)i * n + i];
+    Sd[mo + n + i] = i == n - 2 ? A[(long long)i * n + n - 1] : e[i];
   }
+  form_q<float>(A, Z, n, tau, ring);
+  __syncthreads();
+  for (int i = tid >> 5; i < n; i += nt >> 5)
+    for (int j = tid & 31; j < n; j += 32) Zd[mo + (long long)i * n + j] = Z[(long long)i * n + j];
 }
-
-}  // namespace
 
 TB_OOB_EXPORT(oob_linalg)
 
@@ -1013,13 +788,6 @@ __global__ void __launch_bounds__(kJacobiWarps * 32) k_syev_jacobi(DevBatch B, d
     perm[vo + rank] = lane;
     wout[vo + rank] = di;
   }
-}
-
-__global__ void __launch_bounds__(kEigThreads, 4) k_syev_f32(DevBatch B, float* __restrict__ Ab,
-                                                          float* __restrict__ Zb, double* __restrict__ wout,
-                                                          int* __restrict__ perm, int* __restrict__ status,
-                                                          const int* __restrict__ active) {
-  syev_body<float>(B, Ab, Zb, wout, perm, status, active);
 }
 
 }  // namespace tb

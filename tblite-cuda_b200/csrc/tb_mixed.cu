@@ -7,9 +7,11 @@
 //  * FP64 (1): entered once the mixed phase meets the (loosened) convergence
 //    test; the same contractions as FP64 GEMMs.  A structure retires only
 //    after at least two FP64 iterations and the full-accuracy convergence test.
-// In both phases the eigensolve is the FP32 k_syev_f32 (whose vectors are
-// orthogonal to about n * 1e-7) followed by FP64 refinement of the eigenpairs,
-// GEMMs included: one step in the mixed phase, two in the FP64 phase.  A step
+// The mixed phase reduces F' to tridiagonal form and accumulates Q in FP32
+// (k_reduce_f32; vectors orthogonal to about n * 1e-7), solves the tridiagonal
+// problem in FP64 (k_syev) and refines the eigenpairs by one FP64 step, GEMMs
+// included; structures below kDcMin AOs go through the small FP64 solvers, and
+// the FP64 phase through the FP64 eigensolver alone.  A step
 // is Ogita-Aishima iterative refinement (T. Ogita, K. Aishima, Japan J.
 // Indust. Appl. Math. 35 (2018) 1007-1035, algorithm RefSyEv) with an exact
 // Rayleigh-Ritz solve inside clusters of near-degenerate eigenvalues (their
@@ -55,10 +57,12 @@ __global__ void k_to_f32(DevBatch B, const int4* __restrict__ tiles, int ntiles,
   }
 }
 
-// V[i][j] = Zf[perm[j]][i] in FP64: eigenvector j (ascending) as column j.
+// V[i][j] = Z[perm[j]][i]: eigenvector j (ascending) as column j, from the
+// library's FP32 rows (Zf) or the in-house solver's FP64 rows (Zd).
 __global__ void k_gather_vectors(DevBatch B, const int4* __restrict__ tiles, int ntiles, const float* __restrict__ Zf,
-                                 const int* __restrict__ perm, double* __restrict__ V, const int* __restrict__ mask) {
-  __shared__ float tile[32][33];
+                                 const double* __restrict__ Zd, const int* __restrict__ perm,
+                                 double* __restrict__ V, const int* __restrict__ mask) {
+  __shared__ double tile[32][33];
   for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
     const int4 tl = tiles[t];
     const int m = tl.x;
@@ -66,6 +70,7 @@ __global__ void k_gather_vectors(DevBatch B, const int4* __restrict__ tiles, int
     const int n = B.ooff[m + 1] - B.ooff[m];
     const long long mo = B.moff[m];
     const int* pm = perm + B.ooff[m];
+    const bool lib = on_library(B, n);
     // the 64 x 64 tile as four 32 x 32 transposes
     for (int q = 0; q < 4; ++q) {
       const int i0 = tl.y * MT + 32 * (q >> 1), j0 = tl.z * MT + 32 * (q & 1);
@@ -73,13 +78,14 @@ __global__ void k_gather_vectors(DevBatch B, const int4* __restrict__ tiles, int
       for (int e = threadIdx.x; e < 32 * 32; e += blockDim.x) {
         const int jj = e / 32, ii = e % 32;  // row perm[j0+jj] of Zf read along i (coalesced)
         const int j = j0 + jj, i = i0 + ii;
-        tile[jj][ii] = (j < n && i < n) ? Zf[mo + (long long)pm[j] * n + i] : 0.0f;
+        const long long at = (j < n && i < n) ? mo + (long long)pm[j] * n + i : -1;
+        tile[jj][ii] = at < 0 ? 0.0 : lib ? (double)Zf[at] : Zd[at];
       }
       __syncthreads();
       for (int e = threadIdx.x; e < 32 * 32; e += blockDim.x) {
         const int ii = e / 32, jj = e % 32;
         const int i = i0 + ii, j = j0 + jj;
-        if (i < n && j < n) V[mo + (long long)i * n + j] = (double)tile[jj][ii];
+        if (i < n && j < n) V[mo + (long long)i * n + j] = tile[jj][ii];
       }
     }
   }

@@ -57,3 +57,19 @@ def test_cluster_and_one_cta_give_the_same_bits(gpu_calc):
             assert alone["status"] == r["status"] == 0
             assert alone["energy"] == r["energy"] and alone["iterations"] == r["iterations"]
             np.testing.assert_array_equal(alone["qat"], r["qat"])
+
+
+def test_mixed_form_cluster_and_one_cta_give_the_same_bits(gpu_calc):
+    # FP32 reduction handed to k_syev (68, 224, 446 AOs) and the small solvers (2, 24, 48 AOs)
+    rng = np.random.default_rng(23)
+    mols = [g.water_cluster(k, rng) for k in (4, 8)] + [g.alkane(k, rng) for k in (11, 37, 74)]
+    mols.append(g.Molecule(np.array([0, 0], np.int32), np.array([[0, 0, 0], [0, 0, 1.4]], float)))
+    fill = g.water_clusters(400, seed=3, nmin=11, nmax=12)
+    batch = gpu_calc.singlepoint_batch(mols + fill, precision=1, solver=1)
+    plain = gpu_calc.singlepoint_batch(mols, solver=1, accuracy=0.01)
+    for m, rb, rp in zip(mols, batch, plain):
+        alone = gpu_calc.singlepoint_batch([m], precision=1, solver=1)[0]
+        assert alone["status"] == rb["status"] == rp["status"] == 0
+        assert alone["energy"] == rb["energy"] and alone["iterations"] == rb["iterations"]
+        np.testing.assert_array_equal(alone["qat"], rb["qat"])
+        assert abs(alone["energy"] - rp["energy"]) < 1e-6  # the mixed form's bound
