@@ -1749,7 +1749,7 @@ tb_status iterate_body(tb_batch* b, cudaStream_t st) {
        k_mulliken_cols<<<nchunk, 256, 0, st>>>(B, b->d_chunks32, nchunk, b->P, b->S, b->H0, b->D, b->Q, b->colred,
                                                S.active));
   TB_K("finalize", 0, 0,
-       k_finalize<<<nmol, 256, 0, st>>>(Pc, B, b->colred, b->n0sh, b->mrad, b->q_in, b->dq, b->qsh_out, b->qat_out,
+       k_finalize<<<nmol, 512, 0, st>>>(Pc, B, b->colred, b->n0sh, b->mrad, b->q_in, b->dq, b->qsh_out, b->qat_out,
                                         b->dpat_out, b->qpat_out, econv, pconv, b->opt.max_iter, S,
                                         std::max(kMixedSwitchScale * econv, kMixedSwitchFloorE),
                                         std::max(kMixedSwitchScale * pconv, kMixedSwitchFloorQ), b->gtab, b->atab));
