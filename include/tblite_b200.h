@@ -71,10 +71,11 @@ typedef struct tb_options {
                              cuSOLVER Xsyevd above; 1 in-house only (larger
                              structures: TB_CAPACITY_EXCEEDED); 2 cuSOLVER only */
   int32_t profile;        /* 1: time every kernel class with CUDA events        */
-  int32_t precision;      /* 0 plain FP64; 1 mixed: FP32 eigensolve refined in
-                             FP64 and FP32-product contractions until the SCF
-                             nearly converges, then at least two FP64
-                             iterations before the final convergence test     */
+  int32_t precision;      /* 0 plain FP64; 1 mixed: FP32-product contractions
+                             (cuSOLVER structures: also an FP32 eigensolve
+                             refined in FP64) until the SCF nearly converges,
+                             then at least two FP64 iterations before the
+                             final convergence test                           */
 } tb_options;
 
 /* Per-structure results: the energy/wavefunction outputs of xtb_singlepoint.

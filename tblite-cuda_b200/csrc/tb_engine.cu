@@ -443,7 +443,7 @@ struct tb_batch {
   bool mixed = false;
   float *Af = nullptr, *Zf = nullptr, *wf = nullptr;
   double *Vn = nullptr, *G = nullptr;
-  int *act_lo = nullptr, *act_hi = nullptr;
+  int *act_lo = nullptr, *act_hi = nullptr, *act_ll = nullptr, *act_li = nullptr;
   // stepping state (tb_batch_begin / tb_batch_step) and the captured iteration
   DevParams Pc{};
   int it = 0;
@@ -835,10 +835,13 @@ tb_status batch_build(tb_calculator* calc, const tb_structure* mols, int nmol, c
   size_t o_d4cn = L.add(NA * D8), o_d4w = L.add(kD4MaxRef * NA * D8), o_d4dw = L.add(kD4MaxRef * NA * D8),
          o_d4e = L.add(NA * D8), o_d4dcn = L.add(NA * D8), o_d4g = L.add(3 * NA * D8), o_edisp = L.add(NM * D8);
   size_t o_lwork = L.add(std::max<size_t>(b->lib_bytes, 16)), o_linfo = L.add((2 * b->big.size() + 2) * I4);
-  // mixed-precision form: FP32 eigensolver input/output, refinement buffers, phase state
-  const long long MXN2 = b->mixed ? N2 : 0, MXNO = b->mixed ? NO : 0, MXNM = b->mixed ? NM : 0;
+  // mixed-precision form: phase state; for structures on the library path FP32
+  // eigensolver input/output and refinement buffers
+  const bool mixed_lib = b->mixed && !b->big.empty();
+  const long long MXN2 = mixed_lib ? N2 : 0, MXNO = mixed_lib ? NO : 0, MXNM = b->mixed ? NM : 0;
   size_t o_Af = L.add(MXN2 * 4), o_Zf = L.add(MXN2 * 4), o_wf = L.add(MXNO * 4), o_Vn = L.add(MXN2 * D8),
-         o_G = L.add(MXN2 * D8), o_lo = L.add(MXNM * I4), o_hi = L.add(MXNM * I4), o_phase = L.add(MXNM * I4),
+         o_G = L.add(MXN2 * D8), o_lo = L.add(MXNM * I4), o_hi = L.add(MXNM * I4), o_ll = L.add(MXNM * I4),
+         o_li = L.add(MXNM * I4), o_phase = L.add(MXNM * I4),
          o_n64 = L.add(MXNM * I4);
   b->bytes = L.total;
   b->arena = arena;
@@ -935,6 +938,7 @@ tb_status batch_build(tb_calculator* calc, const tb_structure* mols, int nmol, c
     b->Af = at<float>(base, o_Af); b->Zf = at<float>(base, o_Zf); b->wf = at<float>(base, o_wf);
     b->Vn = at<double>(base, o_Vn); b->G = at<double>(base, o_G);
     b->act_lo = at<int>(base, o_lo); b->act_hi = at<int>(base, o_hi);
+    b->act_ll = at<int>(base, o_ll); b->act_li = at<int>(base, o_li);
   }
   b->d_tiles64 = at<int4>(base, o_t64); b->d_tiles128 = at<int4>(base, o_t128); b->d_tiles32 = at<int4>(base, o_t32); b->d_chunks32 = at<int2>(base, o_c32);
   b->d_gemm64 = at<int4>(base, o_g64);
@@ -1103,26 +1107,44 @@ tb_status launch_gemm(tb_batch* b, cudaStream_t st, const char* prof, double wor
 // contractions leave iteration-to-iteration noise of about 1e-6 in charges.
 constexpr double kMixedSwitchScale = 10.0, kMixedSwitchFloorE = 1e-5, kMixedSwitchFloorQ = 2e-4;
 
+// Symmetric eigensolve with vectors of every active structure that is not on
+// the library path: F' in F, eigenvectors as rows of Z, W as scratch
+// (canonical work 4 N^3).
+tb_status launch_eigen(tb_batch* b, cudaStream_t st, double work) {
+  const DevBatch& B = b->db;
+  MolState& S = b->ms;
+  const tb_status ts = launch_trid_plan(b, S.active, st);
+  if (ts != TB_OK) return ts;
+  TB_K("syev", work, 1,
+       TB_CUDA(launch_syev(b->syev, B, b->F, b->Z, b->W, b->w, b->perm, S.status, S.active, st, &b->launches)));
+  --b->launches;  // launch_syev has counted
+  if (b->njac > 0)
+    TB_K("syev_jacobi", 0, 0,
+         k_syev_jacobi<<<nblk(b->njac, kJacobiWarps), kJacobiWarps * 32, jacobi_smem_bytes(), st>>>(
+             B, b->F, b->Z, b->w, b->perm, S.status, S.active, b->d_jlist, b->njac));
+  return TB_OK;
+}
+
 // Eigen-decomposition and density of one SCF iteration in the mixed-precision
 // form (tb_mixed.cu).  Every matrix is stored in FP64.  Structures in the
-// mixed phase: F', C and P as TF32x3 tensor-core GEMMs (k_gemm_tc, tcgen05),
-// eigenpairs from an FP32 reduction and one FP64 Ogita-Aishima refinement
-// step.  Structures in the FP64 phase (the final iterations) run the plain
-// form's FP64 iteration: FP64 GEMMs and the FP64 eigensolver, so the
-// converged result carries no FP32 error.  Leaves w, focc, kdim and P as the
-// plain form does.
+// mixed phase: F', C and P as TF32x3 tensor-core GEMMs (k_gemm_tc, tcgen05).
+// Structures in the FP64 phase (the final iterations) run the plain form's
+// FP64 iteration, so the converged result carries no FP32 error.  The
+// eigensolve is the FP64 one in both phases, one launch for all; structures on
+// the library path run cuSOLVER's FP32 eigensolver and one FP64 Ogita-Aishima
+// refinement step in the mixed phase.  Leaves w, focc, kdim and P as the plain
+// form does.
 tb_status mixed_core(tb_batch* b, cudaStream_t st, double n3_lo, double n3_hi, double n2occ_lo, double n2occ_hi,
                      int gemm_grid, size_t fermi_smem) {
   const DevBatch& B = b->db;
   MolState& S = b->ms;
   const int nmol = b->nmol, nt = (int)b->tiles64.size();
   const int4* T = b->d_tiles64;
-  const size_t smem32 = syev_smem_bytes(std::max(b->nmax_in, 1), sizeof(float));
-  int *lo = b->act_lo, *hi = b->act_hi;
+  int *lo = b->act_lo, *hi = b->act_hi, *ll = b->act_ll, *li = b->act_li;
   const int nt128 = (int)b->tiles128.size(), tc_grid = std::min(nt128, 148);
   const int4* T128 = b->d_tiles128;
   const size_t tc_smem = gemm_tc_smem_bytes();
-  TB_K("masks", 0, 0, k_phase_masks<<<nblk(nmol, 256), 256, 0, st>>>(nmol, S.active, S.phase, lo, hi));
+  TB_K("masks", 0, 0, k_phase_masks<<<nblk(nmol, 256), 256, 0, st>>>(B, S.active, S.phase, lo, hi, ll, li));
   // F' = X^T F X into F (T = F X in W), each phase in its precision
   TB_K("gemm_tc", 2.0 * n3_lo, 1,
        k_gemm_tc<<<tc_grid, kTcThreads, tc_smem, st>>>(B, T128, nt128, b->F, 0, b->X, 0, nullptr, nullptr, nullptr, b->W, 1.0, 0.0, lo, S.status));
@@ -1130,72 +1152,55 @@ tb_status mixed_core(tb_batch* b, cudaStream_t st, double n3_lo, double n3_hi, d
   TB_K("gemm_tc", 2.0 * n3_lo, 1,
        k_gemm_tc<<<tc_grid, kTcThreads, tc_smem, st>>>(B, T128, nt128, b->X, 1, b->W, 0, nullptr, nullptr, nullptr, b->F, 1.0, 0.0, lo, S.status));
   TB_GEMM(2.0 * n3_hi, b->X, 1, b->W, 0, nullptr, nullptr, nullptr, b->F, 1.0, 0.0, hi, kGemmKUpToI | kGemmSym);
-  // mixed phase: FP32 reduction, then the tridiagonal problem through k_syev
-  // (eigenvectors as rows of Vn; G and W are its scratch); structures below
-  // kDcMin AOs through the small FP64 kernels
-  TB_K("convert", 0, 0, k_to_f32<<<gemm_grid, 256, 0, st>>>(B, T, nt, b->F, b->Af, lo));
-  TB_K("syev_f32", 4.0 * n3_lo, 1,
-       k_reduce_f32<<<nmol, kEigThreads, smem32, st>>>(B, b->Af, b->Zf, b->Vn, b->W, S.status, lo));
-  TB_K("syev_f32", 0.0, 1,
-       TB_CUDA(launch_syev(b->syev, B, b->G, b->Vn, b->W, b->w, b->perm, S.status, lo, st, &b->launches, true, b->F)));
-  --b->launches;  // launch_syev has counted
-  if (b->njac > 0)
-    TB_K("syev_jacobi", 0, 0,
-         k_syev_jacobi<<<nblk(b->njac, kJacobiWarps), kJacobiWarps * 32, jacobi_smem_bytes(), st>>>(
-             B, b->F, b->Vn, b->w, b->perm, S.status, lo, b->d_jlist, b->njac));
-  // FP64 phase: the FP64 eigensolver (eigenvectors as rows of Z, W as its scratch)
+  // eigenpairs (eigenvectors as rows of Z, W as scratch)
   {
-    const tb_status ts = launch_trid_plan(b, hi, st);
+    const tb_status ts = launch_eigen(b, st, 4.0 * (n3_lo + n3_hi));
     if (ts != TB_OK) return ts;
   }
-  TB_K("syev", 4.0 * n3_hi, 1,
-       TB_CUDA(launch_syev(b->syev, B, b->F, b->Z, b->W, b->w, b->perm, S.status, hi, st, &b->launches)));
-  --b->launches;  // launch_syev has counted
-  if (b->njac > 0)
-    TB_K("syev_jacobi", 0, 0,
-         k_syev_jacobi<<<nblk(b->njac, kJacobiWarps), kJacobiWarps * 32, jacobi_smem_bytes(), st>>>(
-             B, b->F, b->Z, b->w, b->perm, S.status, hi, b->d_jlist, b->njac));
-  for (size_t k = 0; k < b->big.size(); ++k) {
-    const int m = b->big[k], n = b->h_ooff[m + 1] - b->h_ooff[m];
-    if (!b->h_active[m] || b->h_status[m] != kStOk) continue;
-    const long long mo = b->h_moff[m], vo = b->h_ooff[m];
-    cudaEvent_t e0 = nullptr;
-    prof_start(b, st, &e0);
-    std::string e;
-    if (b->h_phase[m] == 0)
-      e = b->lib.syev32(st, b->Af + mo, b->Zf + mo, b->wf + vo, b->w + vo, b->perm + vo, n, b->lib_work,
-                        b->lib_bytes, b->lib_info + 2 * k, S.status + m);
-    else
-      e = b->lib.syev(st, b->F + mo, b->Z + mo, b->w + vo, b->perm + vo, n, b->lib_work, b->lib_bytes,
-                      b->lib_info + 2 * k, S.status + m);
-    if (!e.empty()) return fail(TB_CUDA_ERROR, "library eigensolver: " + e);
-    ++b->launches;
-    prof_stop(b, st, b->h_phase[m] == 0 ? "syev_lib_f32" : "syev_lib", e0, 4.0 * n * n * n, 1);
-  }
-  // mixed phase: one FP64 refinement step (GEMMs included) of the FP32
-  // eigenvectors, gathered into FP64 columns in ascending order (Z -> Vn)
-  const size_t oa_smem = oa_smem_bytes(b->nmax);
-  TB_K("refine", 0, 0, k_gather_vectors<<<gemm_grid, 256, 0, st>>>(B, T, nt, b->Zf, b->Vn, b->perm, b->Z, lo));
-  {
+  if (!b->big.empty()) {
+    TB_K("convert", 0, 0, k_to_f32<<<gemm_grid, 256, 0, st>>>(B, T, nt, b->F, b->Af, ll));
+    for (size_t k = 0; k < b->big.size(); ++k) {
+      const int m = b->big[k], n = b->h_ooff[m + 1] - b->h_ooff[m];
+      if (!b->h_active[m] || b->h_status[m] != kStOk) continue;
+      const long long mo = b->h_moff[m], vo = b->h_ooff[m];
+      cudaEvent_t e0 = nullptr;
+      prof_start(b, st, &e0);
+      std::string e;
+      if (b->h_phase[m] == 0)
+        e = b->lib.syev32(st, b->Af + mo, b->Zf + mo, b->wf + vo, b->w + vo, b->perm + vo, n, b->lib_work,
+                          b->lib_bytes, b->lib_info + 2 * k, S.status + m);
+      else
+        e = b->lib.syev(st, b->F + mo, b->Z + mo, b->w + vo, b->perm + vo, n, b->lib_work, b->lib_bytes,
+                        b->lib_info + 2 * k, S.status + m);
+      if (!e.empty()) return fail(TB_CUDA_ERROR, "library eigensolver: " + e);
+      ++b->launches;
+      prof_stop(b, st, b->h_phase[m] == 0 ? "syev_lib_f32" : "syev_lib", e0, 4.0 * n * n * n, 1);
+    }
+    // one FP64 refinement step (GEMMs included) of the FP32 eigenvectors,
+    // gathered into FP64 columns in ascending order (Z -> Vn)
+    const size_t oa_smem = oa_smem_bytes(b->nmax);
+    TB_K("refine", 0, 0, k_gather_vectors<<<gemm_grid, 256, 0, st>>>(B, T, nt, b->Zf, b->perm, b->Z, ll));
     double* V = b->Z;
     double* Vo = b->Vn;
-    const double wk = 2.0 * n3_lo;
-    TB_GEMM(wk,  // G = V^T V
-            V, 1, V, 0, nullptr, nullptr, nullptr, b->G, 1.0, 0.0, lo, 0);
-    TB_GEMM(wk,  // W = F' V
-            b->F, 0, V, 0, nullptr, nullptr, nullptr, b->W, 1.0, 0.0, lo, 0);
-    TB_GEMM(wk,  // Sm = V^T W (in P)
-            V, 1, b->W, 0, nullptr, nullptr, nullptr, b->P, 1.0, 0.0, lo, 0);
-    TB_K("refine", 0, 0, k_oa_step<<<nmol, 256, oa_smem, st>>>(B, b->G, b->P, V, b->w, lo, nullptr));
+    TB_GEMM(0.0,  // G = V^T V
+            V, 1, V, 0, nullptr, nullptr, nullptr, b->G, 1.0, 0.0, ll, 0);
+    TB_GEMM(0.0,  // W = F' V
+            b->F, 0, V, 0, nullptr, nullptr, nullptr, b->W, 1.0, 0.0, ll, 0);
+    TB_GEMM(0.0,  // Sm = V^T W (in P)
+            V, 1, b->W, 0, nullptr, nullptr, nullptr, b->P, 1.0, 0.0, ll, 0);
+    TB_K("refine", 0, 0, k_oa_step<<<nmol, 256, oa_smem, st>>>(B, b->G, b->P, V, b->w, ll, nullptr));
     TB_CUDA(cudaMemcpyAsync(Vo, V, (size_t)b->n2_tot * sizeof(double), cudaMemcpyDeviceToDevice, st));
-    TB_GEMM(wk,  // Vo = V + V E
-            V, 0, b->G, 0, nullptr, nullptr, nullptr, Vo, 1.0, 1.0, lo, 0);
+    TB_GEMM(0.0,  // Vo = V + V E
+            V, 0, b->G, 0, nullptr, nullptr, nullptr, Vo, 1.0, 1.0, ll, 0);
   }
   TB_K("fermi", 0, 0, k_fermi<<<nmol, 128, fermi_smem, st>>>(B, b->w, b->opt.kt, b->focc, b->kdim, S));
-  // C = X V into W (mixed phase: V after the refinement step, in Vn; FP64
-  // phase: the eigenvector rows of Z in ascending order through perm)
+  // C = X V into W: the eigenvector rows of Z in ascending order through perm;
+  // library structures in the mixed phase: the refined columns in Vn
   TB_K("gemm_tc", 2.0 * n3_lo, 1,
-       k_gemm_tc<<<tc_grid, kTcThreads, tc_smem, st>>>(B, T128, nt128, b->X, 0, b->Vn, 0, nullptr, nullptr, nullptr, b->W, 1.0, 0.0, lo, S.status));
+       k_gemm_tc<<<tc_grid, kTcThreads, tc_smem, st>>>(B, T128, nt128, b->X, 0, b->Z, 1, b->perm, nullptr, nullptr, b->W, 1.0, 0.0, li, S.status));
+  if (!b->big.empty())
+    TB_K("gemm_tc", 0.0, 1,
+         k_gemm_tc<<<tc_grid, kTcThreads, tc_smem, st>>>(B, T128, nt128, b->X, 0, b->Vn, 0, nullptr, nullptr, nullptr, b->W, 1.0, 0.0, ll, S.status));
   TB_GEMM(2.0 * n3_hi, b->X, 0, b->Z, 1, b->perm, nullptr, nullptr, b->W, 1.0, 0.0, hi, kGemmKFromI);
   // P = C diag(f) C^T
   TB_K("gemm_tc", 2.0 * n2occ_lo, 1,
@@ -1212,7 +1217,7 @@ tb_status raise_smem_limits() {
   int dev = 0, optin = 0;
   TB_CUDA(cudaGetDevice(&dev));
   TB_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-  const void* ks[] = {(const void*)k_factor, (const void*)k_syev, (const void*)k_syev_wide, (const void*)k_syev_small, (const void*)k_reduce_f32, (const void*)k_fermi, (const void*)k_oa_step,
+  const void* ks[] = {(const void*)k_factor, (const void*)k_syev, (const void*)k_syev_wide, (const void*)k_syev_small, (const void*)k_fermi, (const void*)k_oa_step,
                       (const void*)k_gemm_tc, (const void*)k_fock, (const void*)k_syev_jacobi};
   for (const void* k : ks) {
     cudaFuncAttributes a;
@@ -1712,18 +1717,10 @@ tb_status iterate_body(tb_batch* b, cudaStream_t st) {
     // F' = X^T F X  (T = F X in W, then F' into F): 2 x 2N^3
     TB_GEMM(2.0 * n3, b->F, 0, b->X, 0, nullptr, nullptr, nullptr, b->W, 1.0, 0.0, S.active, kGemmKUpToJ);
     TB_GEMM(2.0 * n3, b->X, 1, b->W, 0, nullptr, nullptr, nullptr, b->F, 1.0, 0.0, S.active, kGemmKUpToI | kGemmSym);
-    // symmetric eigensolve with vectors: canonical 4 N^3 (k_trid_smem + k_syev)
     {
-      const tb_status ts = launch_trid_plan(b, S.active, st);
+      const tb_status ts = launch_eigen(b, st, 4.0 * n3);
       if (ts != TB_OK) return ts;
     }
-    TB_K("syev", 4.0 * n3, 1,
-         TB_CUDA(launch_syev(b->syev, B, b->F, b->Z, b->W, b->w, b->perm, S.status, S.active, st, &b->launches)));
-    --b->launches;  // launch_syev has counted
-    if (b->njac > 0)
-      TB_K("syev_jacobi", 0, 0,
-           k_syev_jacobi<<<nblk(b->njac, kJacobiWarps), kJacobiWarps * 32, jacobi_smem_bytes(), st>>>(
-               B, b->F, b->Z, b->w, b->perm, S.status, S.active, b->d_jlist, b->njac));
     for (size_t k = 0; k < b->big.size(); ++k) {
       const int m = b->big[k], n = b->h_ooff[m + 1] - b->h_ooff[m];
       if (!b->h_active[m] || b->h_status[m] != kStOk) continue;

@@ -179,12 +179,10 @@ __global__ void k_gemm32(DevBatch B, const int4* tiles, int ntiles, const double
 // FP64 eigensolver (tb_syev.cu; structures of kDcMin+ AOs): Sb an n x n scratch
 // per structure (same offsets as Ab); the grid is clusters of C CTAs, the first
 // ncoop of them each on one structure, then one structure per CTA (SyevPlan)
-// given: the tridiagonal problem is in Sb (d | e, 2n entries) and Q^T in Zb; Ab is
-// scratch
 __global__ void k_syev(DevBatch B, double* Ab, double* Zb, double* Sb, double* wout, int* perm, int* status,
-                       const int* active, int ncoop, int given);
+                       const int* active, int ncoop);
 __global__ void k_syev_wide(DevBatch B, double* Ab, double* Zb, double* Sb, double* wout, int* perm, int* status,
-                            const int* active, int ncoop, int given);
+                            const int* active, int ncoop);
 struct SyevPlan {
   int n64 = 0;          // structures of kDcMin+ AOs on the in-house solver lead the order
   int nsmall = 0, small_max = 1;  // structures below kDcMin AOs that k_syev_small solves, the largest
@@ -194,11 +192,9 @@ struct SyevPlan {
   void build(const std::vector<int>& sizes, int lib_above, int jacobi_max);
 };
 // k_syev (and k_syev_small where the plan has small structures) on st; *launches
-// counts them.  The shared-memory limits must have been raised.  given (see
-// k_syev): A is scratch and the small structures' matrices are in Asmall.
+// counts them.  The shared-memory limits must have been raised.
 cudaError_t launch_syev(const SyevPlan& P, const DevBatch& B, double* A, double* Z, double* Sb, double* w, int* perm,
-                        int* status, const int* active, cudaStream_t st, int64_t* launches, bool given = false,
-                        const double* Asmall = nullptr);
+                        int* status, const int* active, cudaStream_t st, int64_t* launches);
 // FP64 structures below kDcMin AOs, one CTA each in shared memory: B.order
 // from position `first` on; dynamic shared memory small_smem_bytes(largest)
 constexpr int kSmallLeaf = 16;  // leaves of its merge tree
@@ -212,11 +208,6 @@ __host__ __device__ constexpr int small_ws_elems(int n) {  // merge workspace; t
 inline size_t small_smem_bytes(int n) { return (3 * (size_t)n * small_ld(n) + 3 * n + small_ws_elems(n)) * sizeof(double); }
 __global__ void k_syev_small(DevBatch B, const double* Ab, double* Zb, double* wout, int* perm, int* status,
                              const int* active, int first);
-// mixed form, structures of kDcMin+ AOs: reduction to tridiagonal form and Q in
-// FP32; Q^T in FP64 into Zd, d | e into the first 2n entries of Sd (k_syev with
-// `given` takes them from there)
-__global__ void k_reduce_f32(DevBatch B, float* Ab, float* Zb, double* Zd, double* Sd, const int* status,
-                             const int* active);
 // small-structure variant: one warp per structure of N <= kJacobiMaxN (cyclic Jacobi
 // in shared memory), structures list[0..nlist), kJacobiWarps structures per CTA;
 // same outputs as k_syev (w ascending, eigenvector j = row perm[j] of Z)
@@ -228,7 +219,7 @@ __global__ void k_syev_jacobi(DevBatch B, double* Ab, double* Zb, double* wout, 
                               const int* active, const int* list, int nlist);
 
 // mixed-precision form (tb_mixed.cu)
-__global__ void k_phase_masks(int nmol, const int* active, const int* phase, int* lo, int* hi);
+__global__ void k_phase_masks(DevBatch B, const int* active, const int* phase, int* lo, int* hi, int* ll, int* li);
 // the same contractions as TF32x3 (split precision) tcgen05 GEMMs over 128 x 128 tiles (tb_tc.cu);
 // kTcThreads threads, dynamic shared memory gemm_tc_smem_bytes(), status marks a structure whose waits ran out
 constexpr int kTcTile = 128;
@@ -238,8 +229,8 @@ __global__ void k_gemm_tc(DevBatch B, const int4* tiles, int ntiles, const doubl
                           double beta, const int* active, int* status);
 size_t gemm_tc_smem_bytes();
 __global__ void k_to_f32(DevBatch B, const int4* tiles, int ntiles, const double* F, float* Af, const int* mask);
-__global__ void k_gather_vectors(DevBatch B, const int4* tiles, int ntiles, const float* Zf, const double* Zd,
-                                 const int* perm, double* V, const int* mask);
+__global__ void k_gather_vectors(DevBatch B, const int4* tiles, int ntiles, const float* Zf, const int* perm,
+                                 double* V, const int* mask);
 // refinement step (Rayleigh-Ritz in clusters + Ogita-Aishima coefficients)
 constexpr int kClusterMax = 64;
 inline size_t oa_smem_bytes(int nmax) {

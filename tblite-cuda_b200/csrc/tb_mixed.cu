@@ -7,18 +7,18 @@
 //  * FP64 (1): entered once the mixed phase meets the (loosened) convergence
 //    test; the same contractions as FP64 GEMMs.  A structure retires only
 //    after at least two FP64 iterations and the full-accuracy convergence test.
-// The mixed phase reduces F' to tridiagonal form and accumulates Q in FP32
-// (k_reduce_f32; vectors orthogonal to about n * 1e-7), solves the tridiagonal
-// problem in FP64 (k_syev) and refines the eigenpairs by one FP64 step, GEMMs
-// included; structures below kDcMin AOs go through the small FP64 solvers, and
-// the FP64 phase through the FP64 eigensolver alone.  A step
-// is Ogita-Aishima iterative refinement (T. Ogita, K. Aishima, Japan J.
-// Indust. Appl. Math. 35 (2018) 1007-1035, algorithm RefSyEv) with an exact
-// Rayleigh-Ritz solve inside clusters of near-degenerate eigenvalues (their
-// treatment of clustered eigenvalues, same journal 36 (2019) 435-459); without
-// it the second step turns the unresolved rotations inside a cluster into
-// large first-order updates and loses orthogonality.  Fermi level, Fock build,
-// Mulliken analysis, energies and Broyden mixing are FP64 throughout.
+// In both phases the eigensolve is the FP64 one (tb_syev.cu; Q and the merges
+// on the FP64 tensor instruction).  It is faster here than the FP32 reduction
+// with an FP64 refinement step of its pairs that it replaced: 64 clusters of
+// 48..384 AOs took 6.9 ms, 0.6 ms of refinement and 8 N^3 flops of FP64 GEMMs an
+// iteration, and 3.5 ms in FP64 on clusters of CTAs.  Structures on the library path keep cuSOLVER's FP32
+// eigensolver in the mixed phase (vectors orthogonal to about n * 1e-7) and
+// one FP64 refinement step of its pairs: Ogita-Aishima iterative refinement
+// (T. Ogita, K. Aishima, Japan J. Indust. Appl. Math. 35 (2018) 1007-1035,
+// algorithm RefSyEv) with an optional exact Rayleigh-Ritz solve inside clusters
+// of near-degenerate eigenvalues (their treatment of clustered eigenvalues,
+// same journal 36 (2019) 435-459).  Fermi level, Fock build, Mulliken analysis,
+// energies and Broyden mixing are FP64 throughout.
 // The kernels here follow the batch conventions of tb_linalg.cu: tile lists of
 // (structure, tile row, tile col), per-structure masks, row-major N x N blocks
 // at moff[m].
@@ -31,13 +31,18 @@ namespace {
 constexpr int MT = 64;
 }  // namespace
 
-// lo[m] = active and in the mixed phase; hi[m] = active and in the FP64 phase.
-__global__ void k_phase_masks(int nmol, const int* __restrict__ active, const int* __restrict__ phase,
-                              int* __restrict__ lo, int* __restrict__ hi) {
-  for (int m = blockIdx.x * blockDim.x + threadIdx.x; m < nmol; m += gridDim.x * blockDim.x) {
-    const int a = active[m];
-    lo[m] = a && phase[m] == 0;
+// lo[m] = active and in the mixed phase; hi[m] = active and in the FP64 phase;
+// ll[m] / li[m] = lo[m] and on the library / in-house eigensolver.
+__global__ void k_phase_masks(DevBatch B, const int* __restrict__ active, const int* __restrict__ phase,
+                              int* __restrict__ lo, int* __restrict__ hi, int* __restrict__ ll,
+                              int* __restrict__ li) {
+  for (int m = blockIdx.x * blockDim.x + threadIdx.x; m < B.nmol; m += gridDim.x * blockDim.x) {
+    const int a = active[m], low = a && phase[m] == 0;
+    const int lib = on_library(B, B.ooff[m + 1] - B.ooff[m]);
+    lo[m] = low;
     hi[m] = a && phase[m] != 0;
+    ll[m] = low && lib;
+    li[m] = low && !lib;
   }
 }
 
@@ -57,12 +62,10 @@ __global__ void k_to_f32(DevBatch B, const int4* __restrict__ tiles, int ntiles,
   }
 }
 
-// V[i][j] = Z[perm[j]][i]: eigenvector j (ascending) as column j, from the
-// library's FP32 rows (Zf) or the in-house solver's FP64 rows (Zd).
+// V[i][j] = Zf[perm[j]][i] in FP64: eigenvector j (ascending) as column j.
 __global__ void k_gather_vectors(DevBatch B, const int4* __restrict__ tiles, int ntiles, const float* __restrict__ Zf,
-                                 const double* __restrict__ Zd, const int* __restrict__ perm,
-                                 double* __restrict__ V, const int* __restrict__ mask) {
-  __shared__ double tile[32][33];
+                                 const int* __restrict__ perm, double* __restrict__ V, const int* __restrict__ mask) {
+  __shared__ float tile[32][33];
   for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
     const int4 tl = tiles[t];
     const int m = tl.x;
@@ -70,7 +73,6 @@ __global__ void k_gather_vectors(DevBatch B, const int4* __restrict__ tiles, int
     const int n = B.ooff[m + 1] - B.ooff[m];
     const long long mo = B.moff[m];
     const int* pm = perm + B.ooff[m];
-    const bool lib = on_library(B, n);
     // the 64 x 64 tile as four 32 x 32 transposes
     for (int q = 0; q < 4; ++q) {
       const int i0 = tl.y * MT + 32 * (q >> 1), j0 = tl.z * MT + 32 * (q & 1);
@@ -78,14 +80,13 @@ __global__ void k_gather_vectors(DevBatch B, const int4* __restrict__ tiles, int
       for (int e = threadIdx.x; e < 32 * 32; e += blockDim.x) {
         const int jj = e / 32, ii = e % 32;  // row perm[j0+jj] of Zf read along i (coalesced)
         const int j = j0 + jj, i = i0 + ii;
-        const long long at = (j < n && i < n) ? mo + (long long)pm[j] * n + i : -1;
-        tile[jj][ii] = at < 0 ? 0.0 : lib ? (double)Zf[at] : Zd[at];
+        tile[jj][ii] = (j < n && i < n) ? Zf[mo + (long long)pm[j] * n + i] : 0.0f;
       }
       __syncthreads();
       for (int e = threadIdx.x; e < 32 * 32; e += blockDim.x) {
         const int ii = e / 32, jj = e % 32;
         const int i = i0 + ii, j = j0 + jj;
-        if (i < n && j < n) V[mo + (long long)i * n + j] = tile[jj][ii];
+        if (i < n && j < n) V[mo + (long long)i * n + j] = (double)tile[jj][ii];
       }
     }
   }

@@ -777,7 +777,7 @@ __global__ void __launch_bounds__(512, 2) k_finalize(DevParams P, DevBatch B, co
     if (S.phase) {
       // mixed-precision form: the mixed phase ends at the loosened test, when
       // its charge error stops falling (less than halved from the previous
-      // iteration after the third: the FP32 eigenpairs no longer improve the
+      // iteration after the third: the FP32 contractions no longer improve the
       // point), or after half the iteration budget; the mixer restarts from
       // the current point, then at least two FP64 iterations run and the full
       // test decides

@@ -1575,7 +1575,7 @@ template <bool W>
 __device__ __forceinline__ void syev_structure(const DevBatch& B, double* __restrict__ Ab, double* __restrict__ Zb,
                                                double* __restrict__ Sb, double* __restrict__ wout,
                                                int* __restrict__ perm, int* __restrict__ status,
-                                               const int* __restrict__ active, int ncoop, int given) {
+                                               const int* __restrict__ active, int ncoop) {
   unsigned csize, crank;
   asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(csize));
   asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(crank));
@@ -1605,12 +1605,7 @@ __device__ __forceinline__ void syev_structure(const DevBatch& B, double* __rest
   __shared__ int q_fail;
   const int tid = threadIdx.x;
 
-  if (given) {  // the mixed form's FP32 reduction: d | e in the scratch slice, Q^T in Z
-    for (int i = tid; i < n; i += kEigThreads) {
-      d[i] = Sc[i];
-      e[i] = i < n - 1 ? Sc[n + i] : 0.0;
-    }
-  } else if (B.trid_max > 0 && n >= B.trid_min && n >= kTridMin && n <= B.trid_max) {
+  if (B.trid_max > 0 && n >= B.trid_min && n >= kTridMin && n <= B.trid_max) {
     // tridiagonalised in shared memory by k_trid_smem: reflectors in A's rows,
     // d | e | tau in the first 3n entries of the scratch slice
     for (int i = tid; i < n; i += kEigThreads) {
@@ -1622,7 +1617,7 @@ __device__ __forceinline__ void syev_structure(const DevBatch& B, double* __rest
   } else {
     tridiag_tiles<W>(A, n, d, e, tau, v, vn, p, w, ring, Sc, g);
   }
-  if (!given) form_q<W>(A, Z, n, tau, v, g);
+  form_q<W>(A, Z, n, tau, v, g);
   group_sync(g);  // Z is complete, A and the scratch are free
 
   unsigned dyn_bytes;
@@ -1663,15 +1658,15 @@ __device__ __forceinline__ void syev_structure(const DevBatch& B, double* __rest
 __global__ void __launch_bounds__(kEigThreads, 2) k_syev(DevBatch B, double* __restrict__ Ab, double* __restrict__ Zb,
                                                          double* __restrict__ Sb, double* __restrict__ wout,
                                                          int* __restrict__ perm, int* __restrict__ status,
-                                                         const int* __restrict__ active, int ncoop, int given) {
-  syev_structure<false>(B, Ab, Zb, Sb, wout, perm, status, active, ncoop, given);
+                                                         const int* __restrict__ active, int ncoop) {
+  syev_structure<false>(B, Ab, Zb, Sb, wout, perm, status, active, ncoop);
 }
 __global__ void __launch_bounds__(kEigThreads, 1) k_syev_wide(DevBatch B, double* __restrict__ Ab,
                                                               double* __restrict__ Zb, double* __restrict__ Sb,
                                                               double* __restrict__ wout, int* __restrict__ perm,
                                                               int* __restrict__ status,
-                                                              const int* __restrict__ active, int ncoop, int given) {
-  syev_structure<true>(B, Ab, Zb, Sb, wout, perm, status, active, ncoop, given);
+                                                              const int* __restrict__ active, int ncoop) {
+  syev_structure<true>(B, Ab, Zb, Sb, wout, perm, status, active, ncoop);
 }
 
 // Structures of B.order from position `first` on, one CTA each.
@@ -1818,8 +1813,7 @@ void SyevPlan::build(const std::vector<int>& sizes, int lib_above, int jacobi_ma
 }
 
 cudaError_t launch_syev(const SyevPlan& P, const DevBatch& B, double* A, double* Z, double* Sb, double* w, int* perm,
-                        int* status, const int* active, cudaStream_t st, int64_t* launches, bool given,
-                        const double* Asmall) {
+                        int* status, const int* active, cudaStream_t st, int64_t* launches) {
   cudaError_t e = cudaSuccess;
   const size_t smem = syev_smem_bytes(P.nmax > 1 ? P.nmax : 1);
   if (P.n64 > 0 && P.nmax >= kDcMin) {
@@ -1838,15 +1832,14 @@ cudaError_t launch_syev(const SyevPlan& P, const DevBatch& B, double* A, double*
     at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = C > 1 ? 1 : 0;
-    e = cudaLaunchKernelEx(&cfg, P.c.wide ? k_syev_wide : k_syev, Bs, A, Z, Sb, w, perm, status, active, P.c.ncoop,
-                           given ? 1 : 0);
+    e = cudaLaunchKernelEx(&cfg, P.c.wide ? k_syev_wide : k_syev, Bs, A, Z, Sb, w, perm, status, active, P.c.ncoop);
     if (e != cudaSuccess) return e;
     if (launches) ++*launches;
   }
   if (P.nsmall > 0) {
     // in the order, the small structures follow n64 (with no order, anywhere)
     const int first = B.order ? P.n64 : 0;
-    k_syev_small<<<B.nmol - first, kEigThreads, small_smem_bytes(P.small_max), st>>>(B, given ? Asmall : A, Z, w, perm, status, active,
+    k_syev_small<<<B.nmol - first, kEigThreads, small_smem_bytes(P.small_max), st>>>(B, A, Z, w, perm, status, active,
                                                                                     first);
     e = cudaGetLastError();
     if (launches) ++*launches;

@@ -60,7 +60,7 @@ def test_cluster_and_one_cta_give_the_same_bits(gpu_calc):
 
 
 def test_mixed_form_cluster_and_one_cta_give_the_same_bits(gpu_calc):
-    # FP32 reduction handed to k_syev (68, 224, 446 AOs) and the small solvers (2, 24, 48 AOs)
+    # k_syev (68, 224, 446 AOs) and the small solvers (2, 24, 48 AOs)
     rng = np.random.default_rng(23)
     mols = [g.water_cluster(k, rng) for k in (4, 8)] + [g.alkane(k, rng) for k in (11, 37, 74)]
     mols.append(g.Molecule(np.array([0, 0], np.int32), np.array([[0, 0, 0], [0, 0, 1.4]], float)))
