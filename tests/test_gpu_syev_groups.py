@@ -43,6 +43,29 @@ def test_orders_at_tile_edges(n):
     np.testing.assert_allclose(H @ V, S @ V * W, atol=tol * scale, rtol=0)
 
 
+@pytest.mark.parametrize("n", [65, 97, 130, 200, 256])
+def test_runs_of_close_eigenvalues(n):
+    # chains of deflated pairs, shorter and longer than the 32 entries tested at once
+    import torch
+    rng = np.random.default_rng(7 * n)
+    q, _ = np.linalg.qr(rng.standard_normal((n, n)))
+    lam = np.concatenate([1.0 + 1e-16 * np.arange(n // 2), np.repeat([2.0, 3.0], (n - n // 2) // 3),
+                          4.0 + 1e-13 * np.arange(n - n // 2 - 2 * ((n - n // 2) // 3))])
+    H = (q * lam) @ q.T
+    H = 0.5 * (H + H.T)
+    h, s = torch.from_numpy(H).cuda(), torch.eye(n, dtype=torch.float64, device="cuda")
+    w = torch.empty(n, dtype=torch.float64, device="cuda")
+    c = torch.empty((n, n), dtype=torch.float64, device="cuda")
+    st = capi.load_library().tb_sygvd_noalloc(C.c_int32(n), *[C.c_void_p(x.data_ptr()) for x in (h, s, w, c)],
+                                              C.c_void_p(0))
+    assert st == 0, capi.last_error()
+    W, V = w.cpu().numpy(), c.cpu().numpy()
+    tol = 8 * n * np.finfo(float).eps  # backward stable: a few n eps of the norm (4)
+    np.testing.assert_allclose(W, np.linalg.eigvalsh(H), atol=4 * tol, rtol=0)
+    np.testing.assert_allclose(V.T @ V, np.eye(n), atol=tol, rtol=0)
+    np.testing.assert_allclose(H @ V, V * W, atol=4 * tol, rtol=0)
+
+
 def test_cluster_and_one_cta_give_the_same_bits(gpu_calc):
     rng = np.random.default_rng(17)
     mols = [g.water_cluster(k, rng) for k in (11, 16, 22, 37, 38, 64)]
