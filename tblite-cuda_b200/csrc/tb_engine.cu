@@ -1611,7 +1611,7 @@ tb_status batch_setup(tb_batch* b, cudaStream_t st) {
   TB_CUDA(cudaMemsetAsync(S.n_active, 0, sizeof(int), st));
   TB_CUDA(cudaMemsetAsync(b->kdim, 0, nmol * sizeof(int), st));  // no occupied orbitals before k_fermi
   // ---- setup (once per structure)
-  TB_K("atoms", 0, 0, k_atoms<<<nblk(B.nat_tot, 128), 128, 0, st>>>(Pc, B, b->cn, b->mrad, b->erep, b->se));
+  TB_K("atoms", 0, 0, k_atoms<<<nblk((long long)B.nat_tot * 32, 128), 128, 0, st>>>(Pc, B, b->cn, b->mrad, b->erep, b->se));
   // D4 dispersion of the fixed geometry (dispersion_get_engrad, src/xtb.cu:274-277)
   if (Pc.d4) {
     cudaEvent_t e0 = nullptr;
@@ -2562,7 +2562,7 @@ tb_status d2h(void* dst, const void* src, size_t bytes) {
 tb_status run_setup_to_integrals(tb_batch* b, bool with_integrals) {
   const DevParams P = params_for(b->calc, 1.0);
   const DevBatch& B = b->db;
-  k_atoms<<<nblk(B.nat_tot, 128), 128>>>(P, B, b->cn, b->mrad, b->erep, b->se);
+  k_atoms<<<nblk((long long)B.nat_tot * 32, 128), 128>>>(P, B, b->cn, b->mrad, b->erep, b->se);
   TB_LAUNCH_CHECK();
   if (!with_integrals) return TB_OK;
   k_adj_count<<<nblk((long long)B.nat_tot * 32, 256), 256>>>(B, P.cutoff, b->cnt);

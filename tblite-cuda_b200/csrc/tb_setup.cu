@@ -19,13 +19,17 @@ __device__ inline double exp_count(double k, double r, double r0) {
   return 1.0 / (1.0 + exp(-k * (r0 / r - 1.0)));
 }
 
-// One thread per atom: CN (ncoord_dexp, src/coulomb.cu:173-246), repulsion
+// One warp per atom, lanes over the partners, reduced across the warp in a
+// fixed order: CN (ncoord_dexp, src/coulomb.cu:173-246), repulsion
 // energy share (get_repulsion_derivs, src/xtb.cu:62-91), multipole damping
 // radius (get_mrad, src/coulomb.cu:387-398) and shell self-energies
-// (get_selfenergy, src/h0.cu:137-170).
+// (get_selfenergy, src/h0.cu:137-170).  Bound by the latency of a pair's
+// chain of sqrt, pow and exp: one thread per atom walked all partners alone (64
+// waters 0.316 ms, now 0.019; 1024 clusters 0.60 and 0.46 ms; octane 0.048 and
+// 0.015).
 __global__ void k_atoms(DevParams P, DevBatch B, double* __restrict__ cn, double* __restrict__ mrad,
                         double* __restrict__ erep, double* __restrict__ se) {
-  const int a = blockIdx.x * blockDim.x + threadIdx.x;
+  const int a = (int)((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
   if (a >= B.nat_tot) return;
   const int m = B.at_mol[a];
   const int a0 = B.aoff[m], a1 = B.aoff[m + 1];
@@ -34,7 +38,7 @@ __global__ void k_atoms(DevParams P, DevBatch B, double* __restrict__ cn, double
   const double ka = 10.0, kb = 20.0, rshift = 2.0;
   const double cn2 = P.cn_cutoff * P.cn_cutoff, rep2 = P.rep_cutoff * P.rep_cutoff;
   double c = 0.0, e = 0.0;
-  for (int b = a0; b < a1; ++b) {
+  for (int b = a0 + lane; b < a1; b += 32) {
     if (b == a) continue;
     const double dx = xa - B.xyz[3 * b], dy = ya - B.xyz[3 * b + 1], dz = za - B.xyz[3 * b + 2];
     const double r2 = dx * dx + dy * dy + dz * dz;
@@ -54,6 +58,9 @@ __global__ void k_atoms(DevParams P, DevBatch B, double* __restrict__ cn, double
       e += 0.5 * zeff * exp(-alpha * r1k) / r1r;
     }
   }
+  c = warp_sum(c);
+  e = warp_sum(e);
+  if (lane != 0) return;
   cn[a] = c;
   erep[a] = e;
   const double t1 = exp(-P.mp_kexp * (c - si.mp_vcn - P.mp_shift));
