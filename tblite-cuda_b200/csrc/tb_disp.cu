@@ -18,10 +18,10 @@
 // Each atom sums its own share of the pair and triple energies and its own
 // gradient terms over the other atoms in a fixed order (no atomics), so a
 // structure gives the same bits alone and in any batch.  Kernels, run once per
-// batch in the setup: k_d4_weights (CN, W, dW/dCN; a thread per atom),
-// k_d4_pairs (two-body; a thread per atom), k_d4_atm (three-body; a warp per
-// atom), k_d4_cnchain (dE/dCN dCN/dR; a thread per atom), k_d4_energy (per
-// structure).
+// batch in the setup: k_d4_weights (CN, W, dW/dCN; a warp per atom),
+// k_d4_pairs (two-body; a warp per atom), k_d4_atm (three-body; a CTA per
+// atom), k_d4_cnchain (dE/dCN dCN/dR; a warp per atom), k_d4_energy (a warp
+// per structure).
 #include <cuda_runtime.h>
 
 #include "tb_common.cuh"
@@ -71,12 +71,12 @@ __device__ inline double d4_qpair(const SpeciesParam& a, const SpeciesParam& b) 
 // CN_A, W_A^i and dW_A^i / dCN_A for every atom of the batch
 __global__ void k_d4_weights(DevParams P, DevBatch B, double* __restrict__ cn, double* __restrict__ W,
                              double* __restrict__ dW) {
-  const int A = blockIdx.x * blockDim.x + threadIdx.x;
+  const int A = (int)((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
   if (A >= B.nat_tot) return;
   const int m = B.at_mol[A], a0 = B.aoff[m], nat = B.aoff[m + 1] - a0;
   const SpeciesParam& sa = P.sp[B.id[A]];
   double c = 0.0;
-  for (int b = 0; b < nat; ++b) {
+  for (int b = lane; b < nat; b += 32) {
     const int Bi = a0 + b;
     if (Bi == A) continue;
     const double v0 = B.xyz[3 * A] - B.xyz[3 * Bi], v1 = B.xyz[3 * A + 1] - B.xyz[3 * Bi + 1],
@@ -85,6 +85,8 @@ __global__ void k_d4_weights(DevParams P, DevBatch B, double* __restrict__ cn, d
     if (r > P.d4_cn_cut || r < 1.0e-6) continue;
     c += d4_count(P, sa, P.sp[B.id[Bi]], r, nullptr);
   }
+  c = warp_sum(c);
+  if (lane != 0) return;
   cn[A] = c;
   double gmax = -1e300;
   for (int i = 0; i < sa.d4_nref; ++i) gmax = fmax(gmax, -P.d4_wf * (c - sa.d4_cn[i]) * (c - sa.d4_cn[i]));
@@ -106,13 +108,13 @@ __global__ void k_d4_weights(DevParams P, DevBatch B, double* __restrict__ cn, d
 // gradient g[A] of A's pairs
 __global__ void k_d4_pairs(DevParams P, DevBatch B, const double* __restrict__ W, const double* __restrict__ dW,
                            double* __restrict__ e_at, double* __restrict__ dEdcn, double* __restrict__ g) {
-  const int A = blockIdx.x * blockDim.x + threadIdx.x;
+  const int A = (int)((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
   if (A >= B.nat_tot) return;
   const int m = B.at_mol[A], a0 = B.aoff[m], nat = B.aoff[m + 1] - a0;
   const int za = B.id[A];
   const SpeciesParam& sa = P.sp[za];
   double e = 0.0, de = 0.0, g0 = 0.0, g1 = 0.0, g2 = 0.0;
-  for (int b = 0; b < nat; ++b) {
+  for (int b = lane; b < nat; b += 32) {
     const int Bi = a0 + b;
     if (Bi == A) continue;
     const double v0 = B.xyz[3 * A] - B.xyz[3 * Bi], v1 = B.xyz[3 * A + 1] - B.xyz[3 * Bi + 1],
@@ -133,27 +135,38 @@ __global__ void k_d4_pairs(DevParams P, DevBatch B, const double* __restrict__ W
     const double f = -C6 * dh / r;
     g0 += f * v0; g1 += f * v1; g2 += f * v2;
   }
+  e = warp_sum(e);
+  de = warp_sum(de);
+  g0 = warp_sum(g0);
+  g1 = warp_sum(g1);
+  g2 = warp_sum(g2);
+  if (lane != 0) return;
   e_at[A] = e;
   dEdcn[A] = de;
   g[3 * A] = g0; g[3 * A + 1] = g1; g[3 * A + 2] = g2;
 }
 
-// three-body: a warp per atom A; lane l takes the atoms B = l, l + 32, ... of
-// A's structure and every C > B (B, C != A); each triple's energy goes one
-// third to each atom, and A adds its own dE/dCN_A and gradient terms.  Lane
-// partials are added by a fixed shuffle tree.
-__global__ void k_d4_atm(DevParams P, DevBatch B, const double* __restrict__ W, const double* __restrict__ dW,
-                         double* __restrict__ e_at, double* __restrict__ dEdcn, double* __restrict__ g) {
-  const int A = (int)((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5);
-  const int lane = threadIdx.x & 31;
-  if (A >= B.nat_tot || P.d4_s9 == 0.0) return;
+// three-body: a CTA per atom A; warp w takes the atoms B = w, w + 4, ... of A's
+// structure, lane l the atoms C = B + 1 + l, ... (B, C != A); each triple's
+// energy goes one third to each atom, and A adds its own dE/dCN_A and gradient
+// terms.  Partials are added in a fixed order.  Bound by the latency of a
+// triple's chain (two C6 sums, pow, divisions): with a warp per atom and lanes
+// over B, whose triples C > B differ in number, the five kernels took 1.48 ms on
+// 16 water clusters and alkanes of 6..40 molecules or carbons, now 0.45.
+__global__ void __launch_bounds__(128) k_d4_atm(DevParams P, DevBatch B, const double* __restrict__ W,
+                                                const double* __restrict__ dW, double* __restrict__ e_at,
+                                                double* __restrict__ dEdcn, double* __restrict__ g) {
+  const int A = blockIdx.x;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
+  if (P.d4_s9 == 0.0) return;
+  __shared__ double red[32];
   const int m = B.at_mol[A], a0 = B.aoff[m], nat = B.aoff[m + 1] - a0;
   const int za = B.id[A];
   const SpeciesParam& sa = P.sp[za];
   const double xa = B.xyz[3 * A], ya = B.xyz[3 * A + 1], zaa = B.xyz[3 * A + 2];
   const double cut = P.d4_atm_cut, p = P.d4_alp / 3.0;
   double e = 0.0, de = 0.0, g0 = 0.0, g1 = 0.0, g2 = 0.0;
-  for (int b = lane; b < nat; b += 32) {
+  for (int b = warp; b < nat; b += nwarp) {
     const int Bi = a0 + b;
     if (Bi == A) continue;
     const double vab0 = xa - B.xyz[3 * Bi], vab1 = ya - B.xyz[3 * Bi + 1], vab2 = zaa - B.xyz[3 * Bi + 2];
@@ -164,7 +177,7 @@ __global__ void k_d4_atm(DevParams P, DevBatch B, const double* __restrict__ W, 
     double dab_a, dab_b;
     const double cab = d4_c6(P, sa, sb, za, zb, W, dW, A, Bi, &dab_a, &dab_b);
     const double Rab = P.d4_a1 * sqrt(d4_qpair(sa, sb)) + P.d4_a2;
-    for (int cc = b + 1; cc < nat; ++cc) {
+    for (int cc = b + 1 + lane; cc < nat; cc += 32) {
       const int Ci = a0 + cc;
       if (Ci == A) continue;
       const double vca0 = B.xyz[3 * Ci] - xa, vca1 = B.xyz[3 * Ci + 1] - ya, vca2 = B.xyz[3 * Ci + 2] - zaa;
@@ -204,12 +217,12 @@ __global__ void k_d4_atm(DevParams P, DevBatch B, const double* __restrict__ W, 
       g2 += dEab * vab2 / rab - dEca * vca2 / rca;
     }
   }
-  e = warp_sum(e);
-  de = warp_sum(de);
-  g0 = warp_sum(g0);
-  g1 = warp_sum(g1);
-  g2 = warp_sum(g2);
-  if (lane == 0) {
+  e = block_sum(e, red);
+  de = block_sum(de, red);
+  g0 = block_sum(g0, red);
+  g1 = block_sum(g1, red);
+  g2 = block_sum(g2, red);
+  if (threadIdx.x == 0) {
     e_at[A] += e;
     dEdcn[A] += de;
     g[3 * A] += g0; g[3 * A + 1] += g1; g[3 * A + 2] += g2;
@@ -218,12 +231,12 @@ __global__ void k_d4_atm(DevParams P, DevBatch B, const double* __restrict__ W, 
 
 // coordination-number chain: g_A += sum_B (dE/dCN_A + dE/dCN_B) dcount_AB/dr (R_A - R_B)/r
 __global__ void k_d4_cnchain(DevParams P, DevBatch B, const double* __restrict__ dEdcn, double* __restrict__ g) {
-  const int A = blockIdx.x * blockDim.x + threadIdx.x;
+  const int A = (int)((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
   if (A >= B.nat_tot) return;
   const int m = B.at_mol[A], a0 = B.aoff[m], nat = B.aoff[m + 1] - a0;
   const SpeciesParam& sa = P.sp[B.id[A]];
   double g0 = 0.0, g1 = 0.0, g2 = 0.0;
-  for (int b = 0; b < nat; ++b) {
+  for (int b = lane; b < nat; b += 32) {
     const int Bi = a0 + b;
     if (Bi == A) continue;
     const double v0 = B.xyz[3 * A] - B.xyz[3 * Bi], v1 = B.xyz[3 * A + 1] - B.xyz[3 * Bi + 1],
@@ -235,16 +248,19 @@ __global__ void k_d4_cnchain(DevParams P, DevBatch B, const double* __restrict__
     const double f = (dEdcn[A] + dEdcn[Bi]) * dcdr / r;
     g0 += f * v0; g1 += f * v1; g2 += f * v2;
   }
-  g[3 * A] += g0; g[3 * A + 1] += g1; g[3 * A + 2] += g2;
+  g0 = warp_sum(g0);
+  g1 = warp_sum(g1);
+  g2 = warp_sum(g2);
+  if (lane == 0) { g[3 * A] += g0; g[3 * A + 1] += g1; g[3 * A + 2] += g2; }
 }
 
-// per-structure dispersion energy: the atoms' shares in order
+// per-structure dispersion energy: one warp, the atoms' shares in a fixed order
 __global__ void k_d4_energy(DevBatch B, const double* __restrict__ e_at, double* __restrict__ e_disp) {
   const int m = blockIdx.x;
-  if (threadIdx.x != 0) return;
   double s = 0.0;
-  for (int a = B.aoff[m]; a < B.aoff[m + 1]; ++a) s += e_at[a];
-  e_disp[m] = s;
+  for (int a = B.aoff[m] + threadIdx.x; a < B.aoff[m + 1]; a += 32) s += e_at[a];
+  s = warp_sum(s);
+  if (threadIdx.x == 0) e_disp[m] = s;
 }
 
 // the dispersion gradient into the total gradient of the flagged structures
@@ -257,11 +273,11 @@ __global__ void k_d4_add_grad(DevBatch B, const int* __restrict__ flag, const do
 
 cudaError_t launch_dispersion(const DevParams& P, const DevBatch& B, int nmol, double* cn, double* W, double* dW,
                               double* e_at, double* dEdcn, double* g, double* e_disp, cudaStream_t st) {
-  const int na = B.nat_tot, t = 128;
-  k_d4_weights<<<(na + t - 1) / t, t, 0, st>>>(P, B, cn, W, dW);
-  k_d4_pairs<<<(na + t - 1) / t, t, 0, st>>>(P, B, W, dW, e_at, dEdcn, g);
-  k_d4_atm<<<(int)(((long long)na * 32 + t - 1) / t), t, 0, st>>>(P, B, W, dW, e_at, dEdcn, g);
-  k_d4_cnchain<<<(na + t - 1) / t, t, 0, st>>>(P, B, dEdcn, g);
+  const int na = B.nat_tot, t = 128, nw = (int)(((long long)na * 32 + t - 1) / t);
+  k_d4_weights<<<nw, t, 0, st>>>(P, B, cn, W, dW);
+  k_d4_pairs<<<nw, t, 0, st>>>(P, B, W, dW, e_at, dEdcn, g);
+  k_d4_atm<<<na, t, 0, st>>>(P, B, W, dW, e_at, dEdcn, g);
+  k_d4_cnchain<<<nw, t, 0, st>>>(P, B, dEdcn, g);
   k_d4_energy<<<nmol, 32, 0, st>>>(B, e_at, e_disp);
   return cudaGetLastError();
 }
