@@ -1116,12 +1116,9 @@ tb_status launch_eigen(tb_batch* b, cudaStream_t st, double work) {
   const tb_status ts = launch_trid_plan(b, S.active, st);
   if (ts != TB_OK) return ts;
   TB_K("syev", work, 1,
-       TB_CUDA(launch_syev(b->syev, B, b->F, b->Z, b->W, b->w, b->perm, S.status, S.active, st, &b->launches)));
+       TB_CUDA(launch_syev(b->syev, B, b->F, b->Z, b->W, b->w, b->perm, S.status, S.active, st, &b->launches,
+                           b->d_jlist, b->njac)));
   --b->launches;  // launch_syev has counted
-  if (b->njac > 0)
-    TB_K("syev_jacobi", 0, 0,
-         k_syev_jacobi<<<nblk(b->njac, kJacobiWarps), kJacobiWarps * 32, jacobi_smem_bytes(), st>>>(
-             B, b->F, b->Z, b->w, b->perm, S.status, S.active, b->d_jlist, b->njac));
   return TB_OK;
 }
 
@@ -1418,7 +1415,7 @@ tb_status calibrate_small(tb_calculator* c) {
         if (variant == 0)
           k_syev_small<<<cnt, kEigThreads, small_smem_bytes(n)>>>(Bk, at<double>(base, oA), at<double>(base, oZ),
                                                                   at<double>(base, ow), at<int>(base, op),
-                                                                  at<int>(base, os), nullptr, 0);
+                                                                  at<int>(base, os), nullptr, 0, nullptr, 0);
         else
           k_syev_jacobi<<<nblk(cnt, kJacobiWarps), kJacobiWarps * 32, jacobi_smem_bytes()>>>(
               Bk, at<double>(base, oA), at<double>(base, oZ), at<double>(base, ow), at<int>(base, op),

@@ -194,7 +194,8 @@ struct SyevPlan {
 // k_syev (and k_syev_small where the plan has small structures) on st; *launches
 // counts them.  The shared-memory limits must have been raised.
 cudaError_t launch_syev(const SyevPlan& P, const DevBatch& B, double* A, double* Z, double* Sb, double* w, int* perm,
-                        int* status, const int* active, cudaStream_t st, int64_t* launches);
+                        int* status, const int* active, cudaStream_t st, int64_t* launches,
+                        const int* jlist = nullptr, int njac = 0);
 // FP64 structures below kDcMin AOs, one CTA each in shared memory: B.order
 // from position `first` on; dynamic shared memory small_smem_bytes(largest)
 constexpr int kSmallLeaf = 16;  // leaves of its merge tree
@@ -207,7 +208,7 @@ __host__ __device__ constexpr int small_ws_elems(int n) {  // merge workspace; t
 }
 inline size_t small_smem_bytes(int n) { return (3 * (size_t)n * small_ld(n) + 3 * n + small_ws_elems(n)) * sizeof(double); }
 __global__ void k_syev_small(DevBatch B, const double* Ab, double* Zb, double* wout, int* perm, int* status,
-                             const int* active, int first);
+                             const int* active, int first, const int* jlist, int njac);
 // small-structure variant: one warp per structure of N <= kJacobiMaxN (cyclic Jacobi
 // in shared memory), structures list[0..nlist), kJacobiWarps structures per CTA;
 // same outputs as k_syev (w ascending, eigenvector j = row perm[j] of Z)
@@ -215,7 +216,7 @@ constexpr int kJacobiMaxN = 32;
 constexpr int kJacobiWarps = 4;
 constexpr int kJacobiPitch = kJacobiMaxN + 1;
 inline size_t jacobi_smem_bytes() { return (size_t)kJacobiWarps * 2 * kJacobiMaxN * kJacobiPitch * sizeof(double); }
-__global__ void k_syev_jacobi(DevBatch B, double* Ab, double* Zb, double* wout, int* perm, int* status,
+__global__ void k_syev_jacobi(DevBatch B, const double* Ab, double* Zb, double* wout, int* perm, int* status,
                               const int* active, const int* list, int nlist);
 
 // mixed-precision form (tb_mixed.cu)
