@@ -39,9 +39,9 @@ typedef enum tb_status {
   TB_NOT_SPD = 2,              /* overlap matrix not positive definite          */
   TB_SCF_NOT_CONVERGED = 3,    /* max_iter reached                              */
   TB_FERMI_NOT_CONVERGED = 4,  /* Fermi level solve hit its iteration cap       */
-  TB_EIGEN_FAILED = 5,         /* tridiagonal solve failed: QL (or a divide-and-
-                                  conquer leaf) hit its sweep cap, or the matrix
-                                  was not finite                                */
+  TB_EIGEN_FAILED = 5,         /* eigensolve failed: the matrix was not finite, or
+                                  the one-warp Jacobi or cuSOLVER did not
+                                  converge                                      */
   TB_CAPACITY_EXCEEDED = 6,    /* request larger than a stated maximum          */
   TB_CUDA_ERROR = 7,           /* CUDA runtime error (see tb_last_error)        */
   TB_PARAM_ERROR = 8           /* parameter file could not be read              */
@@ -163,11 +163,13 @@ const char* tb_last_error(void);
  * one-thread Jacobi, src/lapack/sygvd.cu:74-133).  The per-size eigensolver
  * variant is measured once per calculator, on first need: structures of at
  * most 32 AOs use a one-warp Jacobi solver up to the largest size at which
- * it is measured faster than the one-CTA solver (Householder + implicit QL
- * below 64 AOs, + divide and conquer from 64); above 1216 AOs, and above a
- * size chosen per batch from measured cost models, cuSOLVER Xsyevd (see
- * tb_options.solver).  The choice depends on the size only, so a structure
- * gives the same bits alone and in any batch.
+ * it is measured faster than the one-CTA solver below 64 AOs (Householder +
+ * divide and conquer in shared memory); from 64 AOs the same on one CTA or a
+ * thread block cluster per structure, whichever the batch's sizes favour;
+ * above 1216 AOs, and above a size chosen per batch from measured cost models,
+ * cuSOLVER Xsyevd (see tb_options.solver).  The in-house variant depends on
+ * the size only and the cluster size moves no bits, so a structure gives the
+ * same bits alone and in any batch that leaves it in-house.
  * tb_calculator_set_small_solver: jacobi_max -1 (default) measured choice,
  * 0 never, 1..32 fixed bound.  tb_calculator_tuning writes the measurements
  * and choices as JSON text into buf (NUL-terminated, at most len bytes) and
@@ -177,13 +179,10 @@ tb_status tb_calculator_set_small_solver(tb_calculator* calc, int32_t jacobi_max
 /* Householder tridiagonalisation of the FP64 eigensolver (the dsytrd step of
  * sygvd_solver::solve, src/lapack/sygvd.cu:223-313) held in the shared memory
  * of a thread block cluster: structures of 64..560 AOs, one cluster of 1, 2,
- * 3, 4, 6 or 8 CTAs by size (the choice depends on the size only).  It cuts
- * the latency of a structure's reduction (a 384-AO one: 4 SMs instead of a
- * third of one), but spends more SM time per structure, so it pays where
- * latency bounds the call -- single structures, small batches, the request
- * loop at low load -- and not for large batches.  min_n: structures of at
- * least min_n AOs (and 64..560) take it; 0 (default): the one-CTA kernel
- * reduces every size.  Applies to batches built afterwards.  tb_sygvd_batch
+ * 3, 4, 6 or 8 CTAs by size (the choice depends on the size only).  The
+ * default reduction streams the matrix from L2 on up to 16 CTAs per structure.
+ * min_n: structures of at least min_n AOs (and 64..560) take the shared-memory
+ * one; 0 (default): none.  Applies to batches built afterwards.  tb_sygvd_batch
  * always uses it from 64 AOs. */
 tb_status tb_calculator_set_smem_tridiag(tb_calculator* calc, int32_t min_n);
 

@@ -1347,7 +1347,7 @@ tb_status calibrate_eigensolvers(tb_calculator* c) {
 }
 
 // Measures, once per calculator, the batched throughput of the one-CTA
-// eigensolver (k_syev, implicit QL below 64 AOs) and the one-warp Jacobi
+// eigensolver below 64 AOs (k_syev_small) and the one-warp Jacobi
 // variant (k_syev_jacobi) at N = 8, 12, ..., 32: 592 deterministic random
 // symmetric matrices per size (four per SM), the same inputs for both, the
 // faster of two timed launches each.  The warp variant is chosen up to the
@@ -2986,7 +2986,8 @@ namespace {
 
 // Device workspace of one structure in a batch, following batch_build's
 // layout: 16 N^2 doubles of matrices (S, H0, D, Q, X, W, F, Z, P), 3 more N^2
-// in the mixed-precision form, the pair lists, the Broyden history and the
+// in the mixed-precision form (an upper bound: only structures on the library
+// path need them), the pair lists, the Broyden history and the
 // library workspace above the in-house size bound; 4 KiB per array of slack.
 int64_t workspace_estimate(const tb_options& o, int nat, int nsh, int nao) {
   const double n2 = (double)nao * nao;

@@ -191,8 +191,9 @@ struct SyevPlan {
   // sizes in the batch's order (decreasing; those of the library path first)
   void build(const std::vector<int>& sizes, int lib_above, int jacobi_max);
 };
-// k_syev (and k_syev_small where the plan has small structures) on st; *launches
-// counts them.  The shared-memory limits must have been raised.
+// k_syev, and k_syev_small where the plan has small structures, on st; the njac
+// structures of jlist (one-warp Jacobi) in k_syev_small's launch or, without
+// one, by k_syev_jacobi; *launches counts the launches.  The shared-memory limits must have been raised.
 cudaError_t launch_syev(const SyevPlan& P, const DevBatch& B, double* A, double* Z, double* Sb, double* w, int* perm,
                         int* status, const int* active, cudaStream_t st, int64_t* launches,
                         const int* jlist = nullptr, int njac = 0);

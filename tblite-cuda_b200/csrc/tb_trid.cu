@@ -3,9 +3,8 @@
 // dsytrd step, src/lapack/sygvd.cu:223-313; the eigenvectors follow in k_syev).
 //
 // The matrix lives in the clusters' shared memory for the whole reduction, so
-// the n - 2 Householder steps never touch L2 or DRAM: the one-CTA kernel
-// (k_syev's tridiagonalise) streams the trailing block from L2/DRAM at every
-// step and is bound by those round trips.  Layout:
+// the n - 2 Householder steps never touch L2 or DRAM (k_syev's own reduction,
+// tridiag_tiles, streams the trailing block from L2 at every step).  Layout:
 //  * the upper triangle of tiles (16 x 16 doubles, row-major, the diagonal
 //    tiles stored whole and symmetric); tile row I belongs to CTA owner[I]
 //    (greedy balance of the tile counts), and a CTA stores its tiles ordered
