@@ -23,15 +23,12 @@ __host__ __device__ constexpr int dc_ws_elems(int m) {
   return 8 * m + kDcTileElems + (7 * m * (int)sizeof(int) + (int)sizeof(T) - 1) / (int)sizeof(T);
 }
 // shared memory of k_syev: d, e, tau, v, vn, p, w (7n) + the open panel's pairs (2 n kRing);
-// in FP64 at least d, e and the divide-and-conquer workspace (from tau on) for
-// kDcMin+ rows, so that the solver chosen for a structure depends on its size only
-inline size_t syev_smem_bytes(int n, size_t elem = sizeof(double)) {
+// at least d, e and the divide-and-conquer workspace (from tau on)
+inline size_t syev_smem_bytes(int n) {
   size_t v = (7 + 2 * (size_t)kRing) * (size_t)n;
-  if (elem == sizeof(double) && n >= kDcMin) {
-    const size_t dc = 2 * (size_t)n + (size_t)dc_ws_elems<double>(n);
-    if (dc > v) v = dc;
-  }
-  return v * elem;
+  const size_t dc = 2 * (size_t)n + (size_t)dc_ws_elems<double>(n);
+  if (n >= kDcMin && dc > v) v = dc;
+  return v * sizeof(double);
 }
 constexpr int kSyevMaxN = 1216;
 // k_trid_smem (tb_trid.cu): the tridiagonalisation of FP64 structures of
