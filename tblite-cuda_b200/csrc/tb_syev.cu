@@ -37,6 +37,7 @@ namespace tb {
 namespace {
 
 constexpr double kEps = 2.220446049250313e-16;
+constexpr double kSqrt2 = 1.4142135623730951;
 constexpr int kPanel = 8;    // reflectors per tridiagonalisation panel
 constexpr int kQBlock = 16;  // reflectors per compact-WY block of the Q accumulation
 constexpr int kWarps = kEigThreads / 32;
@@ -685,12 +686,15 @@ __device__ __forceinline__ void form_q(const double* A, double* Z, int n, const 
 // of a halving tree down to leaves of at most kDcLeaf rows; the eigenvector
 // matrix G of each node (rows = eigenvectors in T's index space, an m x m
 // diagonal block of an n x n buffer) is built bottom-up by rank-one merges:
-//  * z = [last column of G_left ; sign(e) * first column of G_right], unit
-//    norm, rho' = |e| |z|^2; eigenvalues sorted;
-//  * deflation (tolerance 8 eps max(|delta|max, rho')): entries with rho'|z_i|
-//    below it keep their eigenpair; adjacent close pairs are rotated so that
-//    one z entry vanishes (LAPACK dlaed2's two tests);
-//  * roots of the secular equation 1 + rho' sum z_i^2 / (delta_i - lambda) = 0
+//  * z = [last column of G_left ; sign(e) * first column of G_right], of norm
+//    sqrt(2) (columns of orthogonal matrices) and left so: divided by its norm,
+//    which rounds the same way in every merge, the rank-one term came out short
+//    by up to 0.8 eps (dense matrices of 256 rows lost 0.65 eps of their
+//    Frobenius norm); eigenvalues sorted;
+//  * deflation (tolerance 8 eps max(|delta|max, 2 rho), 2 rho = rho |z|^2):
+//    entries with sqrt(2) rho |z_i| below it keep their eigenpair; adjacent close pairs
+//    are rotated so that one z entry vanishes (LAPACK dlaed2's two tests);
+//  * roots of the secular equation 1 + rho sum z_i^2 / (delta_i - lambda) = 0
 //    by bracketed two-pole rational interpolation (Bunch, Nielsen and Sorensen
 //    1978), each root kept as (nearest pole, offset) so that delta_i - lambda
 //    keeps full relative accuracy;
@@ -727,7 +731,9 @@ __device__ __forceinline__ double team_mul(double v, unsigned mask) {
 // start solves the equation with the other terms frozen at the interval's
 // middle (for the last root, half way to its upper bound), each step replaces
 // the terms up to p and those beyond by one pole each with the same value and
-// slope; a step out of the bracket bisects it.
+// slope; a step out of the bracket bisects it.  An accepted root takes the Newton
+// step of its last evaluation: below the acceptance bound (8 eps of the terms)
+// the iterates still lie to one side.
 template <int T>
 __device__ __forceinline__ void secular_root(int j, int k, const double* dl, const double* z, double rho, int sub, unsigned mask,
                              int* o_out, double* tau_out) {
@@ -787,7 +793,11 @@ __device__ __forceinline__ void secular_root(int j, int k, const double* dl, con
     dpsi = rho * team_sum<T>(dpsi, mask); dphi = rho * team_sum<T>(dphi, mask);
     const double f = 1.0 + psi + phi;
     const double err = kEps * (8.0 * (fabs(psi) + fabs(phi)) + 3.0 + fabs(tau) * (dpsi + dphi));
-    if (fabs(f) <= err) break;
+    if (fabs(f) <= err) {
+      const double tn = tau - f * dc_rcp(dpsi + dphi);
+      if (tn > lo && tn < hi) tau = tn;
+      break;
+    }
     if (f < 0.0) lo = tau; else hi = tau;
     if (hi - lo <= 2.0 * kEps * fmax(fabs(lo), fabs(hi))) break;
     // psi ~ c1 + s1 / (a - eta), phi ~ c2 + s2 / (b - eta)
@@ -895,7 +905,7 @@ __device__ __noinline__ void dc_merge(int dofs, int eofs, int n, int ld, int lo,
   const int gw = g.rank * kWarps + wid, ngw = g.size * kWarps;
   const int m = hi - lo;
   double* delta = ws;          // m: sorted eigenvalues (rotated pairs updated)
-  double* zs = delta + m;      // m: sorted z (unit norm)
+  double* zs = delta + m;      // m: sorted z
   double* dl = zs + m;         // k: non-deflated delta
   double* zl = dl + m;         // k: their z, then the recomputed z
   double* tv = zl + m;         // k: root offsets
@@ -912,24 +922,20 @@ __device__ __noinline__ void dc_merge(int dofs, int eofs, int n, int ld, int lo,
   int* ori = rq + m;      // k: root origin (index into dl)
   int* srow = ori + m;    // k: row of non-deflated entry
   __shared__ int s_k, s_nrot;
-  __shared__ double red[kWarps];
   const double ev = e[t - 1];
   const double rho = fabs(ev), sg = ev >= 0.0 ? 1.0 : -1.0;
   // children's blocks are diagonal sub-blocks: clear the rest of the node's block
   if (V == Gi)
     for (int r = lo + gw; r < hi; r += ngw)
       for (int c = (r < t ? t : lo) + lane; c < (r < t ? hi : t); c += 32) Gi[(long long)r * ld + c] = 0.0;
-  // z and its norm (in rc until the rotations are formed)
-  double part = 0.0;
+  // z (in rc until the rotations are formed)
   for (int r = lo + tid; r < hi; r += kEigThreads) {
     const double z = r < t ? Gi[(long long)r * ld + t - 1] : sg * Gi[(long long)r * ld + t];
     rc[r - lo] = z;
     rowof[r - lo] = r;  // valid rows even where non-finite eigenvalues leave ranks unset below
     delta[r - lo] = zs[r - lo] = 0.0;
-    part += z * z;
   }
-  const double zz = block_sum_once(part, red);
-  const double zsc = 1.0 / sqrt(zz), rhop = rho * zz;
+  __syncthreads();
   // rank sort of the eigenvalues (ties by index)
   for (int r = lo + tid; r < hi; r += kEigThreads) {
     const double dr = d[r];
@@ -940,7 +946,7 @@ __device__ __noinline__ void dc_merge(int dofs, int eofs, int n, int ld, int lo,
     }
     rowof[rank] = r;
     delta[rank] = dr;
-    zs[rank] = rc[r - lo] * zsc;
+    zs[rank] = rc[r - lo];
   }
   __syncthreads();
   if (tid < 32) {  // deflation scan and compaction, warp 0
@@ -948,11 +954,11 @@ __device__ __noinline__ void dc_merge(int dofs, int eofs, int n, int ld, int lo,
     for (int s = lane; s < m; s += 32) dmax = fmax(dmax, fabs(delta[s]));
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) dmax = fmax(dmax, __shfl_xor_sync(0xffffffffu, dmax, o));
-    const double tol = 8.0 * kEps * fmax(dmax, rhop);
+    const double tol = 8.0 * kEps * fmax(dmax, 2.0 * rho);
     int kc = 0;  // entries with a z of their own, in order (in ndl)
     for (int s0 = 0; s0 < m; s0 += 32) {
       const int s = s0 + lane;
-      const bool keep = s < m && !(rhop * fabs(zs[s]) <= tol);
+      const bool keep = s < m && !(kSqrt2 * rho * fabs(zs[s]) <= tol);
       if (s < m) flg[s] = keep ? 0 : 1;
       const unsigned bal = __ballot_sync(0xffffffffu, keep);
       if (keep) ndl[kc + __popc(bal & ((1u << lane) - 1u))] = s;
@@ -1042,7 +1048,7 @@ __device__ __noinline__ void dc_merge(int dofs, int eofs, int n, int ld, int lo,
   for (int j = gteam; j < k; j += nteam) {
     int o;
     double tj;
-    secular_root<4>(j, k, dl, zl, rhop, sub, mask, &o, &tj);
+    secular_root<4>(j, k, dl, zl, rho, sub, mask, &o, &tj);
     for (int r = sub; r < g.size; r += 4) {
       put_at(ori + j, o, g, r);
       put_at(tv + j, tj, g, r);
@@ -1058,7 +1064,7 @@ __device__ __noinline__ void dc_merge(int dofs, int eofs, int n, int ld, int lo,
 #pragma unroll 4
     for (int j = sub; j < k - 1; j += 4)  // root j over pole j, from the entry's own pole on j + 1
       prod *= ((dl[ori[j]] - di) + tv[j]) * dc_rcp(dl[j + (j >= i)] - di);
-    prod = team_mul(prod, mask) * (((dl[ori[k - 1]] - di) + tv[k - 1]) / rhop);
+    prod = team_mul(prod, mask) * (((dl[ori[k - 1]] - di) + tv[k - 1]) / rho);
     const double z = copysign(sqrt(fmax(prod, 0.0)), zl[i]);
     for (int r = sub; r < g.size; r += 4) put_at(zl + i, z, g, r);
   }
@@ -1134,7 +1140,7 @@ __device__ __noinline__ void dc_leaf(int dofs, int eofs, int lo0, int s, int wof
   const int lane = threadIdx.x & 31, ldw = leaf_ldw(s), sp = leaf_pad(s);
   double* W = ws;
   double* z = W + sp * ldw;
-  double* zs = z + s;      // sorted, unit norm
+  double* zs = z + s;      // sorted
   double* delta = zs + s;  // sorted eigenvalues
   double* dl = delta + s;  // per node from its lo on: the k not deflated
   double* zl = dl + s;
@@ -1178,17 +1184,10 @@ __device__ __noinline__ void dc_leaf(int dofs, int eofs, int lo0, int s, int wof
         if (r >= ra && r < rz) z[r] = f * g[r];
     }
     __syncwarp();
-    double rhop = 0.0;
-    if (act) {
-      double zz = 0.0;
-      for (int i = lo; i < hi; ++i) zz += z[i] * z[i];
-      rhop = rho * zz;
-      delta[lane] = dr;  // unsorted, for the ranks
-      zs[lane] = z[lane] * (1.0 / sqrt(zz));
-    }
-    __syncwarp();
     int rank = lane;
-    const double zr = act ? zs[lane] : 0.0;
+    const double zr = act ? z[lane] : 0.0;
+    if (act) delta[lane] = dr;  // unsorted, for the ranks
+    __syncwarp();
     if (act) {
       rank = lo;
       for (int q = lo; q < hi; ++q) {
@@ -1211,13 +1210,13 @@ __device__ __noinline__ void dc_leaf(int dofs, int eofs, int lo0, int s, int wof
     if (act && j == 0) {  // deflation scan of the node, in order (the tests of dc_merge)
       double dmax = 0.0;
       for (int i = lo; i < hi; ++i) dmax = fmax(dmax, fabs(delta[i]));
-      const double tol = 8.0 * kEps * fmax(dmax, rhop);
+      const double tol = 8.0 * kEps * fmax(dmax, 2.0 * rho);
       unsigned f = 0;
       int n = 0, prev = -1;
       double za = 0.0, da = 0.0;
       for (int i = lo; i < hi; ++i) {
         double zb = zs[i], db = delta[i];
-        if (rhop * fabs(zb) <= tol) { f |= 1u << i; continue; }
+        if (kSqrt2 * rho * fabs(zb) <= tol) { f |= 1u << i; continue; }
         if (prev >= 0) {
           const double t2 = za * za + zb * zb;
           if (fabs(db - da) * fabs(za * zb) <= tol * t2) {
@@ -1254,7 +1253,7 @@ __device__ __noinline__ void dc_leaf(int dofs, int eofs, int lo0, int s, int wof
     if (j < k) {
       int o;
       double tj;
-      secular_root<1>(j, k, dl + lo, zl + lo, rhop, 0, 0u, &o, &tj);
+      secular_root<1>(j, k, dl + lo, zl + lo, rho, 0, 0u, &o, &tj);
       ori[lane] = o;
       tv[lane] = tj;
     }
@@ -1262,7 +1261,7 @@ __device__ __noinline__ void dc_leaf(int dofs, int eofs, int lo0, int s, int wof
     double znew = 0.0;
     if (j < k) {  // Gu and Eisenstat
       const double di = dl[lane];
-      double prod = ((dl[lo + ori[lo + k - 1]] - di) + tv[lo + k - 1]) / rhop;
+      double prod = ((dl[lo + ori[lo + k - 1]] - di) + tv[lo + k - 1]) / rho;
 #pragma unroll 4
       for (int q = 0; q < k - 1; ++q)  // root q over pole q, or past the pole itself q + 1
         prod *= ((dl[lo + ori[lo + q]] - di) + tv[lo + q]) * dc_rcp(dl[lo + q + (q >= j)] - di);
