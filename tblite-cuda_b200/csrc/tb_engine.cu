@@ -1150,6 +1150,7 @@ tb_status mixed_core(tb_batch* b, cudaStream_t st, double n3_lo, double n3_hi, d
        k_gemm_tc<<<tc_grid, kTcThreads, tc_smem, st>>>(B, T128, nt128, b->X, 1, b->W, 0, nullptr, nullptr, nullptr, b->F, 1.0, 0.0, lo, S.status));
   TB_GEMM(2.0 * n3_hi, b->X, 1, b->W, 0, nullptr, nullptr, nullptr, b->F, 1.0, 0.0, hi, kGemmKUpToI | kGemmSym);
   // eigenpairs (eigenvectors as rows of Z, W as scratch)
+  TB_K("convert", 0, 0, k_symmetrize<<<gemm_grid, 256, 0, st>>>(B, T, nt, b->F, li));
   {
     const tb_status ts = launch_eigen(b, st, 4.0 * (n3_lo + n3_hi));
     if (ts != TB_OK) return ts;

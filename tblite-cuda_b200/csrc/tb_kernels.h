@@ -227,6 +227,7 @@ __global__ void k_gemm_tc(DevBatch B, const int4* tiles, int ntiles, const doubl
                           int tb_, const int* perm, const double* ks, const int* kdim, double* Cb, double alpha,
                           double beta, const int* active, int* status);
 size_t gemm_tc_smem_bytes();
+__global__ void k_symmetrize(DevBatch B, const int4* tiles, int ntiles, double* F, const int* mask);
 __global__ void k_to_f32(DevBatch B, const int4* tiles, int ntiles, const double* F, float* Af, const int* mask);
 __global__ void k_gather_vectors(DevBatch B, const int4* tiles, int ntiles, const float* Zf, const int* perm,
                                  double* V, const int* mask);

@@ -46,6 +46,39 @@ __global__ void k_phase_masks(DevBatch B, const int* __restrict__ active, const 
   }
 }
 
+// F' <- (F' + F'^T) / 2 of the masked structures.  The two triangles of a
+// TF32x3 product differ in its last bits (about 1e-7 of the norm); the eigensolvers
+// read one of them, both, or their mean, and get the same symmetric matrix this
+// way.  A CTA takes a 64 x 64 tile on or above the diagonal and its mirror image,
+// as 32 x 32 blocks through shared memory so that rows are read and written whole.
+__global__ void k_symmetrize(DevBatch B, const int4* __restrict__ tiles, int ntiles, double* __restrict__ F,
+                             const int* __restrict__ mask) {
+  __shared__ double up[32][33], low[32][33];
+  for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
+    const int4 tl = tiles[t];
+    const int m = tl.x;
+    if (!mask[m] || tl.z < tl.y) continue;
+    const int n = B.ooff[m + 1] - B.ooff[m];
+    double* f = F + B.moff[m];
+    for (int q = 0; q < 4; ++q) {
+      const int i0 = tl.y * MT + 32 * (q >> 1), j0 = tl.z * MT + 32 * (q & 1);
+      if (i0 > j0 || j0 >= n) continue;
+      __syncthreads();
+      for (int e = threadIdx.x; e < 32 * 32; e += blockDim.x) {
+        const int r = e / 32, c = e % 32;
+        if (i0 + r < n && j0 + c < n) up[r][c] = f[(long long)(i0 + r) * n + j0 + c];
+        if (j0 + r < n && i0 + c < n) low[r][c] = f[(long long)(j0 + r) * n + i0 + c];
+      }
+      __syncthreads();
+      for (int e = threadIdx.x; e < 32 * 32; e += blockDim.x) {
+        const int r = e / 32, c = e % 32;
+        if (i0 + r < n && j0 + c < n) f[(long long)(i0 + r) * n + j0 + c] = 0.5 * (up[r][c] + low[c][r]);
+        if (j0 + r < n && i0 + c < n) f[(long long)(j0 + r) * n + i0 + c] = 0.5 * (up[c][r] + low[r][c]);
+      }
+    }
+  }
+}
+
 // Af = (float) F' for the masked structures, tile by tile.
 __global__ void k_to_f32(DevBatch B, const int4* __restrict__ tiles, int ntiles, const double* __restrict__ F,
                          float* __restrict__ Af, const int* __restrict__ mask) {

@@ -81,3 +81,22 @@ def test_bad_precision_rejected(gpu_calc):
     with pytest.raises(capi.TBError) as e:
         gpu_calc.singlepoint_batch([g.octane()], precision=3)
     assert e.value.status == capi.TB_BAD_INPUT
+
+
+@pytest.mark.parametrize("waters, setter", [([1, 2, 5], "set_small_solver"), ([11, 22, 37, 64], "set_smem_tridiag")])
+def test_mixed_phase_gives_every_eigensolver_one_symmetric_matrix(waters, setter):
+    # After one iteration (the mixed phase) the orbital energies are those of F' as
+    # the TF32x3 products left it.  The eigensolvers read one of its triangles, both
+    # or their mean; two of them agree to their own rounding (a few n eps of the norm,
+    # which is below 4 here) only if the matrix they get is symmetric.
+    calc = capi.Calculator(capi.DEFAULT_PARAMS)
+    rng = np.random.default_rng(71)
+    mols = [g.water_cluster(k, rng) for k in waters]
+    emo = []
+    for on in (32 if setter == "set_small_solver" else 64, 0):
+        getattr(calc, setter)(on)
+        res = calc.singlepoint_batch(mols, precision=1, solver=1, max_iter=1, wavefunction=True)
+        assert all(r["iterations"] == 1 for r in res)
+        emo.append([np.asarray(r["wfn"]["emo"]).ravel() for r in res])
+    for a, b in zip(*emo):
+        np.testing.assert_allclose(a, b, atol=8 * len(a) * np.finfo(float).eps * 4, rtol=0)
