@@ -21,8 +21,6 @@
 // structure and re-read the finished part from L2 for every group.
 #include <cooperative_groups.h>
 
-#include <cmath>
-
 #include "tb_common.cuh"
 #include "tb_kernels.h"
 
@@ -359,20 +357,6 @@ __global__ void __launch_bounds__(kT, 2) k_factor(DevBatch B, const double* __re
     }
     cl.sync();
   }
-}
-
-namespace {
-// Time of one structure of n AOs on C CTAs, in ms: a diagonal block and the
-// two barriers of its column, and the products the CTAs divide.
-double factor_ms(double n, int C) { return 0.03 * std::ceil(n / kB) + 8.0e-9 * n * n * n / C; }
-}  // namespace
-
-void FactorPlan::build(const std::vector<int>& sizes, int lib_above) {
-  *this = FactorPlan();
-  count = (int)sizes.size();
-  int first = 0;  // structures of the library path lead the order and exit at once
-  while (first < count && lib_above != 0 && sizes[first] > lib_above) ++first;
-  if (first < count) c = choose_clusters(sizes, first, count, factor_ms, true, false);
 }
 
 cudaError_t launch_factor(const FactorPlan& P, const DevBatch& B, const double* S, double* W, double* X, int* status,

@@ -31,6 +31,7 @@ inline size_t syev_smem_bytes(int n) {
   return v * sizeof(double);
 }
 constexpr int kSyevMaxN = 1216;
+constexpr int kSyevNarrowMaxN = 449;  // largest order of the two-CTA kernel k_syev
 // k_trid_smem (tb_trid.cu): the tridiagonalisation of FP64 structures of
 // kTridMin..kTridClassMax[last] AOs held in the shared memory of a thread block
 // cluster of kTridClusterSizes[c] CTAs (class c: up to kTridClassMax[c] AOs,
@@ -141,7 +142,7 @@ cudaError_t launch_integrals(const DevParams& P, const DevBatch& B, const int* n
 // How a kernel that takes a structure on one CTA or on a cluster runs a batch:
 // clusters of `cluster` CTAs, the first ncoop structures of the order on one
 // each, then one structure per CTA; one CTA per SM (wide) or two; the modelled
-// span in ms.  ms(n, C): time of a structure of n AOs on C CTAs (tb_syev.cu).
+// span in ms.  ms(n, C): time of a structure of n AOs on C CTAs (tb_plan.cu).
 struct ClusterChoice {
   int cluster = 1, ncoop = 0;
   bool wide = true;

@@ -24,9 +24,6 @@
 // divided, their results exchanged through global memory (walk partials, Z,
 // merge blocks) or the peers' shared memory (roots, recomputed z), with one
 // cluster barrier per Householder step and three per shared merge.
-#include <algorithm>
-#include <functional>
-
 #include <cooperative_groups.h>
 
 #include "tb_common.cuh"
@@ -138,6 +135,7 @@ __device__ __forceinline__ double dc_rcp(double x) {
 // of a cluster without a unit: 138 AOs alone 1.03 ms against 0.87, 384 3.40
 // against 2.87, 722 10.2 against 8.2, for 3% on a batch of one CTA each.
 constexpr int kWalk1 = 224, kWalk2 = 448;  // 16 x 32, 16 x 64, above: 32 x 128
+static_assert(kSyevNarrowMaxN == kWalk2 + 1, "k_syev has no walk of the third shape");
 __host__ __device__ constexpr int parts(int nm, int shift) { return (nm + (1 << shift) - 1) >> shift; }
 
 // Position in the unit list of one warp: units are numbered strip by strip.
@@ -1890,84 +1888,6 @@ __global__ void __launch_bounds__(kEigThreads, 2) k_syev_small(DevBatch B, const
 }
 
 TB_OOB_EXPORT(oob_syev)
-
-namespace {
-// Time of one structure of n AOs on a group of C CTAs, in ms: what each CTA
-// repeats or waits for (the steps' barriers, gathers and scalars, a merge's
-// sort and scan), plus what they divide.  Measured on one structure alone with
-// one CTA per SM, at 138, 384, 722, 1196 AOs: 1.1, 7.8, 41, 156 ms on one CTA;
-// 0.85, 4.8, 23, 84 on two; 0.72, 3.3, 13.5, 47 on four; 0.75, 2.6, 9.0, 29 on
-// eight; 0.74, 2.5, 7.2, 20 on sixteen.
-double syev_ms(double n, int C) {
-  const double serial = n * (4.6e-3 + 2.05e-6 * n), shared = n * n * (6.6e-6 + 8.55e-8 * n);
-  return serial + shared / C;
-}
-}  // namespace
-
-// The combination with the shortest modelled span.  A span is list scheduling of
-// the order (largest first) over as many clusters as the GPU holds at once
-// (kCap: cudaOccupancyMaxActiveClusters on a B200, one and two CTAs per SM) for
-// every cluster size and a geometric set of splits into cluster and one-CTA
-// structures.  Two CTAs on an SM slow each other (kSlowTwo; the narrower
-// kernel alone, kSlowNarrow).  400 water clusters of 48..384 AOs: 13.3 ms on
-// one CTA each, 11.0 on two; 128: 11.1 and 6.2 (on four); 48 chains of
-// 122..1196 AOs: 172 and 40 (on eight) -- with the walks before their one
-// comparison per entry; the ratios since are the same.  Batches of several waves of CTAs keep
-// one CTA per structure: clusters repeat work and would only lose.
-ClusterChoice choose_clusters(const std::vector<int>& sizes, int first, int last, double (*ms)(double, int),
-                              bool two_per_sm, bool one_per_sm) {
-  ClusterChoice best;
-  std::vector<double> busy;  // finish times of the clusters in flight (a heap)
-  auto schedule = [&](int cap, int C, int k, double slow, double limit) {
-    busy.clear();
-    double end = 0.0;
-    for (int i = first; i < last && end < limit;) {
-      const bool coop = C > 1 && i < k;
-      double t = slow * ms(sizes[i], coop ? C : 1);
-      i += coop ? 1 : C;
-      if ((int)busy.size() == cap) {
-        std::pop_heap(busy.begin(), busy.end(), std::greater<double>());
-        t += busy.back();
-        busy.pop_back();
-      }
-      busy.push_back(t);
-      std::push_heap(busy.begin(), busy.end(), std::greater<double>());
-      end = std::max(end, t);
-    }
-    return end;
-  };
-  constexpr int kCap[2][5] = {{148, 74, 33, 15, 7}, {296, 148, 71, 33, 14}};
-  constexpr double kSlowTwo = 1.42, kSlowNarrow = 1.1;
-  const int cnt = last - first;
-  best.span = 1e300;
-  for (int per = two_per_sm ? 2 : 1; per >= (one_per_sm ? 1 : 2); --per)
-    for (int c = 0; c < 5; ++c) {
-      const int C = 1 << c;
-      if (C > 1 && cnt > 4 * 148) break;
-      for (int k = cnt; k >= 1; k = k > 1 ? (3 * k) / 4 : 0) {
-        const int items = C > 1 ? k + (cnt - k + C - 1) / C : cnt;
-        const double slow = per == 1 ? 1.0 : items > kCap[0][c] ? kSlowTwo : kSlowNarrow;
-        const double t = schedule(kCap[per - 1][c], C, first + k, slow, best.span);
-        if (t < 0.97 * best.span) best = {C, C > 1 ? first + k : 0, per == 1, t};
-        if (C == 1) break;
-      }
-    }
-  return best;
-}
-
-void SyevPlan::build(const std::vector<int>& sizes, int lib_above, int jacobi_max) {
-  *this = SyevPlan();
-  int first = 0;  // structures of the library path lead the order and exit at once
-  for (size_t i = 0; i < sizes.size(); ++i) {
-    const int n = sizes[i];
-    if (lib_above != 0 && n > lib_above) { first = n64 = (int)i + 1; continue; }
-    nmax = n > nmax ? n : nmax;
-    if (n >= kDcMin) n64 = (int)i + 1;
-    else if (n > jacobi_max) { ++nsmall; small_max = std::max(small_max, n); }
-  }
-  if (n64 > first)
-    c = choose_clusters(sizes, first, n64, syev_ms, nmax <= kWalk2 + 1, true);
-}
 
 cudaError_t launch_syev(const SyevPlan& P, const DevBatch& B, double* A, double* Z, double* Sb, double* w, int* perm,
                         int* status, const int* active, cudaStream_t st, int64_t* launches, const int* jlist,
