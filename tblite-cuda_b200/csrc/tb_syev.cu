@@ -1859,7 +1859,7 @@ __global__ void __launch_bounds__(kEigThreads, 2) k_syev_small(DevBatch B, const
     __syncthreads();
   }
   for (int i = tid; i < n; i += kEigThreads)
-    if (!(fabs(d[i]) < 1e30)) q_fail = 1;  // non-finite input
+    if (n > 1 && !isfinite(d[i])) q_fail = 1;  // non-finite input (one row is its own eigenvalue, whatever it holds)
   __syncthreads();
   if (q_fail) {
     if (tid == 0) status[m] = kStEigenFailed;  // k_fermi retires the structure

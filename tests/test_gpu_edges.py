@@ -60,3 +60,15 @@ def test_eigensolver_at_the_inhouse_limit():
         np.testing.assert_allclose(w, np.linalg.eigvalsh(Sih @ H @ Sih), atol=1e-10)
         np.testing.assert_allclose(Cm.T @ S @ Cm, np.eye(len(w)), atol=1e-9)
         np.testing.assert_allclose(H @ Cm, S @ Cm * w[None, :], atol=1e-9)
+
+
+@pytest.mark.parametrize("n", [1, 2, 13, 40, 63])
+def test_sygvd_small_matrix_of_any_finite_scale(n):
+    # below 64 AOs only what is not finite is refused (squares of 1e40 are far from overflow)
+    rng = np.random.default_rng(n)
+    a = rng.standard_normal((n, n))
+    H = 0.5e40 * (a + a.T)
+    st, out = capi.sygvd_batch([H], [np.eye(n)])
+    assert st == capi.TB_OK
+    norm = np.abs(H).sum(axis=1).max()
+    np.testing.assert_allclose(out[0][0], np.linalg.eigvalsh(H), atol=8 * n * np.finfo(float).eps * norm, rtol=0)
