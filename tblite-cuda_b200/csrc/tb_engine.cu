@@ -296,10 +296,8 @@ struct tb_calculator {
   // eigensolver cost models for the automatic per-size choice (see choose_lib_above)
   struct EigModel {
     bool ready = false;
-    double a = 0, b = 0;  // in-house latency of one structure: a N^2 + b N^3 seconds
-    double c = 0, d = 0;  // one cuSOLVER call: c + d N seconds
     double t_in[2] = {0, 0}, t_lib[2] = {0, 0};  // the measured points (256/512 and 256/1024 AOs)
-    double scale = 1;  // measured in-house time over SyevPlan's model, mean of the two points
+    SolverModel model;  // cuSOLVER's line through its points; in-house over SyevPlan's model, mean of its two
   } eig;
   // small structures: the one-warp Jacobi variant against the one-CTA
   // eigensolver, measured once per calculator (batched throughput per size)
@@ -484,36 +482,14 @@ tb_status calibrate_eigensolvers(tb_calculator* c);
 tb_status calibrate_small(tb_calculator* c);
 tb_status calibrate_tiles(tb_calculator* c);
 
-// Automatic eigensolver choice for a batch (tb_options.solver = 0): the k
-// largest structures go to cuSOLVER, the rest to the batched in-house solver,
-// with k minimising the modelled time of one SCF iteration's eigensolve:
-//   sum_{i<k} t_lib(N_i) + span(N_k, N_{k+1}, ...)
-// (library calls run one after another, then k_syev runs the rest; t_lib is
-// measured once per calculator, span is the plan's model scaled by the
-// measured in-house times).  Returns lib_above: structures with more AOs go
-// to the library.
-int choose_lib_above(tb_calculator* c, std::vector<int> sizes) {
-  std::sort(sizes.begin(), sizes.end(), std::greater<int>());
-  const int nmol = (int)sizes.size();
-  int k0 = 0;
-  while (k0 < nmol && sizes[k0] > kSyevMaxN) ++k0;
-  if (k0 == nmol) return -1;
-  if (sizes[k0] < 384) return kSyevMaxN;  // small structures: the batched solver always wins
-  if (calibrate_eigensolvers(c) != TB_OK) return kSyevMaxN;
-  const auto& M = c->eig;
-  auto t_lib = [&](double n) { return M.c + M.d * n; };
-  double lib_sum = 0.0, best = 1e300;
-  int best_k = k0;
-  for (int i = 0; i < k0; ++i) lib_sum += t_lib(sizes[i]);
-  for (int k = k0; k <= nmol && lib_sum < best; ++k) {
-    SyevPlan rest;
-    rest.build(std::vector<int>(sizes.begin() + k, sizes.end()), 0, 0);
-    const double in_t = 1e-3 * rest.c.span * M.scale;
-    if (lib_sum + in_t < best) { best = lib_sum + in_t; best_k = k; }
-    if (k < nmol) lib_sum += t_lib(sizes[k]);
-  }
-  if (best_k == nmol) return -1;
-  return best_k == 0 ? kSyevMaxN : sizes[best_k];
+// Automatic eigensolver choice for a batch (tb_options.solver = 0): lib_above,
+// where structures with more AOs go to the library.  The two solvers are measured
+// on the calculator's first batch that offers a choice.
+int choose_lib_above(tb_calculator* c, const std::vector<int>& sizes) {
+  bool choice = false;
+  for (int n : sizes) choice |= n >= kLibMinN && n <= kSyevMaxN;
+  if (choice && calibrate_eigensolvers(c) != TB_OK) return kSyevMaxN;
+  return tb::choose_lib_above(sizes, c->eig.model);
 }
 
 // Build index maps, lay out the workspace, allocate, upload.
@@ -1230,8 +1206,8 @@ tb_status raise_smem_limits() {
 }
 
 // Measures the two eigensolvers once per calculator: the in-house k_syev on
-// one structure (latency, at 256 and 512 AOs, fitted by a N^2 + b N^3) and one
-// cuSOLVER syevd call (at 256 and 1024 AOs, fitted by c + d N: its calls are
+// one structure (latency, at 256 and 512 AOs, against SyevPlan's model) and one
+// cuSOLVER syevd call (at 256 and 1024 AOs, a line between them: its calls are
 // bound by the launches of its steps, 3.9 ms at 384 AOs and 8.5 at 722), on
 // deterministic random symmetric matrices.
 tb_status calibrate_eigensolvers(tb_calculator* c) {
@@ -1328,19 +1304,14 @@ tb_status calibrate_eigensolvers(tb_calculator* c) {
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   if (st != TB_OK) return st;
-  // t = a n^2 + b n^3 through (256, t1), (512, t2); t = c + d n through (256, l1), (1024, l2)
-  const double n1 = 256, n2 = 512, m1 = 256, m2 = NL;
-  const double det = n1 * n1 * n2 * n2 * n2 - n2 * n2 * n1 * n1 * n1;
-  c->eig.a = std::max(0.0, (t1 * n2 * n2 * n2 - t2 * n1 * n1 * n1) / det);
-  c->eig.b = std::max(0.0, (n1 * n1 * t2 - n2 * n2 * t1) / det);
-  c->eig.d = std::max(0.0, (l2 - l1) / (m2 - m1));
-  c->eig.c = l1 - c->eig.d * m1;
+  c->eig.model.lib256 = l1;
+  c->eig.model.lib_slope = std::max(0.0, (l2 - l1) / (NL - 256));
   c->eig.t_in[0] = t1; c->eig.t_in[1] = t2;
   {
     SyevPlan p1, p2;
     p1.build({256}, 0, 0);
     p2.build({512}, 0, 0);
-    c->eig.scale = 500.0 * (t1 / p1.c.span + t2 / p2.c.span);
+    c->eig.model.scale = 500.0 * (t1 / p1.c.span + t2 / p2.c.span);
   }
   c->eig.t_lib[0] = l1; c->eig.t_lib[1] = l2;
   c->eig.ready = true;
@@ -2398,8 +2369,9 @@ int32_t tb_calculator_tuning(const tb_calculator* c, char* buf, int32_t len) {
   o << "]}, \"large\": {\"measured\": " << (c->eig.ready ? "true" : "false")
     << ", \"inhouse_s\": {\"256\": " << c->eig.t_in[0] << ", \"512\": " << c->eig.t_in[1] << "}"
     << ", \"cusolver_s\": {\"256\": " << c->eig.t_lib[0] << ", \"1024\": " << c->eig.t_lib[1] << "}"
-    << ", \"model\": {\"inhouse\": \"" << c->eig.a << " N^2 + " << c->eig.b << " N^3\", \"cusolver\": \""
-    << c->eig.c << " + " << c->eig.d << " N\"}, \"inhouse_limit\": " << kSyevMaxN << "}"
+    << ", \"model\": {\"inhouse_over_plan\": " << c->eig.model.scale << ", \"cusolver\": \""
+    << c->eig.model.lib256 << " + " << c->eig.model.lib_slope << " (N - 256)\", \"smallest\": " << kLibMinN
+    << "}, \"inhouse_limit\": " << kSyevMaxN << "}"
     << ", \"smem_tridiag\": {\"min_n\": " << c->smem_tridiag << ", \"classes\": [";
   for (int k = 0; k < kTridClasses; ++k)
     o << (k ? ", " : "") << "{\"cluster\": " << kTridClusterSizes[k] << ", \"max_n\": " << kTridClassMax[k]

@@ -189,6 +189,17 @@ struct SyevPlan {
   // sizes in the batch's order (decreasing; those of the library path first)
   void build(const std::vector<int>& sizes, int lib_above, int jacobi_max);
 };
+// Measured by a calculator: seconds of a cuSOLVER call for N >= 256 AOs,
+// lib256 + lib_slope (N - 256), and of k_syev over SyevPlan's modelled span.
+struct SolverModel {
+  double lib256 = 0, lib_slope = 0;
+  double scale = 1;
+};
+// Automatic eigensolver choice for a batch: lib_above, where structures with
+// more AOs go to cuSOLVER (-1: all).  Structures below kLibMinN AOs never do
+// while others stay in-house.
+constexpr int kLibMinN = 384;
+int choose_lib_above(std::vector<int> sizes, const SolverModel& M);
 // k_syev, and k_syev_small where the plan has small structures, on st; the njac
 // structures of jlist (one-warp Jacobi) in k_syev_small's launch or, without
 // one, by k_syev_jacobi; *launches counts the launches.  The shared-memory limits must have been raised.

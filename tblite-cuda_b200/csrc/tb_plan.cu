@@ -86,6 +86,34 @@ void SyevPlan::build(const std::vector<int>& sizes, int lib_above, int jacobi_ma
     c = choose_clusters(sizes, first, n64, syev_ms, nmax <= kSyevNarrowMaxN, true);
 }
 
+// The k largest structures go to cuSOLVER, the rest to the batched in-house
+// solvers, with k minimising the modelled time of one SCF iteration's eigensolve:
+//   sum_{i<k} t_lib(N_i) + span(N_k, N_{k+1}, ...)
+// (library calls run one after another, then k_syev runs the rest).  k stops at
+// the first structure below kLibMinN: alone, 256 AOs take 1.4 ms in-house and 2.3
+// in cuSOLVER, 384 AOs 2.4 and 3.9, and in a batch the calls add up while the
+// in-house structures run beside one another.  So every k leaves the structures
+// below 64 AOs in-house; k_syev_small's time for them is a constant of the sum and left out.
+int choose_lib_above(std::vector<int> sizes, const SolverModel& M) {
+  std::sort(sizes.begin(), sizes.end(), std::greater<int>());
+  const int nmol = (int)sizes.size();
+  int k0 = 0;
+  while (k0 < nmol && sizes[k0] > kSyevMaxN) ++k0;
+  if (k0 == nmol) return -1;
+  double lib_sum = 0.0, best = 1e300;  // (the k0 structures above the in-house limit count the same for every k)
+  int best_k = k0;
+  for (int k = k0; lib_sum < best; ++k) {
+    SyevPlan rest;
+    rest.build(std::vector<int>(sizes.begin() + k, sizes.end()), 0, 0);
+    const double in_t = 1e-3 * rest.c.span * M.scale;
+    if (lib_sum + in_t < best) { best = lib_sum + in_t; best_k = k; }
+    if (k == nmol || sizes[k] < kLibMinN) break;
+    lib_sum += M.lib256 + M.lib_slope * (sizes[k] - 256);
+  }
+  if (best_k == nmol) return -1;
+  return best_k == k0 ? kSyevMaxN : sizes[best_k];
+}
+
 namespace {
 // Time of one structure of n AOs on C CTAs, in ms: a diagonal block and the
 // two barriers of its column, and the products the CTAs divide.

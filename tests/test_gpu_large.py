@@ -102,3 +102,16 @@ def test_automatic_solver_choice_matches_inhouse(gpu_calc):
         assert a["status"] == b["status"] == 0
         assert abs(a["energy"] - b["energy"]) < E_TOL
         np.testing.assert_allclose(a["qat"], b["qat"], atol=Q_TOL)
+
+
+def test_automatic_choice_leaves_small_structures_in_house(gpu_calc):
+    # one long chain (1190 AOs) with small molecules beside it: whichever solver the
+    # chain gets, theirs stays the batched one, so their bits are those of a call alone
+    rng = np.random.default_rng(12)
+    small = [g.alkane(n, rng) for n in (2, 3, 7, 9, 10, 11)] + g.water_clusters(14, seed=32, nmin=1, nmax=12)
+    batch = gpu_calc.singlepoint_batch([g.alkane(198, rng)] + small, solver=0)
+    assert batch[0]["status"] == 0 and batch[0]["nao"] == 1190
+    for m, r in zip(small, batch[1:]):
+        alone = gpu_calc.singlepoint_batch([m], solver=0)[0]
+        assert r["status"] == 0 and r["energy"] == alone["energy"] and r["iterations"] == alone["iterations"]
+        np.testing.assert_array_equal(r["qat"], alone["qat"])
