@@ -29,8 +29,13 @@ double syev_ms(double n, int C) {
 // kernel alone, kSlowNarrow).  400 water clusters of 48..384 AOs: 13.3 ms on
 // one CTA each, 11.0 on two; 128: 11.1 and 6.2 (on four); 48 chains of
 // 122..1196 AOs: 172 and 40 (on eight) -- with the walks before their one
-// comparison per entry; the ratios since are the same.  Batches of several waves of CTAs keep
-// one CTA per structure: clusters repeat work and would only lose.
+// comparison per entry; the ratios since are the same.  Where one CTA
+// per structure is within 3% of the CTAs' total work (a batch of several waves of
+// like sizes) no clusters are tried: they repeat work and would only lose.  (The
+// number of structures is no such rule: with clusters for at most 592 of them, 8
+// chains of 602 AOs with 640 of 66..120 took 175 ms a call, now 62; a chain of
+// 1196 with 600 of 66 AOs, in-house, 981 and 165; 620 clusters of 66..384 AOs 136
+// either way.)
 ClusterChoice choose_clusters(const std::vector<int>& sizes, int first, int last, double (*ms)(double, int),
                               bool two_per_sm, bool one_per_sm) {
   ClusterChoice best;
@@ -57,10 +62,14 @@ ClusterChoice choose_clusters(const std::vector<int>& sizes, int first, int last
   constexpr double kSlowTwo = 1.42, kSlowNarrow = 1.1;
   const int cnt = last - first;
   best.span = 1e300;
+  // what no plan can undercut: the one-CTA times over the CTAs (clusters only add work)
+  double least = 0.0;
+  for (int i = first; i < last; ++i) least += ms(sizes[i], 1);
+  least *= std::min(kSlowTwo / kCap[1][0], 1.0 / kCap[0][0]);
   for (int per = two_per_sm ? 2 : 1; per >= (one_per_sm ? 1 : 2); --per)
     for (int c = 0; c < 5; ++c) {
       const int C = 1 << c;
-      if (C > 1 && cnt > 4 * 148) break;
+      if (C > 1 && 0.97 * best.span <= least) break;
       for (int k = cnt; k >= 1; k = k > 1 ? (3 * k) / 4 : 0) {
         const int items = C > 1 ? k + (cnt - k + C - 1) / C : cnt;
         const double slow = per == 1 ? 1.0 : items > kCap[0][c] ? kSlowTwo : kSlowNarrow;

@@ -84,3 +84,16 @@ def test_a_single_large_structure_beside_small_ones_goes_to_the_library(plan):
                                            ([1300, 2000], -1), ([2000, 60], 1216)])
 def test_ends_of_the_range(plan, sizes, expect):
     assert plan(sizes)["lib_above"] == expect
+
+
+@pytest.mark.parametrize("large, small", [([1196], 66), ([1000] * 10, 66), ([384], 100)])
+def test_a_few_large_structures_keep_their_clusters_in_any_number_of_small_ones(plan, large, small):
+    # ten more small structures add little to a plan whose span is its large ones'
+    spans = [plan(large + [small] * k)["span"] for k in (560, 580, 590, 600, 620)]
+    assert max(spans) <= 1.1 * min(spans)
+    assert plan(large + [small] * 600)["cluster"] > 1
+
+
+def test_waves_of_like_structures_take_one_cta_each(plan):
+    assert plan([6 * (11 + i * 53 // 899) for i in range(900)])["cluster"] == 1
+    assert plan([100] * 5000 + [384])["cluster"] == 1
