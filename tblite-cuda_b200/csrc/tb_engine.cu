@@ -883,8 +883,8 @@ tb_status batch_build(tb_calculator* calc, const tb_structure* mols, int nmol, c
   {
     std::vector<int> sizes(nmol);
     for (int i = 0; i < nmol; ++i) sizes[i] = b->h_ooff[order[i] + 1] - b->h_ooff[order[i]];
-    b->syev.build(sizes, lib_above, jacobi_max);
-    b->fac.build(sizes, lib_above);
+    b->syev.build(sizes.data(), nmol, lib_above, jacobi_max);
+    b->fac.build(sizes.data(), nmol, lib_above);
   }
   if (!jlist.empty()) put(o_jlist, jlist.data(), jlist.size() * I4);
   if (!b->trid.list.empty()) put(o_tlist, b->trid.list.data(), b->trid.list.size() * I4);
@@ -1270,7 +1270,7 @@ tb_status calibrate_eigensolvers(tb_calculator* c) {
           TB_CUDA(launch_trid(B, at<double>(base, oA), at<double>(base, oW), at<int>(base, os), nullptr,
                               at<int>(base, ol), 1, kTridClusterSizes[cl], n, 0));
       SyevPlan sp;
-      sp.build({n}, 0, 0);
+      sp.build(&n, 1, 0, 0);
       TB_CUDA(launch_syev(sp, B, at<double>(base, oA), at<double>(base, oZ), at<double>(base, oW),
                           at<double>(base, ow), at<int>(base, op), at<int>(base, os), nullptr, 0, nullptr));
       TB_CUDA(cudaEventRecord(e1));
@@ -1309,8 +1309,9 @@ tb_status calibrate_eigensolvers(tb_calculator* c) {
   c->eig.t_in[0] = t1; c->eig.t_in[1] = t2;
   {
     SyevPlan p1, p2;
-    p1.build({256}, 0, 0);
-    p2.build({512}, 0, 0);
+    const int m1 = 256, m2 = 512;
+    p1.build(&m1, 1, 0, 0);
+    p2.build(&m2, 1, 0, 0);
     c->eig.model.scale = 500.0 * (t1 / p1.c.span + t2 / p2.c.span);
   }
   c->eig.t_lib[0] = l1; c->eig.t_lib[1] = l2;
@@ -2769,8 +2770,8 @@ struct MatBatch {
     for (int m = 0; m < nmat; ++m) order[m] = m;
     std::stable_sort(order.begin(), order.end(), [&](int a, int c) { return n[a] > n[c]; });
     for (int i = 0; i < nmat; ++i) sorted[i] = n[order[i]];
-    syev.build(sorted, kSyevMaxN, 0);
-    fac.build(sorted, kSyevMaxN);
+    syev.build(sorted.data(), nmat, kSyevMaxN, 0);
+    fac.build(sorted.data(), nmat, kSyevMaxN);
     Layout L;
     size_t o_ooff = L.add((nmat + 1) * 4), o_moff = L.add((nmat + 1) * 8), o_t = L.add(tiles.size() * sizeof(int4));
     size_t o_ord = L.add(nmat * 4);

@@ -148,8 +148,8 @@ struct ClusterChoice {
   bool wide = true;
   double span = 0.0;
 };
-ClusterChoice choose_clusters(const std::vector<int>& sizes, int first, int last, double (*ms)(double, int),
-                              bool two_per_sm, bool one_per_sm);
+ClusterChoice choose_clusters(const int* sizes, int first, int last, double (*ms)(double, int), bool two_per_sm,
+                              bool one_per_sm);
 
 // S = L L^T (W[k][i] = L[i][k]) and X = L^-T, 64 x 64 blocks (tb_factor.cu); a
 // structure whose S is not positive definite gets kStNotSpd
@@ -158,8 +158,9 @@ __global__ void k_factor(DevBatch B, const double* S, double* Wb, double* Xb, in
 struct FactorPlan {
   int count = 0;  // structures
   ClusterChoice c;
-  // sizes in the batch's order (decreasing; those of the library path first)
-  void build(const std::vector<int>& sizes, int lib_above);
+  // sizes in the batch's order (decreasing; those of the library path first); one
+  // structure allocates nothing, and so throws nothing
+  void build(const int* sizes, int count, int lib_above);
 };
 size_t factor_smem_bytes();
 // the shared-memory limit must have been raised
@@ -186,8 +187,9 @@ struct SyevPlan {
   int nsmall = 0, small_max = 1;  // structures below kDcMin AOs that k_syev_small solves, the largest
   ClusterChoice c;      // wide: k_syev_wide
   int nmax = 0;         // largest in-house structure
-  // sizes in the batch's order (decreasing; those of the library path first)
-  void build(const std::vector<int>& sizes, int lib_above, int jacobi_max);
+  // sizes in the batch's order (decreasing; those of the library path first); one
+  // structure allocates nothing, and so throws nothing
+  void build(const int* sizes, int count, int lib_above, int jacobi_max);
 };
 // Measured by a calculator: seconds of a cuSOLVER call for N >= 256 AOs,
 // lib256 + lib_slope (N - 256), and of k_syev over SyevPlan's modelled span.

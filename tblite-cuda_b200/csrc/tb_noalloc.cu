@@ -151,7 +151,7 @@ extern "C" tb_status tb_sygvd_noalloc(int32_t n, const double* H, const double* 
   const int nt = (n + 63) / 64, ntiles = nt * nt;
   k_noalloc_init<<<1, 64, 0, st>>>(base, n);
   FactorPlan fp;
-  fp.build({n}, 0);
+  fp.build(&n, 1, 0);
   e = launch_factor(fp, B, S, v.W, v.X, v.status, st);
   if (e != cudaSuccess) return noalloc_fail(TB_CUDA_ERROR, cudaGetErrorString(e));
   // A = X^T H X (T = H X kept in W, whose Cholesky factor is no longer needed)
@@ -160,7 +160,7 @@ extern "C" tb_status tb_sygvd_noalloc(int32_t n, const double* H, const double* 
   k_gemm<<<ntiles, kGemmThreads, 0, st>>>(B, v.tiles, ntiles, v.X, 1, v.W, 0, nullptr, nullptr, nullptr, v.A, 1.0, 0.0,
                                  v.active, kGemmKUpToI | kGemmSym);
   SyevPlan sp;
-  sp.build({n}, 0, 0);
+  sp.build(&n, 1, 0, 0);
   e = launch_syev(sp, B, v.A, v.Z, v.W, w, v.perm, v.status, v.active, st, nullptr);
   if (e != cudaSuccess) return noalloc_fail(TB_CUDA_ERROR, cudaGetErrorString(e));
   // C = X Z with the eigenvectors in ascending order

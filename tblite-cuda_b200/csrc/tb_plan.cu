@@ -36,11 +36,12 @@ double syev_ms(double n, int C) {
 // chains of 602 AOs with 640 of 66..120 took 175 ms a call, now 62; a chain of
 // 1196 with 600 of 66 AOs, in-house, 981 and 165; 620 clusters of 66..384 AOs 136
 // either way.)
-ClusterChoice choose_clusters(const std::vector<int>& sizes, int first, int last, double (*ms)(double, int),
-                              bool two_per_sm, bool one_per_sm) {
+ClusterChoice choose_clusters(const int* sizes, int first, int last, double (*ms)(double, int), bool two_per_sm,
+                              bool one_per_sm) {
   ClusterChoice best;
   std::vector<double> busy;  // finish times of the clusters in flight (a heap)
   auto schedule = [&](int cap, int C, int k, double slow, double limit) {
+    if (last - first == 1) return slow * ms(sizes[first], C);
     busy.clear();
     double end = 0.0;
     for (int i = first; i < last && end < limit;) {
@@ -81,14 +82,14 @@ ClusterChoice choose_clusters(const std::vector<int>& sizes, int first, int last
   return best;
 }
 
-void SyevPlan::build(const std::vector<int>& sizes, int lib_above, int jacobi_max) {
+void SyevPlan::build(const int* sizes, int count, int lib_above, int jacobi_max) {
   *this = SyevPlan();
   int first = 0;  // structures of the library path lead the order and exit at once
-  for (size_t i = 0; i < sizes.size(); ++i) {
+  for (int i = 0; i < count; ++i) {
     const int n = sizes[i];
-    if (lib_above != 0 && n > lib_above) { first = n64 = (int)i + 1; continue; }
+    if (lib_above != 0 && n > lib_above) { first = n64 = i + 1; continue; }
     nmax = n > nmax ? n : nmax;
-    if (n >= kDcMin) n64 = (int)i + 1;
+    if (n >= kDcMin) n64 = i + 1;
     else if (n > jacobi_max) { ++nsmall; small_max = std::max(small_max, n); }
   }
   if (n64 > first)
@@ -113,7 +114,7 @@ int choose_lib_above(std::vector<int> sizes, const SolverModel& M) {
   int best_k = k0;
   for (int k = k0; lib_sum < best; ++k) {
     SyevPlan rest;
-    rest.build(std::vector<int>(sizes.begin() + k, sizes.end()), 0, 0);
+    rest.build(sizes.data() + k, nmol - k, 0, 0);
     const double in_t = 1e-3 * rest.c.span * M.scale;
     if (lib_sum + in_t < best) { best = lib_sum + in_t; best_k = k; }
     if (k == nmol || sizes[k] < kLibMinN) break;
@@ -129,9 +130,9 @@ namespace {
 double factor_ms(double n, int C) { return 0.03 * std::ceil(n / kFactorBlock) + 8.0e-9 * n * n * n / C; }
 }  // namespace
 
-void FactorPlan::build(const std::vector<int>& sizes, int lib_above) {
+void FactorPlan::build(const int* sizes, int nstructures, int lib_above) {
   *this = FactorPlan();
-  count = (int)sizes.size();
+  count = nstructures;
   int first = 0;  // structures of the library path lead the order and exit at once
   while (first < count && lib_above != 0 && sizes[first] > lib_above) ++first;
   if (first < count) c = choose_clusters(sizes, first, count, factor_ms, true, false);

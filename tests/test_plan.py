@@ -1,6 +1,7 @@
 """CPU: the host-side plans (tb_plan.cu), compiled into a program that launches nothing.
 
-The automatic choice sends a structure to cuSOLVER, whose calls run one after
+The plans of one structure allocate nothing, since tb_sygvd_noalloc makes them
+at a C entry.  The automatic choice sends a structure to cuSOLVER, whose calls run one after
 another, only where that shortens the modelled eigensolve; small structures
 beside a large one stay with the batched solvers.  Model coefficients as
 measured on a B200."""
@@ -18,11 +19,23 @@ PROGRAM = r"""
 #include <iostream>
 #include <string>
 #include "tb_plan.cu"
+extern int allocations;
 int main() {
+  {  // the plans of one structure, as tb_sygvd_noalloc makes them
+    tb::SyevPlan p;
+    tb::FactorPlan f;
+    const int before = allocations;
+    for (int n = 1; n <= 256; ++n) {
+      p.build(&n, 1, 0, 0);
+      f.build(&n, 1, 0);
+    }
+    std::printf("%d\n", allocations - before);
+  }
   tb::SolverModel M;
   tb::SyevPlan p, q;
-  p.build({256}, 0, 0);
-  q.build({512}, 0, 0);
+  const int m1 = 256, m2 = 512;
+  p.build(&m1, 1, 0, 0);
+  q.build(&m2, 1, 0, 0);
   M.lib256 = 2.3321e-3;
   M.lib_slope = (12.1454e-3 - 2.3321e-3) / 768;
   M.scale = 500.0 * (1.37712e-3 / p.c.span + 3.61923e-3 / q.c.span);
@@ -32,10 +45,22 @@ int main() {
     for (int& x : s) std::cin >> x;
     std::sort(s.begin(), s.end(), std::greater<int>());
     tb::SyevPlan P;
-    P.build(s, tb::kSyevMaxN, 0);
+    P.build(s.data(), n, tb::kSyevMaxN, 0);
     std::printf("%d %d %d %d %.6f\n", tb::choose_lib_above(s, M), P.c.cluster, P.c.ncoop, (int)P.c.wide, P.c.span);
   }
 }
+"""
+
+COUNT = r"""
+#include <cstdlib>
+#include <new>
+int allocations = 0;
+void* operator new(std::size_t n) {
+  ++allocations;
+  return std::malloc(n);
+}
+void operator delete(void* p) noexcept { std::free(p); }
+void operator delete(void* p, std::size_t) noexcept { std::free(p); }
 """
 
 
@@ -46,12 +71,14 @@ def plan(tmp_path_factory):
         pytest.skip("nvcc not available")
     d = tmp_path_factory.mktemp("plan")
     (d / "plan.cu").write_text(PROGRAM)
-    subprocess.run([nvcc, "-std=c++17", "-O2", "-I", CSRC, str(d / "plan.cu"), "-o", str(d / "plan")], check=True,
-                   capture_output=True, timeout=300)
+    (d / "count.cpp").write_text(COUNT)
+    subprocess.run([nvcc, "-std=c++17", "-O2", "-I", CSRC, str(d / "plan.cu"), str(d / "count.cpp"), "-o",
+                    str(d / "plan")], check=True, capture_output=True, timeout=300)
 
     def run(sizes):
         out = subprocess.run([str(d / "plan")], input=f"{len(sizes)} " + " ".join(map(str, sizes)), text=True,
                              capture_output=True, timeout=60, check=True).stdout.split()
+        assert out.pop(0) == "0"  # allocations of a plan for one structure
         return dict(lib_above=int(out[0]), cluster=int(out[1]), ncoop=int(out[2]), wide=int(out[3]),
                     span=float(out[4]))
 
