@@ -96,3 +96,45 @@ def test_mixed_form_cluster_and_one_cta_give_the_same_bits(gpu_calc):
         assert alone["energy"] == rb["energy"] and alone["iterations"] == rb["iterations"]
         np.testing.assert_array_equal(alone["qat"], rb["qat"])
         assert abs(alone["energy"] - rp["energy"]) < 1e-6  # the mixed form's bound
+
+
+# AOs of batches that k_syev (two CTAs per SM) solves: from one CTA per structure
+# throughout, and with clusters of two for the largest (tests/test_plan.py holds the plans)
+NARROW_LARGE = [446, 384, 228, 224, 222, 132, 66]
+
+
+def narrow_sizes(fill):
+    return NARROW_LARGE + [6 * (11 + i * 62 // (fill - 1)) for i in range(fill)]
+
+
+@pytest.mark.parametrize("fill", [900, 700])
+def test_narrow_kernel_gives_the_bits_of_the_wide_one(gpu_calc, fill):
+    rng = np.random.default_rng(fill)
+    sizes = narrow_sizes(fill)
+    mols = [g.alkane((n - 2) // 6, rng) if n % 6 == 2 else g.water_cluster(n // 6, rng) for n in sizes]
+    batch = gpu_calc.singlepoint_batch(mols, solver=1)
+    assert [r["nao"] for r in batch] == sizes
+    probe = list(range(len(NARROW_LARGE))) + [len(NARROW_LARGE) + i for i in range(0, fill, 90)]
+    for i in probe:  # alone: a cluster of the wide kernel
+        alone = gpu_calc.singlepoint_batch([mols[i]], solver=1)[0]
+        assert alone["status"] == batch[i]["status"] == 0
+        assert alone["energy"] == batch[i]["energy"] and alone["iterations"] == batch[i]["iterations"]
+        np.testing.assert_array_equal(alone["qat"], batch[i]["qat"])
+
+
+def test_narrow_kernel_at_its_largest_orders():
+    rng = np.random.default_rng(449)
+    pairs = []
+    for n in (449, 448, 225, 224):
+        a = rng.standard_normal((n, n))
+        b = 0.1 * rng.standard_normal((n, n))
+        pairs.append((0.5 * (a + a.T), np.eye(n) + b @ b.T / n))
+    many = pairs * 74  # 296 matrices: enough for the narrow kernel
+    st, out = capi.sygvd_batch([p[0] for p in many], [p[1] for p in many])
+    assert st == capi.TB_OK
+    for i, (h, s) in enumerate(pairs):
+        st, alone = capi.sygvd_batch([h], [s])
+        assert st == capi.TB_OK
+        for j in (i, 4 * 73 + i):
+            np.testing.assert_array_equal(out[j][0], alone[0][0])
+            np.testing.assert_array_equal(out[j][1], alone[0][1])

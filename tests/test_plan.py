@@ -124,3 +124,14 @@ def test_a_few_large_structures_keep_their_clusters_in_any_number_of_small_ones(
 def test_waves_of_like_structures_take_one_cta_each(plan):
     assert plan([6 * (11 + i * 53 // 899) for i in range(900)])["cluster"] == 1
     assert plan([100] * 5000 + [384])["cluster"] == 1
+
+
+def test_batches_of_the_narrow_kernel(plan):
+    # what tests/test_gpu_syev_groups.py compares with structures alone, which take the wide one
+    from test_gpu_syev_groups import NARROW_LARGE, narrow_sizes
+    one, two = plan(narrow_sizes(900)), plan(narrow_sizes(700))
+    assert (one["wide"], one["cluster"]) == (0, 1)
+    assert (two["wide"], two["cluster"]) == (0, 2) and two["ncoop"] > len(NARROW_LARGE)
+    assert plan([449, 448, 225, 224] * 74)["wide"] == 0
+    for n in NARROW_LARGE + [449, 448, 225, 224]:
+        assert plan([n])["wide"] == 1
