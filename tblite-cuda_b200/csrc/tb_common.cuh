@@ -108,6 +108,8 @@ __device__ inline bool tb_guard(int site, long long i, long long lo, long long h
   return false;
 }
 #define TB_GUARD(site, i, lo, hi) tb::tb_guard((site), (long long)(i), (long long)(lo), (long long)(hi))
+// brings a warp together after guarded stores that a warp-wide instruction follows
+#define TB_GUARD_CONVERGE() __syncwarp()
 #define TB_OOB_EXPORT(fn)                                                               \
   cudaError_t fn(OobRecord* r, bool reset) {                                           \
     cudaError_t e = cudaMemcpyFromSymbol(r, g_oob, sizeof(OobRecord));                 \
@@ -119,6 +121,7 @@ __device__ inline bool tb_guard(int site, long long i, long long lo, long long h
   }
 #else
 #define TB_GUARD(site, i, lo, hi) true
+#define TB_GUARD_CONVERGE() (void)0
 #define TB_OOB_EXPORT(fn)                         \
   cudaError_t fn(OobRecord* r, bool) {           \
     *r = OobRecord{};                            \

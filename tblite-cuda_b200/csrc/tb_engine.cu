@@ -2259,11 +2259,12 @@ int32_t tb_bounds_check_build(void) {
 
 tb_status tb_bounds_violations(int64_t* count, int32_t* site, int64_t* index, int64_t* lo, int64_t* hi,
                                int32_t reset) {
-  OobRecord r[4];
+  OobRecord r[5];
   cudaError_t e = oob_setup(&r[0], reset != 0);
   if (e == cudaSuccess) e = oob_scf(&r[1], reset != 0);
   if (e == cudaSuccess) e = oob_linalg(&r[2], reset != 0);
   if (e == cudaSuccess) e = oob_syev(&r[3], reset != 0);
+  if (e == cudaSuccess) e = oob_factor(&r[4], reset != 0);
   if (e != cudaSuccess) return fail(TB_CUDA_ERROR, cudaGetErrorString(e));
   int64_t total = 0;
   const OobRecord* first = nullptr;

@@ -303,6 +303,7 @@ __global__ void __launch_bounds__(kT, 2) k_factor(DevBatch B, const double* __re
       invert_diag(T, inv, mj, Y);
       for (int x = threadIdx.x; x < mj * mj; x += kT) {
         const int k = x / mj, i = x - k * mj;
+        if (!TB_GUARD(1, (long long)(j0 + k) * n + j0 + i, 0, (long long)n * n)) continue;
         if (i >= k) W[(long long)(j0 + k) * n + j0 + i] = T[i * kP + k];
         X[(long long)(j0 + k) * n + j0 + i] = Y[k * kP + i];
       }
@@ -325,7 +326,8 @@ __global__ void __launch_bounds__(kT, 2) k_factor(DevBatch B, const double* __re
       });
       __syncthreads();
       solve_block(T, Y, inv, [&](int i, int j, double v) {
-        if (i < mi && j < mj) {
+        if (i < mi && j < mj && TB_GUARD(2, (long long)(j0 + j) * n + i0 + i, 0, (long long)n * n) &&
+            TB_GUARD(3, (long long)(i0 + i) * n + j0 + j, 0, (long long)n * n)) {
           W[(long long)(j0 + j) * n + i0 + i] = v;
           X[(long long)(i0 + i) * n + j0 + j] = 0.0;  // below the diagonal
         }
@@ -351,7 +353,8 @@ __global__ void __launch_bounds__(kT, 2) k_factor(DevBatch B, const double* __re
       acc.zero();
       shared_product(acc, Y, T);
       each(acc, [&](int i, int j, double v) {
-        if (j < mc) X[(long long)(r0 + i) * n + c0 + j] = -v;
+        if (j < mc && TB_GUARD(4, (long long)(r0 + i) * n + c0 + j, 0, (long long)n * n))
+          X[(long long)(r0 + i) * n + c0 + j] = -v;
       });
       __syncthreads();
     }
@@ -375,6 +378,8 @@ cudaError_t launch_factor(const FactorPlan& P, const DevBatch& B, const double* 
   cfg.numAttrs = C > 1 ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, k_factor, B, S, W, X, status, P.c.ncoop);
 }
+
+TB_OOB_EXPORT(oob_factor)
 
 size_t factor_smem_bytes() { return (2 * (size_t)kB * kP + 4 * kSlab * kP) * sizeof(double); }
 

@@ -260,6 +260,7 @@ cudaError_t oob_setup(OobRecord* r, bool reset);
 cudaError_t oob_scf(OobRecord* r, bool reset);
 cudaError_t oob_linalg(OobRecord* r, bool reset);
 cudaError_t oob_syev(OobRecord* r, bool reset);
+cudaError_t oob_factor(OobRecord* r, bool reset);
 
 // D4 dispersion (tb_disp.cu; only when DevParams::d4): per atom cn, W and dW
 // (kD4MaxRef each), energy share e_at, dE/dCN and gradient g [3 nat]; per

@@ -225,12 +225,14 @@ __device__ __noinline__ void walk_read(const double* Mb, int n, int nm, int xo, 
         t += __shfl_xor_sync(0xffffffffu, t, 1);
         t += __shfl_xor_sync(0xffffffffu, t, 2);
         const int r = rb + 8 * k + g;
-        if ((lane & 3) == 0 && r < nm) rowp[r] = t;
+        if ((lane & 3) == 0 && r < nm && TB_GUARD(1, rowp - part + r, 0, (long long)n * n / 2)) rowp[r] = t;
       }
+      TB_GUARD_CONVERGE();
     }
 #pragma unroll
     for (int j = 0; j < Q; ++j)
-      if (cc[j] >= 0) col[(long long)I * nm + cc[j]] = acc[j];
+      if (cc[j] >= 0 && TB_GUARD(2, (long long)I * nm + cc[j], 0, (long long)n * n / 2))
+        col[(long long)I * nm + cc[j]] = acc[j];
   }
 }
 
@@ -309,13 +311,14 @@ __device__ __noinline__ void walk_close(double* Mb, int n, int r0, int nm, int C
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
               const double z = d[i][xx][k];
-              if (cx[k] >= r) {
+              if (cx[k] >= r && TB_GUARD(3, (long long)(r0 + r) * n + r0 + cx[k], 0, (long long)n * n)) {
                 M0[(long long)(16 * (rb0 + i) + 8 * xx) * n + 8 * (k >> 1) + (k & 1)] = z;
                 cs[k] += z * xr;
               }
               if (cx[k] > r) rp[rb0 + i][xx] += z * xc[k];
             }
           }
+        TB_GUARD_CONVERGE();
       }
       // column sums over the eight row lanes g (lane bits 4, 3, 2): lane bit 4
       // ends with y, bit 3 with h
@@ -328,7 +331,9 @@ __device__ __noinline__ void walk_close(double* Mb, int n, int r0, int nm, int C
         double k = (u8 ? k1 : k0) + __shfl_xor_sync(0xffffffffu, s, 8);
         k += __shfl_xor_sync(0xffffffffu, k, 4);
         const int c = cw + (u16 ? 8 : 0) + 2 * t + (u8 ? 1 : 0);
-        if (!(lane & 4) && c < nm) col[(long long)I * nm + c] = k;
+        if (!(lane & 4) && c < nm && TB_GUARD(4, (long long)I * nm + c, 0, (long long)n * n / 2))
+          col[(long long)I * nm + c] = k;
+        TB_GUARD_CONVERGE();
       }
     }
 #pragma unroll
@@ -338,7 +343,9 @@ __device__ __noinline__ void walk_close(double* Mb, int n, int r0, int nm, int C
                  __shfl_xor_sync(0xffffffffu, u1 ? rp[rbk][0] : rp[rbk][1], 1);
       k += __shfl_xor_sync(0xffffffffu, k, 2);
       const int r = rbeg + 16 * rbk + (u1 ? 8 : 0) + g;
-      if (!(lane & 2) && r < nm) row[(long long)J * nm + r] = k;
+      if (!(lane & 2) && r < nm && TB_GUARD(5, row - part + (long long)J * nm + r, 0, (long long)n * n / 2))
+        row[(long long)J * nm + r] = k;
+      TB_GUARD_CONVERGE();
     }
   }
 }
@@ -433,7 +440,8 @@ __device__ __forceinline__ void tridiag_tiles(double* A, int n, double* d, doubl
       // reflector r-1 into row r-1: every CTA has read that row's old values
       // before the last group barrier
       if (g.size == 1 || (r - 1) % g.size == g.rank)
-        for (int j = tid; j < mm; j += kEigThreads) A[(long long)(r - 1) * n + r + j] = v[j];
+        for (int j = tid; j < mm; j += kEigThreads)
+          if (TB_GUARD(6, (long long)(r - 1) * n + r + j, 0, (long long)n * n)) A[(long long)(r - 1) * n + r + j] = v[j];
       const double kk = 0.5 * tk * block_sum_once(part, red[0]);
       const double w0 = p[0] - kk;  // v[0] = 1
       for (int j = tid; j < mm; j += kEigThreads) {
@@ -579,6 +587,7 @@ __device__ __forceinline__ void formq_rows(double* Z, int n, int row0, int c0, i
 #pragma unroll
       for (int y = 0; y < V; ++y) {
         const int c = ct + 8 * y + 2 * t;
+        if (!TB_GUARD(7, (long long)r * n + c0 + c + 1, 0, (long long)n * n)) continue;
         zr[c] = d0[y];
         zr[c + 1] = d1[y];
       }
@@ -602,8 +611,8 @@ __device__ __forceinline__ void formq_rows(double* Z, int n, int row0, int c0, i
 #pragma unroll
     for (int y = 0; y < 2; ++y) {
       const int c = ct + 8 * y + 2 * t;
-      if (valid && c < m) zr[c] = d0[y];
-      if (valid && c + 1 < m) zr[c + 1] = d1[y];
+      if (valid && c < m && TB_GUARD(8, (long long)r * n + c0 + c, 0, (long long)n * n)) zr[c] = d0[y];
+      if (valid && c + 1 < m && TB_GUARD(8, (long long)r * n + c0 + c + 1, 0, (long long)n * n)) zr[c + 1] = d1[y];
     }
   }
 }
@@ -880,8 +889,10 @@ __device__ void dc_gemm(int nrow, int kdim, int ncol, Gen gen, const double* In,
 #pragma unroll
         for (int y = 0; y < 4; ++y) {
           const int c = cb + wcol + 8 * y + 2 * tg;
-          if (c < ncol) Out[(long long)(r0 + j) * ld + c0 + c] = acc[x][y];
-          if (c + 1 < ncol) Out[(long long)(r0 + j) * ld + c0 + c + 1] = acc2[x][y];
+          if (c < ncol && TB_GUARD(11, (long long)(r0 + j) * ld + c0 + c, 0, (long long)ld * ld))
+            Out[(long long)(r0 + j) * ld + c0 + c] = acc[x][y];
+          if (c + 1 < ncol && TB_GUARD(11, (long long)(r0 + j) * ld + c0 + c + 1, 0, (long long)ld * ld))
+            Out[(long long)(r0 + j) * ld + c0 + c + 1] = acc2[x][y];
         }
       }
     }
@@ -1098,7 +1109,8 @@ __device__ __noinline__ void dc_merge(int dofs, int eofs, int n, int ld, int lo,
   auto wgen = [&](int j, int i) { return zl[i] * dc_rcp((dl[i] - dl[ori[j]]) - tv[j]) * inrm[j]; };
   if (Wb) {
     for (int j = gw; j < k; j += ngw)
-      for (int i = lane; i < k; i += 32) Wb[(long long)j * ld + i] = wgen(j, i);
+      for (int i = lane; i < k; i += 32)
+        if (TB_GUARD(12, Wb - Gi + (long long)j * ld + i, 0, (long long)n * ld)) Wb[(long long)j * ld + i] = wgen(j, i);
     group_sync(g);
     dc_gemm(k, k, vcols, [&](int j, int i) { return Wb[(long long)j * ld + i]; }, V, srow, Out, lo, vc0, ld, Wt, Bt, g);
   } else {
@@ -1107,7 +1119,8 @@ __device__ __noinline__ void dc_merge(int dofs, int eofs, int n, int ld, int lo,
   for (int q = gw; q < m - k; q += ngw) {
     const double* src = V + (long long)rowof[ndl[k + q]] * ld;
     double* dst = Out + (long long)(lo + k + q) * ld;
-    for (int c = vc0 + lane; c < vc0 + vcols; c += 32) dst[c] = src[c];
+    for (int c = vc0 + lane; c < vc0 + vcols; c += 32)
+      if (TB_GUARD(13, dst - Out + c, 0, (long long)n * ld)) dst[c] = src[c];
   }
   __syncthreads();
   for (int j = tid; j < m; j += kEigThreads) d[lo + j] = j < k ? dl[ori[j]] + tv[j] : delta[ndl[j]];
@@ -1347,7 +1360,8 @@ __device__ __noinline__ void dc_leaf(int dofs, int eofs, int lo0, int s, int wof
     d[lo0 + lane] = dr;
 #pragma unroll
     for (int r = 0; r < S; ++r)
-      if (r < s) G[(long long)(lo0 + r) * ld + lo0 + lane] = g[r];
+      if (r < s && TB_GUARD(14, (long long)(lo0 + r) * ld + lo0 + lane, 0, (long long)ld * ld))
+        G[(long long)(lo0 + r) * ld + lo0 + lane] = g[r];
   }
   __syncwarp();
 }
@@ -1403,6 +1417,7 @@ __device__ void dc_solve(double* d, double* e, double* Z, double* G0, double* G1
       int lo, hi, pl;
       dc_node(n, dep, b, &lo, &hi, &pl);
       if (hi - lo < 1 || hi - lo > S || pl <= S) continue;
+      if (!TB_GUARD(15, leaf_ws(hi - lo), 0, lsize + 1) || !TB_GUARD(16, (wid + 1) * lsize, 0, lws_cap + 1)) continue;
       dc_leaf<S>(sm_off(d), sm_off(e), lo, hi - lo, sm_off(lws) + wid * lsize, Go, ld);
       for (int r = 0; g.size > 1 && r < g.size; ++r)
         if (r != g.rank && lane < hi - lo) put_at(d + lo + lane, d[lo + lane], g, r);
