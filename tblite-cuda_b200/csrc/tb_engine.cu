@@ -1152,7 +1152,6 @@ tb_status mixed_core(tb_batch* b, cudaStream_t st, double n3_lo, double n3_hi, d
     }
     // one FP64 refinement step (GEMMs included) of the FP32 eigenvectors,
     // gathered into FP64 columns in ascending order (Z -> Vn)
-    const size_t oa_smem = oa_smem_bytes(b->nmax);
     TB_K("refine", 0, 0, k_gather_vectors<<<gemm_grid, 256, 0, st>>>(B, T, nt, b->Zf, b->perm, b->Z, ll));
     double* V = b->Z;
     double* Vo = b->Vn;
@@ -1162,7 +1161,7 @@ tb_status mixed_core(tb_batch* b, cudaStream_t st, double n3_lo, double n3_hi, d
             b->F, 0, V, 0, nullptr, nullptr, nullptr, b->W, 1.0, 0.0, ll, 0);
     TB_GEMM(0.0,  // Sm = V^T W (in P)
             V, 1, b->W, 0, nullptr, nullptr, nullptr, b->P, 1.0, 0.0, ll, 0);
-    TB_K("refine", 0, 0, k_oa_step<<<nmol, 256, oa_smem, st>>>(B, b->G, b->P, V, b->w, ll, nullptr));
+    TB_K("refine", 0, 0, k_oa_step<<<nmol, 256, 0, st>>>(B, b->G, b->P, b->w, ll));
     TB_CUDA(cudaMemcpyAsync(Vo, V, (size_t)b->n2_tot * sizeof(double), cudaMemcpyDeviceToDevice, st));
     TB_GEMM(0.0,  // Vo = V + V E
             V, 0, b->G, 0, nullptr, nullptr, nullptr, Vo, 1.0, 1.0, ll, 0);
@@ -1191,7 +1190,7 @@ tb_status raise_smem_limits() {
   int dev = 0, optin = 0;
   TB_CUDA(cudaGetDevice(&dev));
   TB_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-  const void* ks[] = {(const void*)k_factor, (const void*)k_syev, (const void*)k_syev_wide, (const void*)k_syev_small, (const void*)k_fermi, (const void*)k_oa_step,
+  const void* ks[] = {(const void*)k_factor, (const void*)k_syev, (const void*)k_syev_wide, (const void*)k_syev_small, (const void*)k_fermi,
                       (const void*)k_gemm_tc, (const void*)k_fock, (const void*)k_syev_jacobi};
   for (const void* k : ks) {
     cudaFuncAttributes a;
@@ -2733,8 +2732,7 @@ struct MatBatch {
   size_t lib_bytes = 0;
   int* lib_info = nullptr;
   TridPlan trid;
-  SyevPlan syev;
-  FactorPlan fac;
+  std::vector<int> sorted;  // sizes in db.order: the largest first
   int* d_tlist = nullptr;
   tb_status build(int nmat, const int32_t* n, int smem_tridiag = kTridMin) {
     std::vector<int> ooff(nmat + 1, 0);
@@ -2767,12 +2765,11 @@ struct MatBatch {
     n2 = moff[nmat];
     no = ooff[nmat];
     // largest matrices first: the order k_syev's plan and the factorisations take
-    std::vector<int> order(nmat), sorted(nmat);
+    std::vector<int> order(nmat);
+    sorted.resize(nmat);
     for (int m = 0; m < nmat; ++m) order[m] = m;
     std::stable_sort(order.begin(), order.end(), [&](int a, int c) { return n[a] > n[c]; });
     for (int i = 0; i < nmat; ++i) sorted[i] = n[order[i]];
-    syev.build(sorted.data(), nmat, kSyevMaxN, 0);
-    fac.build(sorted.data(), nmat, kSyevMaxN);
     Layout L;
     size_t o_ooff = L.add((nmat + 1) * 4), o_moff = L.add((nmat + 1) * 8), o_t = L.add(tiles.size() * sizeof(int4));
     size_t o_ord = L.add(nmat * 4);
@@ -2831,7 +2828,11 @@ tb_status tb_sygvd_batch(int32_t nmat, const int32_t* n, const double* H, const 
     const tb_status ss = raise_smem_limits();
     if (ss != TB_OK) return ss;
   }
-  TB_CUDA(launch_factor(mb.fac, B, mb.S, mb.W, mb.X, mb.ms.status, 0));
+  SyevPlan syev;
+  FactorPlan fac;
+  syev.build(mb.sorted.data(), nmat, kSyevMaxN, 0);
+  fac.build(mb.sorted.data(), nmat, kSyevMaxN);
+  TB_CUDA(launch_factor(fac, B, mb.S, mb.W, mb.X, mb.ms.status, 0));
   for (size_t k = 0; k < mb.big.size(); ++k) {
     const int m = mb.big[k];
     const long long mo = mb.h_moff[m];
@@ -2849,7 +2850,7 @@ tb_status tb_sygvd_batch(int32_t nmat, const int32_t* n, const double* H, const 
     TB_CUDA(launch_trid(B, mb.F, mb.W, mb.ms.status, mb.ms.active, mb.d_tlist + mb.trid.off[c], cnt,
                         kTridClusterSizes[c], mb.trid.nmax[c], 0));
   }
-  TB_CUDA(launch_syev(mb.syev, B, mb.F, mb.Z, mb.W, mb.w, mb.perm, mb.ms.status, mb.ms.active, 0, nullptr));
+  TB_CUDA(launch_syev(syev, B, mb.F, mb.Z, mb.W, mb.w, mb.perm, mb.ms.status, mb.ms.active, 0, nullptr));
   std::vector<int> fstat(nmat, 0);
   if (!mb.big.empty()) TB_CUDA(cudaMemcpy(fstat.data(), mb.ms.status, nmat * 4, cudaMemcpyDeviceToHost));
   for (size_t k = 0; k < mb.big.size(); ++k) {

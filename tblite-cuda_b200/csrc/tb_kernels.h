@@ -245,14 +245,8 @@ __global__ void k_symmetrize(DevBatch B, const int4* tiles, int ntiles, double* 
 __global__ void k_to_f32(DevBatch B, const int4* tiles, int ntiles, const double* F, float* Af, const int* mask);
 __global__ void k_gather_vectors(DevBatch B, const int4* tiles, int ntiles, const float* Zf, const int* perm,
                                  double* V, const int* mask);
-// refinement step (Rayleigh-Ritz in clusters + Ogita-Aishima coefficients)
-constexpr int kClusterMax = 64;
-inline size_t oa_smem_bytes(int nmax) {
-  return (3 * (size_t)kClusterMax * kClusterMax + 2 * kClusterMax) * sizeof(double) +
-         2 * ((size_t)nmax + 1) * sizeof(int);
-}
-__global__ void k_oa_step(DevBatch B, double* G, double* Sm, double* V, double* w, const int* mask,
-                          const int* rr_mask);
+// coefficients of one Ogita-Aishima refinement step
+__global__ void k_oa_step(DevBatch B, double* G, const double* Sm, double* w, const int* mask);
 
 // records of the checked build's index guards, one per translation unit
 // (all zero in the normal build); reset clears them after the read

@@ -487,9 +487,9 @@ __device__ __forceinline__ void tridiag_tiles(double* A, int n, double* d, doubl
       else if constexpr (W) walk_close<5, 2>(Mb, n, r + 1, mr, 7, sm_off(PV), sm_off(vn), out, gw, ngw);
       np = 0;
     } else {
-      if (mr <= kWalk1) walk_read<4, 5, W ? 16 : 16>(Mb, n, mr, sm_off(vn), out, gw, ngw);
+      if (mr <= kWalk1) walk_read<4, 5, 16>(Mb, n, mr, sm_off(vn), out, gw, ngw);
       else if (mr <= kWalk2) walk_read<4, 6, 16>(Mb, n, mr, sm_off(vn), out, gw, ngw);
-      else if constexpr (W) walk_read<5, 7, W ? 16 : 8>(Mb, n, mr, sm_off(vn), out, gw, ngw);
+      else if constexpr (W) walk_read<5, 7, 16>(Mb, n, mr, sm_off(vn), out, gw, ngw);
       // the next step's w_i . v and v_i . v, one warp each, in every CTA; the
       // last warps of the group first (the walk's units start at warp 0).  Two
       // buffers: a CTA one step behind may still read the other
