@@ -25,11 +25,13 @@ double syev_ms(double n, int C) {
 // the order (largest first) over as many clusters as the GPU holds at once
 // (kCap: cudaOccupancyMaxActiveClusters on a B200, one and two CTAs per SM) for
 // every cluster size and a geometric set of splits into cluster and one-CTA
-// structures.  Two CTAs on an SM slow each other (kSlowTwo; the narrower
-// kernel alone, kSlowNarrow).  400 water clusters of 48..384 AOs: 13.3 ms on
-// one CTA each, 11.0 on two; 128: 11.1 and 6.2 (on four); 48 chains of
-// 122..1196 AOs: 172 and 40 (on eight) -- with the walks before their one
-// comparison per entry; the ratios since are the same.  Where one CTA
+// structures.  Two CTAs on an SM slow each other (kSlowTwo), and the narrower
+// kernel alone is slower (kSlowNarrow): 148 structures of 150, 300 and 384 AOs take
+// 1.31, 5.31 and 9.19 ms wide, 1.46, 5.70 and 9.94 narrow (1.07 to 1.11 times), 296
+// of them 1.95, 8.02 and 14.1 (1.49 to 1.54 times, all in step; 1.42 is for uneven
+// batches: 400 clusters of 48..384 AOs on one CTA each take 10.8 ms, modelled 11.2).
+// By plan: 400 clusters 8.1 ms (on two), 128 4.5 (8.9 on one, 5.8 on two), 48 chains
+// of 122..1196 AOs 33.5 (on eight; 165 on one).  Where one CTA
 // per structure is within 3% of the CTAs' total work (a batch of several waves of
 // like sizes) no clusters are tried: they repeat work and would only lose.  (The
 // number of structures is no such rule: with clusters for at most 592 of them, 8
