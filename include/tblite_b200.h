@@ -39,9 +39,9 @@ typedef enum tb_status {
   TB_NOT_SPD = 2,              /* overlap matrix not positive definite          */
   TB_SCF_NOT_CONVERGED = 3,    /* max_iter reached                              */
   TB_FERMI_NOT_CONVERGED = 4,  /* Fermi level solve hit its iteration cap       */
-  TB_EIGEN_FAILED = 5,         /* eigensolve failed: the matrix was not finite, or
-                                  the one-warp Jacobi or cuSOLVER did not
-                                  converge                                      */
+  TB_EIGEN_FAILED = 5,         /* eigensolve failed: the matrix was not finite (from
+                                  64 AOs: an eigenvalue of 1e30 or more), or the
+                                  one-warp Jacobi or cuSOLVER did not converge  */
   TB_CAPACITY_EXCEEDED = 6,    /* request larger than a stated maximum          */
   TB_CUDA_ERROR = 7,           /* CUDA runtime error (see tb_last_error)        */
   TB_PARAM_ERROR = 8           /* parameter file could not be read              */
@@ -166,7 +166,8 @@ const char* tb_last_error(void);
  * it is measured faster than the one-CTA solver below 64 AOs (Householder +
  * divide and conquer in shared memory); from 64 AOs the same on one CTA or a
  * thread block cluster per structure, whichever the batch's sizes favour;
- * above 1216 AOs, and above a size chosen per batch from measured cost models,
+ * above 1216 AOs, and from 384 AOs above a size chosen per batch from measured
+ * cost models,
  * cuSOLVER Xsyevd (see tb_options.solver).  The in-house variant depends on
  * the size only and the cluster size moves no bits, so a structure gives the
  * same bits alone and in any batch that leaves it in-house.

@@ -8,7 +8,7 @@
 // below forms S_IJ - sum_k L_Ik L_Jk^T and solves with L_JJ^T by substitution,
 // which gives L_IJ.  (Multiplied by the inverse X_JJ instead, L L^T - S grows by
 // the condition of L_JJ: with functions in pairs 3e-6 apart, 138 of them, the
-// residual of H C = S C w was 4.3e-7 of the largest |w|, by substitution 1.5e-10.)
+// residual of H C = S C w was 4.3e-7 of the largest |w|, by substitution 1.3e-10.)
 // The inverse by block diagonals: X_rc = -X_rr sum_{k=r+1..c} L_kr^T X_kc,
 // every block of a diagonal independent.  The products run on the FP64 tensor
 // instruction; a block's terms are added in the order of k whichever CTA owns
