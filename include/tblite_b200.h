@@ -167,10 +167,9 @@ const char* tb_last_error(void);
  * divide and conquer in shared memory); from 64 AOs the same on one CTA or a
  * thread block cluster per structure, whichever the batch's sizes favour;
  * above 1216 AOs, and from 384 AOs above a size chosen per batch from measured
- * cost models,
- * cuSOLVER Xsyevd (see tb_options.solver).  The in-house variant depends on
- * the size only and the cluster size moves no bits, so a structure gives the
- * same bits alone and in any batch that leaves it in-house.
+ * cost models, cuSOLVER Xsyevd (see tb_options.solver).  The in-house variant
+ * depends on the size only and the cluster size moves no bits, so a structure
+ * gives the same bits alone and in any batch that leaves it in-house.
  * tb_calculator_set_small_solver: jacobi_max -1 (default) measured choice,
  * 0 never, 1..32 fixed bound.  tb_calculator_tuning writes the measurements
  * and choices as JSON text into buf (NUL-terminated, at most len bytes) and
