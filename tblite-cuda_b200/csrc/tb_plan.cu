@@ -32,12 +32,13 @@ double syev_ms(double n, int C) {
 // batches: 400 clusters of 48..384 AOs on one CTA each take 10.8 ms, modelled 11.2).
 // By plan: 400 clusters 8.1 ms (on two), 128 4.5 (8.9 on one, 5.8 on two), 48 chains
 // of 122..1196 AOs 33.5 (on eight; 165 on one).  Where one CTA
-// per structure is within 3% of the CTAs' total work (a batch of several waves of
-// like sizes) no clusters are tried: they repeat work and would only lose.  (The
-// number of structures is no such rule: with clusters for at most 592 of them, 8
-// chains of 602 AOs with 640 of 66..120 took 175 ms a call, now 62; a chain of
-// 1196 with 600 of 66 AOs, in-house, 981 and 165; 620 clusters of 66..384 AOs 136
-// either way.)
+// per structure is within 3% of the CTAs' total work, or more than 592 structures
+// could gain half a millisecond at most, no clusters are tried: they repeat work,
+// and the search takes about as long on the host (0.8 ms for the factorisation of
+// 1024 structures).  (The number alone is no such rule: with clusters for at most
+// 592 structures, 8 chains of 602 AOs with 640 of 66..120 took 175 ms a call, now
+// 62; a chain of 1196 with 600 of 66 AOs, in-house, 981 and 165; 620 clusters of
+// 66..384 AOs 136 either way.)
 ClusterChoice choose_clusters(const int* sizes, int first, int last, double (*ms)(double, int), bool two_per_sm,
                               bool one_per_sm) {
   ClusterChoice best;
@@ -72,7 +73,7 @@ ClusterChoice choose_clusters(const int* sizes, int first, int last, double (*ms
   for (int per = two_per_sm ? 2 : 1; per >= (one_per_sm ? 1 : 2); --per)
     for (int c = 0; c < 5; ++c) {
       const int C = 1 << c;
-      if (C > 1 && 0.97 * best.span <= least) break;
+      if (C > 1 && (0.97 * best.span <= least || (cnt > 4 * 148 && best.span - least < 0.5))) break;
       for (int k = cnt; k >= 1; k = k > 1 ? (3 * k) / 4 : 0) {
         const int items = C > 1 ? k + (cnt - k + C - 1) / C : cnt;
         const double slow = per == 1 ? 1.0 : items > kCap[0][c] ? kSlowTwo : kSlowNarrow;
@@ -112,15 +113,18 @@ int choose_lib_above(std::vector<int> sizes, const SolverModel& M) {
   int k0 = 0;
   while (k0 < nmol && sizes[k0] > kSyevMaxN) ++k0;
   if (k0 == nmol) return -1;
+  int last = k0;  // the first that is not offered
+  while (last < nmol && sizes[last] >= kLibMinN) ++last;
+  const int step = std::max(1, (last - k0) / 64);  // at most 65 plans (2 ms each for 2000 structures)
   double lib_sum = 0.0, best = 1e300;  // (the k0 structures above the in-house limit count the same for every k)
   int best_k = k0;
-  for (int k = k0; lib_sum < best; ++k) {
+  for (int k = k0; lib_sum < best;) {
     SyevPlan rest;
     rest.build(sizes.data() + k, nmol - k, 0, 0);
     const double in_t = 1e-3 * rest.c.span * M.scale;
     if (lib_sum + in_t < best) { best = lib_sum + in_t; best_k = k; }
-    if (k == nmol || sizes[k] < kLibMinN) break;
-    lib_sum += M.lib256 + M.lib_slope * (sizes[k] - 256);
+    if (k == last) break;
+    for (const int end = std::min(last, k + step); k < end; ++k) lib_sum += M.lib256 + M.lib_slope * (sizes[k] - 256);
   }
   if (best_k == nmol) return -1;
   return best_k == k0 ? kSyevMaxN : sizes[best_k];

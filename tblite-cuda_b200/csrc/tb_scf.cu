@@ -633,8 +633,9 @@ __global__ void __launch_bounds__(256) k_mulliken_cols(DevBatch B, const int2* _
 // convergence test of xtb_singlepoint and the iteration bookkeeping.
 // Bound by the latency of the pair sums (a row of the tables per warp): 512
 // threads and four table loads in flight; a 722-AO structure 0.55 -> 0.26 ms,
-// 1024 clusters of 48..384 AOs 0.43 -> 0.32 ms (256 threads before).  The
-// thread count is the same for every batch: the sums' order depends on it.
+// 1024 clusters of 48..384 AOs 0.43 -> 0.32 ms, 4000 waters of 6 AOs 0.115 ->
+// 0.138 (256 threads before).  The thread count is the same for every batch: the
+// sums' order depends on it.
 __global__ void __launch_bounds__(512, 2) k_finalize(DevParams P, DevBatch B, const double* __restrict__ colred, const double* __restrict__ n0sh,
                            const double* __restrict__ mrad, const double* __restrict__ q_in, double* __restrict__ dq,
                            double* __restrict__ qsh_out, double* __restrict__ qat_out, double* __restrict__ dpat_out,
