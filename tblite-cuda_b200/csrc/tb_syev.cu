@@ -1695,7 +1695,7 @@ __device__ __forceinline__ void syev_structure(const DevBatch& B, double* __rest
 // short is between one wave of two and one of three to an SM: 300 structures of 66
 // AOs take 0.99 ms, 444 of them 1.11, the former kernel at three to an SM 0.91 and
 // 0.93; of 96 AOs 1.48 and 1.69 against 1.58 and 1.61; up to 296 and beyond 444
-// structures two are faster by 1.04 to 1.6 times.)
+// structures two are faster, up to 1.6 times.)
 __global__ void __launch_bounds__(kEigThreads, 2) k_syev(DevBatch B, double* __restrict__ Ab, double* __restrict__ Zb,
                                                          double* __restrict__ Sb, double* __restrict__ wout,
                                                          int* __restrict__ perm, int* __restrict__ status,
